@@ -21,7 +21,7 @@ ERR_LAUNCH, ERR_TIMEOUT, ERR_NULL, ERR_DEVICE, ERR_TOO_LARGE = -5, -6, -7, -8, -
 DT_NONE, DT_I8, DT_U8, DT_I32, DT_F32, DT_F16, DT_BF16, DT_F8E4M3, DT_F8E5M2 = range(9)
 
 # qlin_epilogue
-EPI_RAW, EPI_SCALE_PROD, EPI_SCALE_SEQ = 0, 1, 2
+EPI_RAW, EPI_SCALE_PROD, EPI_SCALE_SEQ, EPI_SCALE_ACC16 = 0, 1, 2, 3
 
 # qlin_quant_mode
 (Q_I8_DYN, Q_I8_STATIC, Q_I8_STATIC_CLAMP_FIRST, Q_F8_DYN, Q_I8_GIVEN_SCALE, Q_F8_FAKE_SCALED, Q_I8_STATIC_ROUND_FIRST,

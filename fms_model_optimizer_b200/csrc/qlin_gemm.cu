@@ -149,7 +149,8 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& mb
 template <bool F8>
 __device__ __forceinline__ float dequant_one(const GemmParams& p, uint32_t v, float rs, float cs, float bias,
                                              bool prod, bool has_bias) {
-  const float a = F8 ? __uint_as_float(v) : __int2float_rn(static_cast<int32_t>(v));
+  float a = F8 ? __uint_as_float(v) : __int2float_rn(static_cast<int32_t>(v));
+  if (p.epilogue == QLIN_EPI_SCALE_ACC16) a = round_to(a, QLIN_DT_F16);
   float t;
   if (prod) {
     const float s = round_to(round_to(__fmul_rn(rs, cs), p.prod_round), p.scale_round);
@@ -170,51 +171,138 @@ __device__ __forceinline__ uint32_t pack16(const GemmParams& p, float lo, float 
          (static_cast<uint32_t>(__half_as_ushort(__float2half_rn(hi))) << 16);
 }
 
-// Byte address of output row `row`, column 0 (`elt` bytes per element).  With row-block scatter the block of
-// scatter_rows rows that contains `row` lives in its own buffer (possibly another GPU's).
-__device__ __forceinline__ uint8_t* out_row(const GemmParams& p, int row, int elt) {
+// Byte address of output row `row`, column 0 (`elt` bytes per element) of the output that starts at `dbase`.  With
+// row-block scatter the block of scatter_rows rows that contains `row` lives in its own buffer (possibly another GPU's).
+__device__ __forceinline__ uint8_t* out_row(const GemmParams& p, uint8_t* dbase, int row, int elt) {
   if (p.scatter_rows > 0) {
     const int owner = row / p.scatter_rows;
     return p.scatter_d[owner] + static_cast<int64_t>(row - owner * p.scatter_rows + p.scatter_row0) * p.ldd * elt;
   }
-  return reinterpret_cast<uint8_t*>(p.d) + static_cast<int64_t>(row) * p.ldd * elt;
+  return dbase + static_cast<int64_t>(row) * p.ldd * elt;
 }
 
-// Direct (uncoalesced, bounds-checked) store of NC consecutive columns of one row held by this
-// thread: the path for ragged right edges and for outputs that rule out 16-byte vectors.
-template <bool F8, int NC>
-__device__ __forceinline__ void store_row_direct(const GemmParams& p, const uint32_t (&v)[NC], int row, int col0,
-                                                 const float* s_cs, const float* s_bias, int s_off, float rs) {
-  if (row >= p.M) return;
-  const int ncol = min(NC, p.N - col0);
-  if (ncol <= 0) return;
-  const bool prod = p.epilogue == QLIN_EPI_SCALE_PROD;
-  const bool has_bias = p.bias != nullptr;
-  const int elt = (p.epilogue == QLIN_EPI_RAW || p.out_dtype == QLIN_DT_F32) ? 4 : 2;
-  uint8_t* base = out_row(p, row, elt) + static_cast<int64_t>(col0) * elt;
+// ---- dequantisation of 32 accumulator columns held by one thread -------------------------------------------------
+// Every step of the chain is a loop over 16 column pairs on packed fp32x2 arithmetic and packed conversions, and which
+// rounding a step applies is decided once per step, not once per element.  An epilogue that asked per element (and
+// rounded with the scalar conversions, which issue at a quarter of the rate) took about 17 us for a 128 x 256 tile of a
+// CTA: 53 us of GEMM at 4096 x 768 x 3072 with fp32 output, 32 us at 517 x 4096 x 4096 with fp16 output.
+template <int DT>
+__device__ __forceinline__ float2 round2(float2 t) {
+  if (DT == QLIN_DT_F16) return __half22float2(__float22half2_rn(t));
+  if (DT == QLIN_DT_BF16) {
+    const __nv_bfloat162 b2 = __float22bfloat162_rn(t);
+    const uint32_t bw = *reinterpret_cast<const uint32_t*>(&b2);
+    return make_float2(__uint_as_float(bw << 16), __uint_as_float(bw & 0xFFFF0000u));
+  }
+  return t;
+}
+__device__ __forceinline__ float2 pair_of(const uint32_t (&v)[32], int j) { return make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])); }
+__device__ __forceinline__ void set_pair(uint32_t (&v)[32], int j, float2 t) {
+  v[2 * j] = __float_as_uint(t.x);
+  v[2 * j + 1] = __float_as_uint(t.y);
+}
+template <int DT>
+__device__ __forceinline__ void round32(uint32_t (&v)[32]) {
 #pragma unroll
-  for (int j = 0; j < NC; ++j) {
-    if (j < ncol) {
-      if (p.epilogue == QLIN_EPI_RAW) {
-        reinterpret_cast<uint32_t*>(base)[j] = v[j];
-      } else {
-        const float y = dequant_one<F8>(p, v[j], rs, s_cs[s_off + j], s_bias[s_off + j], prod, has_bias);
-        if (p.out_dtype == QLIN_DT_F32) {
-          reinterpret_cast<float*>(base)[j] = y;
-        } else {
-          reinterpret_cast<uint16_t*>(base)[j] = static_cast<uint16_t>(pack16(p, y, 0.0f) & 0xFFFFu);
-        }
-      }
+  for (int j = 0; j < 16; ++j) set_pair(v, j, round2<DT>(pair_of(v, j)));
+}
+__device__ __forceinline__ void round32_if(uint32_t (&v)[32], int dt) {
+  if (dt == QLIN_DT_F16) {
+    round32<QLIN_DT_F16>(v);
+  } else if (dt == QLIN_DT_BF16) {
+    round32<QLIN_DT_BF16>(v);
+  }
+}
+template <int PROD, int SCALE>
+__device__ __forceinline__ void mul_prod32(uint32_t (&v)[32], float rs, const float* cs) {
+  const float2 rs2 = make_float2(rs, rs);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float2 sc = round2<SCALE>(round2<PROD>(__fmul2_rn(rs2, *reinterpret_cast<const float2*>(cs + 2 * j))));
+    set_pair(v, j, __fmul2_rn(pair_of(v, j), sc));
+  }
+}
+template <int PROD>
+__device__ __forceinline__ void mul_prod32_if(uint32_t (&v)[32], float rs, const float* cs, int scale_round) {
+  if (scale_round == QLIN_DT_F16) {
+    mul_prod32<PROD, QLIN_DT_F16>(v, rs, cs);
+  } else if (scale_round == QLIN_DT_BF16) {
+    mul_prod32<PROD, QLIN_DT_BF16>(v, rs, cs);
+  } else {
+    mul_prod32<PROD, QLIN_DT_F32>(v, rs, cs);
+  }
+}
+// Accumulators in, output values (fp32 bits, already rounded the way the epilogue mode asks) out.
+template <bool F8>
+__device__ __forceinline__ void dequant32(const GemmParams& p, uint32_t (&v)[32], float rs, const float* cs, const float* bias) {
+  if (!F8) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__int2float_rn(static_cast<int32_t>(v[j])));
+  }
+  if (p.epilogue == QLIN_EPI_SCALE_PROD) {
+    if (p.prod_round == QLIN_DT_BF16) {
+      mul_prod32_if<QLIN_DT_BF16>(v, rs, cs, p.scale_round);
+    } else if (p.prod_round == QLIN_DT_F16) {
+      mul_prod32_if<QLIN_DT_F16>(v, rs, cs, p.scale_round);
+    } else {
+      mul_prod32_if<QLIN_DT_F32>(v, rs, cs, p.scale_round);
     }
+  } else {
+    if (p.epilogue == QLIN_EPI_SCALE_ACC16) round32<QLIN_DT_F16>(v);
+    const float2 rs2 = make_float2(rs, rs);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) set_pair(v, j, __fmul2_rn(__fmul2_rn(pair_of(v, j), rs2), *reinterpret_cast<const float2*>(cs + 2 * j)));
+    round32_if(v, p.mid_round);
+  }
+  if (p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) set_pair(v, j, __fadd2_rn(pair_of(v, j), *reinterpret_cast<const float2*>(bias + 2 * j)));
+  }
+  round32_if(v, p.acc_round);
+}
+// 32 values -> 16 words of two 16-bit numbers.
+__device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t* w, bool bf16) {
+  if (bf16) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const __nv_bfloat162 o = __float22bfloat162_rn(pair_of(v, j));
+      w[j] = *reinterpret_cast<const uint32_t*>(&o);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const __half2 o = __float22half2_rn(pair_of(v, j));
+      w[j] = *reinterpret_cast<const uint32_t*>(&o);
+    }
+  }
+}
+
+// Uncoalesced store of up to 32 consecutive columns of one row held by this thread: the path for right edges that do not
+// end on a 16-byte boundary and for outputs that rule out 16-byte vectors.  `v` holds output values (or raw accumulators).
+__device__ __forceinline__ void store_row_direct(const GemmParams& p, uint8_t* dbase, const uint32_t (&v)[32], int row, int col0, bool two_byte) {
+  if (row >= p.M) return;
+  const int ncol = p.N - col0;
+  if (ncol <= 0) return;
+  uint8_t* base = out_row(p, dbase, row, two_byte ? 2 : 4) + static_cast<int64_t>(col0) * (two_byte ? 2 : 4);
+  if (two_byte) {
+    uint32_t w[16];
+    pack32(v, w, p.out_dtype == QLIN_DT_BF16);
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < ncol) reinterpret_cast<uint16_t*>(base)[j] = static_cast<uint16_t>(w[j >> 1] >> (16 * (j & 1)));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < ncol) reinterpret_cast<uint32_t*>(base)[j] = v[j];
   }
 }
 
 // Coalesced store through this warp's 32 x 128-byte staging tile.  `w` holds this thread's row as
 // 32 packed 32-bit words (128 bytes).  The tile is written with a 16-byte-chunk XOR swizzle so both
 // the row-per-lane writes and the row-contiguous reads are bank-conflict free; every global store
-// instruction then covers four full 128-byte lines.
+// instruction then covers four full 128-byte lines.  `chunks` of the row's eight 16-byte pieces lie inside the output.
 __device__ __forceinline__ void store_tile_coalesced(uint8_t* stage, const uint32_t (&w)[32], uint8_t* gbase,
-                                                     int64_t row_pitch_bytes, int rows_valid, int lane) {
+                                                     int64_t row_pitch_bytes, int rows_valid, int lane, int chunks) {
   const uint32_t sbase = smem_u32(stage);
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
@@ -231,12 +319,12 @@ __device__ __forceinline__ void store_tile_coalesced(uint8_t* stage, const uint3
     uint32_t x0, x1, x2, x3;
     const uint32_t addr = sbase + r * 128 + ((c ^ (r & 7)) << 4);
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(addr) : "memory");
-    if (r < rows_valid) *reinterpret_cast<uint4*>(gbase + r * row_pitch_bytes + c * 16) = make_uint4(x0, x1, x2, x3);
+    if (r < rows_valid && c < chunks) *reinterpret_cast<uint4*>(gbase + r * row_pitch_bytes + c * 16) = make_uint4(x0, x1, x2, x3);
   }
   __syncwarp();
 }
 
-// Loads NC columns of the optional initial accumulator C for one row (zeros when absent / outside).
+// Loads 32 columns of the optional initial accumulator C for one row (zeros when absent / outside).
 template <int NC>
 __device__ __forceinline__ void load_c_row(const GemmParams& p, uint32_t (&v)[NC], int row, int col0) {
 #pragma unroll
@@ -248,127 +336,72 @@ __device__ __forceinline__ void load_c_row(const GemmParams& p, uint32_t (&v)[NC
     if (col0 + j < p.N) v[j] = src[j];
 }
 
-// Emits 64 accumulator columns [col0, col0+64) of this thread's row.  `vec_ok` says the output
-// allows 16-byte row-contiguous stores.
+// What the epilogue of a launch does, worked out once per thread.
+struct EpiCtx {
+  uint8_t* dbase;  // output of this tile's problem
+  uint8_t* stage;  // this warp's staging tile
+  bool two_byte, vec_ok, scaled;
+};
+__device__ __forceinline__ EpiCtx make_epi_ctx(const GemmParams& p, uint8_t* stage) {
+  EpiCtx e;
+  e.dbase = reinterpret_cast<uint8_t*>(p.d);
+  e.stage = stage;
+  e.scaled = p.epilogue != QLIN_EPI_RAW;
+  e.two_byte = e.scaled && p.out_dtype != QLIN_DT_F32;
+  e.vec_ok = (p.scatter_rows > 0 || (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0) && ((p.ldd * (e.two_byte ? 2 : 4)) % 16 == 0);
+  return e;
+}
+
+// Emits 32 accumulator columns [col0, col0 + 32) of this thread's row as 4-byte values.
 template <bool F8>
-__device__ __forceinline__ void emit64(const GemmParams& p, const uint32_t (&v)[64], int row0, int lane, int col0,
-                                       const float* s_cs, const float* s_bias, int s_off, float rs, bool vec_ok,
-                                       uint8_t* stage) {
-  const int row = row0 + lane;
-  const bool prod = p.epilogue == QLIN_EPI_SCALE_PROD;
-  const bool has_bias = p.bias != nullptr;
-  const int rows_valid = p.M - row0;
-  if (!vec_ok || col0 + 64 > p.N) {
-    store_row_direct<F8, 64>(p, v, row, col0, s_cs, s_bias, s_off, rs);
-    return;
-  }
-  if (p.epilogue != QLIN_EPI_RAW && p.out_dtype != QLIN_DT_F32) {
-    // 2-byte outputs: 64 columns = one 128-byte staging row
-    uint32_t w[32];
-    if (prod && p.scale_round == QLIN_DT_F16 && p.acc_round == QLIN_DT_F16 && p.out_dtype == QLIN_DT_BF16 &&
-        (p.prod_round == QLIN_DT_BF16 || p.prod_round == QLIN_DT_NONE || p.prod_round == QLIN_DT_F32)) {
-      // The deploy Linear's chain, two columns per instruction: s = fp16(bf16?(rs * cs)); y = fp16(acc * s (+ bias));
-      // the same roundings as dequant_one, done with packed fp32 arithmetic and packed conversions.
-      const bool prod_bf16 = p.prod_round == QLIN_DT_BF16;
-      const float2 rs2 = make_float2(rs, rs);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float2 c2 = *reinterpret_cast<const float2*>(s_cs + s_off + 2 * j);
-        float2 sc = __fmul2_rn(rs2, c2);
-        if (prod_bf16) {
-          const __nv_bfloat162 b2 = __float22bfloat162_rn(sc);
-          const uint32_t bw = *reinterpret_cast<const uint32_t*>(&b2);
-          sc = make_float2(__uint_as_float(bw << 16), __uint_as_float(bw & 0xFFFF0000u));
-        }
-        sc = __half22float2(__float22half2_rn(sc));
-        float2 a2;
-        if (F8) {
-          a2 = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-        } else {
-          a2 = make_float2(__int2float_rn(static_cast<int32_t>(v[2 * j])), __int2float_rn(static_cast<int32_t>(v[2 * j + 1])));
-        }
-        float2 t = __fmul2_rn(a2, sc);
-        if (has_bias) t = __fadd2_rn(t, *reinterpret_cast<const float2*>(s_bias + s_off + 2 * j));
-        t = __half22float2(__float22half2_rn(t));
-        const __nv_bfloat162 o2 = __float22bfloat162_rn(t);
-        w[j] = *reinterpret_cast<const uint32_t*>(&o2);
-      }
-    } else if (!prod && p.out_dtype == QLIN_DT_BF16 && (p.mid_round == QLIN_DT_BF16 || p.mid_round == QLIN_DT_NONE) &&
-               (p.acc_round == QLIN_DT_BF16 || p.acc_round == QLIN_DT_NONE)) {
-      // (acc * rs) * cs, optional bf16 rounding, + bias, bf16: the chain of the FP8 Linear and of the fused ops, two columns
-      // per instruction; the final packed conversion is the last rounding
-      const bool mid_bf16 = p.mid_round == QLIN_DT_BF16;
-      const float2 rs2 = make_float2(rs, rs);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        float2 a2;
-        if (F8) {
-          a2 = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-        } else {
-          a2 = make_float2(__int2float_rn(static_cast<int32_t>(v[2 * j])), __int2float_rn(static_cast<int32_t>(v[2 * j + 1])));
-        }
-        float2 t = __fmul2_rn(__fmul2_rn(a2, rs2), *reinterpret_cast<const float2*>(s_cs + s_off + 2 * j));
-        if (has_bias) {
-          if (mid_bf16) {
-            const __nv_bfloat162 b2 = __float22bfloat162_rn(t);
-            const uint32_t bw = *reinterpret_cast<const uint32_t*>(&b2);
-            t = make_float2(__uint_as_float(bw << 16), __uint_as_float(bw & 0xFFFF0000u));
-          }
-          t = __fadd2_rn(t, *reinterpret_cast<const float2*>(s_bias + s_off + 2 * j));
-        }
-        const __nv_bfloat162 o2 = __float22bfloat162_rn(t);
-        w[j] = *reinterpret_cast<const uint32_t*>(&o2);
-      }
-    } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float y0 = dequant_one<F8>(p, v[2 * j], rs, s_cs[s_off + 2 * j], s_bias[s_off + 2 * j], prod, has_bias);
-      const float y1 =
-          dequant_one<F8>(p, v[2 * j + 1], rs, s_cs[s_off + 2 * j + 1], s_bias[s_off + 2 * j + 1], prod, has_bias);
-      w[j] = pack16(p, y0, y1);
-    }
-    }
-    uint8_t* g = out_row(p, row0, 2) + static_cast<int64_t>(col0) * 2;
-    store_tile_coalesced(stage, w, g, p.ldd * 2, rows_valid, lane);
+__device__ __forceinline__ void emit32_wide(const GemmParams& p, const EpiCtx& e, const uint32_t (&v)[32], int row0, int lane, int col0) {
+  const int left = p.N - col0;
+  if (left <= 0) return;
+  if (e.vec_ok && (left >= 32 || left % 4 == 0)) {
+    uint8_t* g = out_row(p, e.dbase, row0, 4) + static_cast<int64_t>(col0) * 4;
+    store_tile_coalesced(e.stage, v, g, p.ldd * 4, p.M - row0, lane, left >= 32 ? 8 : left / 4);
   } else {
-    // 4-byte outputs: two staging passes of 32 columns
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint32_t w[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int k = h * 32 + j;
-        w[j] = p.epilogue == QLIN_EPI_RAW
-                   ? v[k]
-                   : __float_as_uint(dequant_one<F8>(p, v[k], rs, s_cs[s_off + k], s_bias[s_off + k], prod, has_bias));
-      }
-      uint8_t* g = out_row(p, row0, 4) + static_cast<int64_t>(col0 + h * 32) * 4;
-      store_tile_coalesced(stage, w, g, p.ldd * 4, rows_valid, lane);
-    }
+    store_row_direct(p, e.dbase, v, row0 + lane, col0, false);
   }
 }
 
-// Emits 32 accumulator columns of this thread's row (the chunked kernel's final store): 4-byte
-// outputs go through the coalescing tile, 2-byte outputs (64 bytes per row) are stored directly.
+// Emits 64 accumulator columns [col0, col0 + 64) of this thread's row, given as two halves.
 template <bool F8>
-__device__ __forceinline__ void emit32(const GemmParams& p, const uint32_t (&v)[32], int row0, int lane, int col0,
-                                       const float* s_cs, const float* s_bias, int s_off, float rs, bool vec_ok,
-                                       uint8_t* stage) {
-  const bool four_byte = p.epilogue == QLIN_EPI_RAW || p.out_dtype == QLIN_DT_F32;
-  if (!vec_ok || col0 + 32 > p.N || !four_byte) {
-    store_row_direct<F8, 32>(p, v, row0 + lane, col0, s_cs, s_bias, s_off, rs);
-    return;
+__device__ __forceinline__ void emit64(const GemmParams& p, const EpiCtx& e, uint32_t (&lo)[32], uint32_t (&hi)[32], int row0, int lane, int col0,
+                                       const float* s_cs, const float* s_bias, float rs) {
+  if (e.scaled) {
+    dequant32<F8>(p, lo, rs, s_cs, s_bias);
+    dequant32<F8>(p, hi, rs, s_cs + 32, s_bias + 32);
   }
-  const bool prod = p.epilogue == QLIN_EPI_SCALE_PROD;
-  const bool has_bias = p.bias != nullptr;
-  uint32_t w[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j)
-    w[j] = p.epilogue == QLIN_EPI_RAW
-               ? v[j]
-               : __float_as_uint(dequant_one<F8>(p, v[j], rs, s_cs[s_off + j], s_bias[s_off + j], prod, has_bias));
-  uint8_t* g = out_row(p, row0, 4) + static_cast<int64_t>(col0) * 4;
-  store_tile_coalesced(stage, w, g, p.ldd * 4, p.M - row0, lane);
+  if (e.two_byte) {
+    const int left = p.N - col0;
+    if (left <= 0) return;
+    if (e.vec_ok && (left >= 64 || left % 8 == 0)) {
+      uint32_t w[32];  // 64 columns = one 128-byte staging row
+      pack32(lo, w, p.out_dtype == QLIN_DT_BF16);
+      pack32(hi, w + 16, p.out_dtype == QLIN_DT_BF16);
+      uint8_t* g = out_row(p, e.dbase, row0, 2) + static_cast<int64_t>(col0) * 2;
+      store_tile_coalesced(e.stage, w, g, p.ldd * 2, p.M - row0, lane, left >= 64 ? 8 : left / 8);
+    } else {
+      store_row_direct(p, e.dbase, lo, row0 + lane, col0, true);
+      store_row_direct(p, e.dbase, hi, row0 + lane, col0 + 32, true);
+    }
+  } else {
+    emit32_wide<F8>(p, e, lo, row0, lane, col0);
+    emit32_wide<F8>(p, e, hi, row0, lane, col0 + 32);
+  }
+}
+
+// Emits 32 accumulator columns of this thread's row (the chunked kernel's final store).
+template <bool F8>
+__device__ __forceinline__ void emit32(const GemmParams& p, const EpiCtx& e, uint32_t (&v)[32], int row0, int lane, int col0, const float* s_cs,
+                                       const float* s_bias, float rs) {
+  if (e.scaled) dequant32<F8>(p, v, rs, s_cs, s_bias);
+  if (e.two_byte) {
+    store_row_direct(p, e.dbase, v, row0 + lane, col0, true);
+  } else {
+    emit32_wide<F8>(p, e, v, row0, lane, col0);
+  }
 }
 
 // BATCHED: p.batch problems of the same shape whose operands are stacked along the rows (A is [batch * M, K], B is
@@ -618,16 +651,14 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int q = warp & 3;
     const int half = warp >> 2;  // column slice of this warp
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    uint8_t* stage = smem + C::OUT_OFFSET + warp * kStageOutBytes;
-    const int elt = (p.out_dtype == QLIN_DT_F16 || p.out_dtype == QLIN_DT_BF16) ? 2 : 4;
-    const bool vec_ok = (p.scatter_rows > 0 || (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0) && ((p.ldd * elt) % 16 == 0);
+    EpiCtx epi = make_epi_ctx(p, smem + C::OUT_OFFSET + warp * kStageOutBytes);
     const bool clamp = !F8 && p.max_acc_bits < 32;
     const int32_t lo = clamp ? -(1 << (p.max_acc_bits - 1)) : 0;
     const int32_t hi = clamp ? (1 << (p.max_acc_bits - 1)) - 1 : 0;
     const uint32_t rb = p.trun_bits > 0 ? (1u << (p.trun_bits - 1)) : 0u;
     const uint32_t mask = p.trun_bits > 0 ? ~((1u << p.trun_bits) - 1u) : 0xFFFFFFFFu;
     const bool dl16 = F8 && p.clamp_dl16;
-    const bool scaled = p.epilogue != QLIN_EPI_RAW;
+    const bool scaled = epi.scaled;
     uint32_t ebuf = 0, ebph = 0;
     bool eready = false;
     bool ok = true;
@@ -637,14 +668,7 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       int mb, nb;
       const int bi = BATCHED ? t / per_batch : 0;
       tile_coords(t - bi * per_batch, p.num_m, p.num_n, mb, nb);
-      GemmParams pb;
-      const GemmParams* pp = &p;
-      if constexpr (BATCHED) {
-        pb = p;
-        pb.d = static_cast<uint8_t*>(p.d) + static_cast<int64_t>(bi) * p.batch_stride_d * elt;
-        pp = &pb;
-      }
-      const GemmParams& pe = *pp;
+      if (BATCHED) epi.dbase = static_cast<uint8_t*>(p.d) + static_cast<int64_t>(bi) * p.batch_stride_d * (epi.two_byte ? 2 : 4);
       const int row0 = mb * kBM + q * 32;
       const int row = row0 + lane;
       const int col_w = nb * C::BN + half * C::COLS_PER_WARP;
@@ -673,15 +697,19 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         tc_fence_after();
 #pragma unroll 1
         for (int j = 0; j < C::COLS_PER_WARP; j += 64) {
-          uint32_t v[64];
-          tmem_ld64(tmem_base + lane_base + buf * C::BN + half * C::COLS_PER_WARP + j, v);
+          const int off = half * C::COLS_PER_WARP + j;
+          uint32_t lo[32], hi[32];
+          tmem_ld64(tmem_base + lane_base + buf * C::BN + off, lo, hi);
           if (p.c != nullptr) {
-            uint32_t cv[64];
-            load_c_row<64>(p, cv, row, col_w + j);
+            uint32_t cv[32];
+            load_c_row<32>(p, cv, row, col_w + j);
 #pragma unroll
-            for (int i = 0; i < 64; ++i) v[i] = acc_add<F8>(cv[i], v[i]);
+            for (int i = 0; i < 32; ++i) lo[i] = acc_add<F8>(cv[i], lo[i]);
+            load_c_row<32>(p, cv, row, col_w + j + 32);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) hi[i] = acc_add<F8>(cv[i], hi[i]);
           }
-          emit64<F8>(pe, v, row0, lane, col_w + j, aux->cs, aux->bias, half * C::COLS_PER_WARP + j, rs, vec_ok, stage);
+          emit64<F8>(p, epi, lo, hi, row0, lane, col_w + j, aux->cs + off, aux->bias + off, rs);
         }
         tc_fence_before();
         __syncwarp();
@@ -755,7 +783,7 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           for (int i = 0; i < C::COLS_PER_WARP; ++i) run[i] += tot[i];
         }
         if (!ok) break;
-        emit32<F8>(p, run, row0, lane, col_w, aux->cs, aux->bias, half * C::COLS_PER_WARP, rs, vec_ok, stage);
+        emit32<F8>(p, epi, run, row0, lane, col_w, aux->cs + half * C::COLS_PER_WARP, aux->bias + half * C::COLS_PER_WARP, rs);
       }
     }
     if (!ok && lane == 0) {
@@ -959,10 +987,8 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int q = warp & 3;
     const int half = warp >> 2;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    uint8_t* stage = smem + C::OUT_OFFSET + warp * kStageOutBytes;
-    const int elt = (p.out_dtype == QLIN_DT_F16 || p.out_dtype == QLIN_DT_BF16) ? 2 : 4;
-    const bool vec_ok = (p.scatter_rows > 0 || (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0) && ((p.ldd * elt) % 16 == 0);
-    const bool scaled = p.epilogue != QLIN_EPI_RAW;
+    const EpiCtx epi = make_epi_ctx(p, smem + C::OUT_OFFSET + warp * kStageOutBytes);
+    const bool scaled = epi.scaled;
     uint32_t ebuf = 0, ebph = 0;
     bool ok = true;
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
@@ -994,15 +1020,19 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       tc_fence_after();
 #pragma unroll 1
       for (int j = 0; j < C::COLS_PER_WARP; j += 64) {
-        uint32_t v[64];
-        tmem_ld64(tmem_base + lane_base + buf * C::BN + half * C::COLS_PER_WARP + j, v);
+        const int off = half * C::COLS_PER_WARP + j;
+        uint32_t lo[32], hi[32];
+        tmem_ld64(tmem_base + lane_base + buf * C::BN + off, lo, hi);
         if (p.c != nullptr) {
-          uint32_t cv[64];
-          load_c_row<64>(p, cv, row, col_w + j);
+          uint32_t cv[32];
+          load_c_row<32>(p, cv, row, col_w + j);
 #pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = acc_add<F8>(cv[i], v[i]);
+          for (int i = 0; i < 32; ++i) lo[i] = acc_add<F8>(cv[i], lo[i]);
+          load_c_row<32>(p, cv, row, col_w + j + 32);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) hi[i] = acc_add<F8>(cv[i], hi[i]);
         }
-        emit64<F8>(p, v, row0, lane, col_w + j, aux->cs, aux->bias, half * C::COLS_PER_WARP + j, rs, vec_ok, stage);
+        emit64<F8>(p, epi, lo, hi, row0, lane, col_w + j, aux->cs + off, aux->bias + off, rs);
       }
       tc_fence_before();
       __syncwarp();
@@ -1490,7 +1520,7 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
   if (a->epilogue == QLIN_EPI_RAW) {
     if (a->out_dtype != (f8 ? QLIN_DT_F32 : QLIN_DT_I32))
       return fail(QLIN_ERR_BAD_DTYPE, "qlin_gemm: raw output is int32 for int8 operands and fp32 for fp8 operands");
-  } else if (a->epilogue == QLIN_EPI_SCALE_PROD || a->epilogue == QLIN_EPI_SCALE_SEQ) {
+  } else if (a->epilogue >= QLIN_EPI_SCALE_PROD && a->epilogue <= QLIN_EPI_SCALE_ACC16) {
     if (a->out_dtype != QLIN_DT_F32 && a->out_dtype != QLIN_DT_F16 && a->out_dtype != QLIN_DT_BF16)
       return fail(QLIN_ERR_BAD_DTYPE, "qlin_gemm: scaled output must be fp32, fp16 or bf16");
     if (!is_round_dtype(a->prod_round) || !is_round_dtype(a->scale_round) || !is_round_dtype(a->mid_round) || !is_round_dtype(a->acc_round))

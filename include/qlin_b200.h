@@ -91,6 +91,8 @@ int qlin_device_supported(int device);
  *                       y = round(y, acc_round); d = cast(y, out_dtype)
  *   QLIN_EPI_SCALE_SEQ  y = (acc * rs) * cs; y = round(y, mid_round); y = y + bias[n];
  *                       y = round(y, acc_round); d = cast(y, out_dtype)
+ *   QLIN_EPI_SCALE_ACC16  the same as QLIN_EPI_SCALE_SEQ with acc rounded to fp16 first: QBmmINT8Deploy's
+ *                       acc.to(fp16) * m1_scale * m2_scale (fms_mo/modules/bmm.py:741-752)
  * round(.., QLIN_DT_NONE/F32) is the identity; F16 / BF16 round to nearest even and widen back.
  * Every multiply and add is a separately rounded fp32 operation (no FMA contraction), which is
  * what the reference's eager tensor expressions compute.
@@ -98,7 +100,8 @@ int qlin_device_supported(int device);
 typedef enum qlin_epilogue {
   QLIN_EPI_RAW = 0,
   QLIN_EPI_SCALE_PROD = 1,
-  QLIN_EPI_SCALE_SEQ = 2
+  QLIN_EPI_SCALE_SEQ = 2,
+  QLIN_EPI_SCALE_ACC16 = 3
 } qlin_epilogue;
 
 typedef struct qlin_gemm_args {
