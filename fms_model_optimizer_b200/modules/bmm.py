@@ -178,8 +178,14 @@ class QBmmINT8Deploy(nn.Module):
             m2_nk = m2.transpose(-1, -2).contiguous()
             m1_i8 = self._codes(m1.contiguous(), self.m1_scale, s1, zp1)
             m2_i8_nk = self._codes(m2_nk, self.m2_scale, s2, zp2)
-            acc = ops.bmm_i8(m1_i8.reshape(-1, m, k), m2_i8_nk.reshape(-1, n, k)).view(*lead, m, n)
-            x = acc.to(torch.float16) * self.m1_scale * self.m2_scale
+            a3, b3 = m1_i8.reshape(-1, m, k), m2_i8_nk.reshape(-1, n, k)
+            if all(t.dtype == torch.float32 and t.shape == (1,) for t in (self.m1_scale, self.m2_scale)):
+                # acc.to(fp16) * m1_scale * m2_scale, formed in the GEMM's epilogue (fp32, as PyTorch promotes fp16 with a
+                # one-element fp32 tensor) and written in the result's type when nothing is added to it
+                direct = zp1 == 0 and m1.dtype in (torch.float32, torch.float16, torch.bfloat16)
+                x = ops.bmm_i8(a3, b3, (self.m1_scale, self.m2_scale), m1.dtype if direct else torch.float32).view(*lead, m, n)
+            else:
+                x = ops.bmm_i8(a3, b3).view(*lead, m, n).to(torch.float16) * self.m1_scale * self.m2_scale
             if zp1 != 0:
                 # the reference's correction term as it stands there (fms_mo/modules/bmm.py:741-746), the sum over
                 # dimension 0 of m2's codes included

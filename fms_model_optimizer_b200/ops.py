@@ -231,10 +231,12 @@ def gemm(
     return out
 
 
-def bmm_i8(a: torch.Tensor, b_nk: torch.Tensor) -> torch.Tensor:
+def bmm_i8(a: torch.Tensor, b_nk: torch.Tensor, scales: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
+           out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """Batched int8 product: ``a [B, M, K]`` times ``b_nk [B, N, K]`` (both K-contiguous) -> int32 ``[B, M, N]``, exact.
     One ``qlin_gemm_batched`` call (include/qlin_b200.h); the integer product QBmmINT8Deploy stands for
-    (fms_mo/modules/bmm.py:741-752 simulates it with a float matmul)."""
+    (fms_mo/modules/bmm.py:741-752 simulates it with a float matmul).  With ``scales = (s1, s2)``, one-element fp32 device
+    tensors, the epilogue returns ``(float(fp16(sum)) * s1) * s2`` in ``out_dtype`` (fp32, fp16 or bf16) instead."""
     if a.dim() != 3 or b_nk.dim() != 3 or a.shape[0] != b_nk.shape[0] or a.shape[2] != b_nk.shape[2]:
         raise RuntimeError("bmm_i8 takes a [B,M,K] and b_nk [B,N,K]")
     if a.dtype != torch.int8 or b_nk.dtype != torch.int8 or not a.is_cuda or a.device != b_nk.device:
@@ -242,7 +244,17 @@ def bmm_i8(a: torch.Tensor, b_nk: torch.Tensor) -> torch.Tensor:
     B, M, K = a.shape
     N = b_nk.shape[1]
     dev = a.device
-    out = torch.empty((B, M, N), dtype=torch.int32, device=dev)
+    epilogue, s1, s2 = L.EPI_RAW, None, None
+    if scales is None:
+        out_dtype = torch.int32
+    else:
+        epilogue, (s1, s2) = L.EPI_SCALE_ACC16, scales
+        for t in (s1, s2):
+            if t.dtype != torch.float32 or t.numel() != 1 or t.device != dev:
+                raise RuntimeError("scales are one-element fp32 tensors on the operands' device")
+        if out_dtype not in (torch.float32, torch.float16, torch.bfloat16):
+            raise RuntimeError(f"unsupported output dtype {out_dtype}")
+    out = torch.empty((B, M, N), dtype=out_dtype, device=dev)
     if B == 0 or M == 0 or N == 0:
         return out
     if K % 16 != 0:  # rows of the operands must start on 16-byte boundaries: zero columns add nothing
@@ -251,10 +263,10 @@ def bmm_i8(a: torch.Tensor, b_nk: torch.Tensor) -> torch.Tensor:
     a, b_nk = a.contiguous(), b_nk.contiguous()
     Kp = a.shape[2]
     args = L.GemmArgs(
-        a=_ptr(a), b=_ptr(b_nk), c=None, d=_ptr(out), row_scale=None, col_scale=None, bias=None, status=_ptr(status_word(dev)),
+        a=_ptr(a), b=_ptr(b_nk), c=None, d=_ptr(out), row_scale=_ptr(s1), col_scale=_ptr(s2), bias=None, status=_ptr(status_word(dev)),
         lda=Kp, ldb=Kp, ldc=0, ldd=N, M=M, N=N, K=Kp, kind=L.DT_I8, chunk_k=0, trun_bits=0, max_acc_bits=32, trunc_then_acc=1,
-        clamp_dl16=0, epilogue=L.EPI_RAW, row_scale_stride=0, col_scale_stride=0, prod_round=_ROUND[None], scale_round=_ROUND[None],
-        mid_round=_ROUND[None], acc_round=_ROUND[None], out_dtype=L.DT_I32, max_ctas=int(GEMM_MAX_CTAS),
+        clamp_dl16=0, epilogue=epilogue, row_scale_stride=0, col_scale_stride=0, prod_round=_ROUND[None], scale_round=_ROUND[None],
+        mid_round=_ROUND[None], acc_round=_ROUND[None], out_dtype=_DT[out_dtype], max_ctas=int(GEMM_MAX_CTAS),
     )  # fmt: skip
     with torch.cuda.device(dev):
         rc = _timed("gemm", 2.0 * B * M * N * K, dev,
