@@ -43,6 +43,7 @@ EXPORTED_SYMBOLS = (
     "qlin_gemm",
     "qlin_gemm_batched",
     "qlin_act_quant",
+    "qlin_act_quant_static",
     "qlin_pact2_fwd",
     "qlin_pact2_bwd",
     "qlin_pact2_bwd_workspace_bytes",
@@ -133,6 +134,10 @@ class QuantArgs(C.Structure):
         ("dyn_eps", C.c_float),
         ("f8_format", C.c_int32),
     ]
+
+
+class ScalarSrc(C.Structure):
+    _fields_ = [("ptr", C.c_void_p), ("dtype", C.c_int32)]
 
 
 class Pact2Args(C.Structure):
@@ -319,6 +324,8 @@ def load() -> C.CDLL:
         fn.restype = C.c_int
     lib.qlin_gemm_batched.argtypes = [C.POINTER(GemmArgs), C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]
     lib.qlin_gemm_batched.restype = C.c_int
+    lib.qlin_act_quant_static.argtypes = [C.POINTER(QuantArgs), C.POINTER(ScalarSrc), C.c_void_p]
+    lib.qlin_act_quant_static.restype = C.c_int
     lib.qlin_pact2_bwd_workspace_bytes.argtypes = [C.c_int64]
     lib.qlin_pact2_bwd_workspace_bytes.restype = C.c_size_t
     lib.qlin_pact2_bwd_noalloc_max_numel.restype = C.c_int64

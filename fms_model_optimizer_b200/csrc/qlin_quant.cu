@@ -37,7 +37,30 @@ struct QuantParams {
   int32_t mode, native, native_smooth, smooth_mul, clamp_codes, levels, dl8_flush, scale_in_stride;
   float scale0, zp0, lo, hi, shift, add2, dyn_eps;
   int32_t f8_e5m2;
+  qlin_scalar_src src[4];  // static modes: scale0, zp0, lo, hi read from device memory where a pointer is set
 };
+
+// The static quantisers' scalars: launch arguments, or values in device memory (a module's scale and zero-point buffers:
+// reading them here instead of on the host saves a stream synchronisation per forward pass).
+struct StaticVals {
+  float scale0, zp0, lo, hi;
+};
+__device__ __forceinline__ float load_scalar(const qlin_scalar_src& src, float given) {
+  if (src.ptr == nullptr) return given;
+  switch (src.dtype) {
+    case QLIN_DT_F16:
+      return __half2float(*reinterpret_cast<const __half*>(src.ptr));
+    case QLIN_DT_BF16:
+      return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(src.ptr));
+    case QLIN_DT_I32:
+      return static_cast<float>(*reinterpret_cast<const int32_t*>(src.ptr));
+    default:
+      return *reinterpret_cast<const float*>(src.ptr);
+  }
+}
+__device__ __forceinline__ StaticVals static_vals(const QuantParams& p) {
+  return StaticVals{load_scalar(p.src[0], p.scale0), load_scalar(p.src[1], p.zp0), load_scalar(p.src[2], p.lo), load_scalar(p.src[3], p.hi)};
+}
 
 template <typename XT>
 __device__ __forceinline__ float smooth_apply(const QuantParams& p, float x, float sm, float rsm) {
@@ -85,7 +108,7 @@ __device__ __forceinline__ float from_e4m3(uint8_t c) {
 
 // One element: value after smoothing -> code byte, and the fake-quantised value for dq_out.
 template <typename XT>
-__device__ __forceinline__ uint8_t quant_one(const QuantParams& p, float v, float s, float rs, float& dq) {
+__device__ __forceinline__ uint8_t quant_one(const QuantParams& p, const StaticVals& sv, float v, float s, float rs, float& dq) {
   const bool nat = p.native;
   switch (p.mode) {
     case QLIN_Q_I8_DYN:
@@ -93,14 +116,14 @@ __device__ __forceinline__ uint8_t quant_one(const QuantParams& p, float v, floa
       const float r = rintf(rnd_if<XT>(div_exact(v, s, rs), nat));
       dq = rnd_if<XT>(__fmul_rn(r, s), nat);
       float c = r;
-      if (p.mode == QLIN_Q_I8_GIVEN_SCALE) c = rnd_if<XT>(__fadd_rn(c, p.zp0), nat);
+      if (p.mode == QLIN_Q_I8_GIVEN_SCALE) c = rnd_if<XT>(__fadd_rn(c, sv.zp0), nat);
       int q = static_cast<int>(c);
       if (p.clamp_codes) q = max(-p.levels, min(p.levels, q));
       return static_cast<uint8_t>(q & 0xFF);
     }
     case QLIN_Q_I8_STATIC: {
       float t = rnd_if<XT>(div_exact(v, s, rs), nat);
-      t = rnd_if<XT>(__fadd_rn(t, p.zp0), nat);
+      t = rnd_if<XT>(__fadd_rn(t, sv.zp0), nat);
       t = rnd_if<XT>(__fsub_rn(t, p.shift), nat);
       t = rnd_if<XT>(__fadd_rn(t, p.add2), nat);
       const float r = fminf(fmaxf(rintf(t), -128.0f), 127.0f);
@@ -108,22 +131,22 @@ __device__ __forceinline__ uint8_t quant_one(const QuantParams& p, float v, floa
       return static_cast<uint8_t>(static_cast<int>(r) & 0xFF);
     }
     case QLIN_Q_I8_STATIC_CLAMP_FIRST: {
-      float t = fminf(fmaxf(v, p.lo), p.hi);
+      float t = fminf(fmaxf(v, sv.lo), sv.hi);
       t = rnd_if<XT>(div_exact(t, s, rs), nat);
-      t = rnd_if<XT>(__fsub_rn(t, p.zp0), nat);
+      t = rnd_if<XT>(__fsub_rn(t, sv.zp0), nat);
       const float r = rnd_if<XT>(__fsub_rn(rintf(t), p.shift), nat);
       dq = r;
       return static_cast<uint8_t>(static_cast<int>(r) & 0xFF);
     }
     case QLIN_Q_I8_STATIC_ROUND_FIRST: {  // clamp(rint(v / s + zp), lo, hi) - shift
       float t = rnd_if<XT>(div_exact(v, s, rs), nat);
-      t = rnd_if<XT>(__fadd_rn(t, p.zp0), nat);
-      const float r = fminf(fmaxf(rintf(t), p.lo), p.hi) - p.shift;
+      t = rnd_if<XT>(__fadd_rn(t, sv.zp0), nat);
+      const float r = fminf(fmaxf(rintf(t), sv.lo), sv.hi) - p.shift;
       dq = r;
       return static_cast<uint8_t>(static_cast<int>(r) & 0xFF);
     }
     case QLIN_Q_I8_AFFINE_RCP: {  // torch.quantize_per_tensor: clamp(nearbyint(v * (1 / s)) + zp, -128, 127)
-      const float r = fminf(fmaxf(nearbyintf(__fmul_rn(v, __fdiv_rn(1.0f, s))) + p.zp0, -128.0f), 127.0f);
+      const float r = fminf(fmaxf(nearbyintf(__fmul_rn(v, __fdiv_rn(1.0f, s))) + sv.zp0, -128.0f), 127.0f);
       dq = r;
       return static_cast<uint8_t>(static_cast<int>(r) & 0xFF);
     }
@@ -166,14 +189,14 @@ __device__ __forceinline__ bool is_dynamic(int mode) {
 }
 
 template <typename XT>
-__device__ __forceinline__ float row_scale_of(const QuantParams& p, int row, float amax) {
+__device__ __forceinline__ float row_scale_of(const QuantParams& p, const StaticVals& sv, int row, float amax) {
   if (is_dynamic(p.mode)) return dyn_scale<XT>(p, amax);
   if (p.mode == QLIN_Q_I8_GIVEN_SCALE) return p.scale_in[static_cast<int64_t>(row) * p.scale_in_stride];
   if (p.mode == QLIN_Q_F8_TENSOR) {
     const float a = rnd_if<XT>(__fdiv_rn(p.scale_in[0], p.scale0), p.native);
     return fmaxf(a, rnd_if<XT>(p.dyn_eps, p.native));
   }
-  return p.scale0;
+  return sv.scale0;
 }
 
 // Vector path: cols % 16 == 0 and every row start 16-byte aligned.  MAXC = register-resident
@@ -184,6 +207,7 @@ __global__ void __launch_bounds__(1024) act_quant_vec_kernel(const QuantParams p
   const int nchunks = p.cols >> 4;
   const bool has_smooth = p.smooth != nullptr;
   constexpr int NREG = MAXC > 0 ? MAXC : 1;
+  const StaticVals sv = static_vals(p);
   int iter = 0;
   for (int row = blockIdx.x; row < p.rows; row += gridDim.x, ++iter) {
     const XT* xr = reinterpret_cast<const XT*>(p.x) + static_cast<int64_t>(row) * p.ldx;
@@ -221,7 +245,7 @@ __global__ void __launch_bounds__(1024) act_quant_vec_kernel(const QuantParams p
       }
     }
     if (is_dynamic(p.mode)) amax = block_reduce<OpMax>(amax, red[iter & 1], 0.0f);
-    const float s = row_scale_of<XT>(p, row, amax);
+    const float s = row_scale_of<XT>(p, sv, row, amax);
     const float rs = rcp_for_div(s);
     if (threadIdx.x == 0 && p.scale_out != nullptr) p.scale_out[row] = s;
 
@@ -230,7 +254,7 @@ __global__ void __launch_bounds__(1024) act_quant_vec_kernel(const QuantParams p
       uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const uint32_t c = quant_one<XT>(p, val[i], s, rs, dq[i]);
+        const uint32_t c = quant_one<XT>(p, sv, val[i], s, rs, dq[i]);
         w[i >> 2] |= c << (8 * (i & 3));
       }
       if (p.codes != nullptr)
@@ -738,6 +762,7 @@ template <typename XT>
 __global__ void __launch_bounds__(256) act_quant_scalar_kernel(const QuantParams p) {
   __shared__ float red[2][32];
   const bool has_smooth = p.smooth != nullptr;
+  const StaticVals sv = static_vals(p);
   int iter = 0;
   for (int row = blockIdx.x; row < p.rows; row += gridDim.x, ++iter) {
     const XT* xr = reinterpret_cast<const XT*>(p.x) + static_cast<int64_t>(row) * p.ldx;
@@ -750,22 +775,124 @@ __global__ void __launch_bounds__(256) act_quant_scalar_kernel(const QuantParams
       }
       amax = block_reduce<OpMax>(amax, red[iter & 1], 0.0f);
     }
-    const float s = row_scale_of<XT>(p, row, amax);
+    const float s = row_scale_of<XT>(p, sv, row, amax);
     const float rs = rcp_for_div(s);
     if (threadIdx.x == 0 && p.scale_out != nullptr) p.scale_out[row] = s;
     for (int c = threadIdx.x; c < p.cols; c += blockDim.x) {
       float v = load1(xr + c);
       if (has_smooth) v = smooth_apply<XT>(p, v, p.smooth[c], p.smooth_mul ? 0.0f : p.smooth_rcp[c]);
       float dq;
-      const uint8_t code = quant_one<XT>(p, v, s, rs, dq);
+      const uint8_t code = quant_one<XT>(p, sv, v, s, rs, dq);
       if (p.codes != nullptr) p.codes[static_cast<int64_t>(row) * p.ldq + c] = code;
       if (p.dq_out != nullptr) store1(reinterpret_cast<XT*>(p.dq_out) + static_cast<int64_t>(row) * p.lddq + c, dq);
     }
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Static modes over a dense tensor: every element is independent, so rows do not matter and the tensor is walked flat,
+// 16 elements a thread.  The general kernels above give a row to a block: with the 128-element rows of attention heads
+// 8 of a block's 32 threads work (132 us for a 64 x 2048 x 128 bf16 tensor), rows whose length is no multiple of 16 are
+// read element by element, and the mode is asked per element (11 us for 4096 x 768 fp32).  HBM-bound: s + 1 bytes an element.
+// ------------------------------------------------------------------------------------------------
+constexpr int kStThreads = 256;
+
+// RN(x / s) for a static quantiser, from r = RN(1 / s) (see div_exact).  Where div_exact would take the ordinary division the
+// code does not depend on the digits: below 1e-15 it is the code of zero, above 1e15 (and for infinities and NaN) that of q.
+__device__ __forceinline__ float static_div(float x, float s, float r) {
+  const float q = __fmul_rn(x, r);
+  const float q2 = __fmaf_rn(__fmaf_rn(-s, q, x), r, q);
+  return fabsf(q) < 1e15f ? q2 : q;
+}
+
+template <typename XT, int MODE, bool NATIVE>
+__device__ __forceinline__ uint32_t static_code(const QuantParams& p, const StaticVals& sv, bool exact, float rs, float v) {
+  if (MODE == QLIN_Q_I8_AFFINE_RCP) {  // rs is the reciprocal torch.quantize_per_tensor multiplies with
+    const float c = fminf(fmaxf(nearbyintf(__fmul_rn(v, rs)) + sv.zp0, -128.0f), 127.0f);
+    return static_cast<uint32_t>(static_cast<int>(c)) & 0xFFu;
+  }
+  if (MODE == QLIN_Q_I8_STATIC_CLAMP_FIRST) v = fminf(fmaxf(v, sv.lo), sv.hi);
+  float t = rnd_if<XT>(exact ? __fdiv_rn(v, sv.scale0) : static_div(v, sv.scale0, rs), NATIVE);
+  if (MODE == QLIN_Q_I8_STATIC) {
+    t = rnd_if<XT>(__fadd_rn(t, sv.zp0), NATIVE);
+    t = rnd_if<XT>(__fsub_rn(t, p.shift), NATIVE);
+    t = rnd_if<XT>(__fadd_rn(t, p.add2), NATIVE);
+    // the bounds are whole numbers, so clamping before rounding gives the same code; the low byte of the biased sum is it
+    t = fminf(fmaxf(t, -128.0f), 127.0f);
+    return __float_as_uint(__fadd_rn(t, 12582912.0f)) & 0xFFu;
+  }
+  if (MODE == QLIN_Q_I8_STATIC_CLAMP_FIRST) {
+    t = rnd_if<XT>(__fsub_rn(t, sv.zp0), NATIVE);
+    t = rnd_if<XT>(__fsub_rn(rintf(t), p.shift), NATIVE);
+    return static_cast<uint32_t>(static_cast<int>(t)) & 0xFFu;
+  }
+  t = rnd_if<XT>(__fadd_rn(t, sv.zp0), NATIVE);
+  const float c = fminf(fmaxf(rintf(t), sv.lo), sv.hi) - p.shift;
+  return static_cast<uint32_t>(static_cast<int>(c)) & 0xFFu;
+}
+
+template <typename XT, int MODE, bool NATIVE>
+__global__ void __launch_bounds__(kStThreads) act_quant_static_kernel(const QuantParams p) {
+  const StaticVals sv = static_vals(p);
+  const XT* x = reinterpret_cast<const XT*>(p.x);
+  const int64_t numel = static_cast<int64_t>(p.rows) * p.cols;
+  const int64_t nvec = numel >> 4;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kStThreads + threadIdx.x, stride = static_cast<int64_t>(gridDim.x) * kStThreads;
+  const float rs = MODE == QLIN_Q_I8_AFFINE_RCP ? __fdiv_rn(1.0f, sv.scale0) : rcp_for_div(sv.scale0);
+  const bool exact = rs != rs;  // this scale takes the ordinary division
+  if (p.scale_out != nullptr)
+    for (int64_t r = first; r < p.rows; r += stride) p.scale_out[r] = sv.scale0;
+  for (int64_t i = first; i < nvec; i += stride) {
+    float v[16];
+    load16(x + i * 16, v);
+    uint32_t w[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      uint32_t b[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) b[k] = static_code<XT, MODE, NATIVE>(p, sv, exact, rs, v[4 * g + k]);
+      w[g] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+    }
+    *reinterpret_cast<uint4*>(p.codes + i * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  for (int64_t i = nvec * 16 + first; i < numel; i += stride) p.codes[i] = static_cast<uint8_t>(static_code<XT, MODE, NATIVE>(p, sv, exact, rs, load1(x + i)));
+}
+
+// Returns 1 when the call is not one of a dense tensor quantised with a static mode.
+template <typename XT>
+static int try_static(const QuantParams& p, cudaStream_t stream) {
+  const bool is_static = p.mode == QLIN_Q_I8_STATIC || p.mode == QLIN_Q_I8_STATIC_CLAMP_FIRST || p.mode == QLIN_Q_I8_STATIC_ROUND_FIRST ||
+                         p.mode == QLIN_Q_I8_AFFINE_RCP;
+  if (!is_static || p.smooth != nullptr || p.dq_out != nullptr || p.codes == nullptr) return 1;
+  if (p.rows > 1 && (p.ldx != p.cols || p.ldq != p.cols)) return 1;
+  if (!aligned16(p.x) || !aligned16(p.codes)) return 1;
+  const int64_t nvec = (static_cast<int64_t>(p.rows) * p.cols + 15) / 16;
+  const int64_t want = (nvec + kStThreads - 1) / kStThreads, cap = static_cast<int64_t>(sm_count()) * 8;
+  const int grid = static_cast<int>(want < cap ? want : cap);
+  constexpr bool kIsF32 = sizeof(XT) == 4;
+#define QLIN_ST(MODE)                                                                          \
+  case MODE:                                                                                   \
+    if (!kIsF32 && p.native) {                                                                 \
+      act_quant_static_kernel<XT, MODE, !kIsF32><<<grid, kStThreads, 0, stream>>>(p);          \
+    } else {                                                                                   \
+      act_quant_static_kernel<XT, MODE, false><<<grid, kStThreads, 0, stream>>>(p);            \
+    }                                                                                          \
+    break
+  switch (p.mode) {
+    QLIN_ST(QLIN_Q_I8_STATIC);
+    QLIN_ST(QLIN_Q_I8_STATIC_CLAMP_FIRST);
+    QLIN_ST(QLIN_Q_I8_STATIC_ROUND_FIRST);
+    QLIN_ST(QLIN_Q_I8_AFFINE_RCP);
+  }
+#undef QLIN_ST
+  QLIN_CHECK_LAUNCH("qlin_act_quant");
+  return QLIN_OK;
+}
+
 template <typename XT>
 static int launch_act_quant(const QuantParams& p, cudaStream_t stream) {
+  const int rc_static = try_static<XT>(p, stream);
+  if (rc_static <= 0) return rc_static;
   const int es = static_cast<int>(sizeof(XT));
   bool vec = (p.cols % 16 == 0) && aligned16(p.x) && ((p.ldx * es) % 16 == 0);
   if (p.smooth != nullptr) vec = vec && aligned16(p.smooth) && (p.smooth_mul || aligned16(p.smooth_rcp));
@@ -1017,7 +1144,7 @@ static int launch_wfq(const WfqParams& p, cudaStream_t stream) {
 
 using namespace qlin;
 
-extern "C" int qlin_act_quant(const qlin_quant_args* a, void* stream) {
+static int act_quant_impl(const qlin_quant_args* a, const qlin_scalar_src* src, void* stream) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_act_quant: args is NULL");
   if (a->x == nullptr) return fail(QLIN_ERR_NULL, "qlin_act_quant: x is NULL");
   if (a->codes == nullptr && a->dq_out == nullptr && a->scale_out == nullptr)
@@ -1067,6 +1194,7 @@ extern "C" int qlin_act_quant(const qlin_quant_args* a, void* stream) {
   p.add2 = a->add2;
   p.dyn_eps = a->dyn_eps;
   p.f8_e5m2 = a->f8_format == 1;
+  for (int i = 0; i < 4; ++i) p.src[i] = src != nullptr ? src[i] : qlin_scalar_src{nullptr, 0};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   switch (a->x_dtype) {
     case QLIN_DT_F32:
@@ -1078,6 +1206,18 @@ extern "C" int qlin_act_quant(const qlin_quant_args* a, void* stream) {
     default:
       return fail(QLIN_ERR_BAD_DTYPE, "qlin_act_quant: x_dtype must be F32, F16 or BF16");
   }
+}
+
+extern "C" int qlin_act_quant(const qlin_quant_args* a, void* stream) { return act_quant_impl(a, nullptr, stream); }
+
+extern "C" int qlin_act_quant_static(const qlin_quant_args* a, const qlin_scalar_src src[4], void* stream) {
+  if (a == nullptr || src == nullptr) return fail(QLIN_ERR_NULL, "qlin_act_quant_static: args or src is NULL");
+  if (a->mode != QLIN_Q_I8_STATIC && a->mode != QLIN_Q_I8_STATIC_CLAMP_FIRST && a->mode != QLIN_Q_I8_STATIC_ROUND_FIRST && a->mode != QLIN_Q_I8_AFFINE_RCP)
+    return fail(QLIN_ERR_UNSUPPORTED, "qlin_act_quant_static: mode %d has no static scalars", a->mode);
+  for (int i = 0; i < 4; ++i)
+    if (src[i].ptr != nullptr && src[i].dtype != QLIN_DT_F32 && src[i].dtype != QLIN_DT_F16 && src[i].dtype != QLIN_DT_BF16 && src[i].dtype != QLIN_DT_I32)
+      return fail(QLIN_ERR_BAD_DTYPE, "qlin_act_quant_static: src[%d] must be F32, F16, BF16 or I32", i);
+  return act_quant_impl(a, src, stream);
 }
 
 extern "C" int qlin_weight_fq_perch(const qlin_wfq_args* a, void* stream) {

@@ -290,7 +290,7 @@ class QLinearINT8Deploy(nn.Linear):
                 smooth_native |= 2 if (st == x2.dtype and st != torch.float32) else 0
                 codes, in_scale, _ = ops.act_quant(
                     x2, mode=L.Q_I8_STATIC, smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=smooth_native,
-                    scale0=float(self.input_scale), zp0=float(self.input_zp), shift=128.0, add2=float(self.useSymAct),
+                    scale0=self.input_scale, zp0=self.input_zp, shift=128.0, add2=float(self.useSymAct),
                 )  # fmt: skip
                 in_scale = self.input_scale.detach().float().reshape(-1)
                 scale_dtype = self.input_scale.dtype
@@ -299,7 +299,7 @@ class QLinearINT8Deploy(nn.Linear):
                 smooth_native |= 2 if (st == x2.dtype and st != torch.float32) else 0
                 codes, in_scale, _ = ops.act_quant(
                     x2, mode=L.Q_I8_STATIC_CLAMP_FIRST, smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=smooth_native,
-                    scale0=float(self.quant_stepsize), zp0=float(self.quant_zero_point), lo=float(self.cvs[1]), hi=float(self.cvs[0]),
+                    scale0=self.quant_stepsize, zp0=self.quant_zero_point, lo=self.cvs[1], hi=self.cvs[0],
                     shift=float(128 - self.useSymAct),
                 )  # fmt: skip
                 in_scale = self.input_scale.detach().float().reshape(-1)

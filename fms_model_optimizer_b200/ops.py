@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-from typing import Optional, Sequence, Tuple
+from typing import Optional, Sequence, Tuple, Union
 
 import torch
 
@@ -371,6 +371,18 @@ def smooth_reciprocal(smooth_f32: torch.Tensor) -> torch.Tensor:
     return torch.where(bad, torch.full_like(r, float("nan")), r).contiguous()
 
 
+_STATIC_MODES = (L.Q_I8_STATIC, L.Q_I8_STATIC_CLAMP_FIRST, L.Q_I8_STATIC_ROUND_FIRST, L.Q_I8_AFFINE_RCP)
+
+
+def _scalar_or_src(t, dev: torch.device, src, i: int) -> float:
+    """A static quantiser's scalar: entry ``i`` of ``src`` when ``t`` is a one-element tensor the kernel can read, else the
+    number itself."""
+    if isinstance(t, torch.Tensor) and t.device == dev and t.numel() == 1 and t.dtype in (torch.float32, torch.float16, torch.bfloat16, torch.int32):
+        src[i] = L.ScalarSrc(ptr=t.data_ptr(), dtype=_DT[t.dtype])
+        return 0.0
+    return float(t)
+
+
 def act_quant(
     x: torch.Tensor,
     *,
@@ -385,17 +397,18 @@ def act_quant(
     want_dq: bool = False,
     scale_in: Optional[torch.Tensor] = None,
     dl8_flush: bool = False,
-    scale0: float = 1.0,
-    zp0: float = 0.0,
-    lo: float = 0.0,
-    hi: float = 0.0,
+    scale0: Union[float, torch.Tensor] = 1.0,
+    zp0: Union[float, torch.Tensor] = 0.0,
+    lo: Union[float, torch.Tensor] = 0.0,
+    hi: Union[float, torch.Tensor] = 0.0,
     shift: float = 0.0,
     add2: float = 0.0,
     dyn_eps: float = 1e-5,
     f8_e5m2: bool = False,
 ) -> Tuple[Optional[torch.Tensor], torch.Tensor, Optional[torch.Tensor]]:
     """Row-wise 8-bit quantisation of a 2-D tensor; returns ``(codes, scale[rows], dq)``.
-    See ``qlin_act_quant`` in include/qlin_b200.h for the modes."""
+    See ``qlin_act_quant`` in include/qlin_b200.h for the modes.  In the static modes ``scale0``, ``zp0``, ``lo`` and ``hi``
+    may be one-element tensors; those on x's device are read by the kernel, without a synchronisation."""
     dev = _require_cuda(x, smooth, scale_in)
     if x.dim() != 2:
         raise RuntimeError("act_quant takes a 2-D tensor")
@@ -421,6 +434,10 @@ def act_quant(
     si = _f32(scale_in)
     if rows == 0 or cols == 0:
         return codes, scale, dq
+    src = None
+    if mode in _STATIC_MODES and any(isinstance(t, torch.Tensor) for t in (scale0, zp0, lo, hi)):
+        src = (L.ScalarSrc * 4)()
+        scale0, zp0, lo, hi = (_scalar_or_src(t, dev, src, i) for i, t in enumerate((scale0, zp0, lo, hi)))
     args = L.QuantArgs(
         x=_ptr(x), smooth=_ptr(sm), smooth_rcp=_ptr(rsm), scale_in=_ptr(si), codes=_ptr(codes), scale_out=_ptr(scale), dq_out=_ptr(dq),
         status=None, ldx=x.stride(0), ldq=cols, lddq=cols, rows=rows, cols=cols, x_dtype=_DT[x.dtype], mode=mode,
@@ -432,7 +449,10 @@ def act_quant(
     nbytes = rows * cols * (x.element_size() + (1 if want_codes else 0) + (x.element_size() if want_dq else 0)) + 4 * rows
     nbytes += 4 * cols if sm is not None else 0
     with torch.cuda.device(dev):
-        rc = _timed("act_quant", float(nbytes), dev, lambda: L.load().qlin_act_quant(C.byref(args), _stream(dev)))
+        if src is not None:
+            rc = _timed("act_quant", float(nbytes), dev, lambda: L.load().qlin_act_quant_static(C.byref(args), src, _stream(dev)))
+        else:
+            rc = _timed("act_quant", float(nbytes), dev, lambda: L.load().qlin_act_quant(C.byref(args), _stream(dev)))
         L.check(rc, "qlin_act_quant")
     return codes, scale, dq
 
@@ -782,8 +802,8 @@ def fp8_quant_per_tensor(x2: torch.Tensor, *, e5m2: bool = False, eps: float = 1
     return codes, scale[:1]
 
 
-def _scalar(t) -> float:
-    return float(t.reshape(-1)[0].item()) if isinstance(t, torch.Tensor) else float(t)
+def _scalar(t):
+    return t.reshape(-1)[:1] if isinstance(t, torch.Tensor) else float(t)
 
 
 @torch.library.custom_op("qlin_b200::q_iaddmm_dq", mutates_args=())
@@ -791,7 +811,7 @@ def _q_iaddmm_dq_op(bias: torch.Tensor, m1: torch.Tensor, m2: torch.Tensor, scal
                     scale_w: torch.Tensor) -> torch.Tensor:  # fmt: skip
     """fms_mo::q_iaddmm_dq (fms_mo/custom_ext_kernels/utils.py:748-782): quantise the float ``m1 [m,k]`` with a
     static per-tensor scale and zero point (uint8 codes shifted by 128), int8 GEMM with ``m2 [k,n]``, then
-    ``(scale_i.float() * acc * scale_w + bias).to(m1.dtype)``.  The scale and zero point are read on the host."""
+    ``(scale_i.float() * acc * scale_w + bias).to(m1.dtype)``."""
     assert m2.dtype == torch.int8, f"weight tensor is of incorrect dtype {m2.dtype}"
     native = 3 if (m1.dtype != torch.float32 and scale_i.dtype == m1.dtype) else 0
     codes, _, _ = act_quant(m1, mode=L.Q_I8_STATIC, native_chain=native, scale0=_scalar(scale_i), zp0=_scalar(zp_i), shift=128.0)

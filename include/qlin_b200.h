@@ -244,6 +244,17 @@ typedef struct qlin_quant_args {
 
 int qlin_act_quant(const qlin_quant_args* args, void* stream);
 
+/* qlin_act_quant_static -- the static modes (QLIN_Q_I8_STATIC, _CLAMP_FIRST, _ROUND_FIRST, QLIN_Q_I8_AFFINE_RCP) with scalars
+ * that may live in device memory: src[0..3] stand for scale0, zp0, lo, hi; where ptr is NULL the value in args is used.
+ * The reference's modules keep these in buffers (fms_mo/modules/linear.py:1061-1083); read by the kernel they cost no
+ * synchronisation of the host with the stream. */
+typedef struct qlin_scalar_src {
+  const void* ptr;
+  int32_t dtype; /* QLIN_DT_F32, F16, BF16 or I32 */
+} qlin_scalar_src;
+
+int qlin_act_quant_static(const qlin_quant_args* args, const qlin_scalar_src src[4], void* stream);
+
 /* ------------------------------------------------------------------------------------------------
  * qlin_pact2_fwd / qlin_pact2_bwd -- PACT+ two-sided fake quantisation (QAT activations).
  *
