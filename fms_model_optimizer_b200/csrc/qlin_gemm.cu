@@ -277,26 +277,6 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t* w, boo
   }
 }
 
-// Uncoalesced store of up to 32 consecutive columns of one row held by this thread: the path for right edges that do not
-// end on a 16-byte boundary and for outputs that rule out 16-byte vectors.  `v` holds output values (or raw accumulators).
-__device__ __forceinline__ void store_row_direct(const GemmParams& p, uint8_t* dbase, const uint32_t (&v)[32], int row, int col0, bool two_byte) {
-  if (row >= p.M) return;
-  const int ncol = p.N - col0;
-  if (ncol <= 0) return;
-  uint8_t* base = out_row(p, dbase, row, two_byte ? 2 : 4) + static_cast<int64_t>(col0) * (two_byte ? 2 : 4);
-  if (two_byte) {
-    uint32_t w[16];
-    pack32(v, w, p.out_dtype == QLIN_DT_BF16);
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < ncol) reinterpret_cast<uint16_t*>(base)[j] = static_cast<uint16_t>(w[j >> 1] >> (16 * (j & 1)));
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < ncol) reinterpret_cast<uint32_t*>(base)[j] = v[j];
-  }
-}
-
 // Coalesced store through this warp's 32 x 128-byte staging tile.  `w` holds this thread's row as
 // 32 packed 32-bit words (128 bytes).  The tile is written with a 16-byte-chunk XOR swizzle so both
 // the row-per-lane writes and the row-contiguous reads are bank-conflict free; every global store
@@ -320,6 +300,47 @@ __device__ __forceinline__ void store_tile_coalesced(uint8_t* stage, const uint3
     const uint32_t addr = sbase + r * 128 + ((c ^ (r & 7)) << 4);
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(addr) : "memory");
     if (r < rows_valid && c < chunks) *reinterpret_cast<uint4*>(gbase + r * row_pitch_bytes + c * 16) = make_uint4(x0, x1, x2, x3);
+  }
+  __syncwarp();
+}
+
+// The same through the same staging tile for rows that do not start, or an edge that does not end, on a 16-byte boundary:
+// a warp writes a row at a time, 4 bytes a lane (2 bytes where the rows of a 2-byte output are not 4-byte aligned), so
+// each store instruction still covers consecutive bytes of one row; a thread storing its own row element by element
+// touches 32 rows with every instruction.  `bytes` of the 128-byte row lie inside the output.
+__device__ __forceinline__ void store_tile_narrow(uint8_t* stage, const uint32_t (&w)[32], uint8_t* gbase, int64_t row_pitch_bytes,
+                                                  int rows_valid, int lane, int bytes) {
+  const uint32_t sbase = smem_u32(stage);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t addr = sbase + lane * 128 + ((c ^ (lane & 7)) << 4);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[4 * c]), "r"(w[4 * c + 1]),
+                 "r"(w[4 * c + 2]), "r"(w[4 * c + 3])
+                 : "memory");
+  }
+  __syncwarp();
+  const bool words = ((reinterpret_cast<uintptr_t>(gbase) | static_cast<uintptr_t>(row_pitch_bytes)) & 3u) == 0;
+  const int rows = rows_valid < 32 ? rows_valid : 32;
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    uint8_t* g = gbase + r * row_pitch_bytes;
+    if (words) {
+      uint32_t x;
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(sbase + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) : "memory");
+      if (4 * lane + 4 <= bytes) {
+        reinterpret_cast<uint32_t*>(g)[lane] = x;
+      } else if (4 * lane < bytes) {
+        reinterpret_cast<uint16_t*>(g)[2 * lane] = static_cast<uint16_t>(x);
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = h * 32 + lane;
+        uint16_t x;
+        asm volatile("ld.shared.b16 %0, [%1];" : "=h"(x) : "r"(sbase + r * 128 + (((e >> 3) ^ (r & 7)) << 4) + (e & 7) * 2) : "memory");
+        if (2 * e < bytes) reinterpret_cast<uint16_t*>(g)[e] = x;
+      }
+    }
   }
   __syncwarp();
 }
@@ -348,20 +369,22 @@ __device__ __forceinline__ EpiCtx make_epi_ctx(const GemmParams& p, uint8_t* sta
   e.stage = stage;
   e.scaled = p.epilogue != QLIN_EPI_RAW;
   e.two_byte = e.scaled && p.out_dtype != QLIN_DT_F32;
-  e.vec_ok = (p.scatter_rows > 0 || (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0) && ((p.ldd * (e.two_byte ? 2 : 4)) % 16 == 0);
+  const int elt = e.two_byte ? 2 : 4;
+  e.vec_ok = (p.scatter_rows > 0 || (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0) && ((p.ldd * elt) % 16 == 0) &&
+             (p.batch <= 1 || (p.batch_stride_d * elt) % 16 == 0);
   return e;
 }
 
-// Emits 32 accumulator columns [col0, col0 + 32) of this thread's row as 4-byte values.
-template <bool F8>
-__device__ __forceinline__ void emit32_wide(const GemmParams& p, const EpiCtx& e, const uint32_t (&v)[32], int row0, int lane, int col0) {
-  const int left = p.N - col0;
+// Stores one staging tile: this thread's row of `cols` columns (32 words).
+__device__ __forceinline__ void emit_words(const GemmParams& p, const EpiCtx& e, const uint32_t (&w)[32], int row0, int lane, int col0, int cols) {
+  const int elt = e.two_byte ? 2 : 4;
+  const int left = min(p.N - col0, cols);
   if (left <= 0) return;
-  if (e.vec_ok && (left >= 32 || left % 4 == 0)) {
-    uint8_t* g = out_row(p, e.dbase, row0, 4) + static_cast<int64_t>(col0) * 4;
-    store_tile_coalesced(e.stage, v, g, p.ldd * 4, p.M - row0, lane, left >= 32 ? 8 : left / 4);
+  uint8_t* g = out_row(p, e.dbase, row0, elt) + static_cast<int64_t>(col0) * elt;
+  if (e.vec_ok && (left * elt) % 16 == 0) {
+    store_tile_coalesced(e.stage, w, g, p.ldd * elt, p.M - row0, lane, left * elt / 16);
   } else {
-    store_row_direct(p, e.dbase, v, row0 + lane, col0, false);
+    store_tile_narrow(e.stage, w, g, p.ldd * elt, p.M - row0, lane, left * elt);
   }
 }
 
@@ -374,21 +397,13 @@ __device__ __forceinline__ void emit64(const GemmParams& p, const EpiCtx& e, uin
     dequant32<F8>(p, hi, rs, s_cs + 32, s_bias + 32);
   }
   if (e.two_byte) {
-    const int left = p.N - col0;
-    if (left <= 0) return;
-    if (e.vec_ok && (left >= 64 || left % 8 == 0)) {
-      uint32_t w[32];  // 64 columns = one 128-byte staging row
-      pack32(lo, w, p.out_dtype == QLIN_DT_BF16);
-      pack32(hi, w + 16, p.out_dtype == QLIN_DT_BF16);
-      uint8_t* g = out_row(p, e.dbase, row0, 2) + static_cast<int64_t>(col0) * 2;
-      store_tile_coalesced(e.stage, w, g, p.ldd * 2, p.M - row0, lane, left >= 64 ? 8 : left / 8);
-    } else {
-      store_row_direct(p, e.dbase, lo, row0 + lane, col0, true);
-      store_row_direct(p, e.dbase, hi, row0 + lane, col0 + 32, true);
-    }
+    uint32_t w[32];  // 64 columns = one 128-byte staging row
+    pack32(lo, w, p.out_dtype == QLIN_DT_BF16);
+    pack32(hi, w + 16, p.out_dtype == QLIN_DT_BF16);
+    emit_words(p, e, w, row0, lane, col0, 64);
   } else {
-    emit32_wide<F8>(p, e, lo, row0, lane, col0);
-    emit32_wide<F8>(p, e, hi, row0, lane, col0 + 32);
+    emit_words(p, e, lo, row0, lane, col0, 32);
+    emit_words(p, e, hi, row0, lane, col0 + 32, 32);
   }
 }
 
@@ -398,10 +413,27 @@ __device__ __forceinline__ void emit32(const GemmParams& p, const EpiCtx& e, uin
                                        const float* s_bias, float rs) {
   if (e.scaled) dequant32<F8>(p, v, rs, s_cs, s_bias);
   if (e.two_byte) {
-    store_row_direct(p, e.dbase, v, row0 + lane, col0, true);
+    uint32_t w[32];
+    pack32(v, w, p.out_dtype == QLIN_DT_BF16);
+#pragma unroll
+    for (int j = 16; j < 32; ++j) w[j] = 0u;
+    emit_words(p, e, w, row0, lane, col0, 32);
   } else {
-    emit32_wide<F8>(p, e, v, row0, lane, col0);
+    emit_words(p, e, v, row0, lane, col0, 32);
   }
+}
+
+// The column scales and bias of one column (thread i: column i of the tile) and the row scale of this thread's row, fetched a
+// tile ahead so that their latency is not in the way of the accumulator they belong to.
+struct TileScales {
+  float cs, bias, rs;
+};
+__device__ __forceinline__ TileScales fetch_scales(const GemmParams& p, int col, bool has_col, int row) {
+  TileScales t;
+  t.cs = (p.cs != nullptr && has_col && col < p.N) ? p.cs[static_cast<int64_t>(col) * p.cs_stride] : 1.0f;
+  t.bias = (p.bias != nullptr && has_col && col < p.N) ? p.bias[col] : 0.0f;
+  t.rs = (p.rs != nullptr && row < p.M) ? p.rs[static_cast<int64_t>(row) * p.rs_stride] : 1.0f;
+  return t;
 }
 
 // BATCHED: p.batch problems of the same shape whose operands are stacked along the rows (A is [batch * M, K], B is
@@ -664,6 +696,14 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     bool ok = true;
     const bool elow = CHUNKED && !F8 && p.low_byte_mode != 0;
     const uint32_t enbuf = elow ? C::NBUF - 1 : C::NBUF;
+    TileScales next;
+    auto prefetch = [&](int t) {
+      if (!scaled || t >= num_tiles) return;
+      int mb, nb;
+      tile_coords(BATCHED ? t % per_batch : t, p.num_m, p.num_n, mb, nb);
+      next = fetch_scales(p, nb * C::BN + static_cast<int>(threadIdx.x), static_cast<int>(threadIdx.x) < C::BN, mb * kBM + q * 32 + lane);
+    };
+    prefetch(blockIdx.x);
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       int mb, nb;
       const int bi = BATCHED ? t / per_batch : 0;
@@ -676,13 +716,13 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (scaled) {
         // Stage this tile's column scales and bias once; all lanes then read them as broadcasts.
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
-        for (int i = threadIdx.x; i < C::BN; i += C::EPI_WARPS * 32) {
-          const int n = nb * C::BN + i;
-          aux->cs[i] = (p.cs != nullptr && n < p.N) ? p.cs[static_cast<int64_t>(n) * p.cs_stride] : 1.0f;
-          aux->bias[i] = (p.bias != nullptr && n < p.N) ? p.bias[n] : 0.0f;
+        if (static_cast<int>(threadIdx.x) < C::BN) {
+          aux->cs[threadIdx.x] = next.cs;
+          aux->bias[threadIdx.x] = next.bias;
         }
+        rs = next.rs;
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
-        if (p.rs != nullptr && row < p.M) rs = p.rs[static_cast<int64_t>(row) * p.rs_stride];
+        prefetch(t + gridDim.x);
       }
       if constexpr (!CHUNKED) {
         const uint32_t buf = ebuf, bph = ebph;
@@ -991,6 +1031,15 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const bool scaled = epi.scaled;
     uint32_t ebuf = 0, ebph = 0;
     bool ok = true;
+    TileScales next;
+    auto prefetch = [&](int t) {
+      if (!scaled || t >= num_tiles) return;
+      int mb, nb;
+      tile_coords2(t, num_m2, p.num_n, mb, nb);
+      next = fetch_scales(p, nb * C::BN + static_cast<int>(threadIdx.x), static_cast<int>(threadIdx.x) < C::BN,
+                          mb * 2 * kBM + static_cast<int>(rank) * kBM + q * 32 + lane);
+    };
+    prefetch(pair);
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
       int mb, nb;
       tile_coords2(t, num_m2, p.num_n, mb, nb);
@@ -1000,13 +1049,13 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       float rs = 1.0f;
       if (scaled) {
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
-        for (int i = threadIdx.x; i < C::BN; i += C::EPI_WARPS * 32) {
-          const int n = nb * C::BN + i;
-          aux->cs[i] = (p.cs != nullptr && n < p.N) ? p.cs[static_cast<int64_t>(n) * p.cs_stride] : 1.0f;
-          aux->bias[i] = (p.bias != nullptr && n < p.N) ? p.bias[n] : 0.0f;
+        if (static_cast<int>(threadIdx.x) < C::BN) {
+          aux->cs[threadIdx.x] = next.cs;
+          aux->bias[threadIdx.x] = next.bias;
         }
+        rs = next.rs;
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
-        if (p.rs != nullptr && row < p.M) rs = p.rs[static_cast<int64_t>(row) * p.rs_stride];
+        prefetch(t + num_pairs);
       }
       const uint32_t buf = ebuf, bph = ebph;
       if (++ebuf == C::NBUF) {
@@ -1641,7 +1690,7 @@ extern "C" int qlin_gemm_batched(const qlin_gemm_args* a, int32_t batch, int64_t
   const bool needs_chunks = (a->trun_bits > 0) || (a->kind == QLIN_DT_I8 && a->max_acc_bits < 32) || (a->kind != QLIN_DT_I8 && a->clamp_dl16);
   // dense stacks of unchunked problems: one launch whose tiles walk over all problems
   if (batch > 1 && !needs_chunks && stride_a == static_cast<int64_t>(a->M) * a->lda && stride_b == static_cast<int64_t>(a->N) * a->ldb &&
-      (stride_d * out_elt) % 16 == 0 && a->M > 0 && a->N > 0)
+      a->M > 0 && a->N > 0 && static_cast<int64_t>(batch) * a->M <= 0x7fffffff && static_cast<int64_t>(batch) * a->N <= 0x7fffffff)
     return gemm_impl(a, stream, batch, stride_d);
   qlin_gemm_args one = *a;
   for (int32_t i = 0; i < batch; ++i) {

@@ -53,3 +53,20 @@ def test_dequantise_chains(cuda_dev, M, N, out):
                        scale_round=scale, mid_round=mid, acc_round=accr, out_dtype=out)  # fmt: skip
         assert torch.equal(got.cpu(), want), (epi, prod, scale, mid, accr, with_bias)
     ops.check_status(cuda_dev)
+
+
+@pytest.mark.parametrize("B,M,K,N", [(5, 77, 48, 93), (3, 130, 64, 258), (7, 33, 16, 4), (2, 128, 128, 512), (9, 1, 32, 1)])
+def test_batched_products_of_any_alignment(cuda_dev, B, M, K, N):
+    """One launch over all problems whatever the size of a problem's output: raw sums and the fused fp16 scale chain."""
+    g = torch.Generator().manual_seed(B * M + N)
+    a = torch.randint(-127, 128, (B, M, K), generator=g, dtype=torch.int8)
+    b = torch.randint(-127, 128, (B, N, K), generator=g, dtype=torch.int8)
+    acc = torch.matmul(a.double(), b.double().transpose(1, 2))
+    ad, bd = a.to(cuda_dev), b.to(cuda_dev)
+    assert torch.equal(ops.bmm_i8(ad, bd).cpu(), acc.int())
+    s1, s2 = torch.tensor([0.0137]), torch.tensor([0.071])
+    for dt in (F32, F16, BF16):
+        want = (acc.int().to(F16) * s1 * s2).to(dt)
+        got = ops.bmm_i8(ad, bd, (s1.to(cuda_dev), s2.to(cuda_dev)), dt)
+        assert torch.equal(got.cpu(), want), dt
+    ops.check_status(cuda_dev)
