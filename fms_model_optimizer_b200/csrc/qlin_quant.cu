@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(TPB) act_quant_fast_kernel(const QuantParams p
   for (int i = 0; i < my_rows; ++i) {
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
-    const bool ok = mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
     const XT* xr = reinterpret_cast<const XT*>(ring + static_cast<size_t>(slot) * row_bytes);
     float v[MAXC][16];
     float amax = 0.0f;
@@ -529,13 +529,34 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// Two bf16 values times two fp32 factors, each rounded to bf16 once.
+__device__ __forceinline__ uint32_t mul_pack_bf16x2(uint32_t w, float2 f) {
+  const __nv_bfloat162 h = __float22bfloat162_rn(__fmul2_rn(make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)), f));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// Two fp32 values to e4m3 (the first in the low byte), saturating; NaN gives 0x7F.  For callers whose values cannot exceed
+// 464, where the saturating conversion and torch's (NaN above 464) agree: v / s with s the row's scale is at most 450.
+__device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+// DL8: e4m3 values below 0.0087890625 = 4.5 * 2^-9 become 0, that is the codes 0 to 4 of either sign.
+__device__ __forceinline__ uint32_t flush_dl8_e4m3(uint32_t w) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (((w >> (8 * i)) & 0x7Fu) <= 4u) w &= ~(0xFFu << (8 * i));
+  return w;
+}
+
 template <int MODE, int MAXC, int TPB>
 __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p, int stages, int row_bytes) {
   extern __shared__ __align__(128) uint8_t ring[];
   __shared__ uint64_t full[8];
   __shared__ float red[2][32];
   __shared__ int abort_flag;
-  constexpr bool DYN = MODE == QLIN_Q_I8_DYN;
+  constexpr bool F8 = MODE == QLIN_Q_F8_DYN;
+  constexpr bool DYN = MODE == QLIN_Q_I8_DYN || F8;
   constexpr bool SMREG = TPB <= 256 && MAXC == 1;
   const int nchunks = p.cols >> 4;
   const bool has_smooth = p.smooth != nullptr;
@@ -573,7 +594,7 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
   for (int i = 0; i < my_rows; ++i) {
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
-    const bool ok = mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
     const uint4* xr = reinterpret_cast<const uint4*>(ring + static_cast<size_t>(slot) * row_bytes);
     uint32_t vp[MAXC][8];
     __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
@@ -593,11 +614,7 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
               load16(mulvec + ch * 16, m);
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float lo = __fmul_rn(__uint_as_float(w[j] << 16), m[2 * j]);
-              const float hi = __fmul_rn(__uint_as_float(w[j] & 0xFFFF0000u), m[2 * j + 1]);
-              vp[c][j] = pack_bf16x2(lo, hi);
-            }
+            for (int j = 0; j < 8; ++j) vp[c][j] = mul_pack_bf16x2(w[j], make_float2(m[2 * j], m[2 * j + 1]));
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) vp[c][j] = w[j];
@@ -617,13 +634,17 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
     }
     if (threadIdx.x == 0 && i + stages < my_rows) issue(i + stages);
     float s;
-    if (DYN) {
+    if (F8) {
+      s = fmaxf(Elem<__nv_bfloat16>::rnd(__fdiv_rn(amax, 448.0f)), eps);
+    } else if (DYN) {
       s = Elem<__nv_bfloat16>::rnd(__fdiv_rn(fmaxf(amax, eps), static_cast<float>(p.levels)));
     } else {
       s = p.scale_in[static_cast<int64_t>(row) * p.scale_in_stride];
     }
     if (threadIdx.x == 0 && p.scale_out != nullptr) p.scale_out[row] = s;
     const float rs = __frcp_rn(s);
+    const float2 rs2 = make_float2(rs, rs);
+    const bool slow = F8 && !(s < 1e15f);  // an infinity in the row: the ordinary division makes its codes
 #pragma unroll
     for (int c = 0; c < MAXC; ++c) {
       const int ch = threadIdx.x + c * blockDim.x;
@@ -631,29 +652,48 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
         uint32_t out[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          int q[4];
+          if (F8) {
+            uint32_t h2[2];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint32_t w = vp[c][2 * g + h];
-            const uint32_t t2 = pack_bf16x2(__fmul_rn(__uint_as_float(w << 16), rs), __fmul_rn(__uint_as_float(w & 0xFFFF0000u), rs));
-            float r0, r1;
-            if (DYN) {
-              r0 = fast_rint(__uint_as_float(t2 << 16), q[2 * h]);
-              r1 = fast_rint(__uint_as_float(t2 & 0xFFFF0000u), q[2 * h + 1]);
-            } else {
-              r0 = rintf(__uint_as_float(t2 << 16));
-              r1 = rintf(__uint_as_float(t2 & 0xFFFF0000u));
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t w = vp[c][2 * g + h];
+              uint32_t t2 = mul_pack_bf16x2(w, rs2);
+              if (slow) t2 = pack_bf16x2(__fdiv_rn(__uint_as_float(w << 16), s), __fdiv_rn(__uint_as_float(w & 0xFFFF0000u), s));
+              h2[h] = cvt_e4m3x2(__uint_as_float(t2 << 16), __uint_as_float(t2 & 0xFFFF0000u));
+            }
+            out[g] = __byte_perm(h2[0], h2[1], 0x5410);
+            if (p.dl8_flush) out[g] = flush_dl8_e4m3(out[g]);
+          } else if (DYN) {
+            // the low byte of v / s + 1.5 * 2^23 is the code (|v / s| <= ~128)
+            const float2 magic = make_float2(12582912.0f, 12582912.0f);
+            uint32_t q[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t t2 = mul_pack_bf16x2(vp[c][2 * g + h], rs2);
+              const float2 r2 = __fadd2_rn(make_float2(__uint_as_float(t2 << 16), __uint_as_float(t2 & 0xFFFF0000u)), magic);
+              q[2 * h] = __float_as_uint(r2.x);
+              q[2 * h + 1] = __float_as_uint(r2.y);
+            }
+            if (p.clamp_codes) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) q[k] = static_cast<uint32_t>(max(-p.levels, min(p.levels, static_cast<int>(q[k]) - 0x4B400000)));
+            }
+            out[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+          } else {
+            int q[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t t2 = mul_pack_bf16x2(vp[c][2 * g + h], rs2);
+              const float r0 = rintf(__uint_as_float(t2 << 16)), r1 = rintf(__uint_as_float(t2 & 0xFFFF0000u));
               q[2 * h] = static_cast<int>(Elem<__nv_bfloat16>::rnd(__fadd_rn(r0, p.zp0)));
               q[2 * h + 1] = static_cast<int>(Elem<__nv_bfloat16>::rnd(__fadd_rn(r1, p.zp0)));
             }
-            (void)r0;
-            (void)r1;
-          }
-          if (p.clamp_codes) {
+            if (p.clamp_codes) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) q[k] = max(-p.levels, min(p.levels, q[k]));
+              for (int k = 0; k < 4; ++k) q[k] = max(-p.levels, min(p.levels, q[k]));
+            }
+            out[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
           }
-          out[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
         }
         *reinterpret_cast<uint4*>(p.codes + static_cast<int64_t>(row) * p.ldq + ch * 16) = make_uint4(out[0], out[1], out[2], out[3]);
       }
@@ -737,6 +777,7 @@ static int try_fast(const QuantParams& p, int threads, int nchunks, cudaStream_t
   if (std::is_same<XT, __nv_bfloat16>::value && native && !dq && p.codes != nullptr && (p.smooth == nullptr || p.smooth_exact)) {
     if (p.mode == QLIN_Q_I8_DYN) return launch_bf16_c<QLIN_Q_I8_DYN>(p, threads, nchunks, stream);
     if (p.mode == QLIN_Q_I8_GIVEN_SCALE) return launch_bf16_c<QLIN_Q_I8_GIVEN_SCALE>(p, threads, nchunks, stream);
+    if (p.mode == QLIN_Q_F8_DYN && p.smooth == nullptr) return launch_bf16_c<QLIN_Q_F8_DYN>(p, threads, nchunks, stream);
   }
   if (p.mode == QLIN_Q_I8_DYN) {
     if (kIsF32 || !native)
