@@ -11,6 +11,7 @@ from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 LIB_PATH = PKG_DIR / "lib" / "libqlin_b200.so"
+HOST_PATH = PKG_DIR / "lib" / "_qlin_host.so"
 
 # qlin_status
 OK = 0
@@ -285,6 +286,27 @@ class PeerBarrierArgs(C.Structure):
         ("world", C.c_int32),
         ("timeout_ns", C.c_int64),
     ]
+
+
+_host = None
+
+
+def host():
+    """The tensor-level host code (csrc/host/qlin_host.cpp), loaded once.  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        load()
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m fms_model_optimizer_b200.build_ext`")
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries must be loaded first)
+
+        spec = importlib.util.spec_from_file_location("_qlin_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 _lib = None

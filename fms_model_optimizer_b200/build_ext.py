@@ -1,4 +1,5 @@
-"""Builds libqlin_b200.so (the C-ABI library with every CUDA kernel of this package) in-tree.
+"""Builds libqlin_b200.so (the C-ABI library with every CUDA kernel of this package) and _qlin_host.so (the tensor-level
+host code in C++, linked against it) in-tree.
 
 The library is compiled for sm_100a only with plain ``nvcc``; nothing is JIT-compiled at run time.
 ``python -m fms_model_optimizer_b200.build_ext`` rebuilds it; ``build()`` is also what
@@ -19,6 +20,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "libqlin_b200.so"
+HOST_SRC = CSRC / "host" / "qlin_host.cpp"
+HOST_PATH = LIB_DIR / "_qlin_host.so"
 OBJ_DIR = LIB_DIR / "obj"
 
 NVCC_FLAGS = [
@@ -31,6 +34,33 @@ NVCC_FLAGS = [
     "-fPIC",
     "--expt-relaxed-constexpr",
 ]
+
+
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared"]
+
+
+def _build_host() -> None:
+    """g++ for the host code: PyTorch's headers and libraries, libqlin_b200.so beside it at run time."""
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", Path(sysconfig.get_path("include")), _cuda_include()]
+    tmp = HOST_PATH.with_suffix(".so.tmp")
+    cmd = ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in includes:
+        cmd += ["-isystem", str(inc)]
+    cmd += [str(HOST_SRC), "-o", str(tmp), f"-L{LIB_DIR}", "-l:libqlin_b200.so", f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+            "-Wl,-rpath,$ORIGIN"]  # fmt: skip
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC.name}:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, HOST_PATH)
+
+
+def _cuda_include() -> Path:
+    return Path(_nvcc()).resolve().parent.parent / "include"
 
 
 def _nvcc() -> str:
@@ -51,9 +81,9 @@ def source_digest(extra_flags: tuple = ()) -> str:
     """SHA-256 over the compiler flags and the name and content of every file the library is built from.  File times
     say nothing after a checkout or a copy to another machine, so staleness is decided by content."""
     files = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")))
-    files.append(PKG_DIR.parent / "include" / "qlin_b200.h")
+    files += [PKG_DIR.parent / "include" / "qlin_b200.h", HOST_SRC]
     h = hashlib.sha256()
-    h.update("\0".join([*NVCC_FLAGS, *extra_flags]).encode())
+    h.update("\0".join([*NVCC_FLAGS, *HOST_FLAGS, *extra_flags]).encode())
     for f in files:
         h.update(f.name.encode() + b"\0")
         h.update(f.read_bytes())
@@ -61,14 +91,14 @@ def source_digest(extra_flags: tuple = ()) -> str:
 
 
 def is_stale() -> bool:
-    """True unless the library exists and the digest stored beside it at build time equals the digest of the sources."""
-    if not LIB_PATH.exists() or not STAMP_PATH.exists():
+    """True unless the libraries exist and the digest stored beside them at build time equals the digest of the sources."""
+    if not LIB_PATH.exists() or not HOST_PATH.exists() or not STAMP_PATH.exists():
         return True
     return STAMP_PATH.read_text().strip() != source_digest()
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` and link ``lib/libqlin_b200.so``.  Returns the library path."""
+    """Compile every ``csrc/*.cu`` and link ``lib/libqlin_b200.so``, then the host code.  Returns the library path."""
     if not force and not is_stale():
         return LIB_PATH
     nvcc = _nvcc()
@@ -93,6 +123,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
     os.replace(tmp, LIB_PATH)
+    _build_host()
     STAMP_PATH.write_text(source_digest() + "\n")
     return LIB_PATH
 

@@ -1,0 +1,409 @@
+// Host side of the tensor-level entry points (ops.py) in C++: argument checks, output allocation with PyTorch's caching
+// allocator, the argument block and the call into libqlin_b200.so on the tensors' device and current stream.
+//
+// A deploy-time Linear is two kernels of a few microseconds each when a handful of tokens go through it.  Building the two
+// argument blocks field by field through ctypes, entering device contexts and looking up streams in Python cost about
+// 72 us a call at 1 x 4096 x 14336, four times what the GPU needed; with the same steps here a call takes 22 us, of which
+// the two kernels are 19.
+//
+// No kernel, no fallback and no state of its own: everything a call keeps is one status word per device, which lives as
+// long as the process.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <pybind11/stl.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <mutex>
+#include <optional>
+#include <stdexcept>
+#include <string>
+#include <variant>
+#include <vector>
+
+#include "../../../include/qlin_b200.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+using Scalar = std::variant<Tensor, double>;
+
+[[noreturn]] void raise(const std::string& msg) { throw std::runtime_error(msg); }
+
+void check(int rc, const char* what) {
+  if (rc != QLIN_OK) raise(std::string(what) + " failed with status " + std::to_string(rc) + ": " + qlin_last_error_string());
+}
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kChar:
+      return QLIN_DT_I8;
+    case at::kByte:
+      return QLIN_DT_U8;
+    case at::kInt:
+      return QLIN_DT_I32;
+    case at::kFloat:
+      return QLIN_DT_F32;
+    case at::kHalf:
+      return QLIN_DT_F16;
+    case at::kBFloat16:
+      return QLIN_DT_BF16;
+    case at::kFloat8_e4m3fn:
+      return QLIN_DT_F8E4M3;
+    case at::kFloat8_e5m2:
+      return QLIN_DT_F8E5M2;
+    default:
+      return QLIN_DT_NONE;
+  }
+}
+
+at::ScalarType scalar_type(int code) {
+  switch (code) {
+    case QLIN_DT_I32:
+      return at::kInt;
+    case QLIN_DT_F32:
+      return at::kFloat;
+    case QLIN_DT_F16:
+      return at::kHalf;
+    case QLIN_DT_BF16:
+      return at::kBFloat16;
+    default:
+      raise("unsupported output dtype");
+  }
+}
+
+bool is_float(at::ScalarType t) { return t == at::kFloat || t == at::kHalf || t == at::kBFloat16; }
+
+// All given tensors are on one CUDA device, which is returned.
+at::Device require_cuda(std::initializer_list<const Tensor*> tensors) {
+  std::optional<at::Device> dev;
+  for (const Tensor* t : tensors) {
+    if (t == nullptr || !t->defined()) continue;
+    if (!t->is_cuda()) raise("qlin_b200 ops run on CUDA tensors only (there is no CPU path)");
+    if (!dev) {
+      dev = t->device();
+    } else if (t->device() != *dev) {
+      raise("tensors on different devices: " + dev->str() + " and " + t->device().str());
+    }
+  }
+  if (!dev) raise("no tensor given");
+  return *dev;
+}
+
+const Tensor* ptr_of(const OptTensor& t) { return t ? &*t : nullptr; }
+void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+Tensor empty(at::IntArrayRef sizes, at::ScalarType t, at::Device dev) { return at::empty(sizes, at::TensorOptions().dtype(t).device(dev)); }
+
+// fp32, one-dimensional, contiguous (undefined stays undefined).
+Tensor f32(const OptTensor& t) {
+  if (!t) return Tensor();
+  if (t->scalar_type() == at::kFloat && t->is_contiguous()) return *t;
+  return t->reshape({-1}).to(at::kFloat).contiguous();
+}
+
+// K-contiguous 2-D view or copy whose row stride and base are 16-byte aligned.
+Tensor pad_k(const Tensor& t) {
+  const int64_t es = t.element_size();
+  if (t.stride(1) == 1 && (t.stride(0) * es) % 16 == 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) >= t.size(1)) return t;
+  const int64_t k = t.size(1), kp = (k * es + 15) / 16 * 16 / es;
+  Tensor buf = at::zeros({t.size(0), kp}, t.options());
+  Tensor view = buf.narrow(1, 0, k);
+  view.copy_(t);
+  return view;
+}
+
+// Status word of a device, created on first use and never released (kernels in flight may write it until the process ends).
+Tensor status_word(int index) {
+  static std::mutex* mutex = new std::mutex;
+  static std::vector<Tensor>* words = new std::vector<Tensor>(64);
+  if (index < 0 || index >= 64) raise("device ordinal out of range");
+  std::lock_guard<std::mutex> lock(*mutex);
+  Tensor& w = (*words)[index];
+  if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(index))));
+  return w;
+}
+
+void* stream_of(at::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
+
+// ------------------------------------------------------------------------------------------------ GEMM
+struct Chain {  // chunk function, epilogue and rounding dtypes of a GEMM call
+  int64_t chunk_k;
+  int trun_bits, max_acc_bits, trunc_then_acc, clamp_dl16, epilogue, prod_round, scale_round, mid_round, acc_round;
+};
+
+struct Scatter {
+  std::vector<int64_t> bases;
+  int64_t rows = 0, row0 = 0, ld = 0;
+};
+
+Tensor gemm_impl(const Tensor& a_in, const Tensor& b_in, const OptTensor& c_in, const OptTensor& out_in, const Chain& ch, const OptTensor& row_scale,
+                 const OptTensor& col_scale, const OptTensor& bias, const Scatter* scatter, int64_t max_ctas, int out_code) {
+  const at::Device dev = require_cuda({&a_in, &b_in, ptr_of(c_in), ptr_of(out_in), ptr_of(row_scale), ptr_of(col_scale), ptr_of(bias)});
+  if (a_in.dim() != 2 || b_in.dim() != 2 || a_in.size(1) != b_in.size(1)) raise("incompatible shapes: a [M,K] and b [N,K] are wanted");
+  const at::ScalarType kt = a_in.scalar_type();
+  if (kt != b_in.scalar_type() || (kt != at::kChar && kt != at::kFloat8_e4m3fn && kt != at::kFloat8_e5m2))
+    raise("operands must both be int8, float8_e4m3fn or float8_e5m2");
+  const bool f8 = kt != at::kChar;
+  const int64_t M = a_in.size(0), K = a_in.size(1), N = b_in.size(0);
+  const at::ScalarType raw = f8 ? at::kFloat : at::kInt;
+  const at::ScalarType ot = ch.epilogue == QLIN_EPI_RAW ? raw : (out_code == QLIN_DT_NONE ? at::kFloat : scalar_type(out_code));
+  const c10::cuda::CUDAGuard guard(dev);
+  int64_t ldd = N;
+  Tensor out;
+  if (scatter != nullptr) {
+    if (out_in || c_in) raise("scatter excludes out and c");
+    ldd = scatter->ld > 0 ? scatter->ld : N;
+  } else if (!out_in) {
+    out = empty({M, N}, ot, dev);
+  } else {
+    out = *out_in;
+    if (out.scalar_type() != ot || out.dim() != 2 || out.size(0) != M || out.size(1) != N || out.stride(1) != 1) raise("out has the wrong dtype, shape or layout");
+    ldd = out.stride(0);
+  }
+  if (M == 0 || N == 0) return out;
+  if (K == 0) raise("K must be positive");
+  const Tensor a = pad_k(a_in), b = pad_k(b_in);
+  Tensor c;
+  if (c_in) {
+    if (c_in->scalar_type() != raw || c_in->dim() != 2 || c_in->size(0) != M || c_in->size(1) != N) raise("c must be an [M,N] tensor of the accumulator dtype");
+    c = c_in->stride(1) != 1 ? c_in->contiguous() : *c_in;
+  }
+  const Tensor rs = f32(row_scale), cs = f32(col_scale), bs = f32(bias);
+  if (rs.defined() && rs.numel() != 1 && rs.numel() != M) raise("row_scale must have 1 or M elements");
+  if (cs.defined() && cs.numel() != 1 && cs.numel() != N) raise("col_scale must have 1 or N elements");
+  if (bs.defined() && bs.numel() != N) raise("bias must have N elements");
+  qlin_gemm_args g = {};
+  g.a = data(a);
+  g.b = data(b);
+  g.c = data(c);
+  g.d = data(out);
+  g.row_scale = static_cast<const float*>(data(rs));
+  g.col_scale = static_cast<const float*>(data(cs));
+  g.bias = static_cast<const float*>(data(bs));
+  g.status = static_cast<int32_t*>(status_word(dev.index()).data_ptr());
+  g.lda = a.stride(0);
+  g.ldb = b.stride(0);
+  g.ldc = c.defined() ? c.stride(0) : 0;
+  g.ldd = ldd;
+  g.M = static_cast<int32_t>(M);
+  g.N = static_cast<int32_t>(N);
+  g.K = static_cast<int32_t>(K);
+  g.kind = dtype_code(kt);
+  g.chunk_k = static_cast<int32_t>(ch.chunk_k);
+  g.trun_bits = ch.trun_bits;
+  g.max_acc_bits = ch.max_acc_bits;
+  g.trunc_then_acc = ch.trunc_then_acc;
+  g.clamp_dl16 = ch.clamp_dl16;
+  g.epilogue = ch.epilogue;
+  g.row_scale_stride = rs.defined() && rs.numel() != 1 ? 1 : 0;
+  g.col_scale_stride = cs.defined() && cs.numel() != 1 ? 1 : 0;
+  g.prod_round = ch.prod_round;
+  g.scale_round = ch.scale_round;
+  g.mid_round = ch.mid_round;
+  g.acc_round = ch.acc_round;
+  g.out_dtype = dtype_code(ot);
+  g.max_ctas = static_cast<int32_t>(max_ctas);
+  if (scatter != nullptr) {
+    if (scatter->bases.size() > 8) raise("at most 8 scatter destinations");
+    for (size_t i = 0; i < scatter->bases.size(); ++i) g.scatter_d[i] = reinterpret_cast<void*>(scatter->bases[i]);
+    g.scatter_rows = static_cast<int32_t>(scatter->rows);
+    g.scatter_row0 = static_cast<int32_t>(scatter->row0);
+  }
+  check(qlin_gemm(&g, stream_of(dev)), "qlin_gemm");
+  return out;
+}
+
+OptTensor gemm(const Tensor& a, const Tensor& b, const OptTensor& c, const OptTensor& out, int64_t chunk_k, int trun_bits, int max_acc_bits, bool trunc_then_acc,
+               bool clamp_dl16, int epilogue, const OptTensor& row_scale, const OptTensor& col_scale, const OptTensor& bias, int prod_round,
+               int scale_round, int mid_round, int acc_round, int64_t max_ctas, int out_code, const std::vector<int64_t>& scatter_bases,
+               int64_t scatter_rows, int64_t scatter_row0, int64_t scatter_ld) {
+  const Chain ch{chunk_k, trun_bits, max_acc_bits, trunc_then_acc, clamp_dl16, epilogue, prod_round, scale_round, mid_round, acc_round};
+  Scatter sc;
+  const bool scattered = scatter_rows > 0;
+  if (scattered) sc = Scatter{scatter_bases, scatter_rows, scatter_row0, scatter_ld};
+  Tensor r = gemm_impl(a, b, c, out, ch, row_scale, col_scale, bias, scattered ? &sc : nullptr, max_ctas, out_code);
+  return r.defined() ? OptTensor(r) : std::nullopt;
+}
+
+// ------------------------------------------------------------------------------------------------ row quantiser
+struct QuantOpts {
+  int mode, native_chain, smooth_mul, clamp_codes, levels, dl8_flush, f8_e5m2;
+  float shift, add2, dyn_eps;
+};
+
+bool is_static(int mode) {
+  return mode == QLIN_Q_I8_STATIC || mode == QLIN_Q_I8_STATIC_CLAMP_FIRST || mode == QLIN_Q_I8_STATIC_ROUND_FIRST || mode == QLIN_Q_I8_AFFINE_RCP;
+}
+
+// A scalar of the quantiser: a number, or a one-element tensor.  Tensors on the device are left there in the static modes.
+float scalar(const Scalar& s, at::Device dev, bool may_stay, qlin_scalar_src& src, bool& any) {
+  if (const double* d = std::get_if<double>(&s)) return static_cast<float>(*d);
+  const Tensor& t = std::get<Tensor>(s);
+  const at::ScalarType st = t.scalar_type();
+  if (may_stay && t.device() == dev && t.numel() == 1 && (is_float(st) || st == at::kInt)) {
+    src.ptr = t.data_ptr();
+    src.dtype = dtype_code(st);
+    any = true;
+    return 0.0f;
+  }
+  return static_cast<float>(t.item().toDouble());
+}
+
+void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smooth, const OptTensor& smooth_rcp, const OptTensor& scale_in,
+                    const Scalar* scalars, bool want_codes, bool want_dq, Tensor& codes, Tensor& scale, Tensor& dq) {
+  const at::Device dev = require_cuda({&x_in, ptr_of(smooth), ptr_of(scale_in)});
+  if (x_in.dim() != 2) raise("act_quant takes a 2-D tensor");
+  if (!is_float(x_in.scalar_type())) raise("unsupported activation dtype");
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor x = x_in.stride(1) != 1 ? x_in.contiguous() : x_in;
+  const int64_t rows = x.size(0), cols = x.size(1);
+  at::ScalarType ct = at::kChar;
+  if (o.mode == QLIN_Q_F8_DYN || (o.mode == QLIN_Q_F8_TENSOR && !o.f8_e5m2)) {
+    ct = at::kFloat8_e4m3fn;
+  } else if (o.mode == QLIN_Q_F8_TENSOR) {
+    ct = at::kFloat8_e5m2;
+  }
+  if (want_codes) codes = empty({rows, cols}, ct, dev);
+  if (want_dq) dq = empty({rows, cols}, x.scalar_type(), dev);
+  scale = empty({rows}, at::kFloat, dev);
+  const Tensor sm = f32(smooth);
+  if (sm.defined() && sm.numel() != cols) raise("smooth must have one entry per column");
+  const Tensor rsm = sm.defined() && !o.smooth_mul ? f32(smooth_rcp) : Tensor();
+  const Tensor si = f32(scale_in);
+  if (rows == 0 || cols == 0) return;
+  qlin_quant_args q = {};
+  q.x = data(x);
+  q.smooth = static_cast<const float*>(data(sm));
+  q.smooth_rcp = static_cast<const float*>(data(rsm));
+  q.scale_in = static_cast<const float*>(data(si));
+  q.codes = data(codes);
+  q.scale_out = static_cast<float*>(data(scale));
+  q.dq_out = data(dq);
+  q.ldx = x.stride(0);
+  q.ldq = q.lddq = cols;
+  q.rows = static_cast<int32_t>(rows);
+  q.cols = static_cast<int32_t>(cols);
+  q.x_dtype = dtype_code(x.scalar_type());
+  q.mode = o.mode;
+  q.native_chain = o.native_chain;
+  q.smooth_mul = o.smooth_mul;
+  q.clamp_codes = o.clamp_codes;
+  q.qmax_levels = o.levels;
+  q.dl8_flush = o.dl8_flush;
+  q.scale_in_stride = si.defined() && si.numel() != 1 ? 1 : 0;
+  qlin_scalar_src src[4] = {};
+  bool any = false;
+  const bool st = is_static(o.mode);
+  q.scale0 = scalar(scalars[0], dev, st, src[0], any);
+  q.zp0 = scalar(scalars[1], dev, st, src[1], any);
+  q.lo = scalar(scalars[2], dev, st, src[2], any);
+  q.hi = scalar(scalars[3], dev, st, src[3], any);
+  q.shift = o.shift;
+  q.add2 = o.add2;
+  q.dyn_eps = o.dyn_eps;
+  q.f8_format = o.f8_e5m2;
+  check(any ? qlin_act_quant_static(&q, src, stream_of(dev)) : qlin_act_quant(&q, stream_of(dev)), "qlin_act_quant");
+}
+
+OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
+
+std::tuple<OptTensor, Tensor, OptTensor> act_quant(const Tensor& x, int mode, const OptTensor& smooth, const OptTensor& smooth_rcp, bool smooth_mul,
+                                                   int native_chain, bool clamp_codes, int levels, bool want_codes, bool want_dq, const OptTensor& scale_in,
+                                                   bool dl8_flush, const Scalar& scale0, const Scalar& zp0, const Scalar& lo, const Scalar& hi, double shift,
+                                                   double add2, double dyn_eps, bool f8_e5m2) {
+  const QuantOpts o{mode,      native_chain, smooth_mul, clamp_codes, levels, dl8_flush, f8_e5m2, static_cast<float>(shift), static_cast<float>(add2),
+                    static_cast<float>(dyn_eps)};
+  const Scalar scalars[4] = {scale0, zp0, lo, hi};
+  Tensor codes, scale, dq;
+  act_quant_impl(x, o, smooth, smooth_rcp, scale_in, scalars, want_codes, want_dq, codes, scale, dq);
+  return {opt(codes), scale, opt(dq)};
+}
+
+// Quantises the rows of x [.., K] and multiplies them with weight [N, K]: the two launches of a deploy-time Linear in one
+// call.  row_scale: the scales to dequantise with (none: the ones the quantiser found per row).
+Tensor quant_gemm(const Tensor& x, int mode, const OptTensor& smooth, const OptTensor& smooth_rcp, int native_chain, int levels, bool dl8_flush,
+                  const Scalar& scale0, const Scalar& zp0, const Scalar& lo, const Scalar& hi, double shift, double add2, const Tensor& weight,
+                  const OptTensor& row_scale, const OptTensor& col_scale, const OptTensor& bias, int64_t chunk_k, int trun_bits, int max_acc_bits,
+                  bool clamp_dl16, int epilogue, int prod_round, int scale_round, int mid_round, int acc_round, int64_t max_ctas, int out_code) {
+  const QuantOpts o{mode, native_chain, 0, 0, levels, dl8_flush, 0, static_cast<float>(shift), static_cast<float>(add2), 1e-5f};
+  const Scalar scalars[4] = {scale0, zp0, lo, hi};
+  Tensor codes, scale, dq;
+  const Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+  act_quant_impl(x2, o, smooth, smooth_rcp, std::nullopt, scalars, true, false, codes, scale, dq);
+  const Chain ch{chunk_k, trun_bits, max_acc_bits, 1, clamp_dl16, epilogue, prod_round, scale_round, mid_round, acc_round};
+  Tensor out = gemm_impl(codes, weight, std::nullopt, std::nullopt, ch, row_scale ? row_scale : OptTensor(scale), col_scale, bias, nullptr, max_ctas, out_code);
+  if (x.dim() == 2) return out;
+  std::vector<int64_t> shape = x.sizes().vec();
+  shape.back() = weight.size(0);
+  return out.reshape(shape);
+}
+
+// ------------------------------------------------------------------------------------------------ PACT+
+Tensor clip_f32(const Tensor& t, at::Device dev) {
+  Tensor d = t.detach();
+  if (d.dim() == 1 && d.numel() == 1 && d.scalar_type() == at::kFloat && d.device() == dev) return d;
+  d = d.reshape({-1}).narrow(0, 0, 1);
+  if (d.scalar_type() != at::kFloat || d.device() != dev) d = d.to(at::TensorOptions().device(dev).dtype(at::kFloat));
+  return d.contiguous();
+}
+
+qlin_pact2_args pact_args(const Tensor& x, const Tensor& out, const Tensor& cv, const Tensor& cvn, int num_bits, bool align_zero, int variant) {
+  qlin_pact2_args p = {};
+  p.x = data(x);
+  p.out = data(out);
+  p.clip_val = static_cast<const float*>(data(cv));
+  p.clip_valn = static_cast<const float*>(data(cvn));
+  p.numel = x.numel();
+  p.dtype = dtype_code(x.scalar_type());
+  p.num_bits = num_bits;
+  p.align_zero = align_zero;
+  p.variant = variant;
+  return p;
+}
+
+Tensor pact2_fwd(const Tensor& x_in, const Tensor& clip_val, const OptTensor& clip_valn, int num_bits, bool align_zero, int variant) {
+  const at::Device dev = require_cuda({&x_in});
+  if (!is_float(x_in.scalar_type())) raise("unsupported dtype");
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor x = x_in.detach().contiguous();
+  const Tensor out = at::empty_like(x);
+  const Tensor cv = clip_f32(clip_val, dev), cvn = clip_valn ? clip_f32(*clip_valn, dev) : Tensor();
+  const qlin_pact2_args p = pact_args(x, out, cv, cvn, num_bits, align_zero, variant);
+  check(qlin_pact2_fwd(&p, stream_of(dev)), "qlin_pact2_fwd");
+  return out;
+}
+
+std::tuple<Tensor, Tensor> pact2_bwd(const Tensor& x_in, const Tensor& grad_out, const Tensor& clip_val, const OptTensor& clip_valn, int num_bits,
+                                     bool align_zero, int variant) {
+  const at::Device dev = require_cuda({&x_in, &grad_out});
+  if (!is_float(x_in.scalar_type())) raise("unsupported dtype");
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor x = x_in.detach().contiguous();
+  Tensor g = grad_out.detach().contiguous();
+  if (g.scalar_type() != x.scalar_type()) g = g.to(x.scalar_type());
+  const Tensor gx = at::empty_like(x);
+  const Tensor cv = clip_f32(clip_val, dev), cvn = clip_valn ? clip_f32(*clip_valn, dev) : Tensor();
+  const int64_t ws_floats = std::max<int64_t>(1, static_cast<int64_t>(qlin_pact2_bwd_workspace_bytes(x.numel()) / 4));
+  const Tensor ws = empty({ws_floats}, at::kFloat, dev), grads = empty({2}, at::kFloat, dev);
+  qlin_pact2_args p = pact_args(x, gx, cv, cvn, num_bits, align_zero, variant);
+  p.grad_out = data(g);
+  p.grad_clip = static_cast<float*>(data(grads));
+  p.workspace = data(ws);
+  check(qlin_pact2_bwd(&p, stream_of(dev)), "qlin_pact2_bwd");
+  return {gx, grads};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_qlin_host, m) {
+  using rel = py::call_guard<py::gil_scoped_release>;
+  m.def("status_word", &status_word, rel());
+  m.def("gemm", &gemm, rel());
+  m.def("act_quant", &act_quant, rel());
+  m.def("quant_gemm", &quant_gemm, rel());
+  m.def("pact2_fwd", &pact2_fwd, rel());
+  m.def("pact2_bwd", &pact2_bwd, rel());
+}

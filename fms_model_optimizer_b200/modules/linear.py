@@ -246,73 +246,64 @@ class QLinearINT8Deploy(nn.Linear):
         if not x.is_cuda:
             raise RuntimeError("QLinearINT8Deploy(b200) runs on CUDA tensors only")
         with torch.no_grad():
-            org_dtype = x.dtype
-            tar_shape = tuple(x.shape[:-1]) + (self.weight.shape[0],)
-            x2 = x.reshape(-1, x.shape[-1])
             prep = self._prepared(x.device)
-            smooth = prep["smooth"]
-            chain = x2.dtype if smooth is None else _promote(x2.dtype, self.smoothq_scale.dtype)
-            kw = {}
+            smooth, rcp, w_scale = prep["smooth"], prep["smooth_rcp"], self.w_scale
+            xd = x.dtype
+            chain = xd if smooth is None else _promote(xd, self.smoothq_scale.dtype)
+            levels = 2 ** (self.nbits_a - 1) - 1
             # `x / smoothq_scale` is rounded to the dtype of x when the scale has that dtype (or promotes to it); the
             # static quantisers then divide by their fp32 scale buffers in fp32 (fms_mo/modules/linear.py:1330, :1061-1083)
-            smooth_native = 1 if (smooth is not None and chain == x2.dtype and chain != torch.float32) else 0
+            chain_is_x = chain == xd and chain != torch.float32
+            native = 1 if (smooth is not None and chain_is_x) else 0
+            acc = dict(chunk_k=_normalised_chunk(self.chunk_size), trun_bits=int(self.truncate_lsb), max_acc_bits=int(self.max_acc_bits),
+                       epilogue=L.EPI_SCALE_PROD, scale_round=torch.float16, acc_round=(None if self.acc_dtype == torch.float32 else self.acc_dtype),
+                       col_scale=prep["w_scale"], out_dtype=xd)  # fmt: skip
             if self.useDynMaxQfunc in [-1, -2]:
                 if self.useDynMaxQfunc == -2:
                     raise NotImplementedError("per-channel (dim=-2) dynamic activation quantisation")
                 # qa_dynamic_max_qfunc runs in `chain`; bit 0: the division by smoothq_scale rounds to
                 # the dtype of x, bit 1: the quantise chain does
-                native = smooth_native | (2 if (chain == x2.dtype and chain != torch.float32) else 0)
-                if smooth is None or self.smoothq_scale.dtype == x2.dtype:
+                native |= 2 if chain_is_x else 0
+                if smooth is None or self.smoothq_scale.dtype == xd:
                     native |= 4  # the smoothing scales are values of the activation dtype
-                codes, in_scale, _ = ops.act_quant(
-                    x2, mode=L.Q_I8_DYN, smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=native,
-                    levels=2 ** (self.nbits_a - 1) - 1
-                )
-                scale_dtype = chain
+                quant = dict(mode=L.Q_I8_DYN, native_chain=native, levels=levels)
+                in_scale, scale_dtype = None, chain
             elif self.use_fake_zero_shift:
                 # qa_dyn_max_fake_zero_shift (fms_mo/modules/linear.py:1102-1113): one scale for the whole tensor,
                 # amax / (127 - zp), codes shifted by zp; the largest per-row scale is that scale (rounding is monotonic)
+                x2 = x.reshape(-1, x.shape[-1])
                 zp = int(self.input_zp)
-                native = smooth_native | (2 if (chain == x2.dtype and chain != torch.float32) else 0)
-                if smooth is None or self.smoothq_scale.dtype == x2.dtype:
+                native |= 2 if chain_is_x else 0
+                if smooth is None or self.smoothq_scale.dtype == xd:
                     native |= 4
-                kq = dict(smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=native)
-                _, row_scale, _ = ops.act_quant(x2, mode=L.Q_I8_DYN, levels=2 ** (self.nbits_a - 1) - 1 - zp, want_codes=False, **kq)
+                kq = dict(smooth=smooth, smooth_rcp=rcp, native_chain=native)
+                _, row_scale, _ = ops.act_quant(x2, mode=L.Q_I8_DYN, levels=levels - zp, want_codes=False, **kq)
                 in_scale = row_scale.max().reshape(1)
                 codes, _, _ = ops.act_quant(x2, mode=L.Q_I8_GIVEN_SCALE, scale_in=in_scale, zp0=float(zp), **kq)
                 # iaddmm_int (:1179-1182): bias - input_scale * corr_term, formed in fp32
-                kw["bias"] = prep["bias"] - in_scale * self.corr_term.detach().float().reshape(-1)
-                scale_dtype = self.w_scale.dtype if self.w_scale.dim() > 0 else chain  # a 0-dim scale takes the other operand's dtype
+                bias = prep["bias"] - in_scale * self.corr_term.detach().float().reshape(-1)
+                scale_dtype = w_scale.dtype if w_scale.dim() > 0 else chain  # a 0-dim scale takes the other operand's dtype
+                prod_dtype = _promote(scale_dtype, w_scale.dtype)
+                out = ops.gemm(codes, self.weight, row_scale=in_scale, bias=bias, prod_round=(None if prod_dtype == torch.float32 else prod_dtype), **acc)
+                return out.reshape(tuple(x.shape[:-1]) + (self.weight.shape[0],))
             elif self.usePTnativeQfunc:
                 # qa_raw_qfunc divides by the input_scale buffer: the chain runs in the promoted dtype of the two, which is
                 # the dtype of x for a module converted from a 16-bit model (its scale buffers carry the model's dtype)
-                st = _promote(chain, self.input_scale.dtype)
-                smooth_native |= 2 if (st == x2.dtype and st != torch.float32) else 0
-                codes, in_scale, _ = ops.act_quant(
-                    x2, mode=L.Q_I8_STATIC, smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=smooth_native,
-                    scale0=self.input_scale, zp0=self.input_zp, shift=128.0, add2=float(self.useSymAct),
-                )  # fmt: skip
-                in_scale = self.input_scale.detach().float().reshape(-1)
-                scale_dtype = self.input_scale.dtype
+                in_scale = self.input_scale.detach()
+                st = _promote(chain, in_scale.dtype)
+                native |= 2 if (st == xd and st != torch.float32) else 0
+                quant = dict(mode=L.Q_I8_STATIC, native_chain=native, scale0=in_scale, zp0=self.input_zp, shift=128.0, add2=float(self.useSymAct))
+                scale_dtype = in_scale.dtype
             else:
                 st = _promote(chain, self.quant_stepsize.dtype)
-                smooth_native |= 2 if (st == x2.dtype and st != torch.float32) else 0
-                codes, in_scale, _ = ops.act_quant(
-                    x2, mode=L.Q_I8_STATIC_CLAMP_FIRST, smooth=smooth, smooth_rcp=prep["smooth_rcp"], native_chain=smooth_native,
-                    scale0=self.quant_stepsize, zp0=self.quant_zero_point, lo=self.cvs[1], hi=self.cvs[0],
-                    shift=float(128 - self.useSymAct),
-                )  # fmt: skip
-                in_scale = self.input_scale.detach().float().reshape(-1)
-                scale_dtype = self.input_scale.dtype
-            prod_dtype = _promote(scale_dtype, self.w_scale.dtype)
-            out = ops.gemm(
-                codes, self.weight,
-                chunk_k=_normalised_chunk(self.chunk_size), trun_bits=int(self.truncate_lsb), max_acc_bits=self.max_acc_bits,
-                epilogue=L.EPI_SCALE_PROD, row_scale=in_scale, col_scale=prep["w_scale"], bias=kw.pop("bias", prep["bias"]),
-                prod_round=(None if prod_dtype == torch.float32 else prod_dtype), scale_round=torch.float16,
-                acc_round=(None if self.acc_dtype == torch.float32 else self.acc_dtype), out_dtype=org_dtype, **kw,
-            )  # fmt: skip
-            return out.reshape(tar_shape)
+                native |= 2 if (st == xd and st != torch.float32) else 0
+                quant = dict(mode=L.Q_I8_STATIC_CLAMP_FIRST, native_chain=native, scale0=self.quant_stepsize, zp0=self.quant_zero_point,
+                             lo=self.cvs[1], hi=self.cvs[0], shift=float(128 - self.useSymAct))  # fmt: skip
+                in_scale = self.input_scale.detach()
+                scale_dtype = in_scale.dtype
+            prod_dtype = _promote(scale_dtype, w_scale.dtype)
+            return ops.quant_gemm(x, self.weight, smooth=smooth, smooth_rcp=rcp, row_scale=in_scale, bias=prep["bias"],
+                                  prod_round=(None if prod_dtype == torch.float32 else prod_dtype), **quant, **acc)  # fmt: skip
 
 
 def _normalised_chunk(chunk_size: int) -> int:
@@ -344,19 +335,16 @@ class _LinearFPxFwdBwd(torch.autograd.Function):
         ctx.save_for_backward(x2, weight)
         ctx.cfg = (trun_bits, chunk_size, fp8_dyn, bool(clamp_acc_to_dl16), bias.dtype if bias is not None else None)
         native = 0 if org_dtype == torch.float32 else 3
-        if fp8_dyn == "per_token":
-            xq, xs, _ = ops.act_quant(x2, mode=L.Q_F8_DYN, native_chain=native, dl8_flush=clamp_acc_to_dl16)
-            wq, ws = wq_ws
-        else:
-            xq, xs = ops.fp8_quant_per_tensor(x2, dl8_flush=clamp_acc_to_dl16)
-            wq, ws = ops.fp8_quant_per_tensor(weight.detach(), dl8_flush=clamp_acc_to_dl16)
         rnd = None if org_dtype == torch.float32 else org_dtype
-        out = ops.gemm(
-            xq, wq, chunk_k=_fp8_chunk(chunk_size), trun_bits=(14 if clamp_acc_to_dl16 else int(trun_bits)),
-            clamp_dl16=bool(clamp_acc_to_dl16), epilogue=L.EPI_SCALE_SEQ, row_scale=xs, col_scale=ws,
-            bias=(bias.detach().to(org_dtype) if bias is not None else None), mid_round=rnd, acc_round=rnd, out_dtype=org_dtype,
-        )  # fmt: skip
-        return out.reshape(tar_shape)
+        mul = dict(chunk_k=_fp8_chunk(chunk_size), trun_bits=(14 if clamp_acc_to_dl16 else int(trun_bits)), clamp_dl16=bool(clamp_acc_to_dl16),
+                   epilogue=L.EPI_SCALE_SEQ, bias=(bias.detach().to(org_dtype) if bias is not None else None), mid_round=rnd, acc_round=rnd,
+                   out_dtype=org_dtype)  # fmt: skip
+        if fp8_dyn == "per_token":
+            wq, ws = wq_ws
+            return ops.quant_gemm(x, wq, mode=L.Q_F8_DYN, native_chain=native, dl8_flush=bool(clamp_acc_to_dl16), col_scale=ws, **mul)
+        xq, xs = ops.fp8_quant_per_tensor(x2, dl8_flush=clamp_acc_to_dl16)
+        wq, ws = ops.fp8_quant_per_tensor(weight.detach(), dl8_flush=clamp_acc_to_dl16)
+        return ops.gemm(xq, wq, row_scale=xs, col_scale=ws, **mul).reshape(tar_shape)
 
     @staticmethod
     def backward(ctx, grad_output):

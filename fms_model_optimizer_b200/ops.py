@@ -2,7 +2,8 @@
 
 Every function here takes CUDA tensors, allocates its outputs with PyTorch's caching allocator,
 passes raw device pointers plus the current CUDA stream to the library and returns tensors.  There
-is no CPU path and no fallback kernel: a CPU tensor or a missing library is an error.
+is no CPU path and no fallback kernel: a CPU tensor or a missing library is an error.  The calls made for
+every token (GEMM, row quantiser, the two together, PACT+) do that in C++ (csrc/host/qlin_host.cpp).
 
 The functions are also registered as torch custom ops in the ``qlin_b200`` namespace (see the end
 of the file) so that modules call ``torch.ops.qlin_b200.*`` the way the reference's modules call
@@ -31,8 +32,6 @@ _DT = {
 }
 _ROUND = {None: L.DT_NONE, torch.float32: L.DT_F32, torch.float16: L.DT_F16, torch.bfloat16: L.DT_BF16}
 
-_status_words: dict[int, torch.Tensor] = {}
-
 
 # Measurement hooks used by bench.py: LAUNCHES counts kernel launches made through this module;
 # when PROFILE is a list, every launch is bracketed by CUDA events on the launching stream and
@@ -47,6 +46,15 @@ GEMM_MAX_CTAS = 0
 # QLIN_NVTX=1: every launch of this library sits inside an NVTX range named after its entry point, so that a timeline
 # tool shows the library's calls among PyTorch's (off by default: a range costs a little host time per launch).
 NVTX = os.environ.get("QLIN_NVTX", "0") == "1"
+
+
+def _call(name: str, work: float, dev: torch.device, fn, *args):
+    """One launch through the host library: counted, and bracketed by events or an NVTX range when those are on."""
+    global LAUNCHES
+    if PROFILE is None and not NVTX:
+        LAUNCHES += 1
+        return fn(*args)
+    return _timed(name, work, dev, lambda: fn(*args))
 
 
 def _timed(name: str, work: float, dev: torch.device, call):
@@ -99,10 +107,7 @@ def _stream(dev: torch.device) -> C.c_void_p:
 
 def status_word(dev: torch.device) -> torch.Tensor:
     """Per-device int32 status word handed to the GEMM; stays 0 unless a kernel gave up a wait."""
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    if idx not in _status_words:
-        _status_words[idx] = torch.zeros(1, dtype=torch.int32, device=dev)
-    return _status_words[idx]
+    return L.host().status_word(dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 def check_status(dev: Optional[torch.device] = None) -> None:
@@ -122,18 +127,6 @@ def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     if t.dtype != torch.float32:
         t = t.float()
     return t.contiguous()
-
-
-def _pad_k(t: torch.Tensor) -> torch.Tensor:
-    """Returns a K-contiguous 2-D view/copy whose row stride and base are 16-byte aligned."""
-    es = t.element_size()
-    if t.stride(1) == 1 and (t.stride(0) * es) % 16 == 0 and t.data_ptr() % 16 == 0 and t.stride(0) >= t.shape[1]:
-        return t
-    rows, k = t.shape
-    kp = (k * es + 15) // 16 * 16 // es
-    buf = torch.zeros((rows, kp), dtype=t.dtype, device=t.device)
-    buf[:, :k] = t
-    return buf[:, :k]
 
 
 # --------------------------------------------------------------------------------------------------
@@ -165,70 +158,20 @@ def gemm(
     """``D[M,N] = epilogue(C + sum_chunks f(A_c @ B_c^T))`` with A ``[M,K]`` and B ``[N,K]`` (both
     K-contiguous, int8 or float8_e4m3fn).  See ``qlin_gemm`` in include/qlin_b200.h for the
     chunk and epilogue semantics (tl_matmul_chunk_truncate, fms_mo/custom_ext_kernels/triton_kernels.py:468)."""
-    dev = _require_cuda(a, b_nk, c, out, row_scale, col_scale, bias)
-    if a.dim() != 2 or b_nk.dim() != 2 or a.shape[1] != b_nk.shape[1]:
-        raise RuntimeError(f"incompatible shapes {tuple(a.shape)} x {tuple(b_nk.shape)}^T")
-    if a.dtype != b_nk.dtype or a.dtype not in (torch.int8, torch.float8_e4m3fn, torch.float8_e5m2):
-        raise RuntimeError(f"operands must both be int8, float8_e4m3fn or float8_e5m2, got {a.dtype} and {b_nk.dtype}")
-    f8 = a.dtype != torch.int8
-    M, K = a.shape
-    N = b_nk.shape[0]
-    raw_dtype = torch.float32 if f8 else torch.int32
-    if epilogue == L.EPI_RAW:
-        out_dtype = raw_dtype
-    elif out_dtype is None:
-        out_dtype = torch.float32
-    ldd = N
+    sc_bases, sc_rows, sc_row0, sc_ld = (), 0, 0, 0
     if scatter is not None:
         # (base addresses, rows per destination, first row in each destination[, leading dimension]): the epilogue
         # stores row block m // rows to its own buffer, possibly another GPU's; nothing is returned
-        if out is not None or c is not None:
-            raise RuntimeError("scatter excludes out and c")
-        ldd = int(scatter[3]) if len(scatter) > 3 else N
-    elif out is None:
-        out = torch.empty((M, N), dtype=out_dtype, device=dev)
-    elif out.dtype != out_dtype or out.shape != (M, N) or out.stride(1) != 1:
-        raise RuntimeError("out has the wrong dtype, shape or layout")
-    else:
-        ldd = out.stride(0)
-    if M == 0 or N == 0:
-        return out
-    if K == 0:
-        raise RuntimeError("K must be positive")
-    a = _pad_k(a)
-    b_nk = _pad_k(b_nk)
-    if c is not None:
-        if c.dtype != raw_dtype or c.shape != (M, N):
-            raise RuntimeError("c must be an [M,N] tensor of the accumulator dtype")
-        if c.stride(1) != 1:
-            c = c.contiguous()
-    rs, cs, bs = _f32(row_scale), _f32(col_scale), _f32(bias)
-    if rs is not None and rs.numel() not in (1, M):
-        raise RuntimeError("row_scale must have 1 or M elements")
-    if cs is not None and cs.numel() not in (1, N):
-        raise RuntimeError("col_scale must have 1 or N elements")
-    if bs is not None and bs.numel() != N:
-        raise RuntimeError("bias must have N elements")
-    args = L.GemmArgs(
-        a=_ptr(a), b=_ptr(b_nk), c=_ptr(c), d=_ptr(out),
-        row_scale=_ptr(rs), col_scale=_ptr(cs), bias=_ptr(bs), status=_ptr(status_word(dev)),
-        lda=a.stride(0), ldb=b_nk.stride(0), ldc=(c.stride(0) if c is not None else 0), ldd=ldd,
-        M=M, N=N, K=K, kind=_DT[a.dtype],
-        chunk_k=int(chunk_k), trun_bits=int(trun_bits), max_acc_bits=int(max_acc_bits),
-        trunc_then_acc=int(bool(trunc_then_acc)), clamp_dl16=int(bool(clamp_dl16)), epilogue=int(epilogue),
-        row_scale_stride=(0 if rs is None or rs.numel() == 1 else 1),
-        col_scale_stride=(0 if cs is None or cs.numel() == 1 else 1),
-        prod_round=_ROUND[prod_round], scale_round=_ROUND[scale_round], mid_round=_ROUND[mid_round], acc_round=_ROUND[acc_round],
-        out_dtype=_DT[out_dtype], max_ctas=int(GEMM_MAX_CTAS if max_ctas is None else max_ctas),
+        sc_bases, sc_rows, sc_row0 = list(scatter[0]), int(scatter[1]), int(scatter[2])
+        sc_ld = int(scatter[3]) if len(scatter) > 3 else 0
+        if sc_rows <= 0:
+            raise RuntimeError("scatter needs a positive number of rows per destination")
+    work = 2.0 * a.numel() * (b_nk.shape[0] if b_nk.dim() else 0)
+    return _call(
+        "gemm", work, a.device, L.host().gemm, a, b_nk, c, out, int(chunk_k), int(trun_bits), int(max_acc_bits), bool(trunc_then_acc),
+        bool(clamp_dl16), int(epilogue), row_scale, col_scale, bias, _ROUND[prod_round], _ROUND[scale_round], _ROUND[mid_round], _ROUND[acc_round],
+        int(GEMM_MAX_CTAS if max_ctas is None else max_ctas), (L.DT_NONE if out_dtype is None else _DT[out_dtype]), sc_bases, sc_rows, sc_row0, sc_ld,
     )  # fmt: skip
-    if scatter is not None:
-        bases = list(scatter[0]) + [None] * (8 - len(scatter[0]))
-        args.scatter_d = (C.c_void_p * 8)(*bases)
-        args.scatter_rows, args.scatter_row0 = int(scatter[1]), int(scatter[2])
-    with torch.cuda.device(dev):
-        rc = _timed("gemm", 2.0 * M * N * K, dev, lambda: L.load().qlin_gemm(C.byref(args), _stream(dev)))
-        L.check(rc, "qlin_gemm")
-    return out
 
 
 def bmm_i8(a: torch.Tensor, b_nk: torch.Tensor, scales: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
@@ -371,18 +314,6 @@ def smooth_reciprocal(smooth_f32: torch.Tensor) -> torch.Tensor:
     return torch.where(bad, torch.full_like(r, float("nan")), r).contiguous()
 
 
-_STATIC_MODES = (L.Q_I8_STATIC, L.Q_I8_STATIC_CLAMP_FIRST, L.Q_I8_STATIC_ROUND_FIRST, L.Q_I8_AFFINE_RCP)
-
-
-def _scalar_or_src(t, dev: torch.device, src, i: int) -> float:
-    """A static quantiser's scalar: entry ``i`` of ``src`` when ``t`` is a one-element tensor the kernel can read, else the
-    number itself."""
-    if isinstance(t, torch.Tensor) and t.device == dev and t.numel() == 1 and t.dtype in (torch.float32, torch.float16, torch.bfloat16, torch.int32):
-        src[i] = L.ScalarSrc(ptr=t.data_ptr(), dtype=_DT[t.dtype])
-        return 0.0
-    return float(t)
-
-
 def act_quant(
     x: torch.Tensor,
     *,
@@ -409,52 +340,67 @@ def act_quant(
     """Row-wise 8-bit quantisation of a 2-D tensor; returns ``(codes, scale[rows], dq)``.
     See ``qlin_act_quant`` in include/qlin_b200.h for the modes.  In the static modes ``scale0``, ``zp0``, ``lo`` and ``hi``
     may be one-element tensors; those on x's device are read by the kernel, without a synchronisation."""
-    dev = _require_cuda(x, smooth, scale_in)
-    if x.dim() != 2:
-        raise RuntimeError("act_quant takes a 2-D tensor")
-    if x.dtype not in (torch.float32, torch.float16, torch.bfloat16):
-        raise RuntimeError(f"unsupported activation dtype {x.dtype}")
-    if x.stride(1) != 1:
-        x = x.contiguous()
-    rows, cols = x.shape
-    code_dtype = torch.int8
-    if mode == L.Q_F8_DYN or (mode == L.Q_F8_TENSOR and not f8_e5m2):
-        code_dtype = torch.float8_e4m3fn
-    elif mode == L.Q_F8_TENSOR:
-        code_dtype = torch.float8_e5m2
-    codes = torch.empty((rows, cols), dtype=code_dtype, device=dev) if want_codes else None
-    dq = torch.empty((rows, cols), dtype=x.dtype, device=dev) if want_dq else None
-    scale = torch.empty((rows,), dtype=torch.float32, device=dev)
-    sm = _f32(smooth)
-    if sm is not None and sm.numel() != cols:
-        raise RuntimeError("smooth must have one entry per column")
-    rsm = None
-    if sm is not None and not smooth_mul:
-        rsm = _f32(smooth_rcp) if smooth_rcp is not None else smooth_reciprocal(sm)
-    si = _f32(scale_in)
-    if rows == 0 or cols == 0:
-        return codes, scale, dq
-    src = None
-    if mode in _STATIC_MODES and any(isinstance(t, torch.Tensor) for t in (scale0, zp0, lo, hi)):
-        src = (L.ScalarSrc * 4)()
-        scale0, zp0, lo, hi = (_scalar_or_src(t, dev, src, i) for i, t in enumerate((scale0, zp0, lo, hi)))
-    args = L.QuantArgs(
-        x=_ptr(x), smooth=_ptr(sm), smooth_rcp=_ptr(rsm), scale_in=_ptr(si), codes=_ptr(codes), scale_out=_ptr(scale), dq_out=_ptr(dq),
-        status=None, ldx=x.stride(0), ldq=cols, lddq=cols, rows=rows, cols=cols, x_dtype=_DT[x.dtype], mode=mode,
-        native_chain=int(native_chain), smooth_mul=int(bool(smooth_mul)), clamp_codes=int(bool(clamp_codes)),
-        qmax_levels=int(levels), dl8_flush=int(bool(dl8_flush)),
-        scale_in_stride=(0 if si is None or si.numel() == 1 else 1),
-        scale0=scale0, zp0=zp0, lo=lo, hi=hi, shift=shift, add2=add2, dyn_eps=dyn_eps, f8_format=int(bool(f8_e5m2)),
+    if smooth is not None and not smooth_mul and smooth_rcp is None:
+        _require_cuda(x, smooth)
+        smooth_rcp = smooth_reciprocal(_f32(smooth))
+    es = x.element_size()
+    nbytes = x.numel() * (es + (1 if want_codes else 0) + (es if want_dq else 0))
+    return _call(
+        "act_quant", float(nbytes), x.device, L.host().act_quant, x, int(mode), smooth, smooth_rcp, bool(smooth_mul), int(native_chain), bool(clamp_codes),
+        int(levels), bool(want_codes), bool(want_dq), scale_in, bool(dl8_flush), scale0, zp0, lo, hi, float(shift), float(add2), float(dyn_eps),
+        bool(f8_e5m2),
     )  # fmt: skip
-    nbytes = rows * cols * (x.element_size() + (1 if want_codes else 0) + (x.element_size() if want_dq else 0)) + 4 * rows
-    nbytes += 4 * cols if sm is not None else 0
-    with torch.cuda.device(dev):
-        if src is not None:
-            rc = _timed("act_quant", float(nbytes), dev, lambda: L.load().qlin_act_quant_static(C.byref(args), src, _stream(dev)))
-        else:
-            rc = _timed("act_quant", float(nbytes), dev, lambda: L.load().qlin_act_quant(C.byref(args), _stream(dev)))
-        L.check(rc, "qlin_act_quant")
-    return codes, scale, dq
+
+
+def quant_gemm(
+    x: torch.Tensor,
+    weight: torch.Tensor,
+    *,
+    mode: int = L.Q_I8_DYN,
+    smooth: Optional[torch.Tensor] = None,
+    smooth_rcp: Optional[torch.Tensor] = None,
+    native_chain: int = 0,
+    levels: int = 127,
+    dl8_flush: bool = False,
+    scale0: Union[float, torch.Tensor] = 1.0,
+    zp0: Union[float, torch.Tensor] = 0.0,
+    lo: Union[float, torch.Tensor] = 0.0,
+    hi: Union[float, torch.Tensor] = 0.0,
+    shift: float = 0.0,
+    add2: float = 0.0,
+    row_scale: Optional[torch.Tensor] = None,
+    col_scale: Optional[torch.Tensor] = None,
+    bias: Optional[torch.Tensor] = None,
+    chunk_k: int = 0,
+    trun_bits: int = 0,
+    max_acc_bits: int = 32,
+    clamp_dl16: bool = False,
+    epilogue: int = L.EPI_SCALE_PROD,
+    prod_round: Optional[torch.dtype] = None,
+    scale_round: Optional[torch.dtype] = None,
+    mid_round: Optional[torch.dtype] = None,
+    acc_round: Optional[torch.dtype] = None,
+    out_dtype: torch.dtype = torch.float32,
+) -> torch.Tensor:
+    """``act_quant`` of the rows of ``x [.., K]`` followed by ``gemm`` with ``weight [N, K]``, in one call: the forward pass of a
+    deploy-time Linear.  ``row_scale`` defaults to the scales the quantiser found; the other arguments are theirs."""
+    global LAUNCHES
+    if smooth is not None and smooth_rcp is None:
+        smooth_rcp = smooth_reciprocal(_f32(smooth))
+    if PROFILE is None and not NVTX:
+        LAUNCHES += 2
+        return L.host().quant_gemm(
+            x, mode, smooth, smooth_rcp, native_chain, levels, dl8_flush, scale0, zp0, lo, hi, shift, add2, weight, row_scale, col_scale, bias, chunk_k,
+            trun_bits, max_acc_bits, clamp_dl16, epilogue, _ROUND[prod_round], _ROUND[scale_round], _ROUND[mid_round], _ROUND[acc_round], GEMM_MAX_CTAS,
+            _DT[out_dtype],
+        )  # fmt: skip
+    x2 = x.reshape(-1, x.shape[-1])
+    codes, scale, _ = act_quant(x2, mode=mode, smooth=smooth, smooth_rcp=smooth_rcp, native_chain=native_chain, levels=levels, dl8_flush=dl8_flush,
+                                scale0=scale0, zp0=zp0, lo=lo, hi=hi, shift=shift, add2=add2)  # fmt: skip
+    out = gemm(codes, weight, chunk_k=chunk_k, trun_bits=trun_bits, max_acc_bits=max_acc_bits, clamp_dl16=clamp_dl16, epilogue=epilogue,
+               row_scale=scale if row_scale is None else row_scale, col_scale=col_scale, bias=bias, prod_round=prod_round, scale_round=scale_round,
+               mid_round=mid_round, acc_round=acc_round, out_dtype=out_dtype)  # fmt: skip
+    return out.reshape(*x.shape[:-1], weight.shape[0])
 
 
 def weight_fq_perch(
@@ -560,20 +506,8 @@ def pact2_fwd(x: torch.Tensor, clip_val: torch.Tensor, clip_valn: Optional[torch
               variant: int = L.PACT_TWO_SIDED) -> torch.Tensor:
     """PACTplus2STE.forward with dequantize=True (fms_mo/quant/quantizers.py:1949-2055); ``variant`` selects the
     one-sided (PACTplusSTE, :1016) or symmetric (PACTplusSymSTE_rev1, :1073) member of the family."""
-    dev = _require_cuda(x)
-    xc = x.contiguous()
-    out = torch.empty_like(xc)
-    cv = _clip_f32(clip_val, dev)
-    cvn = _clip_f32(clip_valn, dev) if clip_valn is not None else None
-    args = L.Pact2Args(
-        x=_ptr(xc), grad_out=None, out=_ptr(out), clip_val=_ptr(cv), clip_valn=_ptr(cvn), grad_clip=None,
-        workspace=None, numel=xc.numel(), dtype=_DT[xc.dtype], num_bits=int(num_bits), align_zero=int(bool(align_zero)),
-        variant=int(variant),
-    )  # fmt: skip
-    with torch.cuda.device(dev):
-        rc = _timed("pact2_fwd", 2.0 * xc.numel() * xc.element_size(), dev, lambda: L.load().qlin_pact2_fwd(C.byref(args), _stream(dev)))
-        L.check(rc, "qlin_pact2_fwd")
-    return out
+    return _call("pact2_fwd", 2.0 * x.numel() * x.element_size(), x.device, L.host().pact2_fwd, x, clip_val, clip_valn, int(num_bits), bool(align_zero),
+                 int(variant))  # fmt: skip
 
 
 def pact2_bwd(
@@ -581,26 +515,8 @@ def pact2_bwd(
     align_zero: bool, variant: int = L.PACT_TWO_SIDED,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
     """PACTplus2STE.backward (fms_mo/quant/quantizers.py:2058-2102): returns ``(grad_x, [grad_cv, grad_cvn])``."""
-    dev = _require_cuda(x, grad_out)
-    xc = x.contiguous()
-    gc = grad_out.contiguous()
-    if gc.dtype != xc.dtype:
-        gc = gc.to(xc.dtype)
-    gx = torch.empty_like(xc)
-    cv = _clip_f32(clip_val, dev)
-    cvn = _clip_f32(clip_valn, dev) if clip_valn is not None else None
-    lib = L.load()
-    ws = torch.empty((max(1, lib.qlin_pact2_bwd_workspace_bytes(xc.numel()) // 4),), dtype=torch.float32, device=dev)
-    grads = torch.empty((2,), dtype=torch.float32, device=dev)
-    args = L.Pact2Args(
-        x=_ptr(xc), grad_out=_ptr(gc), out=_ptr(gx), clip_val=_ptr(cv), clip_valn=_ptr(cvn), grad_clip=_ptr(grads),
-        workspace=_ptr(ws), numel=xc.numel(), dtype=_DT[xc.dtype], num_bits=int(num_bits),
-        align_zero=int(bool(align_zero)), variant=int(variant),
-    )  # fmt: skip
-    with torch.cuda.device(dev):
-        rc = _timed("pact2_bwd", 3.0 * xc.numel() * xc.element_size(), dev, lambda: lib.qlin_pact2_bwd(C.byref(args), _stream(dev)))
-        L.check(rc, "qlin_pact2_bwd")
-    return gx, grads
+    return _call("pact2_bwd", 3.0 * x.numel() * x.element_size(), x.device, L.host().pact2_bwd, x, grad_out, clip_val, clip_valn, int(num_bits),
+                 bool(align_zero), int(variant))  # fmt: skip
 
 
 # --------------------------------------------------------------------------------------------------
