@@ -45,6 +45,10 @@ EXPORTED_SYMBOLS = (
     "qlin_gemm_batched",
     "qlin_act_quant",
     "qlin_act_quant_static",
+    "qlin_f8_tensor_quant",
+    "qlin_f8_tensor_colsum_workspace_bytes",
+    "qlin_absmax_parts",
+    "qlin_absmax_parts_count",
     "qlin_pact2_fwd",
     "qlin_pact2_bwd",
     "qlin_pact2_bwd_workspace_bytes",

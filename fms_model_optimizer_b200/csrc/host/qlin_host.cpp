@@ -341,6 +341,60 @@ Tensor quant_gemm(const Tensor& x, int mode, const OptTensor& smooth, const OptT
   return out.reshape(shape);
 }
 
+// ------------------------------------------------------------------------------------------------ per-tensor FP8
+// Partial maxima of |x| over a dense tensor.
+Tensor absmax_parts(const Tensor& x_in) {
+  const at::Device dev = require_cuda({&x_in});
+  if (!is_float(x_in.scalar_type())) raise("unsupported dtype");
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor x = x_in.contiguous();
+  const Tensor parts = empty({qlin_absmax_parts_count(x.numel())}, at::kFloat, dev);
+  check(qlin_absmax_parts(data(x), x.numel(), dtype_code(x.scalar_type()), static_cast<float*>(data(parts)), stream_of(dev)), "qlin_absmax_parts");
+  return parts;
+}
+
+// Codes [rows, cols] and / or [cols, rows] with rows of a multiple of 16 bytes, the scale [1] and, optionally, the column sums.
+std::tuple<OptTensor, OptTensor, Tensor, OptTensor> f8_tensor_quant(const Tensor& x_in, const Tensor& parts, bool e5m2, double eps, bool dl8_flush,
+                                                                    bool want_codes, bool want_t, bool want_colsum) {
+  const at::Device dev = require_cuda({&x_in, &parts});
+  if (x_in.dim() != 2) raise("f8_tensor_quant takes a 2-D tensor");
+  if (!is_float(x_in.scalar_type())) raise("unsupported activation dtype");
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor x = x_in.contiguous();
+  const int64_t rows = x.size(0), cols = x.size(1);
+  const at::ScalarType ct = e5m2 ? at::kFloat8_e5m2 : at::kFloat8_e4m3fn;
+  Tensor codes, codes_t, colsum, ws;
+  const int64_t ldq = (cols + 15) / 16 * 16, ldt = (rows + 15) / 16 * 16;
+  if (want_codes) codes = ldq == cols ? empty({rows, cols}, ct, dev) : empty({rows, ldq}, ct, dev).narrow(1, 0, cols);
+  if (want_t) codes_t = ldt == rows ? empty({cols, rows}, ct, dev) : empty({cols, ldt}, ct, dev).narrow(1, 0, rows);
+  if (want_colsum) {
+    colsum = empty({cols}, at::kFloat, dev);
+    ws = empty({std::max<int64_t>(1, qlin_f8_tensor_colsum_workspace_bytes(static_cast<int32_t>(rows), static_cast<int32_t>(cols)) / 4)}, at::kFloat, dev);
+  }
+  const Tensor scale = empty({1}, at::kFloat, dev);
+  qlin_f8_tensor_args a = {};
+  a.x = data(x);
+  a.amax_parts = static_cast<const float*>(data(parts));
+  a.nparts = static_cast<int32_t>(parts.numel());
+  a.codes = data(codes);
+  a.codes_t = data(codes_t);
+  a.scale_out = static_cast<float*>(data(scale));
+  a.colsum = static_cast<float*>(data(colsum));
+  a.workspace = static_cast<float*>(data(ws));
+  a.ldx = cols;
+  a.ldq = ldq;
+  a.ldt = ldt;
+  a.rows = static_cast<int32_t>(rows);
+  a.cols = static_cast<int32_t>(cols);
+  a.x_dtype = dtype_code(x.scalar_type());
+  a.f8_format = e5m2;
+  a.dl8_flush = dl8_flush;
+  a.f8_max = e5m2 ? 57344.0f : 448.0f;
+  a.eps = static_cast<float>(eps);
+  check(qlin_f8_tensor_quant(&a, stream_of(dev)), "qlin_f8_tensor_quant");
+  return {opt(codes), opt(codes_t), scale, opt(colsum)};
+}
+
 // ------------------------------------------------------------------------------------------------ PACT+
 Tensor clip_f32(const Tensor& t, at::Device dev) {
   Tensor d = t.detach();
@@ -404,6 +458,8 @@ PYBIND11_MODULE(_qlin_host, m) {
   m.def("gemm", &gemm, rel());
   m.def("act_quant", &act_quant, rel());
   m.def("quant_gemm", &quant_gemm, rel());
+  m.def("absmax_parts", &absmax_parts, rel());
+  m.def("f8_tensor_quant", &f8_tensor_quant, rel());
   m.def("pact2_fwd", &pact2_fwd, rel());
   m.def("pact2_bwd", &pact2_bwd, rel());
 }

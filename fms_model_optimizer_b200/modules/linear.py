@@ -332,7 +332,11 @@ class _LinearFPxFwdBwd(torch.autograd.Function):
         org_dtype = x.dtype
         tar_shape = x.shape[:-1] + (weight.shape[0],)
         x2 = x.reshape(-1, x.shape[-1])
-        ctx.save_for_backward(x2, weight)
+        x_parts = w_parts = None
+        if fp8_dyn != "per_token":
+            x_parts, w_parts = ops.absmax_parts(x2), ops.absmax_parts(weight.detach())
+        # the maxima are kept beside the tensors they belong to: the backward pass scales the same tensors again
+        ctx.save_for_backward(x2, weight, x_parts, w_parts)
         ctx.cfg = (trun_bits, chunk_size, fp8_dyn, bool(clamp_acc_to_dl16), bias.dtype if bias is not None else None)
         native = 0 if org_dtype == torch.float32 else 3
         rnd = None if org_dtype == torch.float32 else org_dtype
@@ -342,32 +346,30 @@ class _LinearFPxFwdBwd(torch.autograd.Function):
         if fp8_dyn == "per_token":
             wq, ws = wq_ws
             return ops.quant_gemm(x, wq, mode=L.Q_F8_DYN, native_chain=native, dl8_flush=bool(clamp_acc_to_dl16), col_scale=ws, **mul)
-        xq, xs = ops.fp8_quant_per_tensor(x2, dl8_flush=clamp_acc_to_dl16)
-        wq, ws = ops.fp8_quant_per_tensor(weight.detach(), dl8_flush=clamp_acc_to_dl16)
+        xq, _, xs, _ = ops.fp8_quant_tensor(x2, x_parts, dl8_flush=bool(clamp_acc_to_dl16))
+        wq, _, ws, _ = ops.fp8_quant_tensor(weight.detach(), w_parts, dl8_flush=bool(clamp_acc_to_dl16))
         return ops.gemm(xq, wq, row_scale=xs, col_scale=ws, **mul).reshape(tar_shape)
 
     @staticmethod
     def backward(ctx, grad_output):
-        x2, weight = ctx.saved_tensors
+        x2, weight, x_parts, w_parts = ctx.saved_tensors
         trun_bits, chunk_size, fp8_dyn, dl16, bias_dtype = ctx.cfg
         if fp8_dyn != "per_tensor":
             raise NotImplementedError("the backward of the FP8 Linear runs with dynamic_fp8='per_tensor' only (so does the reference's)")
         dtype_input = x2.dtype
         out_dim, in_dim = weight.shape
         g2 = grad_output.reshape(-1, out_dim).to(dtype_input)
-        xq, xs = ops.fp8_quant_per_tensor(x2, e5m2=True, eps=0.0, dl8_flush=dl16)
-        wq, ws = ops.fp8_quant_per_tensor(weight.detach(), e5m2=True, eps=0.0, dl8_flush=dl16)
-        gq, gs = ops.fp8_quant_per_tensor(g2, e5m2=True, eps=0.0, dl8_flush=dl16)
+        kq = dict(e5m2=True, eps=0.0, dl8_flush=dl16)
+        # both GEMM operands are K-major: grad_weight takes the codes of g and x transposed, grad_input those of g and W transposed
+        _, xq_t, xs, _ = ops.fp8_quant_tensor(x2, x_parts, want_codes=False, want_t=True, **kq)
+        _, wq_t, ws, _ = ops.fp8_quant_tensor(weight.detach(), w_parts, want_codes=False, want_t=True, **kq)
+        gq, gq_t, gs, gsum = ops.fp8_quant_tensor(g2, ops.absmax_parts(g2), want_t=True, want_colsum=bias_dtype is not None, **kq)
         kw = dict(chunk_k=_fp8_chunk(chunk_size), trun_bits=(14 if dl16 else int(trun_bits)), clamp_dl16=dl16, epilogue=L.EPI_SCALE_SEQ)
-
-        def t8(c):  # both GEMM operands are K-major: transpose the one-byte codes
-            return c.view(torch.uint8).t().contiguous().view(torch.float8_e5m2)
-
         # grad_weight[n, k] = sum_m g[m, n] x[m, k];  grad_input[m, k] = sum_n g[m, n] w[n, k]
-        grad_weight = ops.gemm(t8(gq), t8(xq), row_scale=gs, col_scale=xs, out_dtype=weight.dtype, **kw)
-        grad_input = ops.gemm(gq, t8(wq), row_scale=gs, col_scale=ws, out_dtype=dtype_input, **kw)
+        grad_weight = ops.gemm(gq_t, xq_t, row_scale=gs, col_scale=xs, out_dtype=weight.dtype, **kw)
+        grad_input = ops.gemm(gq, wq_t, row_scale=gs, col_scale=ws, out_dtype=dtype_input, **kw)
         grad_input = grad_input.reshape(grad_output.shape[:-1] + (in_dim,))
-        grad_bias = gq.float().sum(0).to(bias_dtype) if bias_dtype is not None else None
+        grad_bias = gsum.to(bias_dtype) if bias_dtype is not None else None
         return grad_input, grad_weight, grad_bias, None, None, None, None, None
 
 

@@ -707,15 +707,26 @@ def tensor_absmax(x: torch.Tensor) -> torch.Tensor:
     return tensor_fq(x, kind=L.PT_INT_SYM, mode=L.W_MAX, want_out=False)[1]
 
 
+def absmax_parts(x: torch.Tensor) -> torch.Tensor:
+    """Partial maxima of ``|x|`` (fp32, on the device) for ``fp8_quant_tensor``; the maximum over them is max|x|."""
+    return _call("absmax_parts", float(x.numel() * x.element_size()), x.device, L.host().absmax_parts, x)
+
+
+def fp8_quant_tensor(x2: torch.Tensor, parts: torch.Tensor, *, e5m2: bool = False, eps: float = 1e-5, dl8_flush: bool = False, want_codes: bool = True,
+                     want_t: bool = False, want_colsum: bool = False):  # fmt: skip
+    """Per-tensor FP8 codes of ``x2 [rows, cols]`` from ``absmax_parts(x2)``: ``(codes, codes_t [cols, rows], scale [1], colsum)``, each but the
+    scale None unless asked for (``qlin_f8_tensor_quant``).  Rows of codes that are no multiple of 16 long carry a padded pitch."""
+    nbytes = float(x2.numel() * (x2.element_size() + int(want_codes) + int(want_t)))
+    return _call("f8_tensor_quant", nbytes, x2.device, L.host().f8_tensor_quant, x2, parts, bool(e5m2), float(eps), bool(dl8_flush), bool(want_codes),
+                 bool(want_t), bool(want_colsum))  # fmt: skip
+
+
 def fp8_quant_per_tensor(x2: torch.Tensor, *, e5m2: bool = False, eps: float = 1e-5, dl8_flush: bool = False):
     """The per-tensor FP8 scaling of LinearFuncFPxFwdBwd (fms_mo/modules/linear.py:1939-1953 forward, e4m3, scale clamped at
     1e-5; :2003-2017 backward, e5m2, no clamp): ``scale = max(amax / fp8_max, eps)``, ``codes = fp8(x / scale)``.
     Returns ``(codes [rows, cols], scale [1] fp32)``; nothing is read back to the host."""
-    amax = tensor_absmax(x2)
-    native = 0 if x2.dtype == torch.float32 else 3
-    codes, scale, _ = act_quant(x2, mode=L.Q_F8_TENSOR, native_chain=native, scale_in=amax, scale0=(57344.0 if e5m2 else 448.0),
-                                dyn_eps=eps, f8_e5m2=e5m2, dl8_flush=dl8_flush)  # fmt: skip
-    return codes, scale[:1]
+    codes, _, scale, _ = fp8_quant_tensor(x2, absmax_parts(x2), e5m2=e5m2, eps=eps, dl8_flush=dl8_flush)
+    return codes.contiguous(), scale
 
 
 def _scalar(t):

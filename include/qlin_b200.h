@@ -256,6 +256,41 @@ typedef struct qlin_scalar_src {
 int qlin_act_quant_static(const qlin_quant_args* args, const qlin_scalar_src src[4], void* stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * qlin_f8_tensor_quant -- one FP8 scale for a whole tensor, codes row-major and / or transposed in one pass.
+ *
+ * Replaces: the per-tensor branches of LinearFuncFPxFwdBwd (fms_mo/modules/linear.py:1939-1953 forward, e4m3, f8_max = 448,
+ *           eps = 1e-5; :2003-2053 backward, e5m2, f8_max = 57344, eps = 0, with the transposes of the codes and the column
+ *           sums of the gradient's codes that its bias gradient is).
+ * scale = max(amax / f8_max, eps); code = fp8(x / scale), each step rounded to the dtype of x; optional DL8 flush.
+ * amax is the largest of the nparts values in amax_parts (device memory), which qlin_absmax_parts fills for a dense tensor
+ * (qlin_absmax_parts_count(numel) of them).
+ * Outputs, all optional but one: codes [rows, cols]; codes_t [cols, rows] with leading dimension ldt, a multiple of 16 (bytes
+ * between rows and ldt are written as zeros); scale_out [1]; colsum [cols] = sum over rows of the codes' values in fp32 (e5m2
+ * only), with a workspace of qlin_f8_tensor_colsum_workspace_bytes(rows, cols) bytes.
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct qlin_f8_tensor_args {
+  const void* x;
+  const float* amax_parts;
+  void* codes;
+  void* codes_t;
+  float* scale_out;
+  float* colsum;
+  float* workspace;
+  int64_t ldx, ldq, ldt;
+  int32_t rows, cols;
+  int32_t nparts;
+  int32_t x_dtype;   /* F32 / F16 / BF16 */
+  int32_t f8_format; /* 0 = e4m3, 1 = e5m2 */
+  int32_t dl8_flush;
+  float f8_max, eps;
+} qlin_f8_tensor_args;
+
+int qlin_f8_tensor_quant(const qlin_f8_tensor_args* args, void* stream);
+int64_t qlin_f8_tensor_colsum_workspace_bytes(int32_t rows, int32_t cols);
+int qlin_absmax_parts(const void* x, int64_t numel, int32_t dtype, float* parts, void* stream);
+int32_t qlin_absmax_parts_count(int64_t numel);
+
+/* ------------------------------------------------------------------------------------------------
  * qlin_pact2_fwd / qlin_pact2_bwd -- PACT+ two-sided fake quantisation (QAT activations).
  *
  * Replaces: PACT2.forward -> PACTplus2STE.forward / .backward
