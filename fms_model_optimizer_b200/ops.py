@@ -419,35 +419,10 @@ def weight_fq_perch(
 ) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor], torch.Tensor]:
     """Per-output-channel symmetric fake quantisation of ``w [rows, cols]``; returns
     ``(dq, codes, clip[rows])``.  See ``qlin_weight_fq_perch`` in include/qlin_b200.h."""
-    dev = _require_cuda(w, clip, smooth)
-    if w.dim() != 2:
-        w = w.reshape(w.shape[0], -1)
-    if w.dtype not in (torch.float32, torch.float16, torch.bfloat16):
-        raise RuntimeError(f"unsupported weight dtype {w.dtype}")
-    if w.stride(1) != 1:
-        w = w.contiguous()
-    rows, cols = w.shape
-    if mode == L.W_GIVEN:
-        if clip is None or clip.numel() != rows:
-            raise RuntimeError("W_GIVEN needs one clip value per row")
-        clip_io = _f32(clip).clone()
-    else:
-        clip_io = torch.empty((rows,), dtype=torch.float32, device=dev)
-    dq = torch.empty((rows, cols), dtype=w.dtype, device=dev) if want_dq else None
-    codes = torch.empty((rows, cols), dtype=torch.int8, device=dev) if want_codes else None
-    sm = _f32(smooth)
-    if rows == 0 or cols == 0:
-        return dq, codes, clip_io
-    args = L.WfqArgs(
-        w=_ptr(w), smooth=_ptr(sm), dq_out=_ptr(dq), codes=_ptr(codes), clip_io=_ptr(clip_io),
-        ldw=w.stride(0), ldo=cols, ldq=cols, rows=rows, cols=cols, dtype=_DT[w.dtype], num_bits=int(num_bits),
-        mode=int(mode), native_mul=int(bool(native_mul)), clip_dtype=(0 if clip_dtype is None or clip_dtype == w.dtype else _DT[clip_dtype]), c0=float(c0), c1=float(c1),
-    )  # fmt: skip
-    nbytes = rows * cols * (w.element_size() * (2 if want_dq else 1) + (1 if want_codes else 0)) + 4 * rows
-    with torch.cuda.device(dev):
-        rc = _timed("weight_fq", float(nbytes), dev, lambda: L.load().qlin_weight_fq_perch(C.byref(args), _stream(dev)))
-        L.check(rc, "qlin_weight_fq_perch")
-    return dq, codes, clip_io
+    nbytes = w.numel() * (w.element_size() * (2 if want_dq else 1) + (1 if want_codes else 0))
+    cd = 0 if clip_dtype is None or clip_dtype == w.dtype else _DT[clip_dtype]
+    return _call("weight_fq", float(nbytes), w.device, L.host().weight_fq_perch, w, int(num_bits), int(mode), clip, smooth, bool(native_mul), cd, bool(want_dq),
+                 bool(want_codes), float(c0), float(c1))  # fmt: skip
 
 
 def tensor_fq(
@@ -517,6 +492,26 @@ def pact2_bwd(
     """PACTplus2STE.backward (fms_mo/quant/quantizers.py:2058-2102): returns ``(grad_x, [grad_cv, grad_cvn])``."""
     return _call("pact2_bwd", 3.0 * x.numel() * x.element_size(), x.device, L.host().pact2_bwd, x, grad_out, clip_val, clip_valn, int(num_bits),
                  bool(align_zero), int(variant))  # fmt: skip
+
+
+# --------------------------------------------------------------------------------------------------
+# Product of a fake-quantised activation and a fake-quantised weight (qlin_fq_*, include/qlin_b200.h)
+# --------------------------------------------------------------------------------------------------
+def fq_linear_fwd(x2, w, bias, clip_val, clip_valn, num_bits: int, align_zero: bool, variant: int, w_clip, w_bits: int):
+    """``F.linear(x2, w, bias)`` for fp32 ``x2 [M, K]`` from a PACT+ quantiser with these clip values and ``w [N, K]`` from the per-channel SAWB+
+    quantiser with clip values ``w_clip [N]``, as one int8 GEMM.  Returns ``(out, *saved)``; ``fq_linear_bwd`` takes ``saved``."""
+    global LAUNCHES
+    LAUNCHES += 3
+    return _call("fq_linear_fwd", 2.0 * x2.numel() * w.shape[0], x2.device, L.host().fq_linear_fwd, x2, w, bias, clip_val, clip_valn, int(num_bits),
+                 bool(align_zero), int(variant), w_clip, int(w_bits))  # fmt: skip
+
+
+def fq_linear_bwd(g2, saved, want_x: bool, want_w: bool, want_b: bool):
+    """Gradients ``(gx [M, K], gw [N, K], gb [N])`` of ``fq_linear_fwd`` for ``g2 [M, N]`` fp32 (None where not wanted)."""
+    global LAUNCHES
+    LAUNCHES += 3 * bool(want_x) + 2 * bool(want_w or want_b) + 3 * bool(want_w) - 1
+    return _call("fq_linear_bwd", 2.0 * g2.numel() * saved[0].shape[0] * (bool(want_x) + bool(want_w)), g2.device, L.host().fq_linear_bwd, g2, *saved,
+                 bool(want_x), bool(want_w), bool(want_b))  # fmt: skip
 
 
 # --------------------------------------------------------------------------------------------------
