@@ -62,7 +62,12 @@ struct Cfg {
   static constexpr int EPI_WARPS = CHUNKED ? 16 : 8;
   static constexpr int PRODUCER_WARP = EPI_WARPS;
   static constexpr int MMA_WARP = EPI_WARPS + 1;
-  static constexpr int THREADS = (EPI_WARPS + 2) * 32;
+  // Issuing the MMAs and the barrier traffic of one chunk takes a warp about 700 cycles, several times what the tensor pipe
+  // needs for it: the chunked kernel shares the issue out, two warps taking every other chunk and, in low-byte mode, a third
+  // keeping the untruncated total.  4096 x 8192 x 4096, 8 bits: chunks of 32 / 64 / 128 730 / 431 / 371 -> 643 / 372 / 256 us.
+  // Without any hand-over of accumulators the issue side would take 246 us at 64 and the epilogue side 302.
+  static constexpr int MMA_WARPS = CHUNKED ? 3 : 1;
+  static constexpr int THREADS = (EPI_WARPS + 1 + MMA_WARPS) * 32;
   static constexpr int A_BYTES = kBM * kBK;
   static constexpr int B_BYTES = BN * kBK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -459,16 +464,23 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     return;
   }
 
+  const int total_k32 = (p.kbytes + 31) / 32;
+  // chunks that tile a 128-byte K block exactly (32, 64 or 128 elements, K a multiple of 128)
+  const bool chunk_fast = CHUNKED && (p.chunk_k32 == 1 || p.chunk_k32 == 2 || p.chunk_k32 == 4) && (total_k32 % 4 == 0);
+  // low-byte mode: the last accumulator holds the tile's untruncated total, the others rotate over the chunks
+  const bool low_mode = CHUNKED && !F8 && p.low_byte_mode != 0;
+  const int mma_warps = low_mode ? 3 : (chunk_fast ? 2 : 1);  // issuing warps: each releases every stage
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&aux->full[s], 1);
-      mbar_init(&aux->empty[s], 1);
+      mbar_init(&aux->empty[s], mma_warps);
     }
     for (int b = 0; b < C::NBUF; ++b) {
       mbar_init(&aux->tfull[b], 1);
       mbar_init(&aux->tempty[b], C::EPI_WARPS);
     }
-    mbar_init(&aux->drain, 1);
+    mbar_init(&aux->drain, mma_warps);
     aux->abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async();
@@ -489,7 +501,6 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int per_batch = p.num_m * p.num_n;
   const int num_tiles = BATCHED ? per_batch * p.batch : per_batch;
   const int num_kb = (p.kbytes + kBK - 1) / kBK;
-  const int total_k32 = (p.kbytes + 31) / 32;
   bool timed_out = false;
 
   if (warp == C::PRODUCER_WARP) {
@@ -534,6 +545,89 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
     __syncwarp();
+  } else if (CHUNKED && chunk_fast && warp >= C::MMA_WARP) {
+    // ------------------------------------------------------------------ MMA issuers of whole chunks
+    // Every issuing warp walks over all stages (so that the stage barriers of all stay in step), issues its share and
+    // commits the stage.  Warp 0 and 1 take the even and the odd chunks, counted over all tiles; warp 2 the total.
+    const int mw = warp - C::MMA_WARP;
+    if (mw < mma_warps) {
+      const uint32_t idesc = F8 ? make_idesc(1u, static_cast<uint32_t>(p.f8_ab_format), kBM, C::BN) : make_idesc(2u, 1u, kBM, C::BN);
+      const uint64_t adesc0 = make_smem_desc_sw128(smem_u32(smem));
+      const uint64_t bdesc0 = make_smem_desc_sw128(smem_u32(smem) + C::A_BYTES);
+      const uint32_t nbuf = low_mode ? C::NBUF - 1 : C::NBUF;
+      const uint32_t d_total = tmem_base + (C::NBUF - 1) * C::BN;
+      const int cpk = 4 / p.chunk_k32;
+      uint32_t s = 0, ph = 0;              // smem stage and its phase
+      uint32_t buf = 0, bph = 0, turn = 0;  // accumulator of the next chunk, its phase, whose chunk it is
+      uint32_t tot_ph = 0;
+      bool ok = true, ready = false, tready = false;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+        if (mw == 2) {  // the epilogue warps must have read the previous tile's total before it is overwritten
+          ok = warp_mbar_wait(&aux->tempty[C::NBUF - 1], tot_ph ^ 1u, abort_flag);
+          if (!ok) break;
+          tot_ph ^= 1u;
+        }
+        for (int kb = 0; kb < num_kb && ok; ++kb) {
+          if (!ready) {
+            ok = warp_mbar_wait(&aux->full[s], ph, abort_flag);
+            if (!ok) break;
+          }
+          tc_fence_after();
+          const uint32_t ns = (s + 1 == C::STAGES) ? 0u : s + 1;
+          const uint32_t nph = (ns == 0u) ? (ph ^ 1u) : ph;
+          const uint32_t peek = warp_mbar_test_begin(&aux->full[ns], nph);
+          const uint64_t adesc = adesc0 + static_cast<uint64_t>(s * (C::STAGE_BYTES >> 4));
+          const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * (C::STAGE_BYTES >> 4));
+          if (mw == 2) {
+            tc_mma4_release<F8 ? 1 : 0>(d_total, adesc, bdesc, idesc, kb > 0 ? 1u : 0u, &aux->empty[s]);
+            if (kb == num_kb - 1) tc_commit_elect(&aux->tfull[C::NBUF - 1]);
+          } else {
+            for (int c = 0; c < cpk && ok; ++c) {
+              const uint32_t nb = (buf + 1 == nbuf) ? 0u : buf + 1;
+              const uint32_t nbph = (nb == 0u) ? (bph ^ 1u) : bph;
+              if (turn == static_cast<uint32_t>(mw)) {
+                if (!tready) {
+                  ok = warp_mbar_wait(&aux->tempty[buf], bph ^ 1u, abort_flag);
+                  if (!ok) break;
+                }
+                tc_fence_after();
+                // this warp's next chunk is the next but one: its accumulator is polled before this chunk is issued
+                const uint32_t nb2 = (nb + 1 == nbuf) ? 0u : nb + 1;
+                const uint32_t nbph2 = (nb2 == 0u) ? (nbph ^ 1u) : nbph;
+                const uint32_t tpeek = warp_mbar_test_begin(&aux->tempty[nb2], nbph2 ^ 1u);
+                const uint64_t off = static_cast<uint64_t>(c * p.chunk_k32 * 2);
+                const uint32_t d = tmem_base + buf * C::BN;
+                if (p.chunk_k32 == 1) {
+                  tc_mma_chunk<F8 ? 1 : 0, 1>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
+                } else if (p.chunk_k32 == 2) {
+                  tc_mma_chunk<F8 ? 1 : 0, 2>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
+                } else {
+                  tc_mma_chunk<F8 ? 1 : 0, 4>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
+                }
+                tready = warp_mbar_test_end(tpeek);
+              }
+              turn ^= 1u;
+              buf = nb;
+              bph = nbph;
+            }
+            if (ok) tc_commit_elect(&aux->empty[s]);
+          }
+          ready = warp_mbar_test_end(peek);
+          s = ns;
+          ph = nph;
+        }
+      }
+      if (!ok && lane == 0) {
+        timed_out = !*abort_flag;
+        *abort_flag = 1;
+      }
+      // Nothing may still be reading shared memory or writing TMEM when the CTA retires.
+      tc_commit_elect(&aux->drain);
+      mbar_wait_drain(&aux->drain, 0);
+    }
+    __syncwarp();
+  } else if (warp > C::MMA_WARP) {
+    // the further issuing warps have nothing to do in this mode
   } else if (warp == C::MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
     // One instruction stream feeds the tensor pipe, so this loop is latency-critical: no
@@ -546,23 +640,8 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint32_t buf = 0, bph = 0;       // TMEM accumulator buffer to use next and its phase
     bool ok = true;
     bool ready = false;
-    bool tready = false;  // next accumulator buffer known to be drained
-    // chunks that tile a 128-byte K block exactly (32, 64 or 128 elements, K a multiple of 128)
-    const bool chunk_fast = CHUNKED && (p.chunk_k32 == 1 || p.chunk_k32 == 2 || p.chunk_k32 == 4) && (total_k32 % 4 == 0);
-    // low-byte mode: the last accumulator holds the tile's untruncated total, the others rotate over the chunks
-    const bool low_mode = CHUNKED && !F8 && p.low_byte_mode != 0;
-    const uint32_t nbuf = low_mode ? C::NBUF - 1 : C::NBUF;
-    const uint32_t d_total = tmem_base + (C::NBUF - 1) * C::BN;
-    uint32_t tot_ph = 0;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       uint32_t accumulate = 0, cur = 0;
-      if (low_mode) {
-        // the epilogue warps must have read the previous tile's total before it is overwritten
-        ok = warp_mbar_wait(&aux->tempty[C::NBUF - 1], tot_ph ^ 1u, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        tot_ph ^= 1u;
-      }
       int chunk_pos = 0;
       int k32_left = total_k32;
       for (int kb = 0; kb < num_kb && ok; ++kb) {
@@ -591,50 +670,6 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           accumulate = 1;
           k32_left -= 4;
           if (k32_left == 0) tc_commit_elect(&aux->tfull[cur]);
-        } else if (CHUNKED && chunk_fast && k32_left >= 4) {
-          // whole chunks inside this 128-byte K block: one fused statement per chunk, the next
-          // accumulator's "empty" barrier polled before the current chunk is issued
-          const int cpk = 4 / p.chunk_k32;
-          for (int c = 0; c < cpk && ok; ++c) {
-            if (!tready) {
-              ok = warp_mbar_wait(&aux->tempty[buf], bph ^ 1u, abort_flag);
-              if (!ok) break;
-            }
-            tc_fence_after();
-            const uint32_t nb = (buf + 1 == nbuf) ? 0u : buf + 1;
-            const uint32_t nbph = (nb == 0u) ? (bph ^ 1u) : bph;
-            const uint32_t tpeek = warp_mbar_test_begin(&aux->tempty[nb], nbph ^ 1u);
-            const uint64_t off = static_cast<uint64_t>(c * p.chunk_k32 * 2);
-            const uint32_t d = tmem_base + buf * C::BN;
-            if constexpr (CHUNKED && !F8) {
-              if (low_mode) {
-                const uint32_t acc_total = (kb == 0 && c == 0) ? 0u : 1u;
-                if (p.chunk_k32 == 1) {
-                  tc_mma_chunk_and_total_i8<1>(d, d_total, adesc + off, bdesc + off, idesc, acc_total, &aux->tfull[buf]);
-                } else if (p.chunk_k32 == 2) {
-                  tc_mma_chunk_and_total_i8<2>(d, d_total, adesc + off, bdesc + off, idesc, acc_total, &aux->tfull[buf]);
-                } else {
-                  tc_mma_chunk_and_total_i8<4>(d, d_total, adesc + off, bdesc + off, idesc, acc_total, &aux->tfull[buf]);
-                }
-                tready = warp_mbar_test_end(tpeek);
-                buf = nb;
-                bph = nbph;
-                continue;
-              }
-            }
-            if (p.chunk_k32 == 1) {
-              tc_mma_chunk<F8 ? 1 : 0, 1>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
-            } else if (p.chunk_k32 == 2) {
-              tc_mma_chunk<F8 ? 1 : 0, 2>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
-            } else {
-              tc_mma_chunk<F8 ? 1 : 0, 4>(d, adesc + off, bdesc + off, idesc, &aux->tfull[buf]);
-            }
-            tready = warp_mbar_test_end(tpeek);
-            buf = nb;
-            bph = nbph;
-          }
-          k32_left -= 4;
-          if (ok) tc_commit_elect(&aux->empty[s]);
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -694,8 +729,9 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint32_t ebuf = 0, ebph = 0;
     bool eready = false;
     bool ok = true;
-    const bool elow = CHUNKED && !F8 && p.low_byte_mode != 0;
+    const bool elow = low_mode;
     const uint32_t enbuf = elow ? C::NBUF - 1 : C::NBUF;
+    uint32_t tot_ph = 0;
     TileScales next;
     auto prefetch = [&](int t) {
       if (!scaled || t >= num_tiles) return;
@@ -813,7 +849,12 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         if (!ok) break;
         if (elow) {
-          // the last chunk's commit covers every MMA of the tile: the total is complete
+          if (!warp_mbar_wait(&aux->tfull[C::NBUF - 1], tot_ph, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tot_ph ^= 1u;
+          tc_fence_after();
           uint32_t tot[C::COLS_PER_WARP];
           tmem_ld32(tmem_base + lane_base + (C::NBUF - 1) * C::BN + half * C::COLS_PER_WARP, tot);
           tc_fence_before();
