@@ -45,6 +45,7 @@ EXPORTED_SYMBOLS = (
     "qlin_gemm_batched",
     "qlin_act_quant",
     "qlin_act_quant_static",
+    "qlin_quant_gemm",
     "qlin_f8_tensor_quant",
     "qlin_f8_tensor_colsum_workspace_bytes",
     "qlin_absmax_parts",

@@ -139,8 +139,16 @@ struct Scatter {
   int64_t rows = 0, row0 = 0, ld = 0;
 };
 
+// A quantiser call whose launch was left to the GEMM that reads its codes.
+struct QuantCall {
+  qlin_quant_args args = {};
+  qlin_scalar_src src[4] = {};
+  bool any_src = false;
+  std::vector<Tensor> keep;  // tensors the argument block points into
+};
+
 Tensor gemm_impl(const Tensor& a_in, const Tensor& b_in, const OptTensor& c_in, const OptTensor& out_in, const Chain& ch, const OptTensor& row_scale,
-                 const OptTensor& col_scale, const OptTensor& bias, const Scatter* scatter, int64_t max_ctas, int out_code) {
+                 const OptTensor& col_scale, const OptTensor& bias, const Scatter* scatter, int64_t max_ctas, int out_code, const QuantCall* quant = nullptr) {
   const at::Device dev = require_cuda({&a_in, &b_in, ptr_of(c_in), ptr_of(out_in), ptr_of(row_scale), ptr_of(col_scale), ptr_of(bias)});
   if (a_in.dim() != 2 || b_in.dim() != 2 || a_in.size(1) != b_in.size(1)) raise("incompatible shapes: a [M,K] and b [N,K] are wanted");
   const at::ScalarType kt = a_in.scalar_type();
@@ -212,7 +220,11 @@ Tensor gemm_impl(const Tensor& a_in, const Tensor& b_in, const OptTensor& c_in, 
     g.scatter_rows = static_cast<int32_t>(scatter->rows);
     g.scatter_row0 = static_cast<int32_t>(scatter->row0);
   }
-  check(qlin_gemm(&g, stream_of(dev)), "qlin_gemm");
+  if (quant != nullptr) {
+    check(qlin_quant_gemm(&quant->args, quant->any_src ? quant->src : nullptr, &g, stream_of(dev)), "qlin_quant_gemm");
+  } else {
+    check(qlin_gemm(&g, stream_of(dev)), "qlin_gemm");
+  }
   return out;
 }
 
@@ -253,7 +265,7 @@ float scalar(const Scalar& s, at::Device dev, bool may_stay, qlin_scalar_src& sr
 }
 
 void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smooth, const OptTensor& smooth_rcp, const OptTensor& scale_in,
-                    const Scalar* scalars, bool want_codes, bool want_dq, Tensor& codes, Tensor& scale, Tensor& dq) {
+                    const Scalar* scalars, bool want_codes, bool want_dq, Tensor& codes, Tensor& scale, Tensor& dq, QuantCall* later = nullptr) {
   const at::Device dev = require_cuda({&x_in, ptr_of(smooth), ptr_of(scale_in)});
   if (x_in.dim() != 2) raise("act_quant takes a 2-D tensor");
   if (!is_float(x_in.scalar_type())) raise("unsupported activation dtype");
@@ -266,7 +278,9 @@ void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smo
   } else if (o.mode == QLIN_Q_F8_TENSOR) {
     ct = at::kFloat8_e5m2;
   }
-  if (want_codes) codes = empty({rows, cols}, ct, dev);
+  // codes that a GEMM reads next get rows of a multiple of 16 bytes
+  const int64_t ldq = later != nullptr ? (cols + 15) / 16 * 16 : cols;
+  if (want_codes) codes = ldq == cols ? empty({rows, cols}, ct, dev) : empty({rows, ldq}, ct, dev).narrow(1, 0, cols);
   if (want_dq) dq = empty({rows, cols}, x.scalar_type(), dev);
   scale = empty({rows}, at::kFloat, dev);
   const Tensor sm = f32(smooth);
@@ -274,7 +288,9 @@ void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smo
   const Tensor rsm = sm.defined() && !o.smooth_mul ? f32(smooth_rcp) : Tensor();
   const Tensor si = f32(scale_in);
   if (rows == 0 || cols == 0) return;
-  qlin_quant_args q = {};
+  QuantCall now;
+  QuantCall& call = later != nullptr ? *later : now;
+  qlin_quant_args& q = call.args;
   q.x = data(x);
   q.smooth = static_cast<const float*>(data(sm));
   q.smooth_rcp = static_cast<const float*>(data(rsm));
@@ -283,7 +299,8 @@ void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smo
   q.scale_out = static_cast<float*>(data(scale));
   q.dq_out = data(dq);
   q.ldx = x.stride(0);
-  q.ldq = q.lddq = cols;
+  q.ldq = ldq;
+  q.lddq = cols;
   q.rows = static_cast<int32_t>(rows);
   q.cols = static_cast<int32_t>(cols);
   q.x_dtype = dtype_code(x.scalar_type());
@@ -294,18 +311,20 @@ void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smo
   q.qmax_levels = o.levels;
   q.dl8_flush = o.dl8_flush;
   q.scale_in_stride = si.defined() && si.numel() != 1 ? 1 : 0;
-  qlin_scalar_src src[4] = {};
-  bool any = false;
   const bool st = is_static(o.mode);
-  q.scale0 = scalar(scalars[0], dev, st, src[0], any);
-  q.zp0 = scalar(scalars[1], dev, st, src[1], any);
-  q.lo = scalar(scalars[2], dev, st, src[2], any);
-  q.hi = scalar(scalars[3], dev, st, src[3], any);
+  q.scale0 = scalar(scalars[0], dev, st, call.src[0], call.any_src);
+  q.zp0 = scalar(scalars[1], dev, st, call.src[1], call.any_src);
+  q.lo = scalar(scalars[2], dev, st, call.src[2], call.any_src);
+  q.hi = scalar(scalars[3], dev, st, call.src[3], call.any_src);
   q.shift = o.shift;
   q.add2 = o.add2;
   q.dyn_eps = o.dyn_eps;
   q.f8_format = o.f8_e5m2;
-  check(any ? qlin_act_quant_static(&q, src, stream_of(dev)) : qlin_act_quant(&q, stream_of(dev)), "qlin_act_quant");
+  if (later != nullptr) {
+    later->keep = {x, sm, rsm, si};
+    return;
+  }
+  check(call.any_src ? qlin_act_quant_static(&q, call.src, stream_of(dev)) : qlin_act_quant(&q, stream_of(dev)), "qlin_act_quant");
 }
 
 OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
@@ -332,9 +351,10 @@ Tensor quant_gemm(const Tensor& x, int mode, const OptTensor& smooth, const OptT
   const Scalar scalars[4] = {scale0, zp0, lo, hi};
   Tensor codes, scale, dq;
   const Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
-  act_quant_impl(x2, o, smooth, smooth_rcp, std::nullopt, scalars, true, false, codes, scale, dq);
+  QuantCall quant;
+  act_quant_impl(x2, o, smooth, smooth_rcp, std::nullopt, scalars, true, false, codes, scale, dq, &quant);
   const Chain ch{chunk_k, trun_bits, max_acc_bits, 1, clamp_dl16, epilogue, prod_round, scale_round, mid_round, acc_round};
-  Tensor out = gemm_impl(codes, weight, std::nullopt, std::nullopt, ch, row_scale ? row_scale : OptTensor(scale), col_scale, bias, nullptr, max_ctas, out_code);
+  Tensor out = gemm_impl(codes, weight, std::nullopt, std::nullopt, ch, row_scale ? row_scale : OptTensor(scale), col_scale, bias, nullptr, max_ctas, out_code, &quant);
   if (x.dim() == 2) return out;
   std::vector<int64_t> shape = x.sizes().vec();
   shape.back() = weight.size(0);

@@ -99,6 +99,7 @@ struct GemmParams {
   int64_t batch_stride_d;    // elements of the output type between the problems' outputs
   int32_t low_byte_mode;  // chunked int8, 8 truncated bits: the total on the tensor core, the chunks' low bytes on the ALU
   int32_t sk_mt, sk_split, sk_stages;  // few-row kernel: padded row count, K splits (= cluster size), pipeline stages
+  int32_t dependent;                   // launched as the dependent of the quantiser that writes A and the row scales
 };
 
 __device__ __forceinline__ float round_to(float y, int dt) {
@@ -508,6 +509,7 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     // The whole warp walks the loop converged; one elected lane issues.  The next stage's
     // barrier is polled (non-blocking) before the current stage is issued, which takes the
     // barrier round trip off the loop's critical path.
+    griddep_wait();
     uint32_t s = 0, ph = 0, issued = 0;
     bool ok = true;
     bool ready = false;
@@ -739,6 +741,7 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       tile_coords(BATCHED ? t % per_batch : t, p.num_m, p.num_n, mb, nb);
       next = fetch_scales(p, nb * C::BN + static_cast<int>(threadIdx.x), static_cast<int>(threadIdx.x) < C::BN, mb * kBM + q * 32 + lane);
     };
+    griddep_wait();  // the row scales may come from the launch before
     prefetch(blockIdx.x);
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       int mb, nb;
@@ -975,6 +978,7 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_BAD_ALIGN));
   } else if (warp == C::PRODUCER_WARP) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
+    griddep_wait();
     uint32_t s = 0, ph = 0;
     bool ok = true, ready = false;
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
@@ -1080,6 +1084,7 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       next = fetch_scales(p, nb * C::BN + static_cast<int>(threadIdx.x), static_cast<int>(threadIdx.x) < C::BN,
                           mb * 2 * kBM + static_cast<int>(rank) * kBM + q * 32 + lane);
     };
+    griddep_wait();  // the row scales may come from the launch before
     prefetch(pair);
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
       int mb, nb;
@@ -1161,6 +1166,11 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 // over the splits in split order through distributed shared memory (a fixed order: the result does not
 // depend on scheduling), dequantises and stores them.  Accumulator lane = output channel, so the
 // stores of one row are contiguous across the warp.
+// Launched as the dependent of the row quantiser, the producer fills the stages with weights before it waits for the
+// codes.  Quantiser and GEMM, bf16 in and out, one after the other -> as a pair: 1 x 4096 x 14336 23.1 -> 18.7 us, 37 x 14336 x
+// 4096 24.7 -> 20.6, 517 x 4096 x 4096 (CTA-pair kernel) 25.8 -> 23.2.  The weights of one launch stream at 4.3 TB/s; tiles of
+// 104 rows on 138 SMs instead of 128 on 112, other K orders per CTA, other L2 promotions and two smaller CTAs per SM
+// were measured within 0.4 us of this at 58.7 MB.
 //   warps 0-3  epilogue (TMEM lanes 32 w ..), warp 4 TMA producer, warp 5 MMA issuer / TMEM owner
 // ------------------------------------------------------------------------------------------------
 constexpr int kSkEpiWarps = 8;  // warp w reads TMEM lanes 32 (w % 4) .., half w / 4 of the 32-row groups
@@ -1241,14 +1251,12 @@ qlin_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
   }
-  // the row scales of the (at most 128) activation rows, read by every epilogue thread
-  float* s_rs = aux->cs;
-  if (threadIdx.x < MT) s_rs[threadIdx.x] = (scaled && p.rs != nullptr && static_cast<int>(threadIdx.x) < p.M) ? p.rs[static_cast<int64_t>(threadIdx.x) * p.rs_stride] : 1.0f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = aux->tmem_base;
   bool timed_out = false;
+  float* s_rs = aux->cs;  // the row scales of the (at most 128) activation rows, read by every epilogue thread
   uint32_t* part = reinterpret_cast<uint32_t*>(smem);  // [MT][128] partial accumulators, over the drained pipeline stages
 
   if (bad) {
@@ -1257,11 +1265,18 @@ qlin_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     // ------------------------------------------------------------------ TMA producer
     uint32_t s = 0, ph = 0, issued = 0;
     bool ok = true;
-    for (int kb = kb0; kb < kb1; ++kb) {
+    const uint32_t tx = static_cast<uint32_t>(stage_bytes);
+    const int pre = min(STG, kb1 - kb0);  // the first fill of the stages: weights now, activations once they are there
+    for (int i = 0; i < pre; ++i) tma_issue_first(&aux->full[i], tx, smem + i * stage_bytes, &tmap_w, tile * kBM, (kb0 + i) * kBK);
+    griddep_wait();
+    for (int i = 0; i < pre; ++i) tma_issue_second(&aux->full[i], smem + i * stage_bytes + kSkWBytes, &tmap_x, 0, (kb0 + i) * kBK);
+    issued = static_cast<uint32_t>(pre);
+    if (pre == STG) ph = 1;
+    for (int kb = kb0 + pre; kb < kb1; ++kb) {
       ok = warp_mbar_wait(&aux->empty[s], ph ^ 1u, abort_flag);
       if (!ok) break;
       uint8_t* sa = smem + s * stage_bytes;
-      tma_issue_stage(&aux->full[s], static_cast<uint32_t>(stage_bytes), sa, &tmap_w, tile * kBM, sa + kSkWBytes, &tmap_x, 0, kb * kBK);
+      tma_issue_stage(&aux->full[s], tx, sa, &tmap_w, tile * kBM, sa + kSkWBytes, &tmap_x, 0, kb * kBK);
       ++issued;
       if (++s == static_cast<uint32_t>(STG)) {
         s = 0;
@@ -1313,6 +1328,10 @@ qlin_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int q = warp & 3;
     const int n_local = q * 32 + lane;
     const int n = tile * kBM + n_local;
+    griddep_wait();
+    if (static_cast<int>(threadIdx.x) < MT)
+      s_rs[threadIdx.x] = (scaled && p.rs != nullptr && static_cast<int>(threadIdx.x) < p.M) ? p.rs[static_cast<int64_t>(threadIdx.x) * p.rs_stride] : 1.0f;
+    asm volatile("bar.sync 1, %0;" ::"n"(kSkEpiWarps * 32) : "memory");
     if (warp_mbar_wait(&aux->tfull[0], 0, abort_flag)) {
       tc_fence_after();
       const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
@@ -1422,6 +1441,32 @@ static int make_operand_map(CUtensorMap* tm, const void* base, int64_t rows, int
   return QLIN_OK;
 }
 
+// A launch with a cluster size and, for a GEMM behind its quantiser, the programmatic dependency.
+struct LaunchCfg {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  LaunchCfg(int grid, int threads, size_t smem, cudaStream_t stream, int cluster, bool dependent) {
+    cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 0;
+    if (cluster > 1) {
+      attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      attr[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(cluster);
+      attr[cfg.numAttrs].val.clusterDim.y = 1;
+      attr[cfg.numAttrs].val.clusterDim.z = 1;
+      ++cfg.numAttrs;
+    }
+    if (dependent) {
+      attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+      ++cfg.numAttrs;
+    }
+  }
+};
+
 template <bool F8, bool CHUNKED, bool BATCHED = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
   using C = Cfg<CHUNKED>;
@@ -1438,8 +1483,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   const int64_t tiles = static_cast<int64_t>(p.num_m) * p.num_n * (BATCHED ? p.batch : 1);
   int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
   if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
-  qlin_gemm_kernel<F8, CHUNKED, BATCHED><<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(ta, tb, p);
-  QLIN_CHECK_LAUNCH("qlin_gemm");
+  LaunchCfg lc(grid, C::THREADS, C::SMEM_BYTES, stream, 1, p.dependent != 0);
+  const cudaError_t le = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_kernel<F8, CHUNKED, BATCHED>, ta, tb, p);
+  if (le != cudaSuccess) {
+    cudaGetLastError();
+    return fail(QLIN_ERR_LAUNCH, "qlin_gemm: %s", cudaGetErrorString(le));
+  }
   return QLIN_OK;
 }
 
@@ -1483,19 +1532,8 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   const int tiles = ((p.M + 2 * kBM - 1) / (2 * kBM)) * p.num_n;
   if (clusters > tiles) clusters = tiles;
   if (p.max_ctas > 0 && clusters > p.max_ctas / 2) clusters = p.max_ctas / 2 > 0 ? p.max_ctas / 2 : 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters), 1, 1);
-  cfg.blockDim = dim3(PairCfg::THREADS, 1, 1);
-  cfg.dynamicSmemBytes = PairCfg::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, qlin_gemm_pair_kernel<F8>, ta, tb, p);
+  LaunchCfg lc(2 * clusters, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream, 2, p.dependent != 0);
+  cudaError_t e = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_pair_kernel<F8>, ta, tb, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(QLIN_ERR_LAUNCH, "qlin_gemm (CTA-pair kernel): %s", cudaGetErrorString(e));
@@ -1553,19 +1591,8 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, GemmParam
   int split = 1;
   while (split < 8 && tiles * split * 2 <= sm_count() && num_kb / (split * 2) >= 4) split *= 2;
   p.sk_split = split;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * split), 1, 1);
-  cfg.blockDim = dim3(kSkThreads, 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>(p.sk_stages) * stage_bytes + sizeof(Aux);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, qlin_gemm_skinny_kernel<F8>, tw, tx, p);
+  LaunchCfg lc(tiles * split, kSkThreads, static_cast<size_t>(p.sk_stages) * stage_bytes + sizeof(Aux), stream, split, p.dependent != 0);
+  cudaError_t e = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_skinny_kernel<F8>, tw, tx, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(QLIN_ERR_LAUNCH, "qlin_gemm (few-row kernel): %s", cudaGetErrorString(e));
@@ -1582,7 +1609,8 @@ static bool is_round_dtype(int dt) {
 using namespace qlin;
 
 // batch > 1: the problems' operands are stacked along the rows (dense), one launch of the batched single-CTA kernel.
-static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64_t stride_d) {
+// dependent: the launch before on the stream is the row quantiser that writes a->a and a->row_scale (and none of the other operands).
+static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64_t stride_d, bool dependent = false) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_gemm: args is NULL");
   if (a->a == nullptr || a->b == nullptr || (a->d == nullptr && a->scatter_rows <= 0))
     return fail(QLIN_ERR_NULL, "qlin_gemm: a, b or d is NULL");
@@ -1669,6 +1697,7 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
 
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   p.sk_mt = p.sk_split = p.sk_stages = 0;
+  p.dependent = dependent ? 1 : 0;
   p.batch = batch;
   p.batch_stride_d = stride_d;
   // int8 chunks with the low byte rounded away, summed after rounding, no clamp, chunks of 32 / 64 / 128 that tile K:
@@ -1720,6 +1749,17 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
 }
 
 extern "C" int qlin_gemm(const qlin_gemm_args* a, void* stream) { return gemm_impl(a, stream, 1, 0); }
+
+extern "C" int qlin_quant_gemm(const qlin_quant_args* q, const qlin_scalar_src src[4], const qlin_gemm_args* g, void* stream) {
+  if (q == nullptr || g == nullptr) return fail(QLIN_ERR_NULL, "qlin_quant_gemm: args is NULL");
+  if (q->codes == nullptr || q->codes != g->a || q->rows != g->M || q->cols != g->K || q->ldq != g->lda)
+    return fail(QLIN_ERR_BAD_SHAPE, "qlin_quant_gemm: the quantiser's codes must be the GEMM's a operand");
+  if (g->b == q->codes || g->c != nullptr || g->scatter_rows != 0)
+    return fail(QLIN_ERR_UNSUPPORTED, "qlin_quant_gemm: no accumulator input and no row-block scatter");
+  const int rc = act_quant_impl(q, src, stream);
+  if (rc != QLIN_OK) return rc;
+  return gemm_impl(g, stream, 1, 0, true);
+}
 
 extern "C" int qlin_gemm_batched(const qlin_gemm_args* a, int32_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_d, void* stream) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_gemm_batched: args is NULL");

@@ -13,6 +13,9 @@ namespace qlin {
 // returns `code`, so call sites can write `return fail(QLIN_ERR_..., "...")`.
 int fail(int code, const char* fmt, ...);
 
+// qlin_act_quant with optional device scalars (one kernel launch, which lets a dependent launch start early).
+int act_quant_impl(const qlin_quant_args* args, const qlin_scalar_src* src, void* stream);
+
 // Number of SMs of the current device (cached per device id).
 int sm_count();
 

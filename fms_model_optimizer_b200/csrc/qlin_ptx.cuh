@@ -123,6 +123,13 @@ __device__ __forceinline__ bool mbar_wait_drain(uint64_t* bar, uint32_t parity) 
   }
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// The row quantisers let the next kernel of the stream start early; a GEMM that was launched as their dependent
+// (qlin_quant_gemm) sets itself up and fetches weights meanwhile, and waits here before it touches anything a quantiser
+// wrote.  Both are no-ops in kernels launched any other way.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- TMA
 // 2-D tiled load global -> shared, completion counted in bytes on `bar`.  x is the innermost
 // (contiguous) coordinate and must keep x * element_size a multiple of 16 bytes.
@@ -224,6 +231,29 @@ __device__ __forceinline__ void tma_issue_stage(uint64_t* full_bar, uint32_t byt
       "}" ::"r"(smem_u32(full_bar)),
       "r"(bytes), "r"(smem_u32(smem_a)), "l"(reinterpret_cast<uint64_t>(tmap_a)), "r"(ya), "r"(smem_u32(smem_b)),
       "l"(reinterpret_cast<uint64_t>(tmap_b)), "r"(yb), "r"(x)
+      : "memory");
+}
+
+// The same in two halves: arm the barrier for the bytes of both boxes and load the first; load the second.
+__device__ __forceinline__ void tma_issue_first(uint64_t* full_bar, uint32_t bytes, void* smem_a, const void* tmap_a, int32_t ya, int32_t x) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred pe;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+      "@pe cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%2], [%3, {%5, %4}], [%0];\n\t"
+      "}" ::"r"(smem_u32(full_bar)),
+      "r"(bytes), "r"(smem_u32(smem_a)), "l"(reinterpret_cast<uint64_t>(tmap_a)), "r"(ya), "r"(x)
+      : "memory");
+}
+__device__ __forceinline__ void tma_issue_second(uint64_t* full_bar, void* smem_b, const void* tmap_b, int32_t yb, int32_t x) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred pe;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {%4, %3}], [%0];\n\t"
+      "}" ::"r"(smem_u32(full_bar)),
+      "r"(smem_u32(smem_b)), "l"(reinterpret_cast<uint64_t>(tmap_b)), "r"(yb), "r"(x)
       : "memory");
 }
 

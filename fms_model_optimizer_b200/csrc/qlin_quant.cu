@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(1024) act_quant_vec_kernel(const QuantParams p
       }
     }
   }
+  griddep_launch();
 }
 
 
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(TPB) act_quant_fast_kernel(const QuantParams p
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
     const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    if (i == my_rows - 1) griddep_launch();  // this block has read all it will read
     const XT* xr = reinterpret_cast<const XT*>(ring + static_cast<size_t>(slot) * row_bytes);
     float v[MAXC][16];
     float amax = 0.0f;
@@ -595,6 +597,7 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
     const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    if (i == my_rows - 1) griddep_launch();  // this block has read all it will read
     const uint4* xr = reinterpret_cast<const uint4*>(ring + static_cast<size_t>(slot) * row_bytes);
     uint32_t vp[MAXC][8];
     __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
@@ -828,6 +831,7 @@ __global__ void __launch_bounds__(256) act_quant_scalar_kernel(const QuantParams
       if (p.dq_out != nullptr) store1(reinterpret_cast<XT*>(p.dq_out) + static_cast<int64_t>(row) * p.lddq + c, dq);
     }
   }
+  griddep_launch();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -897,6 +901,7 @@ __global__ void __launch_bounds__(kStThreads) act_quant_static_kernel(const Quan
     *reinterpret_cast<uint4*>(p.codes + i * 16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   for (int64_t i = nvec * 16 + first; i < numel; i += stride) p.codes[i] = static_cast<uint8_t>(static_code<XT, MODE, NATIVE>(p, sv, exact, rs, load1(x + i)));
+  griddep_launch();
 }
 
 // Returns 1 when the call is not one of a dense tensor quantised with a static mode.
@@ -1185,7 +1190,7 @@ static int launch_wfq(const WfqParams& p, cudaStream_t stream) {
 
 using namespace qlin;
 
-static int act_quant_impl(const qlin_quant_args* a, const qlin_scalar_src* src, void* stream) {
+int qlin::act_quant_impl(const qlin_quant_args* a, const qlin_scalar_src* src, void* stream) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_act_quant: args is NULL");
   if (a->x == nullptr) return fail(QLIN_ERR_NULL, "qlin_act_quant: x is NULL");
   if (a->codes == nullptr && a->dq_out == nullptr && a->scale_out == nullptr)

@@ -255,6 +255,13 @@ typedef struct qlin_scalar_src {
 
 int qlin_act_quant_static(const qlin_quant_args* args, const qlin_scalar_src src[4], void* stream);
 
+/* qlin_quant_gemm -- qlin_act_quant (qlin_act_quant_static when src is not NULL) and the qlin_gemm that multiplies its codes, as two
+ * launches of which the second starts while the first runs (programmatic dependent launch): the forward pass of a
+ * deploy-time Linear, QLinearINT8Deploy.forward (fms_mo/modules/linear.py:1309-1338) and LinearFuncFPxFwdBwd.forward.
+ * g->a must be q->codes (rows, cols and ldq those of M, K and lda); g->row_scale may be q->scale_out.  The other operands of g
+ * must not be written by q.  Results are those of the two calls. */
+int qlin_quant_gemm(const qlin_quant_args* q, const qlin_scalar_src src[4], const qlin_gemm_args* g, void* stream);
+
 /* ------------------------------------------------------------------------------------------------
  * qlin_f8_tensor_quant -- one FP8 scale for a whole tensor, codes row-major and / or transposed in one pass.
  *
