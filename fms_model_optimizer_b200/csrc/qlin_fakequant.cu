@@ -167,6 +167,171 @@ __global__ void __launch_bounds__(kFqThreads) pact2_bwd_kernel(const PactParams 
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// bf16 tensors, at most 8 bits: the same arithmetic on packed pairs.
+//
+// The chain above rounds every step to bf16, one element at a time; a pair takes about a third of the instructions when
+//   * subtraction, addition and multiplication of two bf16 numbers are packed bf16 operations (fp32 keeps 24 >= 2 * 8 + 2
+//     bits, so rounding through fp32, as the reference does, gives the same number),
+//   * a division by the step or by the number of levels (both bf16 numbers: 2^b - 1 and 2^b - 2 need at most 8 bits) is one
+//     fp32 multiplication by the reciprocal and one rounding (a quotient of 8-bit significands is never within 2^-18 of a
+//     rounding boundary),
+//   * clipped lanes are selected with masks, and the two clip gradients are summed in packed fp32 pairs.
+// A step outside [1e-15, 1e15] takes the general functions.  8192 x 4096: forward 40.3 -> 31.7 us, backward 71.3 -> 40.8;
+// HBM would allow 21 and 31. The call with its autograd frames takes 105 us (117 before), bound by the host.
+// ------------------------------------------------------------------------------------------------
+typedef __nv_bfloat162 bf2;
+__device__ __forceinline__ bf2 as_bf2(uint32_t w) { return *reinterpret_cast<const bf2*>(&w); }
+__device__ __forceinline__ uint32_t as_u32(bf2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ float2 widen2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)); }
+__device__ __forceinline__ uint32_t narrow2(float2 f) { return as_u32(__float22bfloat162_rn(f)); }
+__device__ __forceinline__ uint32_t scale_pair(uint32_t w, float2 r) { return narrow2(__fmul2_rn(widen2(w), r)); }
+// rint of both numbers (|v| < 2^22), signs of zeros kept; whole bf16 numbers from 128 on and NaN pass through.
+__device__ __forceinline__ uint32_t rint_pair(uint32_t w) {
+  const float2 m = make_float2(12582912.0f, 12582912.0f), n = make_float2(-12582912.0f, -12582912.0f);
+  return (narrow2(__fadd2_rn(__fadd2_rn(widen2(w), m), n)) & 0x7FFF7FFFu) | (w & 0x80008000u);
+}
+
+struct PactPair {
+  bf2 cv, cvn, ncv, zp, step;
+  float2 rstep, rn;
+};
+__device__ __forceinline__ PactPair pact_pair(const PactScalars& s) {
+  PactPair p;
+  p.cv = __float2bfloat162_rn(s.cv);
+  p.cvn = __float2bfloat162_rn(s.cvn);
+  p.ncv = __float2bfloat162_rn(-s.cv);
+  p.zp = __float2bfloat162_rn(s.zp);
+  p.step = __float2bfloat162_rn(s.step);
+  p.rstep = make_float2(s.rstep, s.rstep);
+  p.rn = make_float2(s.rn, s.rn);
+  return p;
+}
+
+template <int VARIANT>
+__device__ __forceinline__ uint32_t pact_fwd_pair(const PactPair& p, uint32_t xw) {
+  const bf2 x = as_bf2(xw);
+  if (VARIANT == QLIN_PACT_TWO_SIDED) {
+    const bf2 y = __hmax2(__hmin2(x, p.cv), p.cvn);
+    const bf2 t = __hsub2_rn(as_bf2(scale_pair(as_u32(y), p.rstep)), p.zp);
+    return as_u32(__hmul2_rn(__hadd2_rn(as_bf2(rint_pair(as_u32(t))), p.zp), p.step));
+  }
+  if (VARIANT == QLIN_PACT_ONE_SIDED) {
+    const bf2 y = __hmin2(__hmax2(x, p.cvn), p.cv);  // cvn is 0
+    return as_u32(__hmul2_rn(as_bf2(rint_pair(scale_pair(as_u32(y), p.rstep))), p.step));
+  }
+  const bf2 y = __hmax2_nan(__hmin2_nan(x, p.cv), p.ncv);  // a NaN stays one
+  const uint32_t q = rint_pair(scale_pair(as_u32(__hadd2_rn(y, p.cv)), p.rstep));
+  return as_u32(__hsub2_rn(__hmul2_rn(as_bf2(q), p.step), p.cv));
+}
+
+// Returns the pair of input gradients; adds to the clip gradients.
+template <int VARIANT>
+__device__ __forceinline__ uint32_t pact_bwd_pair(const PactPair& p, uint32_t xw, uint32_t gw, float2& ga, float2& gan) {
+  const bf2 x = as_bf2(xw), g = as_bf2(gw);
+  const uint32_t hi = __hge2_mask(x, p.cv);
+  const uint32_t lo = __hle2_mask(x, VARIANT == QLIN_PACT_SYMMETRIC ? p.ncv : p.cvn);
+  const uint32_t in = ~(hi | lo);
+  if (VARIANT == QLIN_PACT_SYMMETRIC) {
+    const uint32_t z = scale_pair(as_u32(__hadd2_rn(x, p.cv)), p.rstep);
+    const bf2 d = __hsub2_rn(as_bf2(rint_pair(z)), as_bf2(z));
+    const uint32_t delz = scale_pair(as_u32(__hadd2_rn(d, d)), p.rn);  // 2 d, exact
+    const uint32_t inner = as_u32(__hmul2_rn(as_bf2(delz), g));
+    const uint32_t low = lo & ~hi;
+    ga = __fadd2_rn(ga, widen2((gw & hi) | ((gw ^ 0x80008000u) & low) | (inner & in)));
+    return gw & in;
+  }
+  const uint32_t z = VARIANT == QLIN_PACT_TWO_SIDED ? scale_pair(as_u32(__hsub2_rn(x, p.cvn)), p.rstep) : scale_pair(xw, p.rstep);
+  const uint32_t delz = scale_pair(as_u32(__hsub2_rn(as_bf2(z), as_bf2(rint_pair(z)))), p.rn);
+  const uint32_t inner = as_u32(__hmul2_rn(as_bf2(gw ^ 0x80008000u), as_bf2(delz)));
+  ga = __fadd2_rn(ga, widen2((gw & hi) | (inner & in)));
+  if (VARIANT == QLIN_PACT_TWO_SIDED) gan = __fadd2_rn(gan, widen2((gw & lo) | ((inner ^ 0x80008000u) & in)));
+  return gw & in;
+}
+
+__device__ __forceinline__ void load_words(const __nv_bfloat16* p, uint32_t (&w)[8]) {
+  const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+  w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+}
+__device__ __forceinline__ void store_words(__nv_bfloat16* p, const uint32_t (&w)[8]) {
+  reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+template <int VARIANT>
+__global__ void __launch_bounds__(kFqThreads) pact2_fwd_bf16_kernel(const PactParams p) {
+  const PactScalars s = pact_scalars<__nv_bfloat16>(p);
+  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(p.x);
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
+  const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 && s.rstep == s.rstep;
+  const int64_t nvec = vec ? (p.numel >> 4) : 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const PactPair pp = pact_pair(s);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec; i += stride) {
+    uint32_t w[8];
+    load_words(x + i * 16, w);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = pact_fwd_pair<VARIANT>(pp, w[j]);
+    store_words(out + i * 16, w);
+  }
+  for (int64_t i = nvec * 16 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.numel; i += stride)
+    store1(out + i, pact_fwd_one<__nv_bfloat16>(s, load1(x + i)));
+}
+
+template <int VARIANT>
+__global__ void __launch_bounds__(kFqThreads) pact2_bwd_bf16_kernel(const PactParams p) {
+  __shared__ float red[2][32];
+  const PactScalars s = pact_scalars<__nv_bfloat16>(p);
+  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(p.x);
+  const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(p.g);
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
+  const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 && s.rstep == s.rstep;
+  const int64_t nvec = vec ? (p.numel >> 4) : 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const PactPair pp = pact_pair(s);
+  float2 ga2 = make_float2(0.0f, 0.0f), gan2 = make_float2(0.0f, 0.0f);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec; i += stride) {
+    uint32_t w[8], gw[8];
+    load_words(x + i * 16, w);
+    load_words(g + i * 16, gw);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = pact_bwd_pair<VARIANT>(pp, w[j], gw[j], ga2, gan2);
+    store_words(out + i * 16, w);
+  }
+  float ga = ga2.x + ga2.y, gan = gan2.x + gan2.y;
+  for (int64_t i = nvec * 16 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.numel; i += stride)
+    store1(out + i, pact_bwd_one<__nv_bfloat16>(s, load1(x + i), load1(g + i), ga, gan));
+  ga = block_reduce<OpSum>(ga, red[0], 0.0f);
+  gan = block_reduce<OpSum>(gan, red[1], 0.0f);
+  if (threadIdx.x == 0) {
+    p.ws[2 * blockIdx.x] = ga;
+    p.ws[2 * blockIdx.x + 1] = gan;
+  }
+}
+
+static void launch_fwd_bf16(const PactParams& p, int grid, cudaStream_t s) {
+  if (p.num_bits > 8) {
+    pact2_fwd_kernel<__nv_bfloat16><<<grid, kFqThreads, 0, s>>>(p);
+  } else if (p.variant == QLIN_PACT_TWO_SIDED) {
+    pact2_fwd_bf16_kernel<QLIN_PACT_TWO_SIDED><<<grid, kFqThreads, 0, s>>>(p);
+  } else if (p.variant == QLIN_PACT_ONE_SIDED) {
+    pact2_fwd_bf16_kernel<QLIN_PACT_ONE_SIDED><<<grid, kFqThreads, 0, s>>>(p);
+  } else {
+    pact2_fwd_bf16_kernel<QLIN_PACT_SYMMETRIC><<<grid, kFqThreads, 0, s>>>(p);
+  }
+}
+static void launch_bwd_bf16(const PactParams& p, int grid, cudaStream_t s) {
+  if (p.num_bits > 8) {
+    pact2_bwd_kernel<__nv_bfloat16><<<grid, kFqThreads, 0, s>>>(p);
+  } else if (p.variant == QLIN_PACT_TWO_SIDED) {
+    pact2_bwd_bf16_kernel<QLIN_PACT_TWO_SIDED><<<grid, kFqThreads, 0, s>>>(p);
+  } else if (p.variant == QLIN_PACT_ONE_SIDED) {
+    pact2_bwd_bf16_kernel<QLIN_PACT_ONE_SIDED><<<grid, kFqThreads, 0, s>>>(p);
+  } else {
+    pact2_bwd_bf16_kernel<QLIN_PACT_SYMMETRIC><<<grid, kFqThreads, 0, s>>>(p);
+  }
+}
+
 // Adds the per-block partial sums in index order.
 __global__ void __launch_bounds__(kFqThreads) pact2_bwd_finish_kernel(const float* ws, int nblocks, float* grad_clip) {
   __shared__ float red[2][32];
@@ -255,7 +420,7 @@ extern "C" int qlin_pact2_fwd(const qlin_pact2_args* a, void* stream) {
       pact2_fwd_kernel<__half><<<grid, kFqThreads, 0, s>>>(p);
       break;
     default:
-      pact2_fwd_kernel<__nv_bfloat16><<<grid, kFqThreads, 0, s>>>(p);
+      launch_fwd_bf16(p, grid, s);
       break;
   }
   QLIN_CHECK_LAUNCH("qlin_pact2_fwd");
@@ -277,7 +442,7 @@ extern "C" int qlin_pact2_bwd(const qlin_pact2_args* a, void* stream) {
         pact2_bwd_kernel<__half><<<grid, kFqThreads, 0, s>>>(p);
         break;
       default:
-        pact2_bwd_kernel<__nv_bfloat16><<<grid, kFqThreads, 0, s>>>(p);
+        launch_bwd_bf16(p, grid, s);
         break;
     }
     QLIN_CHECK_LAUNCH("qlin_pact2_bwd");
@@ -359,7 +524,7 @@ extern "C" int qlin_pact2_bwd_noalloc(const qlin_pact2_args* a, void* stream) {
         pact2_bwd_kernel<__half><<<grid, kFqThreads, 0, s>>>(p);
         break;
       default:
-        pact2_bwd_kernel<__nv_bfloat16><<<grid, kFqThreads, 0, s>>>(p);
+        launch_bwd_bf16(p, grid, s);
         break;
     }
     QLIN_CHECK_LAUNCH("qlin_pact2_bwd_noalloc");
