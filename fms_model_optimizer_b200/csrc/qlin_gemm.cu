@@ -5,10 +5,10 @@
 // Both operands are K-major ("NT"), which is the layout the reference hands to its Triton / CUTLASS
 // kernels (activations [m,k]; weight [n,k] passed as its .t() view).
 //
-// Per CTA (one per SM, 320 or 576 threads):
+// Per CTA (one per SM, 320 or 640 threads):
 //   warp E      TMA producer (E = number of epilogue warps: 8 unchunked, 16 chunked): 128-byte-swizzled [128 x 128B] A tile and [BN x 128B] B tile per stage
 //   warp E+1    MMA issuer: tcgen05.mma.cta_group::1 (M=128, N=BN, K=32 bytes per instruction),
-//               accumulators in tensor memory; owns the TMEM allocation
+//               accumulators in tensor memory; owns the TMEM allocation (chunked: three issuers, see MMA_WARPS)
 //   warps 0..E-1 epilogue: tcgen05.ld of the accumulator, chunk rounding / running sum, dequantise,
 //               global stores.  Warp w reads TMEM lanes 32*(w%4).. and column half w/4.
 // Unchunked: BN=256, two 256-column accumulators so the epilogue of tile i overlaps the mainloop of
