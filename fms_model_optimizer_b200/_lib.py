@@ -50,12 +50,6 @@ EXPORTED_SYMBOLS = (
     "qlin_f8_tensor_colsum_workspace_bytes",
     "qlin_absmax_parts",
     "qlin_absmax_parts_count",
-    "qlin_fq_codes",
-    "qlin_fq_fold",
-    "qlin_fq_row_planes",
-    "qlin_fq_col_planes",
-    "qlin_fq_col_workspace_bytes",
-    "qlin_fq_combine",
     "qlin_pact2_fwd",
     "qlin_pact2_bwd",
     "qlin_pact2_bwd_workspace_bytes",

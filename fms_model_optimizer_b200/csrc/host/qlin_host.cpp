@@ -512,108 +512,6 @@ std::tuple<OptTensor, OptTensor, Tensor> weight_fq_perch(const Tensor& w_in, int
   return {opt(dq), opt(codes), clip_io};
 }
 
-// ------------------------------------------------------------------------------------------------ fake-quantised product
-int64_t up16(int64_t v) { return (v + 15) / 16 * 16; }
-
-Tensor int_gemm(const Tensor& a, const Tensor& b) {
-  const Chain raw{0, 0, 32, 1, 0, QLIN_EPI_RAW, 0, 0, 0, 0};
-  return gemm_impl(a, b, std::nullopt, std::nullopt, raw, std::nullopt, std::nullopt, std::nullopt, nullptr, 0, QLIN_DT_NONE);
-}
-
-// F.linear(x, w, bias) for fake-quantised fp32 x [M, K] and w [N, K].  Returns the output and what the backward pass needs:
-// the codes of x and of w transposed, the weight scales and {step, z + h}.
-std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> fq_linear_fwd(const Tensor& x_in, const Tensor& w_in, const OptTensor& bias_in, const Tensor& clip_val,
-                                                                 const OptTensor& clip_valn, int num_bits, bool align_zero, int variant, const Tensor& w_clip,
-                                                                 int w_bits) {
-  const at::Device dev = require_cuda({&x_in, &w_in, ptr_of(bias_in), &clip_val, ptr_of(clip_valn), &w_clip});
-  const c10::cuda::CUDAGuard guard(dev);
-  void* const st = stream_of(dev);
-  const Tensor x = x_in.detach().contiguous(), w = w_in.detach().contiguous();
-  const Tensor bias = bias_in ? bias_in->detach().contiguous() : Tensor();
-  const Tensor cv = clip_f32(clip_val, dev), cvn = clip_valn ? clip_f32(*clip_valn, dev) : Tensor();
-  const Tensor wc = f32(w_clip.detach());
-  if (x.dim() != 2 || w.dim() != 2 || x.size(1) != w.size(1) || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || wc.numel() != w.size(0))
-    raise("fq_linear takes fp32 x [M, K], w [N, K] and one clip value per row of w");
-  const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-  const Tensor xq = empty({M, K}, at::kChar, dev), wq = empty({N, K}, at::kChar, dev);
-  const Tensor x_t = empty({K, up16(M)}, at::kChar, dev).narrow(1, 0, M), w_t = empty({K, up16(N)}, at::kChar, dev).narrow(1, 0, N);
-  qlin_fq_codes_args c = {};
-  c.act.clip_val = static_cast<const float*>(data(cv));
-  c.act.clip_valn = static_cast<const float*>(data(cvn));
-  c.act.num_bits = num_bits;
-  c.act.align_zero = align_zero;
-  c.act.variant = variant;
-  c.w_bits = w_bits;
-  c.v = static_cast<const float*>(data(x));
-  c.codes = data(xq);
-  c.codes_t = data(x_t);
-  c.ldt = x_t.stride(0);
-  c.rows = static_cast<int32_t>(M);
-  c.cols = static_cast<int32_t>(K);
-  check(qlin_fq_codes(&c, st), "qlin_fq_codes");
-  c.w_clip = static_cast<const float*>(data(wc));
-  c.v = static_cast<const float*>(data(w));
-  c.codes = data(wq);
-  c.codes_t = data(w_t);
-  c.ldt = w_t.stride(0);
-  c.rows = static_cast<int32_t>(N);
-  check(qlin_fq_codes(&c, st), "qlin_fq_codes");
-  const Tensor ws = empty({N}, at::kFloat, dev), folded = empty({N}, at::kFloat, dev), step = empty({1}, at::kFloat, dev);
-  const Tensor scal = empty({2}, at::kDouble, dev);
-  check(qlin_fq_fold(static_cast<const int8_t*>(data(wq)), static_cast<int32_t>(N), static_cast<int32_t>(K), &c.act, c.w_clip, w_bits,
-                     static_cast<const float*>(data(bias)), static_cast<float*>(data(ws)), static_cast<float*>(data(folded)),
-                     static_cast<float*>(data(step)), static_cast<double*>(data(scal)), st),
-        "qlin_fq_fold");
-  const Chain seq{0, 0, 32, 1, 0, QLIN_EPI_SCALE_SEQ, 0, 0, 0, 0};
-  Tensor out = gemm_impl(xq, wq, std::nullopt, std::nullopt, seq, step, ws, folded, nullptr, 0, QLIN_DT_F32);
-  return {out, x_t, w_t, ws, scal};
-}
-
-// Gradients of fq_linear_fwd for g [M, N]: with respect to x (g . w), to w (g^T . x) and to the bias (column sums).
-std::tuple<OptTensor, OptTensor, OptTensor> fq_linear_bwd(const Tensor& g_in, const Tensor& x_t, const Tensor& w_t, const Tensor& ws, const Tensor& scal,
-                                                          bool want_x, bool want_w, bool want_b) {
-  const at::Device dev = require_cuda({&g_in, &x_t, &w_t, &ws, &scal});
-  const c10::cuda::CUDAGuard guard(dev);
-  void* const st = stream_of(dev);
-  const Tensor g = g_in.detach().contiguous();
-  const int64_t M = g.size(0), N = g.size(1), K = x_t.size(0);
-  const float* gp = static_cast<const float*>(data(g));
-  Tensor gx, gw, gb;
-  if (want_x) {
-    const Tensor planes = empty({4 * M, N}, at::kChar, dev), back = empty({M}, at::kDouble, dev);
-    check(qlin_fq_row_planes(gp, static_cast<const float*>(data(ws)), static_cast<int32_t>(M), static_cast<int32_t>(N), data(planes),
-                             static_cast<double*>(data(back)), st),
-          "qlin_fq_row_planes");
-    const Tensor acc = int_gemm(planes, w_t);
-    gx = empty({M, K}, at::kFloat, dev);
-    check(qlin_fq_combine(static_cast<const int32_t*>(data(acc)), static_cast<int32_t>(M), static_cast<int32_t>(K), static_cast<const double*>(data(back)),
-                          nullptr, nullptr, static_cast<float*>(data(gx)), st),
-          "qlin_fq_combine");
-  }
-  if (want_w || want_b) {
-    const int32_t m = static_cast<int32_t>(M), n = static_cast<int32_t>(N);
-    const int64_t ldt = up16(M);
-    const Tensor wsp = empty({qlin_fq_col_workspace_bytes(m, n)}, at::kByte, dev), sum = empty({N}, at::kDouble, dev);
-    Tensor planes, back;
-    if (want_w) {
-      planes = empty({4 * N, ldt}, at::kChar, dev);
-      back = empty({N}, at::kDouble, dev);
-    }
-    if (want_b) gb = empty({N}, at::kFloat, dev);
-    check(qlin_fq_col_planes(gp, m, n, data(wsp), data(planes), ldt, static_cast<double*>(data(back)), static_cast<double*>(data(sum)),
-                             static_cast<float*>(data(gb)), st),
-          "qlin_fq_col_planes");
-    if (want_w) {
-      const Tensor acc = int_gemm(planes.narrow(1, 0, M), x_t);
-      gw = empty({N, K}, at::kFloat, dev);
-      check(qlin_fq_combine(static_cast<const int32_t*>(data(acc)), n, static_cast<int32_t>(K), static_cast<const double*>(data(back)),
-                            static_cast<const double*>(data(sum)), static_cast<const double*>(data(scal)), static_cast<float*>(data(gw)), st),
-            "qlin_fq_combine");
-    }
-  }
-  return {opt(gx), opt(gw), opt(gb)};
-}
-
 }  // namespace
 
 PYBIND11_MODULE(_qlin_host, m) {
@@ -625,8 +523,6 @@ PYBIND11_MODULE(_qlin_host, m) {
   m.def("absmax_parts", &absmax_parts, rel());
   m.def("f8_tensor_quant", &f8_tensor_quant, rel());
   m.def("weight_fq_perch", &weight_fq_perch, rel());
-  m.def("fq_linear_fwd", &fq_linear_fwd, rel());
-  m.def("fq_linear_bwd", &fq_linear_bwd, rel());
   m.def("pact2_fwd", &pact2_fwd, rel());
   m.def("pact2_bwd", &pact2_bwd, rel());
 }

@@ -17,7 +17,7 @@ from torch import nn
 
 from .. import _lib as L
 from .. import ops
-from ..quant.quantizers import PACT, PACT2, SAWB, PACTplusSym, get_activation_quantizer, get_weight_quantizer
+from ..quant.quantizers import get_activation_quantizer, get_weight_quantizer
 
 _FLOATS = (torch.float32, torch.float16, torch.bfloat16)
 
@@ -587,55 +587,11 @@ class QLinearINT8Train(nn.Linear):
         return s
 
 
-class _FakeQuantMatmul(torch.autograd.Function):
-    """``F.linear`` of a fake-quantised activation and a fake-quantised weight through their codes (``ops.fq_linear_fwd`` /
-    ``fq_linear_bwd``).  The gradients are those of ``F.linear``; a backward pass that is itself differentiated runs as PyTorch
-    operations on the saved operands."""
-
-    @staticmethod
-    def forward(ctx, qinput, qweight, bias, act, w_clip, w_bits):
-        x2 = qinput.reshape(-1, qinput.shape[-1])
-        out, *saved = ops.fq_linear_fwd(x2, qweight, bias, *act, w_clip, w_bits)
-        ctx.save_for_backward(qinput, qweight, *saved)
-        return out.reshape(*qinput.shape[:-1], qweight.shape[0])
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        qinput, qweight, *saved = ctx.saved_tensors
-        need_x, need_w, need_b = ctx.needs_input_grad[:3]
-        g2 = grad_output.reshape(-1, qweight.shape[0])
-        if torch.is_grad_enabled():
-            gx = grad_output.matmul(qweight) if need_x else None
-            gw = g2.t().matmul(qinput.reshape(-1, qinput.shape[-1])) if need_w else None
-            return gx, gw, (g2.sum(0) if need_b else None), None, None, None
-        gx, gw, gb = ops.fq_linear_bwd(g2, saved, need_x, need_w, need_b)
-        return (gx.reshape(qinput.shape) if need_x else None), gw, gb, None, None, None
-
-
-def _has_hooks(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks)
-
-
-def _pact_args(q: nn.Module):
-    """``(clip_val, clip_valn, num_bits, align_zero, variant)`` of a PACT+ quantizer whose outputs are whole numbers times a step, else None."""
-    if type(q) is PACT2:
-        args = (q.clip_val, q.clip_valn, q.num_bits, bool(q.align_zero), L.PACT_TWO_SIDED)
-    elif type(q) is PACT:
-        args = (q.clip_val, None, q.num_bits, False, L.PACT_ONE_SIDED)
-    elif type(q) is PACTplusSym:
-        args = (q.clip_val, None, q.num_bits, bool(q.intg_zp), L.PACT_SYMMETRIC)
-    else:
-        return None
-    clips = [t for t in args[:2] if t is not None]
-    return args if 2 <= args[2] <= 8 and all(t.numel() == 1 and t.is_cuda and t.dtype == torch.float32 for t in clips) else None
-
-
 class QLinear(nn.Linear):
     """Fake-quant Linear for QAT / DQ (fms_mo/modules/linear.py:51-393, forward :248-305):
     ``F.linear(Qa(x / s), Qw(W * s), bias)`` with the SmoothQuant scale ``s`` of :345-368.  The two
-    quantizers run as single CUDA kernels (forward and backward).  The matmul is a plain library GEMM, as in the
-    reference, except for large fp32 products of PACT+ activations and per-channel SAWB+ weights, which run on their
-    integer codes (``_codes_route``)."""
+    quantizers run as single CUDA kernels (forward and backward); the matmul itself stays a plain
+    library GEMM, as in the reference."""
 
     def __init__(self, in_features, out_features, bias=True, num_bits_feature=32, qa_mode=None, num_bits_weight=32,
                  qw_mode=None, **kwargs):  # fmt: skip
@@ -695,45 +651,9 @@ class QLinear(nn.Linear):
         else:  # the reference divides and multiplies by a tensor holding 1.0 here: the identity, bit for bit
             qinput = self.quantize_feature(x).to(x.dtype)
             qweight = self.quantize_weight(self.weight).to(self.weight.dtype)
-        act = self._codes_route(qinput, qweight)
-        if act is not None:
-            output = _FakeQuantMatmul.apply(qinput, qweight, self.bias, act, self.quantize_weight.clip_val.detach().clone(), self.quantize_weight.num_bits)
-        else:
-            output = nn.functional.linear(qinput, qweight, self.bias)
+        output = nn.functional.linear(qinput, qweight, self.bias)
         self.num_module_called += 1
         return output
-
-    def _codes_route(self, qinput, qweight):
-        """The activation quantizer's arguments when ``qinput`` and ``qweight`` are known to be integer codes times scales and the
-        product is worth a dozen launches, else None.
-
-        fp32 only: a 16-bit library GEMM is as fast.  The quantizers must be exactly the PACT+ and per-channel SAWB+ modules,
-        without hooks that could change what they return.  Settings under which ``F.linear`` would do something else
-        (autocast, TF32, functional transforms, forward-mode differentiation, tracing) keep it.  Below ``_FQ_MIN_MACS`` multiply-adds the
-        launches cost as much as the library GEMM or more.  Codes against library, forward / forward + backward, us: at 1.2e9
-        (2048 x 768 x 768) 122 : 82 / 348 : 272, at 2.4e9 (4096 x 768 x 768) 128 : 138 / 363 : 383, at 4.8e9 (2048 x 3072 x 768)
-        122 : 239 / 348 : 631, at 9.7e9 (4096 x 768 x 3072) 122 : 401 / 346 : 1139.  The gradient's four byte planes, twice, stay below 1 GB, and the int32 sums of a
-        plane below 2^30."""
-        Qa, Qw = self.quantize_feature, self.quantize_weight
-        n, k = self.weight.shape
-        m = qinput.numel() // k
-        if not (qinput.is_cuda and qinput.dtype == qweight.dtype == torch.float32 and (self.bias is None or self.bias.dtype == torch.float32)):
-            return None
-        if k % 16 != 0 or n % 16 != 0 or m * n * k < _FQ_MIN_MACS or m * n > 1 << 27 or max(m, n, k) > 65536:
-            return None
-        if type(Qw) is not SAWB or not Qw.perCh or not Qw.dequantize or Qw.clip_val.dtype != torch.float32 or _has_hooks(Qa) or _has_hooks(Qw):
-            return None
-        if torch.is_autocast_enabled("cuda") or torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
-            return None
-        if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
-            return None
-        if torch.jit.is_tracing() or torch.compiler.is_compiling():
-            return None
-        return _pact_args(Qa)
-
-
-# multiply-adds from which the codes' product beats the fp32 library GEMM, forward alone and with its gradients
-_FQ_MIN_MACS = 1 << 32
 
 
 def lower_qmodel_b200(model: nn.Module, use_dyn_max_act=False, max_acc_bits=32, clamp_acc_to_dl16=False,

@@ -495,26 +495,6 @@ def pact2_bwd(
 
 
 # --------------------------------------------------------------------------------------------------
-# Product of a fake-quantised activation and a fake-quantised weight (qlin_fq_*, include/qlin_b200.h)
-# --------------------------------------------------------------------------------------------------
-def fq_linear_fwd(x2, w, bias, clip_val, clip_valn, num_bits: int, align_zero: bool, variant: int, w_clip, w_bits: int):
-    """``F.linear(x2, w, bias)`` for fp32 ``x2 [M, K]`` from a PACT+ quantiser with these clip values and ``w [N, K]`` from the per-channel SAWB+
-    quantiser with clip values ``w_clip [N]``, as one int8 GEMM.  Returns ``(out, *saved)``; ``fq_linear_bwd`` takes ``saved``."""
-    global LAUNCHES
-    LAUNCHES += 3
-    return _call("fq_linear_fwd", 2.0 * x2.numel() * w.shape[0], x2.device, L.host().fq_linear_fwd, x2, w, bias, clip_val, clip_valn, int(num_bits),
-                 bool(align_zero), int(variant), w_clip, int(w_bits))  # fmt: skip
-
-
-def fq_linear_bwd(g2, saved, want_x: bool, want_w: bool, want_b: bool):
-    """Gradients ``(gx [M, K], gw [N, K], gb [N])`` of ``fq_linear_fwd`` for ``g2 [M, N]`` fp32 (None where not wanted)."""
-    global LAUNCHES
-    LAUNCHES += 3 * bool(want_x) + 2 * bool(want_w or want_b) + 3 * bool(want_w) - 1
-    return _call("fq_linear_bwd", 2.0 * g2.numel() * saved[0].shape[0] * (bool(want_x) + bool(want_w)), g2.device, L.host().fq_linear_bwd, g2, *saved,
-                 bool(want_x), bool(want_w), bool(want_b))  # fmt: skip
-
-
-# --------------------------------------------------------------------------------------------------
 # Decoder-block fusions: (residual add +) RMSNorm / SiLU * up, then per-token quantisation for up to
 # three Linears that share the input; rotary embedding.
 # --------------------------------------------------------------------------------------------------

@@ -359,55 +359,6 @@ int qlin_pact2_bwd_noalloc(const qlin_pact2_args* args, void* stream);
 int64_t qlin_pact2_bwd_noalloc_max_numel(void);
 
 /* ------------------------------------------------------------------------------------------------
- * qlin_fq_* -- the pieces around the int8 GEMMs that multiply a fake-quantised activation with a fake-quantised weight.
- *
- * Stands in for: F.linear(qinput, qweight, bias) of QLinear.forward (fms_mo/modules/linear.py:248-305) and its gradients, for
- * fp32 tensors that a PACT+ quantiser of at most 8 bits (qlin_pact2_fwd) and the per-channel SAWB+ quantiser
- * (qlin_weight_fq_perch) produced.  With value = (q + z) * step, weight = c * w_scale[n] and
- * h = 2^(num_bits - 1):
- *   qlin_fq_codes       codes[r,c] = q - h (act) or c (w_clip: [rows] fp32, scale = clip * 2 / (2^w_bits - 2)) and the same
- *                       transposed with ldt bytes between rows (a multiple of 16; zeros beyond `rows`)
- *   qlin_fq_fold        w_scale [n]; bias_out[n] = bias[n] + step * w_scale[n] * (z + h) * sum_k c[n,k] (bias may be NULL);
- *                       step_out [1] fp32 (NaN where step is 0 or not finite); scal[2] = {step, z + h} fp64
- *   qlin_fq_row_planes  planes[4][rows][cols]: the signed bytes, lowest first, of rint(g[m,n] * w_scale[n] * 2^e_m) with the
- *                       largest |value| of a row in [2^29, 2^30); back[m] = 2^-e_m, NaN for a row with an infinity or NaN
- *   qlin_fq_col_planes  planes[4][cols][ldt] the same of g transposed (no w_scale), one exponent per column; colsum [cols] fp64 sums
- *                       over the rows, grad_bias (optional) the same in fp32; planes may be NULL; workspace of
- *                       qlin_fq_col_workspace_bytes(rows, cols) bytes
- *   qlin_fq_combine     out[r,c] = ((sum_b 2^(8b) acc[b][r][c]) * back[r] + add[r] * scal[1]) * scal[0], formed in fp64;
- *                       without scal the factor is 1, without add the addend 0
- * cols are multiples of 16; buffers are dense and 16-byte aligned.
- * ---------------------------------------------------------------------------------------------- */
-typedef struct qlin_fq_act {
-  const float* clip_val;  /* [1] fp32 */
-  const float* clip_valn; /* [1] fp32, two-sided only */
-  int32_t num_bits;
-  int32_t align_zero;
-  int32_t variant;        /* qlin_pact_variant */
-} qlin_fq_act;
-
-typedef struct qlin_fq_codes_args {
-  const float* v;
-  const float* w_clip;    /* weights: [rows]; NULL for activations */
-  void* codes;
-  void* codes_t;
-  int64_t ldt;
-  int32_t rows, cols;
-  int32_t w_bits;
-  qlin_fq_act act;
-} qlin_fq_codes_args;
-
-int qlin_fq_codes(const qlin_fq_codes_args* args, void* stream);
-int qlin_fq_fold(const int8_t* codes, int32_t n, int32_t k, const qlin_fq_act* act, const float* w_clip, int32_t w_bits, const float* bias,
-                 float* w_scale, float* bias_out, float* step_out, double* scal, void* stream);
-int qlin_fq_row_planes(const float* g, const float* w_scale, int32_t rows, int32_t cols, void* planes, double* back, void* stream);
-int qlin_fq_col_planes(const float* g, int32_t rows, int32_t cols, void* workspace, void* planes, int64_t ldt, double* back, double* colsum,
-                       float* grad_bias, void* stream);
-int64_t qlin_fq_col_workspace_bytes(int32_t rows, int32_t cols);
-int qlin_fq_combine(const int32_t* acc, int32_t rows, int32_t cols, const double* back, const double* add, const double* scal, float* out,
-                    void* stream);
-
-/* ------------------------------------------------------------------------------------------------
  * qlin_weight_fq_perch -- per-output-channel symmetric weight fake quantisation with the
  * clip value computed in the same pass.
  *
