@@ -482,7 +482,7 @@ std::tuple<OptTensor, OptTensor, Tensor> weight_fq_perch(const Tensor& w_in, int
   Tensor clip_io;
   if (mode == QLIN_W_GIVEN) {
     if (!clip || clip->numel() != rows) raise("W_GIVEN needs one clip value per row");
-    clip_io = f32(clip->detach()).clone();
+    clip_io = f32(clip->detach().reshape({-1})).clone();
   } else {
     clip_io = empty({rows}, at::kFloat, dev);
   }
