@@ -385,6 +385,8 @@ def quant_gemm(
     """``act_quant`` of the rows of ``x [.., K]`` followed by ``gemm`` with ``weight [N, K]``, in one call: the forward pass of a
     deploy-time Linear.  ``row_scale`` defaults to the scales the quantiser found; the other arguments are theirs."""
     global LAUNCHES
+    if x.dtype not in (torch.float32, torch.float16, torch.bfloat16):  # before anything is looked up for the GEMM
+        raise RuntimeError(f"unsupported activation dtype {x.dtype}")
     if smooth is not None and smooth_rcp is None:
         smooth_rcp = smooth_reciprocal(_f32(smooth))
     if PROFILE is None and not NVTX:
