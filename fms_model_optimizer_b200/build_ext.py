@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -41,8 +42,6 @@ HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared"]
 
 def _build_host() -> None:
     """g++ for the host code: PyTorch's headers and libraries, libqlin_b200.so beside it at run time."""
-    import sysconfig
-
     import torch
 
     root = Path(torch.__file__).resolve().parent
@@ -77,13 +76,21 @@ def _sources() -> list[Path]:
 STAMP_PATH = LIB_DIR / "libqlin_b200.stamp"
 
 
+def _host_environment() -> list[str]:
+    """What the host library's binary interface depends on besides its source: PyTorch, its CUDA and C++ ABI, Python."""
+    import torch
+
+    return [str(v) for v in (torch.__version__, torch.version.cuda, torch._C._GLIBCXX_USE_CXX11_ABI, sysconfig.get_config_var("SOABI"))]
+
+
 def source_digest(extra_flags: tuple = ()) -> str:
-    """SHA-256 over the compiler flags and the name and content of every file the library is built from.  File times
-    say nothing after a checkout or a copy to another machine, so staleness is decided by content."""
+    """SHA-256 over the compiler flags, the name and content of every file the libraries are built from and the environment of
+    the host library.  File times say nothing after a checkout or a copy to another machine, so staleness is decided by
+    content."""
     files = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")))
     files += [PKG_DIR.parent / "include" / "qlin_b200.h", HOST_SRC]
     h = hashlib.sha256()
-    h.update("\0".join([*NVCC_FLAGS, *HOST_FLAGS, *extra_flags]).encode())
+    h.update("\0".join([*NVCC_FLAGS, *HOST_FLAGS, *_host_environment(), *extra_flags]).encode())
     for f in files:
         h.update(f.name.encode() + b"\0")
         h.update(f.read_bytes())
