@@ -284,6 +284,12 @@ __global__ void __launch_bounds__(1024) act_quant_vec_kernel(const QuantParams p
   griddep_launch();
 }
 
+// Waits for a ring slot whose bytes every lane reads next: lane 0 polls, the warp barrier orders the other lanes' reads behind it.
+__device__ __forceinline__ bool ring_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const bool ok = warp_mbar_wait(bar, parity, abort_flag);
+  __syncwarp();
+  return ok;
+}
 
 // ------------------------------------------------------------------------------------------------
 // Specialised fast path of the dynamic quantisers (the per-token int8 / e4m3 quantise of the deploy
@@ -375,7 +381,7 @@ __global__ void __launch_bounds__(TPB) act_quant_fast_kernel(const QuantParams p
   for (int i = 0; i < my_rows; ++i) {
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
-    const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    const bool ok = ring_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
     if (i == my_rows - 1) griddep_launch();  // this block has read all it will read
     const XT* xr = reinterpret_cast<const XT*>(ring + static_cast<size_t>(slot) * row_bytes);
     float v[MAXC][16];
@@ -596,7 +602,7 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
   for (int i = 0; i < my_rows; ++i) {
     const int slot = i % stages;
     const int row = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
-    const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    const bool ok = ring_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
     if (i == my_rows - 1) griddep_launch();  // this block has read all it will read
     const uint4* xr = reinterpret_cast<const uint4*>(ring + static_cast<size_t>(slot) * row_bytes);
     uint32_t vp[MAXC][8];
@@ -764,7 +770,7 @@ __global__ void __launch_bounds__(256) act_quant_bf16_rows_kernel(const QuantPar
     const int slot = i % stages;
     const int row0 = (static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)) * kRows4;
     const int n = min(kRows4, p.rows - row0);
-    const bool ok = warp_mbar_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
+    const bool ok = ring_wait(&full[slot], static_cast<uint32_t>((i / stages) & 1), &abort_flag);
     if (i == my_groups - 1) griddep_launch();  // this block has read all it will read
     uint32_t v[kRows4][8];
     uint32_t am[kRows4];
