@@ -298,6 +298,7 @@ void act_quant_impl(const Tensor& x_in, const QuantOpts& o, const OptTensor& smo
   q.codes = data(codes);
   q.scale_out = static_cast<float*>(data(scale));
   q.dq_out = data(dq);
+  q.status = static_cast<int32_t*>(status_word(dev.index()).data_ptr());
   q.ldx = x.stride(0);
   q.ldq = ldq;
   q.lddq = cols;

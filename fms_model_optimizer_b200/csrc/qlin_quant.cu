@@ -290,6 +290,12 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, uint32_t parity, volati
   __syncwarp();
   return ok;
 }
+// After a wait that ran out (thread 0): sets the status word and waits, with a limit, for the copies still in flight into the slots of
+// iterations i .. i + stages - 1, so that none lands in shared memory that is no longer this block's.
+__device__ __forceinline__ void ring_give_up(int32_t* status, uint64_t* full, int stages, int i, int n) {
+  if (status != nullptr) atomicExch(status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
+  for (int j = i; j < n && j < i + stages; ++j) mbar_wait_drain(&full[j % stages], static_cast<uint32_t>((j / stages) & 1));
+}
 
 // ------------------------------------------------------------------------------------------------
 // Specialised fast path of the dynamic quantisers (the per-token int8 / e4m3 quantise of the deploy
@@ -433,7 +439,7 @@ __global__ void __launch_bounds__(TPB) act_quant_fast_kernel(const QuantParams p
     bool any_bad;
     amax = block_reduce_flag<OpMax>(amax, red[i & 1], 0.0f, !ok, any_bad);
     if (any_bad) {
-      if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
+      if (threadIdx.x == 0) ring_give_up(p.status, full, stages, i, my_rows);
       break;
     }
     if (smooth_div && !(amax < 1e15f)) {
@@ -638,7 +644,7 @@ __global__ void __launch_bounds__(TPB) act_quant_bf16_kernel(const QuantParams p
     bool any_bad;
     amax = block_reduce_flag<OpMax>(amax, red[i & 1], 0.0f, !ok, any_bad);
     if (any_bad) {
-      if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
+      if (threadIdx.x == 0) ring_give_up(p.status, full, stages, i, my_rows);
       break;
     }
     if (threadIdx.x == 0 && i + stages < my_rows) issue(i + stages);
@@ -792,7 +798,7 @@ __global__ void __launch_bounds__(256) act_quant_bf16_rows_kernel(const QuantPar
     }
     if (lane == 0) red[i & 1][warp] = make_uint4(am[0], am[1], am[2], am[3]);
     if (__syncthreads_or(ok ? 0 : 1)) {
-      if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
+      if (threadIdx.x == 0) ring_give_up(p.status, full, stages, i, my_groups);
       break;
     }
     if (threadIdx.x == 0 && i + stages < my_groups) issue(i + stages);  // every slice of the slot is in registers

@@ -106,18 +106,18 @@ def _stream(dev: torch.device) -> C.c_void_p:
 
 
 def status_word(dev: torch.device) -> torch.Tensor:
-    """Per-device int32 status word handed to the GEMM; stays 0 unless a kernel gave up a wait."""
+    """Per-device int32 status word handed to the GEMM and the row quantiser; stays 0 unless a kernel gave up a wait."""
     return L.host().status_word(dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 def check_status(dev: Optional[torch.device] = None) -> None:
-    """Synchronises and raises if any GEMM on ``dev`` reported a timed-out wait."""
+    """Synchronises and raises if any GEMM or row quantiser on ``dev`` reported a timed-out wait."""
     dev = dev if dev is not None else torch.device("cuda", torch.cuda.current_device())
     word = status_word(dev)
     val = int(word.item())
     if val != 0:
         word.zero_()
-        raise RuntimeError(f"qlin_gemm reported device status {val} (a bounded wait ran out)")
+        raise RuntimeError(f"a kernel reported device status {val} (a bounded wait ran out)")
 
 
 def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -385,7 +385,7 @@ def quant_gemm(
     """``act_quant`` of the rows of ``x [.., K]`` followed by ``gemm`` with ``weight [N, K]``, in one call: the forward pass of a
     deploy-time Linear.  ``row_scale`` defaults to the scales the quantiser found; the other arguments are theirs."""
     global LAUNCHES
-    if x.dtype not in (torch.float32, torch.float16, torch.bfloat16):  # before anything is looked up for the GEMM
+    if x.dtype not in _ROUND:  # before anything is looked up for the GEMM
         raise RuntimeError(f"unsupported activation dtype {x.dtype}")
     if smooth is not None and smooth_rcp is None:
         smooth_rcp = smooth_reciprocal(_f32(smooth))
