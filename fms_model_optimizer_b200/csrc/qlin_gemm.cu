@@ -743,7 +743,8 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     };
     griddep_wait();  // the row scales may come from the launch before
     prefetch(blockIdx.x);
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+    int t = blockIdx.x;
+    for (; t < num_tiles && ok; t += gridDim.x) {
       int mb, nb;
       const int bi = BATCHED ? t / per_batch : 0;
       tile_coords(t - bi * per_batch, p.num_m, p.num_n, mb, nb);
@@ -874,6 +875,13 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       timed_out = !*abort_flag;
       *abort_flag = 1;
     }
+    // a warp that gave up still takes part in the barriers of the tiles that are left: another may have seen its accumulator
+    // complete a moment before the abort and be on its way to them
+    if (!ok && scaled)
+      for (t += gridDim.x; t < num_tiles; t += gridDim.x) {
+        asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
+      }
   }
 
   if (timed_out && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
@@ -1086,7 +1094,8 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     };
     griddep_wait();  // the row scales may come from the launch before
     prefetch(pair);
-    for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+    int t = pair;
+    for (; t < num_tiles && ok; t += num_pairs) {
       int mb, nb;
       tile_coords2(t, num_m2, p.num_n, mb, nb);
       const int row0 = mb * 2 * kBM + static_cast<int>(rank) * kBM + q * 32;
@@ -1137,6 +1146,13 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       timed_out = !*abort_flag;
       *abort_flag = 1;
     }
+    // a warp that gave up still takes part in the barriers of the tiles that are left: another may have seen its accumulator
+    // complete a moment before the abort and be on its way to them
+    if (!ok && scaled)
+      for (t += num_pairs; t < num_tiles; t += num_pairs) {
+        asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
+      }
   }
 
   if (timed_out && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_TIMEOUT));
