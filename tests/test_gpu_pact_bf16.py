@@ -2,9 +2,8 @@
 still takes): outputs and input gradients bit for bit over every bf16 number, NaN, infinities and subnormal numbers included,
 for all three quantisers, several widths and clip values (one of them with a step that takes the ordinary division).
 
-Clip gradients: both sides add the same terms in fp32 in another order; over n terms either sum is within n * 2^-24 * sum |term|
-of the exact one, which is asserted against the 64-bit sum of the terms the input gradients imply only through each
-other: |a - b| <= 2 n 2^-24 sum |g|."""
+Clip gradients: both sides add the same terms, each at most |g|, in fp32 in another order; either sum of n terms is within
+n * 2^-24 * sum |g| of the exact one, so they differ by at most twice that, which is asserted."""
 
 import pytest
 import torch
