@@ -51,15 +51,18 @@ struct Aux {
   float bias[256];
 };
 
-template <bool CHUNKED>
+// SHORT_K: the batched products of attention, whose tiles are a K block or two deep.  They are written as fast as the epilogue
+// goes: sixteen warps and three stages (64 x 2048 x 128 x 2048: 130 us with eight warps and four stages, 108 with sixteen).
+// The CTA-pair kernel, whose main loop counts, lost 3 to 7 % with sixteen warps and the five stages that they leave room for.
+template <bool CHUNKED, bool SHORT_K = false>
 struct Cfg {
   static constexpr int BN = CHUNKED ? 128 : 256;
   static constexpr int NBUF = CHUNKED ? 4 : 2;
-  static constexpr int STAGES = CHUNKED ? 5 : 4;
+  static constexpr int STAGES = CHUNKED ? 5 : (SHORT_K ? 3 : 4);
   // Epilogue warps: w % 4 selects the 32 TMEM lanes a warp may read, w / 4 its column slice.  The
   // chunked kernel drains an accumulator per K-chunk, a chain of short dependent steps, and hides
   // that latency with twice as many, narrower warps.
-  static constexpr int EPI_WARPS = CHUNKED ? 16 : 8;
+  static constexpr int EPI_WARPS = CHUNKED || SHORT_K ? 16 : 8;
   static constexpr int PRODUCER_WARP = EPI_WARPS;
   static constexpr int MMA_WARP = EPI_WARPS + 1;
   // Issuing the MMAs and the barrier traffic of one chunk takes a warp about 700 cycles, several times what the tensor pipe
@@ -100,6 +103,19 @@ struct GemmParams {
   int32_t low_byte_mode;  // chunked int8, 8 truncated bits: the total on the tensor core, the chunks' low bytes on the ALU
   int32_t sk_mt, sk_split, sk_stages;  // few-row kernel: padded row count, K splits (= cluster size), pipeline stages
   int32_t dependent;                   // launched as the dependent of the quantiser that writes A and the row scales
+  int32_t chain;                       // Chain of the epilogue (tiled stores)
+};
+
+// The epilogues that calls of this package ask for, compiled without a decision inside; any other combination of roundings
+// takes kChainAny, which decides per step of 16 columns.
+enum Chain : int32_t {
+  kChainAny = 0,
+  kChainRaw,         // accumulators as they are
+  kChainProdBf16,    // SCALE_PROD, product rounded to bf16 then fp16, result to fp16: the deployed Linear of a bf16 model
+  kChainProdF16,     // the same with the product rounded to fp16 once: fp16 and fp32 models
+  kChainSeqBf16,     // SCALE_SEQ with both steps rounded to bf16: the FP8 Linear of a bf16 model
+  kChainSeq,         // SCALE_SEQ without rounding steps
+  kChainAcc16Tensor  // SCALE_ACC16 with one scale per operand: the batched product of attention
 };
 
 __device__ __forceinline__ float round_to(float y, int dt) {
@@ -429,6 +445,202 @@ __device__ __forceinline__ void emit32(const GemmParams& p, const EpiCtx& e, uin
   }
 }
 
+// ---- the epilogue with tiled stores -------------------------------------------------------------------------------
+// A loop over steps of 16 accumulator columns: the next step's tcgen05.ld is in flight while this step's values are scaled,
+// rounded and packed; 64 bytes of every row (32 columns of a 2-byte type, 16 of a 4-byte type) make a piece of 32 rows,
+// written to one of this warp's two 2 KB buffers with the 64-byte swizzle and stored by one TMA instruction, which also cuts
+// off rows and columns beyond the output.  Bound by instruction issue and its latencies, not by stores: straight-line code over
+// 64 columns with staged 16-byte stores (emit64, still used for outputs TMA cannot address) took up to 1300 instructions a
+// warp and tile, fetched anew for every tile.  Kernel times before and after: attention scores 64 x 2048 x 128 x 2048 210 -> 108
+// us (537 MB written at 5.0 TB/s), 4096 x 768 x 3072 with fp32 output 25.5 -> 21.5, 517 x 4096 x 4096 fp16 20.5 -> 18.8.
+template <int N>
+__device__ __forceinline__ float2 pair_n(const uint32_t (&v)[N], int j) { return make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])); }
+template <int N>
+__device__ __forceinline__ void set_pair_n(uint32_t (&v)[N], int j, float2 t) {
+  v[2 * j] = __float_as_uint(t.x);
+  v[2 * j + 1] = __float_as_uint(t.y);
+}
+template <int DT>
+__device__ __forceinline__ void round16(uint32_t (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) set_pair_n(v, j, round2<DT>(pair_n(v, j)));
+}
+__device__ __forceinline__ void round16_if(uint32_t (&v)[16], int dt) {
+  if (dt == QLIN_DT_F16) {
+    round16<QLIN_DT_F16>(v);
+  } else if (dt == QLIN_DT_BF16) {
+    round16<QLIN_DT_BF16>(v);
+  }
+}
+template <int PROD, int SCALE>
+__device__ __forceinline__ void mul_prod16(uint32_t (&v)[16], float rs, const float* cs) {
+  const float2 rs2 = make_float2(rs, rs);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 sc = round2<SCALE>(round2<PROD>(__fmul2_rn(rs2, *reinterpret_cast<const float2*>(cs + 2 * j))));
+    set_pair_n(v, j, __fmul2_rn(pair_n(v, j), sc));
+  }
+}
+template <int PROD>
+__device__ __forceinline__ void mul_prod16_if(uint32_t (&v)[16], float rs, const float* cs, int scale_round) {
+  if (scale_round == QLIN_DT_F16) {
+    mul_prod16<PROD, QLIN_DT_F16>(v, rs, cs);
+  } else if (scale_round == QLIN_DT_BF16) {
+    mul_prod16<PROD, QLIN_DT_BF16>(v, rs, cs);
+  } else {
+    mul_prod16<PROD, QLIN_DT_F32>(v, rs, cs);
+  }
+}
+// Accumulators of 16 columns in, output values (fp32 bits, rounded the way the epilogue asks) out: dequant32, step by step.
+// `cst` is the one column scale of kChainAcc16Tensor.  A last rounding that packing to OUT repeats is left to it.
+template <bool F8, int CH, int OUT>
+__device__ __forceinline__ void dequant16(const GemmParams& p, uint32_t (&v)[16], float rs, float cst, const float* cs, const float* bias) {
+  if (CH == kChainRaw) return;
+  if (!F8) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__int2float_rn(static_cast<int32_t>(v[j])));
+  }
+  const float2 rs2 = make_float2(rs, rs);
+  if (CH == kChainProdBf16) {
+    mul_prod16<QLIN_DT_BF16, QLIN_DT_F16>(v, rs, cs);
+  } else if (CH == kChainProdF16) {
+    mul_prod16<QLIN_DT_F16, QLIN_DT_F32>(v, rs, cs);
+  } else if (CH == kChainAcc16Tensor) {
+    round16<QLIN_DT_F16>(v);
+    const float2 cs2 = make_float2(cst, cst);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) set_pair_n(v, j, __fmul2_rn(__fmul2_rn(pair_n(v, j), rs2), cs2));
+    return;
+  } else if (CH == kChainAny && p.epilogue == QLIN_EPI_SCALE_PROD) {
+    if (p.prod_round == QLIN_DT_BF16) {
+      mul_prod16_if<QLIN_DT_BF16>(v, rs, cs, p.scale_round);
+    } else if (p.prod_round == QLIN_DT_F16) {
+      mul_prod16_if<QLIN_DT_F16>(v, rs, cs, p.scale_round);
+    } else {
+      mul_prod16_if<QLIN_DT_F32>(v, rs, cs, p.scale_round);
+    }
+  } else {
+    if (CH == kChainAny && p.epilogue == QLIN_EPI_SCALE_ACC16) round16<QLIN_DT_F16>(v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) set_pair_n(v, j, __fmul2_rn(__fmul2_rn(pair_n(v, j), rs2), *reinterpret_cast<const float2*>(cs + 2 * j)));
+    if (CH == kChainSeqBf16) round16<QLIN_DT_BF16>(v);
+    if (CH == kChainAny) round16_if(v, p.mid_round);
+  }
+  if (p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) set_pair_n(v, j, __fadd2_rn(pair_n(v, j), *reinterpret_cast<const float2*>(bias + 2 * j)));
+  }
+  if ((CH == kChainProdBf16 || CH == kChainProdF16) && OUT != QLIN_DT_F16) round16<QLIN_DT_F16>(v);
+  if (CH == kChainSeqBf16 && OUT != QLIN_DT_BF16) round16<QLIN_DT_BF16>(v);
+  if (CH == kChainAny) round16_if(v, p.acc_round);
+}
+
+constexpr int kPieceBytes = 2048;  // 32 rows x 64 bytes
+__device__ __forceinline__ void piece_write(uint32_t sbase, int lane, int chunk, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+  const uint32_t addr = sbase + lane * 64 + ((chunk ^ ((lane >> 1) & 3)) << 4);
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+}
+
+// What the epilogue of one warp needs for a tile: its 32 rows from `row0` and `cols` (a multiple of 32) columns from `col0` of
+// problem `bi`, held in TMEM from `taddr`; scales and bias of those columns in shared memory.
+struct TilePart {
+  const CUtensorMap* tmap_d;
+  uint8_t* stage;  // this warp's two pieces
+  uint32_t taddr;
+  int cols, row0, col0, bi, lane;
+  float rs, cst;
+  const float* cs;
+  const float* bias;
+};
+
+// `piece` counts the pieces this warp has written; `release` is called once the accumulator has been read.
+template <bool F8, int CH, int OUT, typename Release>
+__device__ __forceinline__ void drain_tile(const GemmParams& p, const TilePart& t, uint32_t& piece, Release release) {
+  uint32_t va[16], vb[16];
+  tmem_issue16(t.taddr, va);
+  auto put = [&](uint32_t (&v)[16], int half, int col) {
+    const uint32_t sbase = smem_u32(t.stage) + (piece & 1) * kPieceBytes;
+    constexpr bool two_byte = OUT != QLIN_DT_F32;
+    uint32_t w[two_byte ? 8 : 16];
+    if (two_byte) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (OUT == QLIN_DT_BF16) {
+          const __nv_bfloat162 o = __float22bfloat162_rn(pair_n(v, j));
+          w[j] = *reinterpret_cast<const uint32_t*>(&o);
+        } else {
+          const __half2 o = __float22half2_rn(pair_n(v, j));
+          w[j] = *reinterpret_cast<const uint32_t*>(&o);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = v[j];
+    }
+    if (!two_byte || half == 0) {  // the buffer's previous store, two pieces ago, has been read
+      if (t.lane == 0) tma_store_wait_read<1>();
+      __syncwarp();
+    }
+#pragma unroll
+    for (int c = 0; c < (two_byte ? 2 : 4); ++c) piece_write(sbase, t.lane, (two_byte ? 2 * half : 0) + c, w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+    if (!two_byte || half == 1) {
+      fence_proxy_async();
+      __syncwarp();
+      const int x = two_byte ? col - 16 : col;
+      if (t.lane == 0) {
+        if (t.row0 < p.M && x < p.N) tma_store_3d(t.tmap_d, t.stage + (piece & 1) * kPieceBytes, x, t.row0, t.bi);
+        tma_store_commit();  // a piece outside the output is an empty group: the wait above counts pieces
+      }
+      ++piece;
+    }
+  };
+#pragma unroll 1
+  for (int j = 0; j < t.cols; j += 32) {
+    tmem_wait16(va);
+    tmem_issue16(t.taddr + j + 16, vb);
+    dequant16<F8, CH, OUT>(p, va, t.rs, t.cst, t.cs + j, t.bias + j);
+    put(va, 0, t.col0 + j);
+    tmem_wait16(vb);
+    if (j + 32 < t.cols) {
+      tmem_issue16(t.taddr + j + 32, va);
+    } else {
+      release();
+    }
+    dequant16<F8, CH, OUT>(p, vb, t.rs, t.cst, t.cs + j + 16, t.bias + j + 16);
+    put(vb, 1, t.col0 + j + 16);
+  }
+}
+
+// Which chain and output type a launch has are kernel arguments, so every warp of the grid takes the same branch.
+template <bool F8, int CH, typename Release>
+__device__ __forceinline__ void drain_tile_to(const GemmParams& p, const TilePart& t, uint32_t& piece, Release release) {
+  if (p.out_dtype == QLIN_DT_BF16) {
+    drain_tile<F8, CH, QLIN_DT_BF16>(p, t, piece, release);
+  } else if (p.out_dtype == QLIN_DT_F16) {
+    drain_tile<F8, CH, QLIN_DT_F16>(p, t, piece, release);
+  } else {
+    drain_tile<F8, CH, QLIN_DT_F32>(p, t, piece, release);
+  }
+}
+template <bool F8, typename Release>
+__device__ __forceinline__ void drain_tile_any(const GemmParams& p, const TilePart& t, uint32_t& piece, Release release) {
+  if (p.chain == kChainRaw) {
+    drain_tile<F8, kChainRaw, QLIN_DT_F32>(p, t, piece, release);
+  } else if (p.chain == kChainSeq) {
+    drain_tile_to<F8, kChainSeq>(p, t, piece, release);
+  } else if (F8 && p.chain == kChainSeqBf16) {
+    drain_tile<F8, kChainSeqBf16, QLIN_DT_BF16>(p, t, piece, release);
+  } else if (!F8 && p.chain == kChainProdBf16) {
+    drain_tile<F8, kChainProdBf16, QLIN_DT_BF16>(p, t, piece, release);
+  } else if (!F8 && p.chain == kChainProdF16) {
+    drain_tile_to<F8, kChainProdF16>(p, t, piece, release);
+  } else if (!F8 && p.chain == kChainAcc16Tensor) {
+    drain_tile_to<F8, kChainAcc16Tensor>(p, t, piece, release);
+  } else {
+    drain_tile_to<F8, kChainAny>(p, t, piece, release);
+  }
+}
+
 // The column scales and bias of one column (thread i: column i of the tile) and the row scale of this thread's row, fetched a
 // tile ahead so that their latency is not in the way of the accumulator they belong to.
 struct TileScales {
@@ -446,11 +658,12 @@ __device__ __forceinline__ TileScales fetch_scales(const GemmParams& p, int col,
 // [batch * N, K]); a tile of problem b starts at row b * M of A and row b * N of B, its rows and columns beyond the
 // problem's M and N belong to the next problem (or lie outside and read as zeros) and are dropped by the epilogue's
 // bounds checks, and its output goes to D + b * batch_stride_d.
-template <bool F8, bool CHUNKED, bool BATCHED = false>
-__global__ void __launch_bounds__(Cfg<CHUNKED>::THREADS, 1)
+// TILED: outputs that TMA can address are stored by drain_tile_any (tmap_d); the others, and chunked problems, by emit64 / emit32.
+template <bool F8, bool CHUNKED, bool BATCHED = false, bool TILED = false>
+__global__ void __launch_bounds__(Cfg<CHUNKED, BATCHED && TILED>::THREADS, 1)
 qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const GemmParams p) {
-  using C = Cfg<CHUNKED>;
+                 const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
+  using C = Cfg<CHUNKED, BATCHED && TILED>;
   extern __shared__ __align__(1024) uint8_t smem[];
   Aux* aux = reinterpret_cast<Aux*>(smem + C::AUX_OFFSET);
   volatile int* abort_flag = &aux->abort_flag;
@@ -493,6 +706,7 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (warp == C::PRODUCER_WARP && lane == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    if (TILED) tma_prefetch_desc(&tmap_d);
   }
   tc_fence_before();
   __syncthreads();
@@ -715,6 +929,82 @@ qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tc_commit_elect(&aux->drain);
     mbar_wait_drain(&aux->drain, 0);
     __syncwarp();
+  } else if constexpr (TILED) {
+    // ------------------------------------------------------------------ epilogue warps, tiled stores
+    const int q = warp & 3;
+    const int half = warp >> 2;  // column half of this warp
+    TilePart part;
+    part.tmap_d = &tmap_d;
+    part.stage = smem + C::OUT_OFFSET + warp * kStageOutBytes;
+    part.cols = C::COLS_PER_WARP;
+    part.lane = lane;
+    part.rs = part.cst = 1.0f;
+    part.cs = aux->cs + half * C::COLS_PER_WARP;
+    part.bias = aux->bias + half * C::COLS_PER_WARP;
+    const bool staged = p.chain != kChainRaw && p.chain != kChainAcc16Tensor;  // the chain takes a scale or bias per column
+    uint32_t ebuf = 0, ebph = 0, piece = 0;
+    bool ok = true;
+    TileScales next;
+    auto prefetch = [&](int t) {
+      if (!staged || t >= num_tiles) return;
+      int mb, nb;
+      tile_coords(BATCHED ? t % per_batch : t, p.num_m, p.num_n, mb, nb);
+      next = fetch_scales(p, nb * C::BN + half * C::COLS_PER_WARP + static_cast<int>(threadIdx.x & 127), (threadIdx.x & 127) < C::COLS_PER_WARP, mb * kBM + q * 32 + lane);
+    };
+    griddep_wait();  // the row scales may come from the launch before
+    if (p.chain == kChainAcc16Tensor) {
+      part.rs = p.rs != nullptr ? *p.rs : 1.0f;
+      part.cst = p.cs != nullptr ? *p.cs : 1.0f;
+    }
+    prefetch(blockIdx.x);
+    int t = blockIdx.x;
+    for (; t < num_tiles && ok; t += gridDim.x) {
+      int mb, nb;
+      const int bi = BATCHED ? t / per_batch : 0;
+      tile_coords(t - bi * per_batch, p.num_m, p.num_n, mb, nb);
+      if (staged) {
+        // Stage the column scales and bias of this half once; all lanes then read them as broadcasts.
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        if ((threadIdx.x & 127) < C::COLS_PER_WARP) {
+          aux->cs[half * C::COLS_PER_WARP + (threadIdx.x & 127)] = next.cs;
+          aux->bias[half * C::COLS_PER_WARP + (threadIdx.x & 127)] = next.bias;
+        }
+        part.rs = next.rs;
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        prefetch(t + gridDim.x);
+      }
+      const uint32_t buf = ebuf, bph = ebph;
+      if (++ebuf == C::NBUF) {
+        ebuf = 0;
+        ebph ^= 1u;
+      }
+      if (!warp_mbar_wait(&aux->tfull[buf], bph, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      part.taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::BN + half * C::COLS_PER_WARP;
+      part.row0 = mb * kBM + q * 32;
+      part.col0 = nb * C::BN + half * C::COLS_PER_WARP;
+      part.bi = bi;
+      drain_tile_any<F8>(p, part, piece, [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&aux->tempty[buf]);
+      });
+    }
+    if (lane == 0) tma_store_wait_read<0>();  // the stores read this CTA's shared memory
+    if (!ok && lane == 0) {
+      timed_out = !*abort_flag;
+      *abort_flag = 1;
+    }
+    // a warp that gave up still takes part in the barriers of the tiles that are left: another may have seen its accumulator
+    // complete a moment before the abort and be on its way to them
+    if (!ok && staged)
+      for (t += gridDim.x; t < num_tiles; t += gridDim.x) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+      }
   } else {
     // ------------------------------------------------------------------ epilogue warps
     const int q = warp & 3;
@@ -933,9 +1223,10 @@ __device__ __forceinline__ void tile_coords2(int t, int num_m, int num_n, int& m
   nb = r / gsz;
 }
 
-template <bool F8>
+template <bool F8, bool TILED>
 __global__ void __launch_bounds__(PairCfg::THREADS, 1)
-qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
+                      const GemmParams p) {
   using C = PairCfg;
   extern __shared__ __align__(1024) uint8_t smem[];
   Aux* aux = reinterpret_cast<Aux*>(smem + C::AUX_OFFSET);
@@ -969,6 +1260,7 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   if (warp == C::PRODUCER_WARP && lane == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    if (TILED) tma_prefetch_desc(&tmap_d);
   }
   tc_fence_before();
   __syncthreads();
@@ -1075,6 +1367,79 @@ qlin_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       mbar_wait_drain(&aux->drain, 0);
     }
     __syncwarp();
+  } else if constexpr (TILED) {
+    // ------------------------------------------------------------------ epilogue warps (both CTAs), tiled stores
+    const int q = warp & 3;
+    const int half = warp >> 2;  // column half of this warp
+    TilePart part;
+    part.tmap_d = &tmap_d;
+    part.stage = smem + C::OUT_OFFSET + warp * kStageOutBytes;
+    part.cols = C::COLS_PER_WARP;
+    part.lane = lane;
+    part.rs = part.cst = 1.0f;
+    part.cs = aux->cs + half * C::COLS_PER_WARP;
+    part.bias = aux->bias + half * C::COLS_PER_WARP;
+    const bool staged = p.chain != kChainRaw && p.chain != kChainAcc16Tensor;  // the chain takes a scale or bias per column
+    uint32_t ebuf = 0, ebph = 0, piece = 0;
+    bool ok = true;
+    TileScales next;
+    auto prefetch = [&](int t) {
+      if (!staged || t >= num_tiles) return;
+      int mb, nb;
+      tile_coords2(t, num_m2, p.num_n, mb, nb);
+      next = fetch_scales(p, nb * C::BN + static_cast<int>(threadIdx.x), true, mb * 2 * kBM + static_cast<int>(rank) * kBM + q * 32 + lane);
+    };
+    griddep_wait();  // the row scales may come from the launch before
+    if (p.chain == kChainAcc16Tensor) {
+      part.rs = p.rs != nullptr ? *p.rs : 1.0f;
+      part.cst = p.cs != nullptr ? *p.cs : 1.0f;
+    }
+    prefetch(pair);
+    int t = pair;
+    for (; t < num_tiles && ok; t += num_pairs) {
+      int mb, nb;
+      tile_coords2(t, num_m2, p.num_n, mb, nb);
+      if (staged) {
+        // Stage the column scales and bias of this half once; all lanes then read them as broadcasts.
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        aux->cs[threadIdx.x] = next.cs;
+        aux->bias[threadIdx.x] = next.bias;
+        part.rs = next.rs;
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        prefetch(t + num_pairs);
+      }
+      const uint32_t buf = ebuf, bph = ebph;
+      if (++ebuf == C::NBUF) {
+        ebuf = 0;
+        ebph ^= 1u;
+      }
+      if (!warp_mbar_wait(&aux->tfull[buf], bph, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      part.taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::BN + half * C::COLS_PER_WARP;
+      part.row0 = mb * 2 * kBM + static_cast<int>(rank) * kBM + q * 32;
+      part.col0 = nb * C::BN + half * C::COLS_PER_WARP;
+      part.bi = 0;
+      drain_tile_any<F8>(p, part, piece, [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(&aux->tempty[buf], 0));
+      });
+    }
+    if (lane == 0) tma_store_wait_read<0>();  // the stores read this CTA's shared memory
+    if (!ok && lane == 0) {
+      timed_out = !*abort_flag;
+      *abort_flag = 1;
+    }
+    // a warp that gave up still takes part in the barriers of the tiles that are left: another may have seen its accumulator
+    // complete a moment before the abort and be on its way to them
+    if (!ok && staged)
+      for (t += num_pairs; t < num_tiles; t += num_pairs) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+      }
   } else {
     // ------------------------------------------------------------------ epilogue warps (both CTAs)
     const int q = warp & 3;
@@ -1457,6 +1822,42 @@ static int make_operand_map(CUtensorMap* tm, const void* base, int64_t rows, int
   return QLIN_OK;
 }
 
+// The output of `batch` problems as a [batch, M, N] tensor read in pieces of 32 rows x 64 bytes.  Returns false where TMA cannot
+// address it (base, row pitch or problem stride off a 16-byte boundary) or rows end inside 16 bytes that are not all theirs.
+static bool make_output_map(CUtensorMap* tm, const GemmParams& p) {
+  const bool two_byte = p.epilogue != QLIN_EPI_RAW && p.out_dtype != QLIN_DT_F32;
+  const int64_t elt = two_byte ? 2 : 4;
+  const int64_t pitch = p.ldd * elt, stride = p.batch > 1 ? p.batch_stride_d * elt : pitch * p.M;
+  if (!aligned16(p.d) || pitch % 16 != 0 || stride % 16 != 0 || (p.N * elt) % 16 != 0 || stride >= (int64_t{1} << 40) || pitch >= (int64_t{1} << 40)) return false;
+  EncodeTiledFn enc = get_encode_fn();
+  if (enc == nullptr) return false;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.N), static_cast<cuuint64_t>(p.M), static_cast<cuuint64_t>(p.batch > 1 ? p.batch : 1)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch), static_cast<cuuint64_t>(stride)};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(64 / elt), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(tm, two_byte ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, p.d, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+static bool no_round(int dt) { return dt == QLIN_DT_NONE || dt == QLIN_DT_F32; }
+
+// The compiled epilogue that rounds where this launch's does.
+static int32_t pick_chain(const GemmParams& p, bool f8) {
+  if (p.epilogue == QLIN_EPI_RAW) return kChainRaw;
+  if (p.epilogue == QLIN_EPI_SCALE_PROD && !f8 && p.acc_round == QLIN_DT_F16) {
+    if (p.prod_round == QLIN_DT_BF16 && p.scale_round == QLIN_DT_F16 && p.out_dtype == QLIN_DT_BF16) return kChainProdBf16;
+    // rounding to fp16 twice is rounding once
+    if ((no_round(p.prod_round) || p.prod_round == QLIN_DT_F16) && p.scale_round == QLIN_DT_F16) return kChainProdF16;
+  }
+  if (p.epilogue == QLIN_EPI_SCALE_SEQ) {
+    if (no_round(p.mid_round) && no_round(p.acc_round)) return kChainSeq;
+    if (f8 && p.mid_round == QLIN_DT_BF16 && p.acc_round == QLIN_DT_BF16 && p.out_dtype == QLIN_DT_BF16) return kChainSeqBf16;
+  }
+  if (p.epilogue == QLIN_EPI_SCALE_ACC16 && !f8 && p.rs_stride == 0 && p.cs_stride == 0 && p.bias == nullptr && no_round(p.mid_round) && no_round(p.acc_round))
+    return kChainAcc16Tensor;
+  return kChainAny;
+}
+
 // A launch with a cluster size and, for a GEMM behind its quantiser, the programmatic dependency.
 struct LaunchCfg {
   cudaLaunchConfig_t cfg = {};
@@ -1483,16 +1884,16 @@ struct LaunchCfg {
   }
 };
 
-template <bool F8, bool CHUNKED, bool BATCHED = false>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
-  using C = Cfg<CHUNKED>;
+template <bool F8, bool CHUNKED, bool BATCHED, bool TILED>
+static int launch_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, cudaStream_t stream) {
+  using C = Cfg<CHUNKED, BATCHED && TILED>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return fail(QLIN_ERR_DEVICE, "device ordinal %d out of range", dev);
+  const auto kernel = qlin_gemm_kernel<F8, CHUNKED, BATCHED, TILED>;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(qlin_gemm_kernel<F8, CHUNKED, BATCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return fail(QLIN_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured[dev] = true;
   }
@@ -1500,16 +1901,24 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
   if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
   LaunchCfg lc(grid, C::THREADS, C::SMEM_BYTES, stream, 1, p.dependent != 0);
-  const cudaError_t le = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_kernel<F8, CHUNKED, BATCHED>, ta, tb, p);
+  const cudaError_t le = cudaLaunchKernelEx(&lc.cfg, kernel, ta, tb, td, p);
   if (le != cudaSuccess) {
     cudaGetLastError();
     return fail(QLIN_ERR_LAUNCH, "qlin_gemm: %s", cudaGetErrorString(le));
   }
   return QLIN_OK;
 }
+// `td`: the output's map, or null for outputs that TMA does not store.
+template <bool F8, bool CHUNKED, bool BATCHED = false>
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* td, const GemmParams& p, cudaStream_t stream) {
+  if constexpr (!CHUNKED) {
+    if (td != nullptr) return launch_as<F8, false, BATCHED, true>(ta, tb, *td, p, stream);
+  }
+  return launch_as<F8, CHUNKED, BATCHED, false>(ta, tb, ta, p, stream);
+}
 
 // Largest number of two-CTA clusters of the pair kernel that can be resident at once (cached per device).
-template <bool F8>
+template <bool F8, bool TILED>
 static int pair_max_clusters() {
   static int cached[64] = {};
   int dev = 0;
@@ -1517,7 +1926,8 @@ static int pair_max_clusters() {
   if (dev < 0 || dev >= 64) return 0;
   if (cached[dev] != 0) return cached[dev] > 0 ? cached[dev] : 0;
   cached[dev] = -1;
-  if (cudaFuncSetAttribute(qlin_gemm_pair_kernel<F8>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES) != cudaSuccess) {
+  const auto kernel = qlin_gemm_pair_kernel<F8, TILED>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1533,7 +1943,7 @@ static int pair_max_clusters() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, qlin_gemm_pair_kernel<F8>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1541,20 +1951,24 @@ static int pair_max_clusters() {
   return n > 0 ? n : 0;
 }
 
-template <bool F8>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
-  int clusters = pair_max_clusters<F8>();
+template <bool F8, bool TILED>
+static int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, cudaStream_t stream) {
+  int clusters = pair_max_clusters<F8, TILED>();
   if (clusters <= 0) return 1;  // not available: the caller takes the single-CTA kernel
   const int tiles = ((p.M + 2 * kBM - 1) / (2 * kBM)) * p.num_n;
   if (clusters > tiles) clusters = tiles;
   if (p.max_ctas > 0 && clusters > p.max_ctas / 2) clusters = p.max_ctas / 2 > 0 ? p.max_ctas / 2 : 1;
   LaunchCfg lc(2 * clusters, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream, 2, p.dependent != 0);
-  cudaError_t e = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_pair_kernel<F8>, ta, tb, p);
+  const cudaError_t e = cudaLaunchKernelEx(&lc.cfg, qlin_gemm_pair_kernel<F8, TILED>, ta, tb, td, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(QLIN_ERR_LAUNCH, "qlin_gemm (CTA-pair kernel): %s", cudaGetErrorString(e));
   }
   return QLIN_OK;
+}
+template <bool F8>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* td, const GemmParams& p, cudaStream_t stream) {
+  return td != nullptr ? launch_pair_as<F8, true>(ta, tb, *td, p, stream) : launch_pair_as<F8, false>(ta, tb, ta, p, stream);
 }
 
 // The CTA-pair kernel is used for unchunked problems of at least 256 rows unless QLIN_GEMM_PAIR=0.
@@ -1722,6 +2136,10 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
                      (chunk_k32 == 1 || chunk_k32 == 2 || chunk_k32 == 4) && total_k32 % 4 == 0 && low_byte_enabled())
                         ? 1
                         : 0;
+  // unchunked products whose output TMA can address are stored by it; an accumulator input or row-block scatter keeps emit64
+  p.chain = pick_chain(p, f8);
+  CUtensorMap tmap_d;
+  const CUtensorMap* td = !chunked && p.c == nullptr && p.scatter_rows <= 0 && make_output_map(&tmap_d, p) ? &tmap_d : nullptr;
   if (batch > 1) {
     if (chunked || a->c != nullptr || a->scatter_rows != 0) return fail(QLIN_ERR_UNSUPPORTED, "qlin_gemm_batched: one launch takes unchunked problems without accumulator input or scatter");
     if (static_cast<int64_t>(batch) * a->M > 0x7fffffff || static_cast<int64_t>(batch) * a->N > 0x7fffffff)
@@ -1731,7 +2149,7 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
     if (rc != QLIN_OK) return rc;
     rc = make_operand_map(&tb, a->b, static_cast<int64_t>(batch) * a->N, a->K, a->ldb, bn);
     if (rc != QLIN_OK) return rc;
-    return f8 ? launch<true, false, true>(ta, tb, p, s) : launch<false, false, true>(ta, tb, p, s);
+    return f8 ? launch<true, false, true>(ta, tb, td, p, s) : launch<false, false, true>(ta, tb, td, p, s);
   }
   if (!chunked && a->M <= kBM && a->scatter_rows == 0 && a->max_ctas <= 0 && skinny_enabled()) {
     // weight rows as the MMA's M dimension, the few activation rows (padded to 32) as its N dimension
@@ -1757,11 +2175,11 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
     CUtensorMap tb_half;  // each CTA of a pair loads 128 of the tile's 256 B rows
     rc = make_operand_map(&tb_half, a->b, a->N, a->K, a->ldb, PairCfg::BN / 2);
     if (rc != QLIN_OK) return rc;
-    rc = f8 ? launch_pair<true>(ta, tb_half, p, s) : launch_pair<false>(ta, tb_half, p, s);
+    rc = f8 ? launch_pair<true>(ta, tb_half, td, p, s) : launch_pair<false>(ta, tb_half, td, p, s);
     if (rc <= 0) return rc;
   }
-  if (f8) return chunked ? launch<true, true>(ta, tb, p, s) : launch<true, false>(ta, tb, p, s);
-  return chunked ? launch<false, true>(ta, tb, p, s) : launch<false, false>(ta, tb, p, s);
+  if (f8) return chunked ? launch<true, true>(ta, tb, td, p, s) : launch<true, false>(ta, tb, td, p, s);
+  return chunked ? launch<false, true>(ta, tb, td, p, s) : launch<false, false>(ta, tb, td, p, s);
 }
 
 extern "C" int qlin_gemm(const qlin_gemm_args* a, void* stream) { return gemm_impl(a, stream, 1, 0); }
