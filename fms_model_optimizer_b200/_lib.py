@@ -67,6 +67,11 @@ EXPORTED_SYMBOLS = (
     "qlin_peer_barrier",
     "qlin_col_absmax",
     "qlin_shard_reduce",
+    "qlin_qat_flag_count",
+    "qlin_qat_colsum_workspace_bytes",
+    "qlin_qat_codes",
+    "qlin_qat_split",
+    "qlin_qat_product",
 )
 
 

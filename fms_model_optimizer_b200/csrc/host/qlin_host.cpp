@@ -9,9 +9,11 @@
 // No kernel, no fallback and no state of its own: everything a call keeps is one status word per device, which lives as
 // long as the process.
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/stl.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <mutex>
@@ -513,6 +515,145 @@ std::tuple<OptTensor, OptTensor, Tensor> weight_fq_perch(const Tensor& w_in, int
   return {opt(dq), opt(codes), clip_io};
 }
 
+// ------------------------------------------------------------------------------------------------ QAT Linear
+// out = x w^T + bias for fake-quantised fp32 operands on the tensor cores (qlin_qat_*), with its gradients.
+struct QatShape {
+  int64_t tokens, in, out;
+};
+
+// The operands' arguments of one pass; `floats` is [2 * out + 1]: scales, their reciprocals, the step.
+qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, const Tensor& flags, const QatShape& n) {
+  qlin_qat_args a = {};
+  a.x = static_cast<const float*>(data(x));
+  a.w = static_cast<const float*>(data(w));
+  a.scale = static_cast<float*>(data(floats));
+  a.rcp = a.scale + n.out;
+  a.step = a.scale + 2 * n.out;
+  a.flags = static_cast<int32_t*>(data(flags));
+  a.status = static_cast<int32_t*>(status_word(x.device().index()).data_ptr());
+  a.tokens = static_cast<int32_t>(n.tokens);
+  a.in = static_cast<int32_t>(n.in);
+  a.out = static_cast<int32_t>(n.out);
+  return a;
+}
+
+class QatProduct : public torch::autograd::Function<QatProduct> {
+ public:
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias, const Tensor& clip_x,
+                        const OptTensor& clipn_x, const Tensor& clip_w, int64_t bits_x, int64_t bits_w, int64_t variant) {
+    const at::Device dev = x.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const QatShape n{x.numel() / x.size(-1), x.size(-1), w.size(0)};
+    const Tensor floats = empty({2 * n.out + 1}, at::kFloat, dev), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
+    const Tensor xc = empty({n.tokens, n.in}, at::kBFloat16, dev), wc = empty({n.out, n.in}, at::kBFloat16, dev);
+    std::vector<int64_t> shape = x.sizes().vec();
+    shape.back() = n.out;
+    const Tensor out = empty(shape, at::kFloat, dev);
+    const Tensor bs = bias ? bias->detach().contiguous() : Tensor(), cv = clip_f32(clip_x, dev), cvn = clipn_x ? clip_f32(*clipn_x, dev) : Tensor();
+    const Tensor cw = clip_w.detach().contiguous();
+    qlin_qat_args a = qat_args(x, w, floats, flags, n);
+    a.bias = static_cast<const float*>(data(bs));
+    a.clip_x = static_cast<const float*>(data(cv));
+    a.clipn_x = static_cast<const float*>(data(cvn));
+    a.clip_w = static_cast<const float*>(data(cw));
+    a.x_codes = data(xc);
+    a.w_codes = data(wc);
+    a.d = static_cast<float*>(data(out));
+    a.num_bits_x = static_cast<int32_t>(bits_x);
+    a.num_bits_w = static_cast<int32_t>(bits_w);
+    a.variant = static_cast<int32_t>(variant);
+    check(qlin_qat_codes(&a, 0, stream_of(dev)), "qlin_qat_codes");
+    check(qlin_qat_product(&a, 0, stream_of(dev)), "qlin_qat_product");
+    // the step and scales are kept, not the clip values they came from: a later forward pass may have replaced those
+    ctx->save_for_backward({x, w, floats});
+    ctx->saved_data["bits"] = std::vector<int64_t>{bits_x, bits_w, variant};
+    ctx->saved_data["bias"] = bias.has_value();
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const torch::autograd::variable_list saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1], &floats = saved[2];
+    const QatShape n{x.numel() / x.size(-1), x.size(-1), w.size(0)};
+    const bool want_x = ctx->needs_input_grad(0), want_w = ctx->needs_input_grad(1);
+    const bool want_b = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
+    Tensor gx, gw, gb;
+    const Tensor& go = grads[0];
+    if (go.defined()) {
+      const Tensor g = go.reshape({n.tokens, n.out});
+      if (at::GradMode::is_enabled()) {  // gradients that are differentiated again
+        if (want_x) gx = g.matmul(w).view(x.sizes());
+        if (want_w) gw = g.t().matmul(x.reshape({n.tokens, n.in}));
+      } else if (want_x || want_w) {
+        const at::Device dev = x.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const Tensor gc = g.contiguous(), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
+        const std::vector<int64_t> bits = ctx->saved_data["bits"].toIntVector();
+        Tensor planes = empty({3, n.tokens, n.out}, at::kBFloat16, dev);
+        // both operands' codes are made, and checked, whichever gradient is wanted
+        Tensor xc = empty({n.tokens, n.in}, at::kBFloat16, dev), wc = empty({n.in, n.out}, at::kBFloat16, dev);
+        qlin_qat_args a = qat_args(x, w, floats, flags, n);
+        a.g = static_cast<const float*>(data(gc));
+        a.x_codes = data(xc);
+        a.w_codes = data(wc);
+        a.g_planes = data(planes);
+        a.num_bits_x = static_cast<int32_t>(bits[0]);
+        a.num_bits_w = static_cast<int32_t>(bits[1]);
+        a.variant = static_cast<int32_t>(bits[2]);
+        Tensor ws;
+        if (want_b) {
+          gb = empty({n.out}, at::kFloat, dev);
+          ws = empty({qlin_qat_colsum_workspace_bytes(a.tokens, a.out) / 4}, at::kFloat, dev);
+          a.colsum = static_cast<float*>(data(gb));
+          a.workspace = static_cast<float*>(data(ws));
+        }
+        check(qlin_qat_codes(&a, 1, stream_of(dev)), "qlin_qat_codes");
+        check(qlin_qat_split(&a, stream_of(dev)), "qlin_qat_split");
+        if (want_w) {
+          gw = empty({n.out, n.in}, at::kFloat, dev);
+          a.d = static_cast<float*>(data(gw));
+          check(qlin_qat_product(&a, 2, stream_of(dev)), "qlin_qat_product");
+        }
+        xc.reset();
+        if (want_x) {
+          gx = empty(x.sizes(), at::kFloat, dev);
+          a.d = static_cast<float*>(data(gx));
+          a.x_codes = nullptr;
+          check(qlin_qat_product(&a, 1, stream_of(dev)), "qlin_qat_product");
+        }
+      }
+      if (want_b && !gb.defined()) gb = g.sum(0);
+    }
+    return {gx, gw, gb, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// Calls with fewer multiply-adds than this, or with a side shorter than 128, stay with the library.  Device time of forward and
+// backward, library -> tensor cores: 256 x 768 x 768 (2^27.2) 65 -> 67 us, 700 x 768 x 768 (2^28.6) 95 -> 73, 256 x 768 x 3072
+// (2^29.2) 159 -> 101, 4096 x 768 x 768 364 -> 135.
+constexpr double kQatMinWork = 268435456.0;
+constexpr int64_t kQatMinSide = 128;
+
+// Whether qat_linear takes these operands: fp32 in fp32 arithmetic (no TF32, no autocast), dense, aligned, and large enough.
+bool qat_takes(const Tensor& x, const Tensor& w, const OptTensor& bias, const Tensor& clip_w) {
+  if (!x.is_cuda() || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || w.device() != x.device() || w.dim() != 2 || x.dim() < 1) return false;
+  if (x.size(-1) != w.size(1) || !x.is_contiguous() || !w.is_contiguous() || x.layout() != at::kStrided || w.layout() != at::kStrided) return false;
+  if (bias && (bias->scalar_type() != at::kFloat || bias->device() != x.device() || bias->dim() != 1 || bias->size(0) != w.size(0))) return false;
+  if (clip_w.scalar_type() != at::kFloat || clip_w.device() != x.device() || clip_w.numel() != w.size(0)) return false;
+  const int64_t in = w.size(1), out = w.size(0);
+  if (in < kQatMinSide || out < kQatMinSide || x.numel() < kQatMinSide * in || in % 8 != 0 || out % 8 != 0 || x.numel() / in > 0x7fffffff - 256 || in > 0x7fffff00 || out > 0x7fffff00) return false;
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0 || reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 != 0) return false;
+  if (at::autocast::is_autocast_enabled(at::kCUDA)) return false;
+  const at::Float32Precision prec = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);
+  if (prec != at::Float32Precision::NONE && prec != at::Float32Precision::IEEE) return false;
+  return static_cast<double>(x.numel()) * static_cast<double>(out) >= kQatMinWork;
+}
+
+Tensor qat_linear(const Tensor& x, const Tensor& w, const OptTensor& bias, const Tensor& clip_x, const OptTensor& clipn_x, const Tensor& clip_w, int64_t bits_x,
+                  int64_t bits_w, int64_t variant) {
+  return QatProduct::apply(x, w, bias, clip_x.detach(), clipn_x ? OptTensor(clipn_x->detach()) : std::nullopt, clip_w, bits_x, bits_w, variant);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_qlin_host, m) {
@@ -526,4 +667,6 @@ PYBIND11_MODULE(_qlin_host, m) {
   m.def("weight_fq_perch", &weight_fq_perch, rel());
   m.def("pact2_fwd", &pact2_fwd, rel());
   m.def("pact2_bwd", &pact2_bwd, rel());
+  m.def("qat_takes", &qat_takes, rel());
+  m.def("qat_linear", &qat_linear, rel());
 }

@@ -1806,6 +1806,8 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+void* tensor_map_encoder() { return reinterpret_cast<void*>(get_encode_fn()); }
+
 // [rows, kbytes] byte matrix with `ld_bytes` between rows, read in boxes of [box_rows x 128 bytes].
 static int make_operand_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t kbytes, int64_t ld_bytes,
                             int box_rows) {

@@ -16,6 +16,9 @@ int fail(int code, const char* fmt, ...);
 // qlin_act_quant with optional device scalars (one kernel launch, which lets a dependent launch start early).
 int act_quant_impl(const qlin_quant_args* args, const qlin_scalar_src* src, void* stream);
 
+// cuTensorMapEncodeTiled of the driver, or null.
+void* tensor_map_encoder();
+
 // Number of SMs of the current device (cached per device id).
 int sm_count();
 

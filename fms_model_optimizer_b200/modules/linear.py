@@ -17,7 +17,7 @@ from torch import nn
 
 from .. import _lib as L
 from .. import ops
-from ..quant.quantizers import get_activation_quantizer, get_weight_quantizer
+from ..quant.quantizers import PACT, PACT2, SAWB, PACTplusSym, get_activation_quantizer, get_weight_quantizer
 
 _FLOATS = (torch.float32, torch.float16, torch.bfloat16)
 
@@ -587,6 +587,20 @@ class QLinearINT8Train(nn.Linear):
         return s
 
 
+def _ordinary_call(*tensors) -> bool:
+    """No tensor subclass, functorch transform, forward-mode level, dispatch or function mode, tracer or compiler is at work."""
+    if any(t is not None and type(t) not in (torch.Tensor, nn.Parameter) for t in tensors):
+        return False
+    return not (
+        torch.compiler.is_compiling()
+        or torch._C._are_functorch_transforms_active()
+        or torch._C._len_torch_dispatch_stack()
+        or torch._C._len_torch_function_stack()
+        or torch._C._get_tracing_state() is not None
+        or torch.autograd.forward_ad._current_level >= 0
+    )
+
+
 class QLinear(nn.Linear):
     """Fake-quant Linear for QAT / DQ (fms_mo/modules/linear.py:51-393, forward :248-305):
     ``F.linear(Qa(x / s), Qw(W * s), bias)`` with the SmoothQuant scale ``s`` of :345-368.  The two
@@ -651,9 +665,29 @@ class QLinear(nn.Linear):
         else:  # the reference divides and multiplies by a tensor holding 1.0 here: the identity, bit for bit
             qinput = self.quantize_feature(x).to(x.dtype)
             qweight = self.quantize_weight(self.weight).to(self.weight.dtype)
-        output = nn.functional.linear(qinput, qweight, self.bias)
+        output = self._product(qinput, qweight)
         self.num_module_called += 1
         return output
+
+    def _product(self, qinput, qweight):
+        """``F.linear`` of the quantised operands: on the tensor cores, at fp32 accuracy (csrc/qlin_qat.cu), where both are whole
+        numbers of a quantizer's steps with an integral zero point and the call is an ordinary one -- no transform, mode or
+        tracer that would have to see the product -- and by the library otherwise."""
+        Qa, Qw = self.quantize_feature, self.quantize_weight
+        variant = None
+        if type(Qw) is SAWB and Qw.perCh and Qw.dequantize:
+            if type(Qa) is PACT2 and Qa.align_zero:
+                variant = L.PACT_TWO_SIDED
+            elif type(Qa) is PACT:
+                variant = L.PACT_ONE_SIDED
+            elif type(Qa) is PACTplusSym and Qa.intg_zp:
+                variant = L.PACT_SYMMETRIC
+        if variant is None or not (2 <= Qa.num_bits <= 8) or not _ordinary_call(qinput, qweight, self.bias):
+            return nn.functional.linear(qinput, qweight, self.bias)
+        host = L.host()
+        if not host.qat_takes(qinput, qweight, self.bias, Qw.clip_val):
+            return nn.functional.linear(qinput, qweight, self.bias)
+        return host.qat_linear(qinput, qweight, self.bias, Qa.clip_val, getattr(Qa, "clip_valn", None), Qw.clip_val, Qa.num_bits, Qw.num_bits, variant)
 
 
 def lower_qmodel_b200(model: nn.Module, use_dyn_max_act=False, max_acc_bits=32, clamp_acc_to_dl16=False,

@@ -591,6 +591,47 @@ typedef struct qlin_peer_barrier_args {
 
 int qlin_peer_barrier(const qlin_peer_barrier_args* args, void* stream);
 
+/* ------------------------------------------------------------------------------------------------
+ * qlin_qat_* -- the fp32 product of a QAT Linear (QLinear.forward, fms_mo/modules/linear.py:248-305) and its gradients on
+ * bf16 tensor cores, at fp32 accuracy.  x [tokens, in] and w [out, in] are the fake-quantised operands of a PACT+ activation
+ * quantizer and of a per-channel symmetric weight quantizer: whole numbers of steps.  They enter as those whole numbers, a
+ * gradient g [tokens, out] as three bf16 parts.  Operands the arithmetic cannot carry (no whole number of steps, scales out of
+ * range, infinite, NaN or tiny gradients) raise a flag, and the product is then computed in fp32 from x, w and g.
+ * Forward: qlin_qat_codes(a, 0), qlin_qat_product(a, 0).  Backward: qlin_qat_codes(a, 1) with the step and scales of the forward
+ * pass, qlin_qat_split, qlin_qat_product(a, 1) for gx and (a, 2) for gw.  in and out are multiples of 8; x, w and d dense and 16-byte
+ * aligned; g dense.  `flags` holds qlin_qat_flag_count() words for each pass, which the calls of that pass write before they read.
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct qlin_qat_args {
+  const float* x;       /* [tokens, in] */
+  const float* w;       /* [out, in] */
+  const float* g;       /* [tokens, out] */
+  const float* bias;    /* optional [out]; forward */
+  const float* clip_x;  /* [1]; forward */
+  const float* clipn_x; /* [1], QLIN_PACT_TWO_SIDED; forward */
+  const float* clip_w;  /* [out]; forward */
+  float* step;          /* [1]: written by the forward pass, read by both */
+  float* scale;         /* [out], 16-byte aligned: likewise */
+  float* rcp;           /* [out]: likewise */
+  void* x_codes;        /* bf16 [tokens, in]; qlin_qat_codes leaves them out when NULL */
+  void* w_codes;        /* bf16 [out, in], backward [in, out]; likewise */
+  void* g_planes;       /* bf16 [3, tokens, out] */
+  float* d;             /* the product */
+  float* colsum;        /* optional [out]: qlin_qat_split's column sums of g */
+  float* workspace;     /* qlin_qat_colsum_workspace_bytes, 16-byte aligned, when colsum is given */
+  int32_t* flags;
+  int32_t* status;      /* optional device status word, written only on failure */
+  int32_t tokens, in, out;
+  int32_t num_bits_x, num_bits_w;
+  int32_t variant;      /* qlin_pact_variant of x's quantizer */
+} qlin_qat_args;
+
+int32_t qlin_qat_flag_count(void);
+int64_t qlin_qat_colsum_workspace_bytes(int32_t tokens, int32_t out);
+int qlin_qat_codes(const qlin_qat_args* args, int32_t backward, void* stream);
+int qlin_qat_split(const qlin_qat_args* args, void* stream);
+/* which: 0 out = x w^T + bias, 1 gx = g w, 2 gw = g^T x */
+int qlin_qat_product(const qlin_qat_args* args, int32_t which, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

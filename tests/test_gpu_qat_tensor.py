@@ -1,0 +1,146 @@
+"""The QAT product on the tensor cores (csrc/qlin_qat.cu) at the sizes and values where it can go wrong: edges of its 256 x 128 / 192 / 256
+tiles and 64-term stages, operands that it must hand to fp32, a clip value that changes between forward and backward, gradients
+that are differentiated again, and the rule that leaves a call to the library.
+
+Bound: a product of n terms summed in fp32 in any order is within 8 sqrt(n) 2^-24 of the sum of the terms' absolute values."""
+
+import pytest
+import torch
+
+from fms_model_optimizer_b200 import _lib as L
+from fms_model_optimizer_b200.modules import QLinear
+from fms_model_optimizer_b200.modules.linear import _ordinary_call
+
+gpu = pytest.mark.gpu
+
+
+def _operands(t, k, n, clips=(3.0, -2.5)):
+    g = torch.Generator(device="cuda").manual_seed(t + k + n)
+    lin = QLinear(k, n, num_bits_feature=8, qa_mode="pact+", num_bits_weight=8, qw_mode="sawb+perCh", act_clip_init_val=clips[0], act_clip_init_valn=clips[1],
+                  device="cuda").train()  # fmt: skip
+    with torch.no_grad():
+        lin.weight.copy_(torch.randn(n, k, generator=g, device="cuda") * 0.02)
+        x = lin.quantize_feature(torch.randn(t, k, generator=g, device="cuda")).detach().requires_grad_(True)
+        w = lin.quantize_weight(lin.weight).detach().requires_grad_(True)
+    return lin, x, w, torch.randn(t, n, generator=g, device="cuda")
+
+
+def _run(lin, x, w):
+    Qa, Qw = lin.quantize_feature, lin.quantize_weight
+    return L.host().qat_linear(x, w, lin.bias, Qa.clip_val, Qa.clip_valn, Qw.clip_val, 8, 8, L.PACT_TWO_SIDED)
+
+
+def _check(lin, x, w, go, out, grads):
+    xd, wd, gd = x.detach().double(), w.detach().double(), go.double()
+    bd = lin.bias.detach().double()
+    for got, want, terms, n in (
+        (out.detach(), xd @ wd.t() + bd, xd.abs() @ wd.abs().t() + bd.abs(), x.shape[1] + 1),
+        (grads[0], gd @ wd, gd.abs() @ wd.abs(), w.shape[0]),
+        (grads[1], gd.t() @ xd, gd.abs().t() @ xd.abs(), x.shape[0]),
+        (grads[2], gd.sum(0), gd.abs().sum(0), x.shape[0]),
+    ):
+        assert bool(((got.double() - want).abs() <= 8 * n**0.5 * 2.0**-24 * terms + 1e-38).all())
+
+
+@gpu
+@pytest.mark.parametrize("t,k,n", [(1, 8, 8), (65, 64, 136), (257, 128, 264), (256, 72, 384), (1000, 200, 392), (63, 1032, 8), (3001, 520, 1048), (130, 4104, 776)])
+def test_edges(cuda_dev, t, k, n):
+    lin, x, w, go = _operands(t, k, n)
+    out = _run(lin, x, w)
+    _check(lin, x, w, go, out, torch.autograd.grad(out, [x, w, lin.bias], go))
+
+
+@gpu
+@pytest.mark.parametrize("what", ["tiny gradient", "activation off the steps", "weight off the steps", "scales replaced", "gradient off 16 bytes"])
+def test_operands_the_codes_cannot_carry(cuda_dev, what):
+    t, k, n = 300, 264, 200
+    lin, x, w, go = _operands(t, k, n)
+    with torch.no_grad():
+        if what == "tiny gradient":
+            go *= 1e-34
+        elif what == "activation off the steps":
+            x[7, 9] += 0.003
+        elif what == "weight off the steps":
+            w[11, 13] *= 1.01
+    out = _run(lin, x, w)
+    if what == "scales replaced":  # as by another forward pass with new weights before this one's backward
+        lin.quantize_weight.clip_val.mul_(1.5)
+        with torch.no_grad():
+            lin.quantize_feature.clip_val.mul_(0.5)
+    if what == "gradient off 16 bytes":
+        buf = torch.empty(t * n + 1, device="cuda")
+        buf[1:] = go.flatten()
+        go = buf[1:].view(t, n)
+    _check(lin, x, w, go, out, torch.autograd.grad(out, [x, w, lin.bias], go))
+
+
+@gpu
+def test_infinite_operands_give_what_fp32_gives(cuda_dev):
+    lin, x, w, go = _operands(300, 264, 200)
+    go[3, 5], go[8, 9], go[11] = float("inf"), float("nan"), 0
+    out = _run(lin, x, w)
+    got = torch.autograd.grad(out, [x, w], go)
+    want = torch.autograd.grad(torch.nn.functional.linear(x, w, lin.bias), [x, w], go)
+    for a, b in zip(got, want):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b))
+        ok = torch.isfinite(b)
+        assert torch.allclose(a[ok], b[ok], rtol=1e-4, atol=1e-5)
+
+
+@gpu
+def test_gradients_of_gradients_and_single_gradients(cuda_dev):
+    lin, x, w, go = _operands(200, 136, 144)
+    for leaf in (x, w, lin.bias):  # one gradient at a time
+        (a,) = torch.autograd.grad(_run(lin, x, w), [leaf], go)
+        (b,) = torch.autograd.grad(torch.nn.functional.linear(x, w, lin.bias), [leaf], go)
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4 * float(b.abs().max()))
+    res = []
+    for f in (lambda: _run(lin, x, w), lambda: torch.nn.functional.linear(x, w, lin.bias)):
+        gx, gw = torch.autograd.grad(f(), [x, w], go, create_graph=True)
+        res.append(torch.autograd.grad((gx * gx).sum() + (gw * gw).sum(), [x, w]))
+    for a, b in zip(*res):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4 * float(b.abs().max()))
+
+
+@gpu
+def test_rule(cuda_dev):
+    host = L.host()
+    lin, x, w, _ = _operands(1024, 512, 512)
+    cw = lin.quantize_weight.clip_val
+    assert host.qat_takes(x, w, lin.bias, cw) and host.qat_takes(x.view(4, 256, 512), w, None, cw)
+    assert not host.qat_takes(x[:100], w, lin.bias, cw)  # too small
+    assert not host.qat_takes(x[:, :256], w[:, :256], lin.bias, cw)  # not dense
+    assert not host.qat_takes(x.half(), w.half(), None, cw)
+    assert not host.qat_takes(x.cpu(), w.cpu(), None, cw.cpu())
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert not host.qat_takes(x, w, lin.bias, cw)
+    before = torch.backends.cuda.matmul.fp32_precision
+    torch.backends.cuda.matmul.fp32_precision = "tf32"
+    try:
+        assert not host.qat_takes(x, w, lin.bias, cw)
+    finally:
+        torch.backends.cuda.matmul.fp32_precision = before
+    assert type(lin._product(x, w).grad_fn).__name__ != type(torch.nn.functional.linear(x, w, lin.bias).grad_fn).__name__
+
+
+def test_calls_that_something_watches_stay_with_the_library():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+
+    x = torch.ones(2, 2)
+    assert _ordinary_call(x, torch.nn.Parameter(x.clone()), None)
+    assert not _ordinary_call(x, x.as_subclass(Sub))
+    with Watch():
+        assert not _ordinary_call(x)
+    seen = []
+    torch.func.vmap(lambda t: (seen.append(_ordinary_call(t)), t)[1])(x)
+    with torch.autograd.forward_ad.dual_level():
+        seen.append(_ordinary_call(x))
+    torch.jit.trace(lambda t: (seen.append(_ordinary_call(t)), t + 1)[1], x, check_trace=False)
+    assert seen == [False, False, False]
