@@ -56,14 +56,22 @@ __device__ __forceinline__ uint32_t bq_pack(float lo, float hi) {
 // Packed pair arithmetic: two bf16 values of one word as float2, multiplied by two fp32 factors with one packed
 // instruction and rounded back to a bf16 pair with one packed conversion (the same roundings as the scalar forms).
 __device__ __forceinline__ float2 bq_unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)); }
-__device__ __forceinline__ uint32_t bq_mul_pack(uint32_t w, float2 f) {
-  const __nv_bfloat162 h = __float22bfloat162_rn(__fmul2_rn(bq_unpack(w), f));
+__device__ __forceinline__ uint32_t bq_pack2(float2 v) {
+  const __nv_bfloat162 h = __float22bfloat162_rn(v);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
+__device__ __forceinline__ uint32_t bq_mul_pack(uint32_t w, float2 f) { return bq_pack2(__fmul2_rn(bq_unpack(w), f)); }
 __device__ __forceinline__ float bq_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bq_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-// SiLU rounded to bf16; the fast exponential and division are exact to well below half a bf16 place
-__device__ __forceinline__ float bq_silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
+// SiLU before its rounding to bf16: v / (1 + exp(-v)) with the approximate exponential and reciprocal, exact to well below half a
+// bf16 place.  Both flush: an exponential below the normal numbers leaves the sum at 1, a reciprocal below them is the 0 that
+// the division gives there, and neither needs the scaling around the instruction that the forms which keep them take.
+__device__ __forceinline__ float bq_silu(float v) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(v, -1.4426950408889634f)));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fadd_rn(1.0f, e)));
+  return __fmul_rn(v, r);
+}
 
 __device__ __forceinline__ void bq_load8(const __nv_bfloat16* p, uint32_t (&w)[8]) {
   const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
@@ -96,15 +104,43 @@ __device__ __forceinline__ void bq_store_f32_all(float* mc, float v) {
   asm volatile("multimem.st.relaxed.sys.global.f32 [%0], %1;" ::"l"(mc), "f"(v) : "memory");
 }
 
-template <int TPB>
-__global__ void __launch_bounds__(TPB) block_quant_kernel(const BlockQuantParams p, int mul_in_smem) {
+// The sum over a block of NW warps (a power of two), in the order of block_reduce: its steps over lanes that hold zeros fall away.
+template <int NW>
+__device__ __forceinline__ float bq_block_sum(float v, float* slot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_reduce<OpSum>(v);
+  if (lane == 0) slot[warp] = v;
+  __syncthreads();
+  float r = slot[lane & (NW - 1)];
+#pragma unroll
+  for (int o = NW / 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
+}
+
+// What bounds it: instruction issue (64 to 68 % of the issue slots, 33 instructions an element with SiLU) and a chain of loads,
+// reductions and stores per row.  So the next row is loaded while this one is reduced and stored, the outputs' maxima go
+// through one barrier (their bit patterns as whole numbers, one redux instruction a warp), and the scales of the outputs,
+// two divisions each, are computed side by side in three lanes.  Before that a row's loads followed the last row's stores
+// and each output had a reduction of its own.  Before and after, L2 flushed: 16384 x 4096, addend, norm and three outputs
+// 188 -> 170 us (3.6 TB/s), two outputs 145 -> 131, plain rows 65 -> 58; SiLU 16384 x 14336 346 -> 301 (3.9 TB/s); 2048 rows of
+// them 39 -> 35, 31 -> 29, 16 -> 16 and 55 -> 47.
+// Resident blocks an SM.  One output fits 64 registers a thread, 1024 threads; the values of two or three between their maximum
+// and their codes, beside the next row, need 80.  At 64 they spill: 16384 x 4096, addend, norm and three outputs 207 us at 1024
+// threads, 170 at 768; two outputs 143 and 131.
+constexpr int bq_resident(int tpb, int nout) { return (nout >= 2 && tpb <= 256 ? 768 : 1024) / tpb; }
+
+// NOUT: the most outputs this instance takes (their values stay in registers between the maximum and the codes)
+template <int TPB, int NOUT>
+__global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT)) block_quant_kernel(const BlockQuantParams p, int mul_in_smem) {
   // The reciprocal SmoothQuant vectors are the same for every row: with `mul_in_smem` the block copies them into shared
   // memory once, quarter-transposed ([output][quarter][slice] of four floats) so that the four 16-byte reads of a
   // thread's slice are conflict free, instead of re-reading them through L1 for every row and output.
+  constexpr int NW = TPB / 32;
   extern __shared__ __align__(16) float mul_s[];
-  __shared__ float red[2][32];
+  __shared__ float red_sum[2][32];
+  __shared__ uint32_t red_max[2][NOUT][32];
   const int nchunks = p.cols >> 4;
-  const int ch = threadIdx.x;
+  const int ch = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool active = ch < nchunks;
   if (mul_in_smem) {
     for (int o = 0; o < p.nout; ++o) {
@@ -118,24 +154,34 @@ __global__ void __launch_bounds__(TPB) block_quant_kernel(const BlockQuantParams
   }
   const float eps = Elem<__nv_bfloat16>::rnd(p.dyn_eps);
   const float inv_cols = 1.0f / static_cast<float>(p.cols);
-  int flip = 0;
-  for (int row = blockIdx.x; row < p.rows; row += gridDim.x) {
-    uint32_t h[8];
+  const bool ahead_r = active && p.r != nullptr && p.prologue != QLIN_BLOCK_PLAIN && !p.r_multimem;
+  uint32_t h[8], a[8], nx[8], na[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) h[j] = 0u;
+  for (int j = 0; j < 8; ++j) h[j] = a[j] = nx[j] = na[j] = 0u;
+  if (active && blockIdx.x < p.rows) {
+    bq_load8(p.x + static_cast<int64_t>(blockIdx.x) * p.ldx + ch * 16, nx);
+    if (ahead_r) bq_load8(p.r + static_cast<int64_t>(blockIdx.x) * p.ldr + ch * 16, na);
+  }
+  int flip = 0;
+  for (int row = blockIdx.x; row < p.rows; row += gridDim.x, flip ^= 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = nx[j], a[j] = na[j];
+    // issued as soon as this row's inputs are used up, so that the next row needs no registers of its own before
+    const auto load_next = [&]() {
+      if (active && p.rows - row > static_cast<int>(gridDim.x)) {
+        const int64_t next = row + static_cast<int>(gridDim.x);
+        bq_load8(p.x + next * p.ldx + ch * 16, nx);
+        if (ahead_r) bq_load8(p.r + next * p.ldr + ch * 16, na);
+      }
+    };
     if (p.prologue == QLIN_BLOCK_NORM) {
       float ssq = 0.0f;
       if (active) {
-        bq_load8(p.x + static_cast<int64_t>(row) * p.ldx + ch * 16, h);
         if (p.r != nullptr) {
-          uint32_t a[8];
           const __nv_bfloat16* rp = p.r + static_cast<int64_t>(row) * p.ldr + ch * 16;
           if (p.r_multimem) {
             bq_load8_reduce(rp, a);  // the switch adds the row-parallel shards' partial outputs
-          } else {
-            bq_load8(rp, a);
-          }
-          if (p.r_parts > 1 && !p.r_multimem) {  // sum of the shards' partial outputs: fp32 in index order, one rounding
+          } else if (p.r_parts > 1) {  // sum of the shards' partial outputs: fp32 in index order, one rounding
             float acc[16];
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[2 * j] = bq_lo(a[j]), acc[2 * j + 1] = bq_hi(a[j]);
@@ -148,91 +194,107 @@ __global__ void __launch_bounds__(TPB) block_quant_kernel(const BlockQuantParams
             for (int j = 0; j < 8; ++j) a[j] = bq_pack(acc[2 * j], acc[2 * j + 1]);
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) h[j] = bq_pack(__fadd_rn(bq_lo(h[j]), bq_lo(a[j])), __fadd_rn(bq_hi(h[j]), bq_hi(a[j])));
+          for (int j = 0; j < 8; ++j) h[j] = bq_pack2(__fadd2_rn(bq_unpack(h[j]), bq_unpack(a[j])));
           if (p.x_out != nullptr) bq_store8(p.x_out + static_cast<int64_t>(row) * p.ldxo + ch * 16, h);
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) ssq += bq_lo(h[j]) * bq_lo(h[j]) + bq_hi(h[j]) * bq_hi(h[j]);
       }
-      ssq = block_reduce<OpSum>(ssq, red[flip], 0.0f);
-      flip ^= 1;
+      load_next();
+      ssq = bq_block_sum<NW>(ssq, red_sum[flip]);
       const float rstd = rsqrtf(ssq * inv_cols + p.norm_eps);
       if (active) {
         uint32_t w[8];
         bq_load8(p.norm_w + ch * 16, w);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = bq_pack(bq_lo(h[j]) * rstd * bq_lo(w[j]), bq_hi(h[j]) * rstd * bq_hi(w[j]));
+        for (int j = 0; j < 8; ++j) h[j] = bq_pack2(__fmul2_rn(__fmul2_rn(bq_unpack(h[j]), make_float2(rstd, rstd)), bq_unpack(w[j])));
       }
-    } else if (active) {
-      bq_load8(p.x + static_cast<int64_t>(row) * p.ldx + ch * 16, h);
+    } else {
       if (p.prologue == QLIN_BLOCK_SILU_MUL) {
-        uint32_t u[8];
-        bq_load8(p.r + static_cast<int64_t>(row) * p.ldr + ch * 16, u);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t sl = bq_pack(bq_silu(bq_lo(h[j])), bq_silu(bq_hi(h[j])));
-          h[j] = bq_pack(__fmul_rn(bq_lo(sl), bq_lo(u[j])), __fmul_rn(bq_hi(sl), bq_hi(u[j])));
+          h[j] = bq_pack2(__fmul2_rn(bq_unpack(sl), bq_unpack(a[j])));
         }
       }
+      load_next();
     }
     if (active && p.h_out != nullptr) bq_store8(p.h_out + static_cast<int64_t>(row) * p.ldh + ch * 16, h);
 
-    for (int o = 0; o < p.nout; ++o) {
-      uint32_t v[8];
+    uint32_t v[NOUT][8];
+#pragma unroll
+    for (int o = 0; o < NOUT; ++o) {
+      if (o >= p.nout) break;
       __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
       if (active) {
         if (p.mul[o] != nullptr) {
-          float m[16];
-          if (mul_in_smem) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float4 f = reinterpret_cast<const float4*>(mul_s)[(o * 4 + q) * nchunks + ch];
-              m[4 * q] = f.x, m[4 * q + 1] = f.y, m[4 * q + 2] = f.z, m[4 * q + 3] = f.w;
-            }
-          } else {
-            load16(p.mul[o] + ch * 16, m);
+          for (int q = 0; q < 4; ++q) {
+            const float4 f = mul_in_smem ? reinterpret_cast<const float4*>(mul_s)[(o * 4 + q) * nchunks + ch] : reinterpret_cast<const float4*>(p.mul[o])[ch * 4 + q];
+            v[o][2 * q] = bq_mul_pack(h[2 * q], make_float2(f.x, f.y));
+            v[o][2 * q + 1] = bq_mul_pack(h[2 * q + 1], make_float2(f.z, f.w));
           }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = bq_mul_pack(h[j], make_float2(m[2 * j], m[2 * j + 1]));
         } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = h[j];
+          for (int j = 0; j < 8; ++j) v[o][j] = h[j];
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v[j])));
+        for (int j = 0; j < 8; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v[o][j])));
       }
-      float s;
-      if (p.mode == QLIN_BLOCK_GIVEN_SCALE) {
-        s = p.scale_in[row];
-        // the shards of a row-parallel Linear each reported the scale of their slice: the row's scale is the largest
-        for (int k = 1; k < p.scale_in_parts; ++k) s = fmaxf(s, p.scale_in[k * p.scale_in_stride + row]);
-        if (threadIdx.x == 0 && p.scale_out[o] != nullptr) p.scale_out[o][row] = s;
-      } else {
-        float amax = fmaxf(__low2float(amax2), __high2float(amax2));
-        amax = block_reduce<OpMax>(amax, red[flip], 0.0f);
-        flip ^= 1;
-        s = Elem<__nv_bfloat16>::rnd(__fdiv_rn(fmaxf(amax, eps), static_cast<float>(p.levels)));
+      if (p.mode != QLIN_BLOCK_GIVEN_SCALE) {  // non-negative and never NaN: the order of the bit patterns is that of the values
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(amax2), __high2float(amax2))));
+        if (lane == 0) red_max[flip][o][warp] = top;
+      }
+    }
+    float s[NOUT], rs[NOUT];
+    if (p.mode == QLIN_BLOCK_GIVEN_SCALE) {  // one output
+      s[0] = p.scale_in[row];
+      // the shards of a row-parallel Linear each reported the scale of their slice: the row's scale is the largest
+      for (int k = 1; k < p.scale_in_parts; ++k) s[0] = fmaxf(s[0], p.scale_in[k * p.scale_in_stride + row]);
+      rs[0] = __frcp_rn(s[0]);
+#pragma unroll
+      for (int o = 1; o < NOUT; ++o) s[o] = s[0], rs[o] = rs[0];
+      if (threadIdx.x == 0 && p.scale_out[0] != nullptr) p.scale_out[0][row] = s[0];
+    } else if (p.nout > 0) {
+      __syncthreads();
+      uint32_t top[NOUT];
+#pragma unroll
+      for (int o = 0; o < NOUT; ++o) top[o] = o < p.nout ? __reduce_max_sync(0xffffffffu, red_max[flip][o][lane & (NW - 1)]) : 0u;
+      uint32_t mine = top[0];
+#pragma unroll
+      for (int o = 1; o < NOUT; ++o) mine = lane == o ? top[o] : mine;
+      const float amax = __uint_as_float(mine);
+      const float sl = Elem<__nv_bfloat16>::rnd(__fdiv_rn(fmaxf(amax, eps), static_cast<float>(p.levels)));
+      const float rsl = __frcp_rn(sl);
+#pragma unroll
+      for (int o = 0; o < NOUT; ++o) s[o] = NOUT == 1 ? sl : __shfl_sync(0xffffffffu, sl, o), rs[o] = NOUT == 1 ? rsl : __shfl_sync(0xffffffffu, rsl, o);
+#pragma unroll
+      for (int o = 0; o < NOUT; ++o) {
+        if (o >= p.nout) break;
         if (p.dst_multimem) {
           if (threadIdx.x == 0) {
-            bq_store_f32_all(reinterpret_cast<float*>(p.dst_base[0] + p.scale_off[o]) + p.dst_row0 + row, s);
-            if (p.ndst > 1) reinterpret_cast<float*>(p.dst_base[1] + p.scale_off[o])[p.dst_row0 + row] = s;
+            bq_store_f32_all(reinterpret_cast<float*>(p.dst_base[0] + p.scale_off[o]) + p.dst_row0 + row, s[o]);
+            if (p.ndst > 1) reinterpret_cast<float*>(p.dst_base[1] + p.scale_off[o])[p.dst_row0 + row] = s[o];
           }
         } else if (p.ndst > 0) {
           if (static_cast<int>(threadIdx.x) < p.ndst)
-            reinterpret_cast<float*>(p.dst_base[threadIdx.x] + p.scale_off[o])[p.dst_row0 + row] = s;
+            reinterpret_cast<float*>(p.dst_base[threadIdx.x] + p.scale_off[o])[p.dst_row0 + row] = s[o];
         } else if (threadIdx.x == 0 && p.scale_out[o] != nullptr) {
-          p.scale_out[o][row] = s;
+          p.scale_out[o][row] = s[o];
         }
       }
-      if (p.mode == QLIN_BLOCK_SCALE_ONLY || !active) continue;
-      const float rs = __frcp_rn(s);
-      const float2 rs2 = make_float2(rs, rs);
+    }
+    if (p.mode == QLIN_BLOCK_SCALE_ONLY || !active) continue;
+#pragma unroll
+    for (int o = 0; o < NOUT; ++o) {
+      if (o >= p.nout) break;
+      const float2 rs2 = make_float2(rs[o], rs[o]);
       const float2 magic = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the sum's low mantissa byte is rint's code
       uint32_t out[4];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const float2 qa = __fadd2_rn(bq_unpack(bq_mul_pack(v[2 * g], rs2)), magic);
-        const float2 qb = __fadd2_rn(bq_unpack(bq_mul_pack(v[2 * g + 1], rs2)), magic);
+        const float2 qa = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g], rs2)), magic);
+        const float2 qb = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g + 1], rs2)), magic);
         out[g] = __byte_perm(__byte_perm(__float_as_uint(qa.x), __float_as_uint(qa.y), 0x0040),
                              __byte_perm(__float_as_uint(qb.x), __float_as_uint(qb.y), 0x0040), 0x5410);
       }
@@ -295,20 +357,19 @@ __global__ void __launch_bounds__(256) rope_kernel(const RopeParams p) {
   }
 }
 
-template <int TPB>
-static int launch_block_quant_tpb(const BlockQuantParams& p, cudaStream_t s) {
+template <int TPB, int NOUT>
+static int launch_block_quant_n(const BlockQuantParams& p, cudaStream_t s) {
   static bool configured[64] = {};
   constexpr int kSmemMax = TPB >= 1024 ? 98304 : 49152;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(block_quant_kernel<TPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
+    if (cudaFuncSetAttribute(block_quant_kernel<TPB, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
       return fail(QLIN_ERR_LAUNCH, "cudaFuncSetAttribute failed for qlin_block_quant");
     configured[dev] = true;
   }
-  // resident blocks per SM by registers (64 per thread): 1024 threads
-  const int per_sm = TPB >= 1024 ? 2 : (TPB >= 512 ? 2 : 2 * (1024 / TPB));
-  int grid = sm_count() * per_sm;
+  // the blocks that are resident: each walks over its rows and loads ahead
+  int grid = sm_count() * bq_resident(TPB, NOUT);
   if (grid > p.rows) grid = p.rows;
   if (p.max_ctas > 0) {  // the cap counts blocks of 256 threads
     int cap = TPB >= 256 ? p.max_ctas : p.max_ctas * (256 / TPB);
@@ -316,10 +377,16 @@ static int launch_block_quant_tpb(const BlockQuantParams& p, cudaStream_t s) {
     if (grid > cap) grid = cap;
   }
   const int smem = p.nout * p.cols * 4;
-  const bool in_smem = smem > 0 && smem <= kSmemMax && p.rows >= 4 * grid;
-  block_quant_kernel<TPB><<<grid, TPB, in_smem ? smem : 0, s>>>(p, in_smem ? 1 : 0);
+  const bool in_smem = smem > 0 && smem <= kSmemMax && p.rows >= 8 * grid;
+  block_quant_kernel<TPB, NOUT><<<grid, TPB, in_smem ? smem : 0, s>>>(p, in_smem ? 1 : 0);
   QLIN_CHECK_LAUNCH("qlin_block_quant");
   return QLIN_OK;
+}
+
+template <int TPB>
+static int launch_block_quant_tpb(const BlockQuantParams& p, cudaStream_t s) {
+  if (p.nout <= 1) return launch_block_quant_n<TPB, 1>(p, s);
+  return p.nout == 2 ? launch_block_quant_n<TPB, 2>(p, s) : launch_block_quant_n<TPB, 3>(p, s);
 }
 
 static int launch_block_quant(const BlockQuantParams& p, int nchunks, cudaStream_t s) {

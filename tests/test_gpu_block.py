@@ -59,6 +59,27 @@ def test_norm_prologue_with_residual(cuda_dev):
     assert xo2 is None and torch.equal(h2, h) and all(torch.equal(a, b) for a, b in zip(codes, codes2))
 
 
+@pytest.mark.parametrize("max_ctas", [1, 2, 5])
+@pytest.mark.parametrize("nout,K", [(1, 4096), (1, 14336), (2, 4096), (3, 4096), (2, 528), (3, 8192), (0, 2048)])
+def test_blocks_that_walk_over_rows(cuda_dev, max_ctas, nout, K):
+    """A block that owns several rows loads ahead and reuses its reduction slots: same results as one block a row, in place too."""
+    T = 19
+    g = torch.Generator().manual_seed(K + nout)
+    x, r = (torch.randn(T, K, generator=g) * 2).bfloat16().to(cuda_dev), torch.randn(T, K, generator=g).bfloat16().to(cuda_dev)
+    x[3], r[3] = 0, 0
+    w = (1 + 0.1 * torch.randn(K, generator=g)).bfloat16().to(cuda_dev)
+    rcps = [ops.smooth_reciprocal(_smooth(K, 11 + i).float().to(cuda_dev)) for i in range(nout)]
+    for kw in (dict(), dict(prologue=L.BLOCK_SILU_MUL, r=r), dict(prologue=L.BLOCK_NORM, r=r, norm_w=w), dict(prologue=L.BLOCK_NORM, norm_w=w)):
+        want = ops.block_quant(x, smooth_rcps=rcps, want_h=True, store_sum="norm_w" in kw, **kw)
+        xin = x.clone()
+        into = dict(sum_into=xin) if kw.get("prologue") == L.BLOCK_NORM and "r" in kw else {}
+        got = ops.block_quant(xin, smooth_rcps=rcps, want_h=True, max_ctas=max_ctas, **kw, **into)
+        for a, b in zip((*got[0], *got[1], got[3]), (*want[0], *want[1], want[3])):
+            assert torch.equal(a, b)
+        if into:
+            assert torch.equal(xin, want[2])
+
+
 def test_silu_mul_prologue_and_two_pass_given_scale(cuda_dev):
     T, K = 23, 7168
     g = torch.Generator().manual_seed(2)
