@@ -6,12 +6,15 @@
 // codes of the gradient both ways, those of x and W transposed, and the column sums of the gradient's codes; both GEMM
 // operands are K-major.
 //
-// HBM-bound: s bytes read and one or two bytes written per element.  A block walks over 128 x 64 tiles; a thread quantises
-// two 16-element slices, the transposed copy goes through a swizzled shared tile of 4-byte words, read back as 8 rows x 4
-// columns per thread and turned with byte permutes, so both outputs are written in runs of 64 and 128 bytes.
+// Bound by HBM and, at a few tiles a block, by the latency of a tile: s bytes read and one or two bytes written per element.  The
+// resident blocks walk over 128 x 64 tiles; a thread quantises two 16-element slices and loads each slice of its next tile as soon
+// as it has used this one's (the first tile's before the maximum is known); the transposed copy goes through a swizzled
+// shared tile of 4-byte words, read back as 8 rows x 4 columns per thread and turned with byte permutes, so both outputs are
+// written in runs of 64 and 128 bytes.
 //
-// 4096 x 4096 bf16, before: 9.3 us statistics + 2.9 us finish + 73 us generic quantiser + 66 us byte transpose (and 42 us for
-// the column sums through an fp32 copy); now 9.3 us for the partial maxima and 17.5 us for the codes, either or both ways.
+// Codes, or codes both ways, L2 flushed, before (half as many blocks again as fit, no load ahead, four-way conflicts in the
+// stores to shared memory) and after: 4096 x 4096 bf16 22.5 -> 18.4 and 24.6 -> 20.5 us, 8192 x 8192 bf16 63.5 -> 43.0 and
+// 79.9 -> 53.3 (5.0 TB/s), fp32 71.7 -> 65.6 and 88.1 -> 77.9.
 #include <type_traits>
 
 #include <cuda_fp8.h>
@@ -134,10 +137,69 @@ __device__ __forceinline__ void transpose4(const uint32_t (&a)[4], uint32_t (&ou
   out[3] = __byte_perm(t2, t3, 0x7632);
 }
 
+// Sixteen elements as they lie in memory.
 template <typename XT>
-__global__ void __launch_bounds__(kF8Threads) f8_tensor_quant_kernel(const F8TensorParams p) {
-  __shared__ uint32_t tile[kF8TileM * (kF8TileN / 4)];  // word (row, c4) at row * 16 + (c4 ^ (row / 8))
+struct F8Raw {
+  static constexpr int kWords = 4 * static_cast<int>(sizeof(XT));
+  uint32_t w[kWords];
+};
+__device__ __forceinline__ uint32_t f8_bits(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ uint32_t f8_bits(__half v) { return __half_as_ushort(v); }
+__device__ __forceinline__ uint32_t f8_bits(__nv_bfloat16 v) { return __bfloat16_as_ushort(v); }
+
+// Columns col .. col + 15 of `row`, zeros outside the tensor.
+template <typename XT>
+__device__ __forceinline__ void f8_fetch(const F8TensorParams& p, bool vec, int row, int col, F8Raw<XT>& raw) {
+  constexpr int kPer = 4 / static_cast<int>(sizeof(XT));  // elements a word
+  const XT* src = reinterpret_cast<const XT*>(p.x) + static_cast<int64_t>(row) * p.ldx + col;
+  if (row < p.rows && vec && col + 16 <= p.cols) {
+#pragma unroll
+    for (int i = 0; i < F8Raw<XT>::kWords / 4; ++i) {
+      const uint4 q = reinterpret_cast<const uint4*>(src)[i];
+      raw.w[4 * i] = q.x, raw.w[4 * i + 1] = q.y, raw.w[4 * i + 2] = q.z, raw.w[4 * i + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < F8Raw<XT>::kWords; ++i) raw.w[i] = 0u;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (row < p.rows && col + j < p.cols) raw.w[j / kPer] |= f8_bits(src[j]) << (16 * (j % kPer));
+  }
+}
+__device__ __forceinline__ void f8_widen(const F8Raw<float>& r, float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r.w[j]);
+}
+__device__ __forceinline__ void f8_widen(const F8Raw<__half>& r, float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r.w[j]));
+    v[2 * j] = f.x, v[2 * j + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void f8_widen(const F8Raw<__nv_bfloat16>& r, float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[2 * j] = __uint_as_float(r.w[j] << 16), v[2 * j + 1] = __uint_as_float(r.w[j] & 0xFFFF0000u);
+}
+
+// Resident blocks an SM; a block walks over its tiles, and each slice of the next one is loaded as soon as this tile's is used up.
+template <typename XT>
+constexpr int f8_resident() { return sizeof(XT) == 4 ? 3 : 4; }
+
+template <typename XT>
+__global__ void __launch_bounds__(kF8Threads, f8_resident<XT>()) f8_tensor_quant_kernel(const F8TensorParams p) {
+  __shared__ uint32_t tile[kF8TileM * (kF8TileN / 4)];  // word (row, c4) at row * 16 + (c4 ^ (row / 8) ^ (row / 2 % 4)): stores without conflicts, loads two-way
   __shared__ float red[32];
+  const int tiles_n = (p.cols + kF8TileN - 1) / kF8TileN, tiles_m = (p.rows + kF8TileM - 1) / kF8TileM;
+  const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
+  const bool vec_x = (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && (p.ldx * static_cast<int64_t>(sizeof(XT))) % 16 == 0;
+  F8Raw<XT> raw[2];
+  const auto fetch = [&](int64_t t, int h) {
+    const int id = threadIdx.x + h * kF8Threads;
+    f8_fetch(p, vec_x, static_cast<int>(t / tiles_n) * kF8TileM + (id >> 2), static_cast<int>(t % tiles_n) * kF8TileN + (id & 3) * 16, raw[h]);
+  };
+  fetch(blockIdx.x, 0);  // under way while the maximum is found; the grid has no more blocks than tiles
+  fetch(blockIdx.x, 1);
   float am = 0.0f;
   for (int i = threadIdx.x; i < p.nparts; i += kF8Threads) am = fmaxf(am, p.parts[i]);
   am = block_reduce<OpMax>(am, red, 0.0f);
@@ -146,34 +208,20 @@ __global__ void __launch_bounds__(kF8Threads) f8_tensor_quant_kernel(const F8Ten
   const float rs = rcp_for_div(s);
   const bool fast = rs == rs;
   const bool e5m2 = p.e5m2 != 0, flush = p.dl8_flush != 0;
-  const XT* x = reinterpret_cast<const XT*>(p.x);
-  const bool vec_x = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (p.ldx * static_cast<int64_t>(sizeof(XT))) % 16 == 0;
   const bool vec_q = (reinterpret_cast<uintptr_t>(p.codes) & 15u) == 0 && p.ldq % 16 == 0;
   const bool turn = p.codes_t != nullptr || p.colsum_ws != nullptr;
-  const int tiles_n = (p.cols + kF8TileN - 1) / kF8TileN, tiles_m = (p.rows + kF8TileM - 1) / kF8TileM;
-  const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
     const int tm = static_cast<int>(t / tiles_n), tn = static_cast<int>(t % tiles_n);
     const int row0 = tm * kF8TileM, col0 = tn * kF8TileN;
-    float v[2][16];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int id = threadIdx.x + h * kF8Threads;
-      const int row = row0 + (id >> 2), col = col0 + (id & 3) * 16;
-      const XT* src = x + static_cast<int64_t>(row) * p.ldx + col;
-      if (row < p.rows && vec_x && col + 16 <= p.cols) {
-        load16(src, v[h]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[h][j] = (row < p.rows && col + j < p.cols) ? load1(src + j) : 0.0f;
-      }
-    }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int id = threadIdx.x + h * kF8Threads;
       const int r = id >> 2, row = row0 + r, col = col0 + (id & 3) * 16;
+      float v[16];
+      f8_widen(raw[h], v);
+      if (t + gridDim.x < tiles) fetch(t + gridDim.x, h);
       uint32_t w[4];
-      f8_codes16<XT>(v[h], s, rs, fast, e5m2, flush, w);
+      f8_codes16<XT>(v, s, rs, fast, e5m2, flush, w);
       if (row >= p.rows || col >= p.cols) {  // padding of the transposed rows: zeros (a zero scale makes NaN of 0 / s)
 #pragma unroll
         for (int g = 0; g < 4; ++g) w[g] = 0u;
@@ -190,7 +238,7 @@ __global__ void __launch_bounds__(kF8Threads) f8_tensor_quant_kernel(const F8Ten
       }
       if (turn) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) tile[r * 16 + ((((id & 3) * 4) + g) ^ (r >> 3))] = w[g];
+        for (int g = 0; g < 4; ++g) tile[r * 16 + ((((id & 3) * 4) + g) ^ (r >> 3) ^ ((r >> 1) & 3))] = w[g];
       }
     }
     if (!turn) continue;
@@ -199,8 +247,8 @@ __global__ void __launch_bounds__(kF8Threads) f8_tensor_quant_kernel(const F8Ten
     uint32_t a[4], b[4], lo[4], hi[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      a[i] = tile[(rg * 8 + i) * 16 + (c4 ^ rg)];
-      b[i] = tile[(rg * 8 + 4 + i) * 16 + (c4 ^ rg)];
+      a[i] = tile[(rg * 8 + i) * 16 + (c4 ^ rg ^ (i >> 1))];
+      b[i] = tile[(rg * 8 + 4 + i) * 16 + (c4 ^ rg ^ (2 + (i >> 1)))];
     }
     transpose4(a, lo);
     transpose4(b, hi);
@@ -249,7 +297,7 @@ static int abs_parts(int64_t numel) {
 template <typename XT>
 static int launch_f8_tensor(const F8TensorParams& p, cudaStream_t stream) {
   const int64_t tiles = static_cast<int64_t>((p.rows + kF8TileM - 1) / kF8TileM) * ((p.cols + kF8TileN - 1) / kF8TileN);
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 6;
+  const int64_t cap = static_cast<int64_t>(sm_count()) * f8_resident<XT>();
   f8_tensor_quant_kernel<XT><<<static_cast<int>(tiles < cap ? tiles : cap), kF8Threads, 0, stream>>>(p);
   QLIN_CHECK_LAUNCH("qlin_f8_tensor_quant");
   return QLIN_OK;

@@ -52,3 +52,17 @@ def test_per_tensor_codes(cuda_dev, rows, cols, dtype, kind):
                 ok = (colsum.double() - ref).abs() <= bound
                 assert bool((ok | ~torch.isfinite(ref)).all())
     ops.check_status(cuda_dev)
+
+
+@pytest.mark.parametrize("rows,cols,pitch", [(2085, 3000, 3000), (2560, 2048, 2048), (130, 64 * 620 + 16, 64 * 620 + 19)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+def test_blocks_that_walk_over_tiles(cuda_dev, rows, cols, pitch, dtype):
+    """More tiles than resident blocks: the next tile is loaded while this one is written; ragged edges, rows off 16 bytes."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, pitch, generator=g, device="cuda").to(dtype)[:, :cols]
+    parts = ops.absmax_parts(x.contiguous())
+    for e5m2, eps in ((False, 1e-5), (True, 0.0)):
+        want, ws = _general(x.contiguous(), e5m2, eps, False)
+        codes, codes_t, scale, _ = ops.fp8_quant_tensor(x, parts, e5m2=e5m2, eps=eps, want_t=True, want_colsum=e5m2)
+        assert torch.equal(scale, ws) and torch.equal(codes.view(torch.uint8), want.view(torch.uint8))
+        assert torch.equal(codes_t.view(torch.uint8), codes.view(torch.uint8).t())
