@@ -521,7 +521,7 @@ struct QatShape {
   int64_t tokens, in, out;
 };
 
-// The operands' arguments of one pass; `floats` is [2 * out + 1]: scales, their reciprocals, the step.
+// The operands' arguments of one pass; `floats` is [2 * out + 2]: scales, their reciprocals, the step and its clip value.
 qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, const Tensor& flags, const QatShape& n) {
   qlin_qat_args a = {};
   a.x = static_cast<const float*>(data(x));
@@ -529,6 +529,7 @@ qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, c
   a.scale = static_cast<float*>(data(floats));
   a.rcp = a.scale + n.out;
   a.step = a.scale + 2 * n.out;
+  a.clip_kept = a.step + 1;
   a.flags = static_cast<int32_t*>(data(flags));
   a.status = static_cast<int32_t*>(status_word(x.device().index()).data_ptr());
   a.tokens = static_cast<int32_t>(n.tokens);
@@ -544,7 +545,7 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
     const at::Device dev = x.device();
     const c10::cuda::CUDAGuard guard(dev);
     const QatShape n{x.numel() / x.size(-1), x.size(-1), w.size(0)};
-    const Tensor floats = empty({2 * n.out + 1}, at::kFloat, dev), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
+    const Tensor floats = empty({2 * n.out + 2}, at::kFloat, dev), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
     const Tensor xc = empty({n.tokens, n.in}, at::kBFloat16, dev), wc = empty({n.out, n.in}, at::kBFloat16, dev);
     std::vector<int64_t> shape = x.sizes().vec();
     shape.back() = n.out;

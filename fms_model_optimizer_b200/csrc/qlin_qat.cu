@@ -19,8 +19,8 @@
 // tensor cycles) are limited by what three of them keep in flight from L2; then the split of the gradient (HBM).  Forward and
 // backward of 4096 x 768 x 3072: 1124 us of device time with the library's fp32 GEMMs, 212 with this.
 //
-// What the argument rests on is checked where the operands are made: a value that is no such multiple (another quantizer's
-// output, a hook's), a scale out of range, an infinity or NaN in the gradient, or a gradient element so small (below 2^-100)
+// What the argument rests on is checked where the operands are made: a value that is not bit for bit what the quantizer makes of a
+// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, or a gradient element so small (below 2^-100)
 // that its third part could leave bf16's range raises a flag on the device, and the last kernel of each product, which is
 // always launched, then computes it in fp32 from the operands themselves.  With no flag up it returns at once.
 #include <cuda.h>
@@ -34,7 +34,6 @@ namespace qlin {
 
 // ------------------------------------------------------------------------------------------------ operands
 constexpr float kMaxCode = 256.0f;                // whole numbers up to here are bf16 numbers
-constexpr float kCodeSlack = 3.0517578125e-5f;    // 2^-15 of a step: the rounding of a symmetric quantizer's k * step - clip
 constexpr float kTiny = 7.888609052210118e-31f;   // 2^-100
 constexpr float kHuge = 8.5070591730234616e37f;   // 2^126
 constexpr int kPrepThreads = 256;
@@ -46,6 +45,7 @@ struct QatCodesParams {
   const float* clip;    // activations: clip_val [1]; weights: one per row
   const float* clipn;   // two-sided activations: clip_valn [1]
   float* scale;         // activations: step [1]; weights: s [rows]
+  float* clip_kept;     // symmetric activations: the clip value of the forward pass [1]
   float* rcp;           // weights: 1 / s [rows]
   int32_t* flags;       // one per block
   int64_t ldo;
@@ -74,11 +74,19 @@ __device__ __forceinline__ bool scale_ok(float s) {
   return a > 1e-18f && a < 1e18f;
 }
 
-// The whole number of steps in x; `bad` is raised where x is not one (NaN passes as NaN).
+// The whole number of steps in x; `bad` is raised where x is not the fp32 product of one (NaN passes as NaN).
 __device__ __forceinline__ float code_of(float x, float step, float rstep, bool& bad) {
-  const float u = div_exact(x, step, rstep);
-  const float c = rintf(u);
-  bad |= !(fabsf(u - c) <= kCodeSlack && fabsf(c) <= kMaxCode) && x == x;
+  const float c = rintf(div_exact(x, step, rstep));
+  bad |= !(x == __fmul_rn(c, step) && fabsf(c) <= kMaxCode) && x == x;
+  return c;
+}
+
+// The symmetric quantizer's values are not products but k * step - clip with k = 0 .. 2 half, up to 2^-15 of a step off the
+// multiple k - half of the step that they stand for.  So `bad` is raised where x is not that expression of a whole number.
+__device__ __forceinline__ float code_of_sym(float x, float step, float rstep, float clip, float half, bool& bad) {
+  const float k = rintf(div_exact(__fadd_rn(x, clip), step, rstep));
+  const float c = k - half;
+  bad |= !(x == __fsub_rn(__fmul_rn(k, step), clip) && fabsf(c) <= kMaxCode) && x == x;
   return c;
 }
 
@@ -91,21 +99,27 @@ __device__ __forceinline__ uint32_t pack_codes(float a, float b) {
 __global__ void __launch_bounds__(kPrepThreads) qat_act_codes_kernel(const QatCodesParams p) {
   const float step = p.given ? *p.scale : act_step(p), rstep = rcp_for_div(step);
   bool bad = !scale_ok(step);
+  const bool sym = p.variant == QLIN_PACT_SYMMETRIC;
+  const float clip = !sym ? 0.0f : (p.given ? *p.clip_kept : *p.clip), half = static_cast<float>((1 << (p.num_bits - 1)) - 1);
+  const auto code = [&](float v) { return sym ? code_of_sym(v, step, rstep, clip, half, bad) : code_of(v, step, rstep, bad); };
   const int per_row = p.cols / 8;
   const int64_t total = static_cast<int64_t>(p.rows) * per_row;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kPrepThreads + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * kPrepThreads) {
     const float4 a = reinterpret_cast<const float4*>(p.x)[2 * i], b = reinterpret_cast<const float4*>(p.x)[2 * i + 1];
     uint4 o;
-    o.x = pack_codes(code_of(a.x, step, rstep, bad), code_of(a.y, step, rstep, bad));
-    o.y = pack_codes(code_of(a.z, step, rstep, bad), code_of(a.w, step, rstep, bad));
-    o.z = pack_codes(code_of(b.x, step, rstep, bad), code_of(b.y, step, rstep, bad));
-    o.w = pack_codes(code_of(b.z, step, rstep, bad), code_of(b.w, step, rstep, bad));
+    o.x = pack_codes(code(a.x), code(a.y));
+    o.y = pack_codes(code(a.z), code(a.w));
+    o.z = pack_codes(code(b.x), code(b.y));
+    o.w = pack_codes(code(b.z), code(b.w));
     reinterpret_cast<uint4*>(p.codes)[i] = o;
   }
   const int any = __syncthreads_or(bad);
   if (threadIdx.x == 0) {
     p.flags[blockIdx.x] = any;
-    if (blockIdx.x == 0 && !p.given) *p.scale = step;
+    if (blockIdx.x == 0 && !p.given) {
+      *p.scale = step;
+      if (sym) *p.clip_kept = clip;
+    }
   }
 }
 
@@ -737,6 +751,7 @@ extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* st
   if (a->flags == nullptr || a->step == nullptr || a->scale == nullptr || a->rcp == nullptr ||
       (!backward && (a->clip_x == nullptr || a->clip_w == nullptr || (a->variant == QLIN_PACT_TWO_SIDED && a->clipn_x == nullptr))))
     return fail(QLIN_ERR_NULL, "qlin_qat_codes: a pointer is NULL");
+  if (a->variant == QLIN_PACT_SYMMETRIC && a->clip_kept == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_codes: the symmetric quantizer needs clip_kept");
   if (!aligned16(a->x) || !aligned16(a->w) || !aligned16(a->x_codes) || !aligned16(a->w_codes)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_codes: 16-byte alignment");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   QatCodesParams p = {};
@@ -749,6 +764,7 @@ extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* st
     p.clip = a->clip_x;
     p.clipn = a->clipn_x;
     p.scale = a->step;
+    p.clip_kept = a->clip_kept;
     p.flags = a->flags;
     p.rows = a->tokens;
     p.cols = a->in;

@@ -623,6 +623,7 @@ typedef struct qlin_qat_args {
   int32_t tokens, in, out;
   int32_t num_bits_x, num_bits_w;
   int32_t variant;      /* qlin_pact_variant of x's quantizer */
+  float* clip_kept;     /* [1], QLIN_PACT_SYMMETRIC: written by the forward pass, read by both */
 } qlin_qat_args;
 
 int32_t qlin_qat_flag_count(void);

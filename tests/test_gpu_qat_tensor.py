@@ -4,6 +4,8 @@ that are differentiated again, and the rule that leaves a call to the library.
 
 Bound: a product of n terms summed in fp32 in any order is within 8 sqrt(n) 2^-24 of the sum of the terms' absolute values."""
 
+import ctypes as C
+
 import pytest
 import torch
 
@@ -14,10 +16,13 @@ from fms_model_optimizer_b200.modules.linear import _ordinary_call
 gpu = pytest.mark.gpu
 
 
-def _operands(t, k, n, clips=(3.0, -2.5)):
+MODES = {"two-sided": L.PACT_TWO_SIDED, "one-sided": L.PACT_ONE_SIDED, "symmetric": L.PACT_SYMMETRIC}
+
+
+def _operands(t, k, n, clips=(3.0, -2.5), mode="two-sided"):
     g = torch.Generator(device="cuda").manual_seed(t + k + n)
-    lin = QLinear(k, n, num_bits_feature=8, qa_mode="pact+", num_bits_weight=8, qw_mode="sawb+perCh", act_clip_init_val=clips[0], act_clip_init_valn=clips[1],
-                  device="cuda").train()  # fmt: skip
+    lin = QLinear(k, n, num_bits_feature=8, qa_mode="pactsym+" if mode == "symmetric" else "pact+", num_bits_weight=8, qw_mode="sawb+perCh",
+                  act_clip_init_val=clips[0], act_clip_init_valn=clips[1], non_neg=mode == "one-sided", device="cuda").train()  # fmt: skip
     with torch.no_grad():
         lin.weight.copy_(torch.randn(n, k, generator=g, device="cuda") * 0.02)
         x = lin.quantize_feature(torch.randn(t, k, generator=g, device="cuda")).detach().requires_grad_(True)
@@ -25,9 +30,40 @@ def _operands(t, k, n, clips=(3.0, -2.5)):
     return lin, x, w, torch.randn(t, n, generator=g, device="cuda")
 
 
-def _run(lin, x, w):
+def _run(lin, x, w, mode="two-sided"):
     Qa, Qw = lin.quantize_feature, lin.quantize_weight
-    return L.host().qat_linear(x, w, lin.bias, Qa.clip_val, Qa.clip_valn, Qw.clip_val, 8, 8, L.PACT_TWO_SIDED)
+    return L.host().qat_linear(x, w, lin.bias, Qa.clip_val, getattr(Qa, "clip_valn", None), Qw.clip_val, 8, 8, MODES[mode])
+
+
+class _Args(C.Structure):  # qlin_qat_args
+    _fields_ = [(f, C.c_void_p) for f in ("x", "w", "g", "bias", "clip_x", "clipn_x", "clip_w", "step", "scale", "rcp", "x_codes", "w_codes", "g_planes", "d", "colsum",
+                                          "workspace", "flags", "status")]  # fmt: skip
+    _fields_ += [(f, C.c_int32) for f in ("tokens", "inp", "out", "num_bits_x", "num_bits_w", "variant")] + [("clip_kept", C.c_void_p)]
+
+
+def _flags(lin, x, w, go, mode="two-sided", replaced=None):
+    """Whether (x, w) of the forward pass and (x, w, gradient) of the backward pass raise their flags, through the C entry points.
+    ``replaced`` is called between the passes."""
+    lib, t, k, n = L.load(), x.shape[0], x.shape[1], w.shape[0]
+    Qa, Qw = lin.quantize_feature, lin.quantize_weight
+    buf = {"x_codes": torch.empty(t * k, dtype=torch.bfloat16, device="cuda"), "w_codes": torch.empty(n * k, dtype=torch.bfloat16, device="cuda"),
+           "g_planes": torch.empty(3 * t * n, dtype=torch.bfloat16, device="cuda"), "step": torch.empty(1, device="cuda"), "scale": torch.empty(n, device="cuda"),
+           "rcp": torch.empty(n, device="cuda"), "clip_kept": torch.empty(1, device="cuda"), "x": x.detach(), "w": w.detach(), "g": go, "clip_x": Qa.clip_val.detach(),
+           "clip_w": Qw.clip_val}  # fmt: skip
+    if mode == "two-sided":
+        buf["clipn_x"] = Qa.clip_valn.detach()
+    res = []
+    for backward in (0, 1):
+        flags = torch.zeros(lib.qlin_qat_flag_count(), dtype=torch.int32, device="cuda")
+        a = _Args(flags=flags.data_ptr(), tokens=t, inp=k, out=n, num_bits_x=8, num_bits_w=8, variant=MODES[mode], **{f: v.data_ptr() for f, v in buf.items()})
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        L.check(lib.qlin_qat_codes(C.byref(a), C.c_int32(backward), stream), "qlin_qat_codes")
+        if backward:
+            L.check(lib.qlin_qat_split(C.byref(a), stream), "qlin_qat_split")
+        res += [bool(v) for v in (flags.view(3, -1) != 0).any(1).tolist()[: 3 if backward else 2]]
+        if replaced is not None:
+            replaced()
+    return tuple(res)
 
 
 def _check(lin, x, w, go, out, grads):
@@ -72,6 +108,28 @@ def test_operands_the_codes_cannot_carry(cuda_dev, what):
         buf[1:] = go.flatten()
         go = buf[1:].view(t, n)
     _check(lin, x, w, go, out, torch.autograd.grad(out, [x, w, lin.bias], go))
+
+
+@gpu
+@pytest.mark.parametrize("mode", list(MODES))
+def test_operands_that_a_hook_changed(cuda_dev, mode):
+    """An operand scaled far below a step, and one element a single place off, are multiplied as they are."""
+    t, k, n = 300, 264, 200
+    lin, x, w, go = _operands(t, k, n, mode=mode)
+    assert _flags(lin, x, w, go, mode) == (False,) * 5
+    with torch.no_grad():
+        lin.bias.zero_()
+    for what in ("x", "w"):
+        sx, sw = (1e-7, 1.0) if what == "x" else (1.0, 1e-7)
+        xs, ws = (x.detach() * sx).requires_grad_(True), (w.detach() * sw).requires_grad_(True)
+        assert _flags(lin, xs, ws, go, mode) == (what == "x", what == "w", what == "x", what == "w", False)
+        out = _run(lin, xs, ws, mode)
+        _check(lin, xs, ws, go, out, torch.autograd.grad(out, [xs, ws, lin.bias], go))
+        x1, w1 = x.detach().clone(), w.detach().clone()
+        e = (x1 if what == "x" else w1).view(-1)
+        i = int(e.abs().argmax())
+        e[i] = torch.nextafter(e[i], torch.zeros((), device="cuda"))
+        assert _flags(lin, x1, w1, go, mode) == (what == "x", what == "w", what == "x", what == "w", False)
 
 
 @gpu
