@@ -20,9 +20,12 @@
 // backward of 4096 x 768 x 3072: 1124 us of device time with the library's fp32 GEMMs, 212 with this.
 //
 // What the argument rests on is checked where the operands are made: a value that is not bit for bit what the quantizer makes of a
-// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, or a gradient element so small (below 2^-100)
-// that its third part could leave bf16's range raises a flag on the device, and the last kernel of each product, which is
+// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element so large that a sum of its products with
+// codes could leave fp32's range (which the product with the operand itself need not), or one so small (below 2^-100) that its third
+// part could leave bf16's range raises a flag on the device, and the last kernel of each product, which is
 // always launched, then computes it in fp32 from the operands themselves.  With no flag up it returns at once.
+#include <cmath>
+
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -35,7 +38,8 @@ namespace qlin {
 // ------------------------------------------------------------------------------------------------ operands
 constexpr float kMaxCode = 256.0f;                // whole numbers up to here are bf16 numbers
 constexpr float kTiny = 7.888609052210118e-31f;   // 2^-100
-constexpr float kHuge = 8.5070591730234616e37f;   // 2^126
+// |g s| below 2^(kSumExp - e), 2^e >= the longer contraction: a sum of 2^e products with codes of up to 2^8 stays below 2^126.
+constexpr int kSumExp = 118;
 constexpr int kPrepThreads = 256;
 constexpr int kQatFlagSlots = 1184;  // flags of each kernel that makes an operand
 
@@ -183,6 +187,7 @@ struct QatSplitParams {
   int32_t* flags;
   float* sums;            // optional [row blocks][cols]: each block's column sums
   int32_t rows, cols, block_rows;
+  float huge;
 };
 constexpr int kSplitThreads = 128;  // eight columns a thread
 
@@ -215,8 +220,8 @@ __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplit
       for (int j = 0; j < 8; j += 2) {
         float2 t = __fmul2_rn(make_float2(v[j], v[j + 1]), make_float2(s[j], s[j + 1]));
         // not finite, too large or too small (a NaN fails every comparison); an exact zero is fine
-        bad |= !(fabsf(t.x) >= kTiny && fabsf(t.x) <= kHuge) && !(v[j] == 0.0f);
-        bad |= !(fabsf(t.y) >= kTiny && fabsf(t.y) <= kHuge) && !(v[j + 1] == 0.0f);
+        bad |= !(fabsf(t.x) >= kTiny && fabsf(t.x) <= p.huge) && !(v[j] == 0.0f);
+        bad |= !(fabsf(t.y) >= kTiny && fabsf(t.y) <= p.huge) && !(v[j + 1] == 0.0f);
         sum[j] += v[j];
         sum[j + 1] += v[j + 1];
 #pragma unroll
@@ -731,6 +736,11 @@ static int split_block_rows(const qlin_qat_args* a) {
   return need > 16 ? need : 16;
 }
 static int split_row_blocks(const qlin_qat_args* a) { return (a->tokens + split_block_rows(a) - 1) / split_block_rows(a); }
+static float split_huge(const qlin_qat_args* a) {
+  int e = 0;
+  while ((int64_t{1} << e) < (a->tokens > a->out ? a->tokens : a->out)) ++e;
+  return std::ldexp(1.0f, kSumExp - e);
+}
 static int split_grid(const qlin_qat_args* a) { return split_row_blocks(a) * split_strips(a); }
 
 }  // namespace qlin
@@ -797,7 +807,7 @@ extern "C" int qlin_qat_split(const qlin_qat_args* a, void* stream) {
   if (!aligned16(a->g_planes) || !aligned16(a->scale)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_split: 16-byte alignment");
   if (a->colsum != nullptr && (a->workspace == nullptr || !aligned16(a->workspace))) return fail(QLIN_ERR_NULL, "qlin_qat_split: column sums need a workspace");
   QatSplitParams p = {a->g, a->scale, static_cast<__nv_bfloat16*>(a->g_planes), a->flags + 2 * kQatFlagSlots, a->colsum != nullptr ? a->workspace : nullptr, a->tokens, a->out,
-                      split_block_rows(a)};
+                      split_block_rows(a), split_huge(a)};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   qat_split_kernel<<<split_grid(a), kSplitThreads, 0, s>>>(p);
   QLIN_CHECK_LAUNCH("qlin_qat_split");

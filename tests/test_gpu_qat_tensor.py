@@ -133,6 +133,27 @@ def test_operands_that_a_hook_changed(cuda_dev, mode):
 
 
 @gpu
+def test_large_gradients_stay_finite(cuda_dev):
+    """Gradients whose product with the operand is an fp32 number, but not with the operand's codes or as g times a scale of 1."""
+    t, k, n = 300, 264, 200
+    lin, x, w, go = _operands(t, k, n)
+    with torch.no_grad():
+        w[5] = 0  # its scale counts as 1
+        big = go.clone()
+        big[:, 5] *= 1.4e36
+        all_big = go * (2.0**122 / float(go.abs().max()))
+        large = go * (2.0**108 / float((go * lin.quantize_weight.clip_val.view(1, -1) / 127).abs().max()))
+        large[:, 5] = 0
+        lin.quantize_weight.clip_val[5] = 0
+    for g, flag in ((big, True), (all_big, True), (large, False)):
+        assert _flags(lin, x, w, g)[4] == flag
+        out = _run(lin, x, w)
+        grads = torch.autograd.grad(out, [x, w, lin.bias], g)
+        assert all(bool(torch.isfinite(v).all()) for v in grads)
+        _check(lin, x, w, g, out, grads)
+
+
+@gpu
 def test_infinite_operands_give_what_fp32_gives(cuda_dev):
     lin, x, w, go = _operands(300, 264, 200)
     go[3, 5], go[8, 9], go[11] = float("inf"), float("nan"), 0
