@@ -13,6 +13,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/stl.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -538,6 +540,14 @@ qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, c
   return a;
 }
 
+// A gradient that the kernels can read: memory of its own on the operands' device, and nothing at work that has to see operators.
+bool plain_gradient(const Tensor& g, const at::Device& dev) {
+  const c10::DispatchKeySet seen({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                  c10::DispatchKey::Batched, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
+  return g.device() == dev && g.layout() == at::kStrided && g.scalar_type() == at::kFloat && g.has_storage() && !g.key_set().has_any(seen) &&
+         !c10::impl::TorchDispatchModeTLS::any_modes_set() && !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
 class QatProduct : public torch::autograd::Function<QatProduct> {
  public:
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias, const Tensor& clip_x,
@@ -582,7 +592,8 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
     const Tensor& go = grads[0];
     if (go.defined()) {
       const Tensor g = go.reshape({n.tokens, n.out});
-      if (at::GradMode::is_enabled()) {  // gradients that are differentiated again
+      // gradients that are differentiated again, that are batched, or that a mode or a subclass follows
+      if (at::GradMode::is_enabled() || !plain_gradient(g, x.device())) {
         if (want_x) gx = g.matmul(w).view(x.sizes());
         if (want_w) gw = g.t().matmul(x.reshape({n.tokens, n.in}));
       } else if (want_x || want_w) {

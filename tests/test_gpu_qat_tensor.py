@@ -182,6 +182,36 @@ def test_gradients_of_gradients_and_single_gradients(cuda_dev):
 
 
 @gpu
+def test_batched_gradients_and_modes_in_the_backward_pass(cuda_dev):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    lin, x, w, go = _operands(200, 136, 144)
+    gos = torch.stack([go, -2 * go, go.flip(0)])
+    got = torch.autograd.grad(_run(lin, x, w), [x, w, lin.bias], gos, is_grads_batched=True)
+    for i in range(3):
+        want = torch.autograd.grad(torch.nn.functional.linear(x, w, lin.bias), [x, w, lin.bias], gos[i])
+        for a, b in zip(got, want):
+            assert torch.allclose(a[i], b, rtol=1e-4, atol=1e-4 * float(b.abs().max()))
+    lin, x, _, go = _operands(1024, 512, 512)  # through the module, where its product is this one
+    x = x.detach()
+    assert type(lin._product(x, lin.weight).grad_fn).__name__ != "AddmmBackward0"
+    (got,) = torch.autograd.grad(lin(x), [lin.weight], torch.stack([go, go * 2]), is_grads_batched=True)
+    (want,) = torch.autograd.grad(lin(x), [lin.weight], go)
+    assert torch.allclose(got[0], want, rtol=1e-4, atol=1e-3) and torch.allclose(got[1], 2 * want, rtol=1e-4, atol=1e-3)
+    out = lin(x)
+    with Watch() as mode:
+        torch.autograd.grad(out, [lin.weight], go)
+    assert any("mm" in f for f in mode.seen)
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
