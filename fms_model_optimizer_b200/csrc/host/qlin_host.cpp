@@ -540,12 +540,17 @@ qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, c
   return a;
 }
 
-// A gradient that the kernels can read: memory of its own on the operands' device, and nothing at work that has to see operators.
-bool plain_gradient(const Tensor& g, const at::Device& dev) {
+// What the kernels can read in the backward pass: fp32 memory of its own on the device, and nothing at work that has to see operators.
+bool plain(const Tensor& g, const at::Device& dev) {
   const c10::DispatchKeySet seen({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                   c10::DispatchKey::Batched, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
   return g.device() == dev && g.layout() == at::kStrided && g.scalar_type() == at::kFloat && g.has_storage() && !g.key_set().has_any(seen) &&
          !c10::impl::TorchDispatchModeTLS::any_modes_set() && !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
+// The same for what was saved: hooks on saved tensors may bring it back with other strides, from another address or device.
+bool plain_saved(const Tensor& t, const at::Device& dev) {
+  return plain(t, dev) && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
 }
 
 class QatProduct : public torch::autograd::Function<QatProduct> {
@@ -592,12 +597,12 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
     const Tensor& go = grads[0];
     if (go.defined()) {
       const Tensor g = go.reshape({n.tokens, n.out});
+      const at::Device dev = go.device();
       // gradients that are differentiated again, that are batched, or that a mode or a subclass follows
-      if (at::GradMode::is_enabled() || !plain_gradient(g, x.device())) {
-        if (want_x) gx = g.matmul(w).view(x.sizes());
+      if (at::GradMode::is_enabled() || !plain(g, dev) || !plain_saved(x, dev) || !plain_saved(w, dev) || !plain_saved(floats, dev)) {
+        if (want_x) gx = g.matmul(w).reshape(x.sizes());
         if (want_w) gw = g.t().matmul(x.reshape({n.tokens, n.in}));
       } else if (want_x || want_w) {
-        const at::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
         const Tensor gc = g.contiguous(), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
         const std::vector<int64_t> bits = ctx->saved_data["bits"].toIntVector();

@@ -212,6 +212,32 @@ def test_batched_gradients_and_modes_in_the_backward_pass(cuda_dev):
 
 
 @gpu
+@pytest.mark.parametrize("what", ["strides", "address", "expanded", "fewer bits"])
+def test_saved_tensors_that_come_back_changed(cuda_dev, what):
+    """Hooks on saved tensors that return the operands column by column, off a 16-byte boundary, as an expanded row, or rounded."""
+
+    def unpack(t):
+        if t.dim() != 2:
+            return t
+        if what == "strides":
+            return t.t().contiguous().t()
+        if what == "expanded":
+            return t[:1].expand(t.shape)
+        if what == "fewer bits":
+            return t.bfloat16().float()
+        buf = torch.empty(t.numel() + 1, device="cuda")
+        buf[1:] = t.reshape(-1)
+        return buf[1:].view(t.shape)
+
+    lin, x, w, go = _operands(200, 136, 144)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), unpack):
+        out = _run(lin, x, w)
+    got = torch.autograd.grad(out, [x, w, lin.bias], go)
+    for a, b in zip(got, (go @ unpack(w.detach()), go.t() @ unpack(x.detach()), go.sum(0))):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4 * float(b.abs().max()))
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
