@@ -203,6 +203,8 @@ __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplit
   if (c < p.cols) {  // cols is a multiple of 8
     const float4 sa = *reinterpret_cast<const float4*>(p.scale + c), sb = *reinterpret_cast<const float4*>(p.scale + c + 4);
     const float s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bad |= !scale_ok(s[j]);  // also for products that the weight's codes are no part of
     float sum[8] = {};
 #pragma unroll 4
     for (int row = rb * p.block_rows; row < row1; ++row) {
@@ -612,7 +614,7 @@ struct QatFallbackParams {
   const float* b;
   const float* bias;
   float* d;
-  const int32_t* flags;        // three groups of kQatFlagSlots, of which the first n are in use
+  const int32_t* flags;        // three groups of kQatFlagSlots; the first n of each belong to this product's operands
   int64_t a_m, a_k, b_n, b_k;  // element strides
   int32_t M, N, K, n[3];
 };
@@ -857,8 +859,9 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
     f.a = a->g, f.a_m = 1, f.a_k = O, f.b = a->x, f.b_n = 1, f.b_k = I;
   }
   f.M = p.M, f.N = p.N, f.K = p.K;
-  f.n[0] = act_grid(a);
-  f.n[1] = weight_grid(a);
+  // a product looks at the flags of its own two operands: the others may have been left out
+  f.n[0] = which == 1 ? 0 : act_grid(a);
+  f.n[1] = which == 2 ? 0 : weight_grid(a);
   f.n[2] = which == 0 ? 0 : split_grid(a);
   if (pa == nullptr || pb == nullptr || f.a == nullptr || f.b == nullptr || a->flags == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_product: a pointer is NULL");
   const int num_kb = (p.K + 63) / 64;

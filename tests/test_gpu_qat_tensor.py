@@ -41,29 +41,48 @@ class _Args(C.Structure):  # qlin_qat_args
     _fields_ += [(f, C.c_int32) for f in ("tokens", "inp", "out", "num_bits_x", "num_bits_w", "variant")] + [("clip_kept", C.c_void_p)]
 
 
-def _flags(lin, x, w, go, mode="two-sided", replaced=None):
-    """Whether (x, w) of the forward pass and (x, w, gradient) of the backward pass raise their flags, through the C entry points.
-    ``replaced`` is called between the passes."""
+def _passes(lin, x, w, go, mode="two-sided", left_out=(), between=lambda: None):
+    """Both passes through the C entry points: (flags of x and w in the forward pass, of x, w and the gradient in the backward pass) and
+    (whether out, gx and gw were computed again in fp32).  The second is seen by putting zeros in the operands' place once their codes are
+    made.  The flags start as memory that nobody cleared.  ``between`` is called between the passes."""
     lib, t, k, n = L.load(), x.shape[0], x.shape[1], w.shape[0]
     Qa, Qw = lin.quantize_feature, lin.quantize_weight
-    buf = {"x_codes": torch.empty(t * k, dtype=torch.bfloat16, device="cuda"), "w_codes": torch.empty(n * k, dtype=torch.bfloat16, device="cuda"),
-           "g_planes": torch.empty(3 * t * n, dtype=torch.bfloat16, device="cuda"), "step": torch.empty(1, device="cuda"), "scale": torch.empty(n, device="cuda"),
-           "rcp": torch.empty(n, device="cuda"), "clip_kept": torch.empty(1, device="cuda"), "x": x.detach(), "w": w.detach(), "g": go, "clip_x": Qa.clip_val.detach(),
-           "clip_w": Qw.clip_val}  # fmt: skip
+    dev = dict(device="cuda")
+    f32 = {"step": torch.empty(1, **dev), "scale": torch.empty(n, **dev), "rcp": torch.empty(n, **dev), "clip_kept": torch.empty(1, **dev), "x": x.detach(), "w": w.detach(),
+           "g": go, "clip_x": Qa.clip_val.detach(), "clip_w": Qw.clip_val, "d": None}  # fmt: skip
     if mode == "two-sided":
-        buf["clipn_x"] = Qa.clip_valn.detach()
-    res = []
+        f32["clipn_x"] = Qa.clip_valn.detach()
+    codes = {"x_codes": t * k, "w_codes": n * k, "g_planes": 3 * t * n}
+    codes = {f: torch.empty(c, dtype=torch.bfloat16, **dev) for f, c in codes.items()}
+    kept = {f: v for f, v in codes.items() if f not in left_out}
+    zeros = torch.zeros(max(t * k, n * k, t * n), **dev)
+    flags = torch.ones(lib.qlin_qat_flag_count(), dtype=torch.int32, **dev)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def args(**other):
+        ptr = {f: v.data_ptr() for f, v in {**f32, **codes, **other}.items() if v is not None}
+        return C.byref(_Args(flags=flags.data_ptr(), tokens=t, inp=k, out=n, num_bits_x=8, num_bits_w=8, variant=MODES[mode], **ptr))
+
+    raised, again = [], []
     for backward in (0, 1):
-        flags = torch.zeros(lib.qlin_qat_flag_count(), dtype=torch.int32, device="cuda")
-        a = _Args(flags=flags.data_ptr(), tokens=t, inp=k, out=n, num_bits_x=8, num_bits_w=8, variant=MODES[mode], **{f: v.data_ptr() for f, v in buf.items()})
-        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
-        L.check(lib.qlin_qat_codes(C.byref(a), C.c_int32(backward), stream), "qlin_qat_codes")
+        if left_out and backward:
+            codes = kept
+            flags.fill_(1)
+        L.check(lib.qlin_qat_codes(args(), C.c_int32(backward), stream), "qlin_qat_codes")
         if backward:
-            L.check(lib.qlin_qat_split(C.byref(a), stream), "qlin_qat_split")
-        res += [bool(v) for v in (flags.view(3, -1) != 0).any(1).tolist()[: 3 if backward else 2]]
-        if replaced is not None:
-            replaced()
-    return tuple(res)
+            L.check(lib.qlin_qat_split(args(), stream), "qlin_qat_split")
+        if not left_out:
+            counts = flags.view(3, -1)[: 2 + backward].clone()
+            used = [((t * k // 8 + 255) // 256), ((n + 63) // 64) * ((k + 63) // 64), ((t + 15) // 16) * ((n + 1023) // 1024)]
+            raised += [bool((counts[i, : used[i]] != 0).any()) for i in range(2 + backward)]
+        for which in (1, 2) if backward else (0,):
+            if left_out and (not backward or {1: "w_codes", 2: "x_codes"}[which] in left_out):
+                continue
+            d = torch.full((max(t * k, n * k, t * n),), float("nan"), **dev)
+            L.check(lib.qlin_qat_product(args(d=d, x=zeros, w=zeros, g=zeros), C.c_int32(which), stream), "qlin_qat_product")
+            again.append(bool((d.nan_to_num(1.0)[: (t * n, t * k, n * k)[which]] == 0).all()))
+        between()
+    return tuple(raised), tuple(again)
 
 
 def _check(lin, x, w, go, out, grads):
@@ -116,20 +135,22 @@ def test_operands_that_a_hook_changed(cuda_dev, mode):
     """An operand scaled far below a step, and one element a single place off, are multiplied as they are."""
     t, k, n = 300, 264, 200
     lin, x, w, go = _operands(t, k, n, mode=mode)
-    assert _flags(lin, x, w, go, mode) == (False,) * 5
+    assert _passes(lin, x, w, go, mode) == ((False,) * 5, (False,) * 3)
     with torch.no_grad():
         lin.bias.zero_()
     for what in ("x", "w"):
         sx, sw = (1e-7, 1.0) if what == "x" else (1.0, 1e-7)
         xs, ws = (x.detach() * sx).requires_grad_(True), (w.detach() * sw).requires_grad_(True)
-        assert _flags(lin, xs, ws, go, mode) == (what == "x", what == "w", what == "x", what == "w", False)
+        flags = (what == "x", what == "w", what == "x", what == "w", False)
+        again = (True, what == "w", what == "x")
+        assert _passes(lin, xs, ws, go, mode) == (flags, again)
         out = _run(lin, xs, ws, mode)
         _check(lin, xs, ws, go, out, torch.autograd.grad(out, [xs, ws, lin.bias], go))
         x1, w1 = x.detach().clone(), w.detach().clone()
         e = (x1 if what == "x" else w1).view(-1)
         i = int(e.abs().argmax())
         e[i] = torch.nextafter(e[i], torch.zeros((), device="cuda"))
-        assert _flags(lin, x1, w1, go, mode) == (what == "x", what == "w", what == "x", what == "w", False)
+        assert _passes(lin, x1, w1, go, mode) == (flags, again)
 
 
 @gpu
@@ -146,11 +167,19 @@ def test_large_gradients_stay_finite(cuda_dev):
         large[:, 5] = 0
         lin.quantize_weight.clip_val[5] = 0
     for g, flag in ((big, True), (all_big, True), (large, False)):
-        assert _flags(lin, x, w, g)[4] == flag
+        assert _passes(lin, x, w, g) == ((False,) * 4 + (flag,), (False, flag, flag))
         out = _run(lin, x, w)
         grads = torch.autograd.grad(out, [x, w, lin.bias], g)
         assert all(bool(torch.isfinite(v).all()) for v in grads)
         _check(lin, x, w, g, out, grads)
+
+
+@gpu
+def test_operand_that_is_left_out(cuda_dev):
+    """A caller of the C entry points that wants one gradient makes the codes of one operand; the other's flags are not looked at."""
+    lin, x, w, go = _operands(300, 264, 200)
+    for left_out in ("x_codes", "w_codes"):
+        assert _passes(lin, x, w, go, left_out=(left_out,))[1] == (False,)
 
 
 @gpu
