@@ -523,14 +523,13 @@ struct QatShape {
   int64_t tokens, in, out;
 };
 
-// The operands' arguments of one pass; `floats` is [2 * out + 2]: scales, their reciprocals, the step and its clip value.
+// The operands' arguments of one pass; `floats` is [out + 2]: scales, the step and its clip value.
 qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, const Tensor& flags, const QatShape& n) {
   qlin_qat_args a = {};
   a.x = static_cast<const float*>(data(x));
   a.w = static_cast<const float*>(data(w));
   a.scale = static_cast<float*>(data(floats));
-  a.rcp = a.scale + n.out;
-  a.step = a.scale + 2 * n.out;
+  a.step = a.scale + n.out;
   a.clip_kept = a.step + 1;
   a.flags = static_cast<int32_t*>(data(flags));
   a.status = static_cast<int32_t*>(status_word(x.device().index()).data_ptr());
@@ -560,7 +559,7 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
     const at::Device dev = x.device();
     const c10::cuda::CUDAGuard guard(dev);
     const QatShape n{x.numel() / x.size(-1), x.size(-1), w.size(0)};
-    const Tensor floats = empty({2 * n.out + 2}, at::kFloat, dev), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
+    const Tensor floats = empty({n.out + 2}, at::kFloat, dev), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
     const Tensor xc = empty({n.tokens, n.in}, at::kBFloat16, dev), wc = empty({n.out, n.in}, at::kBFloat16, dev);
     std::vector<int64_t> shape = x.sizes().vec();
     shape.back() = n.out;
@@ -606,7 +605,7 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
         const c10::cuda::CUDAGuard guard(dev);
         const Tensor gc = g.contiguous(), flags = empty({qlin_qat_flag_count()}, at::kInt, dev);
         const std::vector<int64_t> bits = ctx->saved_data["bits"].toIntVector();
-        Tensor planes = empty({3, n.tokens, n.out}, at::kBFloat16, dev);
+        const Tensor planes = empty({3, n.tokens, n.out}, at::kBFloat16, dev), rcp = empty({n.out}, at::kFloat, dev);
         // both operands' codes are made, and checked, whichever gradient is wanted
         Tensor xc = empty({n.tokens, n.in}, at::kBFloat16, dev), wc = empty({n.in, n.out}, at::kBFloat16, dev);
         qlin_qat_args a = qat_args(x, w, floats, flags, n);
@@ -614,6 +613,7 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
         a.x_codes = data(xc);
         a.w_codes = data(wc);
         a.g_planes = data(planes);
+        a.rcp = static_cast<float*>(data(rcp));
         a.num_bits_x = static_cast<int32_t>(bits[0]);
         a.num_bits_w = static_cast<int32_t>(bits[1]);
         a.variant = static_cast<int32_t>(bits[2]);

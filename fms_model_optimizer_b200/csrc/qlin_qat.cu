@@ -50,7 +50,6 @@ struct QatCodesParams {
   const float* clipn;   // two-sided activations: clip_valn [1]
   float* scale;         // activations: step [1]; weights: s [rows]
   float* clip_kept;     // symmetric activations: the clip value of the forward pass [1]
-  float* rcp;           // weights: 1 / s [rows]
   int32_t* flags;       // one per block
   int64_t ldo;
   int32_t rows, cols, num_bits, variant, transposed, given;  // given: `scale` holds the step or scales of the forward pass
@@ -153,10 +152,7 @@ __global__ void __launch_bounds__(kPrepThreads) qat_weight_codes_kernel(const Qa
         } else {
           *reinterpret_cast<uint2*>(p.codes + static_cast<int64_t>(row) * p.ldo + c0 + c) = make_uint2(lo, hi);
         }
-        if (c0 + c == 0 && !p.given) {
-          p.scale[row] = sp;
-          p.rcp[row] = __fdiv_rn(1.0f, sp);
-        }
+        if (c0 + c == 0 && !p.given) p.scale[row] = sp;
       }
     }
     if (p.transposed) {
@@ -186,6 +182,7 @@ struct QatSplitParams {
   __nv_bfloat16* planes;  // [3][rows][cols]
   int32_t* flags;
   float* sums;            // optional [row blocks][cols]: each block's column sums
+  float* rcp;             // [cols]: 1 / s
   int32_t rows, cols, block_rows;
   float huge;
 };
@@ -205,6 +202,10 @@ __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplit
     const float s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
 #pragma unroll
     for (int j = 0; j < 8; ++j) bad |= !scale_ok(s[j]);  // also for products that the weight's codes are no part of
+    if (rb == 0) {  // made here so that it undoes the very scale that the planes carry
+#pragma unroll
+      for (int j = 0; j < 8; ++j) p.rcp[c + j] = __fdiv_rn(1.0f, s[j]);
+    }
     float sum[8] = {};
 #pragma unroll 4
     for (int row = rb * p.block_rows; row < row1; ++row) {
@@ -760,7 +761,7 @@ extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* st
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_codes: args is NULL");
   if (!qat_shape_ok(a)) return fail(QLIN_ERR_BAD_SHAPE, "qlin_qat: in and out must be positive multiples of 8");
   if (a->num_bits_x < 2 || a->num_bits_x > 8 || a->num_bits_w < 2 || a->num_bits_w > 8) return fail(QLIN_ERR_UNSUPPORTED, "qlin_qat: 2 to 8 bits");
-  if (a->flags == nullptr || a->step == nullptr || a->scale == nullptr || a->rcp == nullptr ||
+  if (a->flags == nullptr || a->step == nullptr || a->scale == nullptr ||
       (!backward && (a->clip_x == nullptr || a->clip_w == nullptr || (a->variant == QLIN_PACT_TWO_SIDED && a->clipn_x == nullptr))))
     return fail(QLIN_ERR_NULL, "qlin_qat_codes: a pointer is NULL");
   if (a->variant == QLIN_PACT_SYMMETRIC && a->clip_kept == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_codes: the symmetric quantizer needs clip_kept");
@@ -790,7 +791,6 @@ extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* st
     p.num_bits = a->num_bits_w;
     p.clip = a->clip_w;
     p.scale = a->scale;
-    p.rcp = a->rcp;
     p.flags = a->flags + kQatFlagSlots;
     p.rows = a->out;
     p.cols = a->in;
@@ -805,10 +805,10 @@ extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* st
 extern "C" int qlin_qat_split(const qlin_qat_args* a, void* stream) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_split: args is NULL");
   if (!qat_shape_ok(a)) return fail(QLIN_ERR_BAD_SHAPE, "qlin_qat: in and out must be positive multiples of 8");
-  if (a->g == nullptr || a->g_planes == nullptr || a->scale == nullptr || a->flags == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_split: a pointer is NULL");
+  if (a->g == nullptr || a->g_planes == nullptr || a->scale == nullptr || a->rcp == nullptr || a->flags == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_split: a pointer is NULL");
   if (!aligned16(a->g_planes) || !aligned16(a->scale)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_split: 16-byte alignment");
   if (a->colsum != nullptr && (a->workspace == nullptr || !aligned16(a->workspace))) return fail(QLIN_ERR_NULL, "qlin_qat_split: column sums need a workspace");
-  QatSplitParams p = {a->g, a->scale, static_cast<__nv_bfloat16*>(a->g_planes), a->flags + 2 * kQatFlagSlots, a->colsum != nullptr ? a->workspace : nullptr, a->tokens, a->out,
+  QatSplitParams p = {a->g, a->scale, static_cast<__nv_bfloat16*>(a->g_planes), a->flags + 2 * kQatFlagSlots, a->colsum != nullptr ? a->workspace : nullptr, a->rcp, a->tokens, a->out,
                       split_block_rows(a), split_huge(a)};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   qat_split_kernel<<<split_grid(a), kSplitThreads, 0, s>>>(p);

@@ -611,7 +611,7 @@ typedef struct qlin_qat_args {
   const float* clip_w;  /* [out]; forward */
   float* step;          /* [1]: written by the forward pass, read by both */
   float* scale;         /* [out], 16-byte aligned: likewise */
-  float* rcp;           /* [out]: likewise */
+  float* rcp;           /* [out]: reciprocals of `scale`, written by qlin_qat_split, read by product 2 */
   void* x_codes;        /* bf16 [tokens, in]; qlin_qat_codes leaves them out when NULL */
   void* w_codes;        /* bf16 [out, in], backward [in, out]; likewise */
   void* g_planes;       /* bf16 [3, tokens, out] */

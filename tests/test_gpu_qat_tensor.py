@@ -267,6 +267,19 @@ def test_saved_tensors_that_come_back_changed(cuda_dev, what):
 
 
 @gpu
+def test_saved_scales_that_come_back_rounded(cuda_dev):
+    """Hooks that keep saved tensors in bf16.  The activations are bf16 numbers, so the weight's gradient does not change; what the
+    function saves besides the operands is its own affair."""
+    lin, x, w, go = _operands(300, 264, 200, clips=(127 / 64, -128 / 64))
+    assert torch.equal(x, x.bfloat16().float())
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().bfloat16(), lambda t: t.float()):
+        out = _run(lin, x, w)
+    (got,) = torch.autograd.grad(out, [w], go)
+    terms = go.double().abs().t() @ x.detach().double().abs()
+    assert bool(((got.double() - go.double().t() @ x.detach().double()).abs() <= 8 * 300**0.5 * 2.0**-24 * terms + 1e-38).all())
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
