@@ -68,6 +68,7 @@ EXPORTED_SYMBOLS = (
     "qlin_col_absmax",
     "qlin_shard_reduce",
     "qlin_qat_flag_count",
+    "qlin_qat_max_out",
     "qlin_qat_colsum_workspace_bytes",
     "qlin_qat_codes",
     "qlin_qat_split",

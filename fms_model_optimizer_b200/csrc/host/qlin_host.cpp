@@ -658,7 +658,7 @@ bool qat_takes(const Tensor& x, const Tensor& w, const OptTensor& bias, const Te
   if (bias && (bias->scalar_type() != at::kFloat || bias->device() != x.device() || bias->dim() != 1 || bias->size(0) != w.size(0))) return false;
   if (clip_w.scalar_type() != at::kFloat || clip_w.device() != x.device() || clip_w.numel() != w.size(0)) return false;
   const int64_t in = w.size(1), out = w.size(0);
-  if (in < kQatMinSide || out < kQatMinSide || x.numel() < kQatMinSide * in || in % 8 != 0 || out % 8 != 0 || x.numel() / in > 0x7fffffff - 256 || in > 0x7fffff00 || out > 0x7fffff00) return false;
+  if (in < kQatMinSide || out < kQatMinSide || x.numel() < kQatMinSide * in || in % 8 != 0 || out % 8 != 0 || x.numel() / in > 0x7fffffff - 256 || in > 0x7fffff00 || out > qlin_qat_max_out()) return false;
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0 || reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 != 0) return false;
   if (at::autocast::is_autocast_enabled(at::kCUDA)) return false;
   const at::Float32Precision prec = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);

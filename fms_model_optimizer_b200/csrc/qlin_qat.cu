@@ -750,12 +750,13 @@ static int split_grid(const qlin_qat_args* a) { return split_row_blocks(a) * spl
 
 using namespace qlin;
 
+extern "C" int32_t qlin_qat_flag_count(void) { return 3 * kQatFlagSlots; }
+extern "C" int32_t qlin_qat_max_out(void) { return 8 * kSplitThreads * kQatFlagSlots; }
+
 static bool qat_shape_ok(const qlin_qat_args* a) {
-  return a->tokens > 0 && a->out <= 8 * kSplitThreads * kQatFlagSlots && a->in > 0 && a->out > 0 && a->in % 8 == 0 && a->out % 8 == 0 && static_cast<int64_t>(a->tokens) * a->in < (int64_t{1} << 40) &&
+  return a->tokens > 0 && a->out <= qlin_qat_max_out() && a->in > 0 && a->out > 0 && a->in % 8 == 0 && a->out % 8 == 0 && static_cast<int64_t>(a->tokens) * a->in < (int64_t{1} << 40) &&
          static_cast<int64_t>(a->tokens) * a->out < (int64_t{1} << 40);
 }
-
-extern "C" int32_t qlin_qat_flag_count(void) { return 3 * kQatFlagSlots; }
 
 extern "C" int qlin_qat_codes(const qlin_qat_args* a, int32_t backward, void* stream) {
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_codes: args is NULL");

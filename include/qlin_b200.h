@@ -627,6 +627,7 @@ typedef struct qlin_qat_args {
 } qlin_qat_args;
 
 int32_t qlin_qat_flag_count(void);
+int32_t qlin_qat_max_out(void); /* the most outputs that the calls below take */
 int64_t qlin_qat_colsum_workspace_bytes(int32_t tokens, int32_t out);
 int qlin_qat_codes(const qlin_qat_args* args, int32_t backward, void* stream);
 int qlin_qat_split(const qlin_qat_args* args, void* stream);

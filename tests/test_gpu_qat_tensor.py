@@ -280,6 +280,19 @@ def test_saved_scales_that_come_back_rounded(cuda_dev):
 
 
 @gpu
+def test_more_outputs_than_the_flags_cover(cuda_dev):
+    """Wider than the gradient's split goes: the library's call, as every other one that the rule leaves out."""
+    t, k, n = 128, 128, 1212424
+    g = torch.Generator(device="cuda").manual_seed(0)
+    lin = QLinear(k, n, num_bits_feature=8, qa_mode="pact+", num_bits_weight=8, qw_mode="sawb+perCh", device="cuda").train()
+    x = torch.randn(t, k, generator=g, device="cuda")
+    out = lin(x).detach()[:, -100:]
+    with torch.no_grad():
+        want = lin.quantize_feature(x).double() @ lin.quantize_weight(lin.weight)[-100:].double().t() + lin.bias[-100:]
+    assert torch.allclose(out.double(), want, rtol=1e-4, atol=1e-4)
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
