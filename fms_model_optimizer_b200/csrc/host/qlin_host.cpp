@@ -539,7 +539,7 @@ qlin_qat_args qat_args(const Tensor& x, const Tensor& w, const Tensor& floats, c
   return a;
 }
 
-// What the kernels can read in the backward pass: fp32 memory of its own on the device, and nothing at work that has to see operators.
+// What the kernels can read: fp32 memory on the device that holds the values as they are, and nothing at work that has to see operators.
 bool plain(const Tensor& g, const at::Device& dev) {
   const c10::DispatchKeySet seen({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                   c10::DispatchKey::Batched, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
@@ -547,8 +547,8 @@ bool plain(const Tensor& g, const at::Device& dev) {
          !c10::impl::TorchDispatchModeTLS::any_modes_set() && !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 
-// The same for what was saved: hooks on saved tensors may bring it back with other strides, from another address or device.
-bool plain_saved(const Tensor& t, const at::Device& dev) {
+// The same, dense and aligned, for operands: hooks on saved tensors may bring them back with other strides, from another address or device.
+bool plain_operand(const Tensor& t, const at::Device& dev) {
   return plain(t, dev) && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
 }
 
@@ -598,7 +598,7 @@ class QatProduct : public torch::autograd::Function<QatProduct> {
       const Tensor g = go.reshape({n.tokens, n.out});
       const at::Device dev = go.device();
       // gradients that are differentiated again, that are batched, or that a mode or a subclass follows
-      if (at::GradMode::is_enabled() || !plain(g, dev) || !plain_saved(x, dev) || !plain_saved(w, dev) || !plain_saved(floats, dev)) {
+      if (at::GradMode::is_enabled() || !plain(g, dev) || !plain_operand(x, dev) || !plain_operand(w, dev) || !plain_operand(floats, dev)) {
         if (want_x) gx = g.matmul(w).reshape(x.sizes());
         if (want_w) gw = g.t().matmul(x.reshape({n.tokens, n.in}));
       } else if (want_x || want_w) {
@@ -659,7 +659,7 @@ bool qat_takes(const Tensor& x, const Tensor& w, const OptTensor& bias, const Te
   if (clip_w.scalar_type() != at::kFloat || clip_w.device() != x.device() || clip_w.numel() != w.size(0)) return false;
   const int64_t in = w.size(1), out = w.size(0);
   if (in < kQatMinSide || out < kQatMinSide || x.numel() < kQatMinSide * in || in % 8 != 0 || out % 8 != 0 || x.numel() / in > 0x7fffffff - 256 || in > 0x7fffff00 || out > qlin_qat_max_out()) return false;
-  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0 || reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 != 0) return false;
+  if (!plain_operand(x, x.device()) || !plain_operand(w, x.device()) || (bias && !plain(*bias, x.device()))) return false;
   if (at::autocast::is_autocast_enabled(at::kCUDA)) return false;
   const at::Float32Precision prec = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);
   if (prec != at::Float32Precision::NONE && prec != at::Float32Precision::IEEE) return false;

@@ -293,6 +293,20 @@ def test_more_outputs_than_the_flags_cover(cuda_dev):
 
 
 @gpu
+@pytest.mark.parametrize("which", ["x", "w", "bias"])
+def test_operands_that_are_stored_negated(cuda_dev, which):
+    lin, x, w, _ = _operands(1024, 512, 512)
+    with torch.no_grad():
+        x, w, b = x.detach(), w.detach(), lin.bias.detach()
+        if which == "bias":
+            lin.bias = torch.nn.Parameter(torch._neg_view(b), requires_grad=False)
+        args = (torch._neg_view(x) if which == "x" else x, torch._neg_view(w) if which == "w" else w)
+        got = lin._product(*args).double()
+    want = (-x if which == "x" else x).double() @ (-w if which == "w" else w).double().t() + (-b if which == "bias" else b)
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-4)
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
