@@ -4,8 +4,8 @@
 //
 // x and w are fake-quantised: x = c step and w = d s[n] with whole numbers c, d of at most 8 bits and a sign, which bf16 holds
 // exactly (up to 256, so the codes 256 and -1 that some clip pairs reach fit, and so does a NaN).  With the zero point taken
-// off beforehand there is no offset that could cancel.  The gradient is any fp32 number: g s[n], rounded once, is the sum of
-// three bf16 numbers (8 + 8 + 8 bits, each rounded from what the ones before left over).  So the forward product is one
+// off beforehand there is no offset that could cancel.  The gradient is any fp32 number: g s[n] (times a power of two that keeps small
+// parts in range), rounded once, is the sum of three bf16 numbers (8 + 8 + 8 bits, each rounded from what the ones before left over).  So the forward product is one
 // bf16 GEMM whose sums are whole numbers, and each gradient is three, with every product exact and the sums in fp32.
 //
 // The tensor core truncates as it adds, which shows after a few hundred terms.  So no accumulator of a gradient lives longer
@@ -20,10 +20,10 @@
 // backward of 4096 x 768 x 3072: 1124 us of device time with the library's fp32 GEMMs, 212 with this.
 //
 // What the argument rests on is checked where the operands are made: a value that is not bit for bit what the quantizer makes of a
-// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element so large that a sum of its products with
-// codes could leave fp32's range (which the product with the operand itself need not), or one so small (below 2^-100) that its third
-// part could leave bf16's range raises a flag on the device, and the last kernel of each product, which is
-// always launched, then computes it in fp32 from the operands themselves.  With no flag up it returns at once.
+// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element so large that a sum of
+// its products with codes could leave fp32's range (which the product with the operand itself need not), or a tiny one beside a scale at
+// which its lost digits could show raises a flag on the device, and the last kernel of each product, which is always launched, then
+// computes it in fp32 from the operands themselves.  With no flag up it returns at once.
 #include <cmath>
 
 #include <cuda.h>
@@ -37,9 +37,16 @@ namespace qlin {
 
 // ------------------------------------------------------------------------------------------------ operands
 constexpr float kMaxCode = 256.0f;                // whole numbers up to here are bf16 numbers
-constexpr float kTiny = 7.888609052210118e-31f;   // 2^-100
-// |g s| below 2^(kSumExp - e), 2^e >= the longer contraction: a sum of 2^e products with codes of up to 2^8 stays below 2^126.
+// A gradient enters as t = g s 2^kShift, and the products take the power of two out again.  Let 2^e be at least the longer contraction.
+// Above: |t| up to 2^(kSumExp - e), so that a sum of 2^e products with codes of up to 2^8 stays below 2^126.  Below: from 2^-100 on
+// the third part is a normal bf16 number.  A smaller t loses at most 2^-124, its sums 2^(e - 115), gx 2^(e - 115 - kShift) and gw
+// that times step / s: below half of the smallest fp32 number, which no result can show, while step / s is at most
+// 2^(kShift - 36 - e).  So tiny elements (the tails of a GELU's or a softmax's gradient) cost nothing, and only a tiny element
+// in a column whose step / s is above that raises the flag.  At e = 12: |g s| up to 2^34, step / s up to 2^24.
+constexpr int kShift = 72;
 constexpr int kSumExp = 118;
+constexpr float kTiny = 7.888609052210118e-31f;   // 2^-100
+constexpr float kShiftUp = 4722366482869645213696.0f, kShiftDown = 1.0f / kShiftUp;  // 2^72, 2^-72
 constexpr int kPrepThreads = 256;
 constexpr int kQatFlagSlots = 1184;  // flags of each kernel that makes an operand
 
@@ -184,11 +191,12 @@ struct QatSplitParams {
   float* sums;            // optional [row blocks][cols]: each block's column sums
   float* rcp;             // [cols]: 1 / s
   int32_t rows, cols, block_rows;
-  float huge;
+  const float* step;      // optional [1]: without it no tiny element is left out
+  float huge, far;        // the largest |t|; the largest step / s at which tiny elements go unseen
 };
 constexpr int kSplitThreads = 128;  // eight columns a thread
 
-// g s[n] as three bf16 numbers, and the column sums of g.  Bound by HBM: 4 bytes read and 6 written an element.
+// g s[n] 2^kShift as three bf16 numbers, and the column sums of g.  Bound by HBM: 4 bytes read and 6 written an element.
 __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplitParams p) {
   const int strips = (p.cols + 8 * kSplitThreads - 1) / (8 * kSplitThreads);
   const int c = (static_cast<int>(blockIdx.x % strips) * kSplitThreads + static_cast<int>(threadIdx.x)) * 8;
@@ -199,12 +207,14 @@ __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplit
   bool bad = false;
   if (c < p.cols) {  // cols is a multiple of 8
     const float4 sa = *reinterpret_cast<const float4*>(p.scale + c), sb = *reinterpret_cast<const float4*>(p.scale + c + 4);
-    const float s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+    float s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+    uint32_t far = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) bad |= !scale_ok(s[j]);  // also for products that the weight's codes are no part of
-    if (rb == 0) {  // made here so that it undoes the very scale that the planes carry
-#pragma unroll
-      for (int j = 0; j < 8; ++j) p.rcp[c + j] = __fdiv_rn(1.0f, s[j]);
+    for (int j = 0; j < 8; ++j) {
+      bad |= !scale_ok(s[j]);  // also for products that the weight's codes are no part of
+      if (rb == 0) p.rcp[c + j] = __fdiv_rn(1.0f, s[j]);  // made here so that it undoes the very scale that the planes carry
+      if (p.step == nullptr || !(fabsf(*p.step) <= p.far * fabsf(s[j]))) far |= 1u << j;
+      s[j] *= kShiftUp;
     }
     float sum[8] = {};
 #pragma unroll 4
@@ -222,9 +232,9 @@ __global__ void __launch_bounds__(kSplitThreads) qat_split_kernel(const QatSplit
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
         float2 t = __fmul2_rn(make_float2(v[j], v[j + 1]), make_float2(s[j], s[j + 1]));
-        // not finite, too large or too small (a NaN fails every comparison); an exact zero is fine
-        bad |= !(fabsf(t.x) >= kTiny && fabsf(t.x) <= p.huge) && !(v[j] == 0.0f);
-        bad |= !(fabsf(t.y) >= kTiny && fabsf(t.y) <= p.huge) && !(v[j + 1] == 0.0f);
+        // not finite or too large (a NaN fails every comparison), or too small where that shows; an exact zero is fine
+        bad |= !(fabsf(t.x) <= p.huge) || ((far >> j & 1) && fabsf(t.x) < kTiny && v[j] != 0.0f);
+        bad |= !(fabsf(t.y) <= p.huge) || ((far >> (j + 1) & 1) && fabsf(t.y) < kTiny && v[j + 1] != 0.0f);
         sum[j] += v[j];
         sum[j + 1] += v[j + 1];
 #pragma unroll
@@ -265,8 +275,8 @@ __global__ void __launch_bounds__(256) qat_colsum_kernel(const float* sums, int 
 }
 
 // ------------------------------------------------------------------------------------------------ product
-// D[M,N] = (sum over planes and K of A_plane[m,k] B[n,k]) * row[m] * col[n] * scalar + bias[n] in fp32, one CTA pair per 256 x BN
-// tile.  A stage holds 64 K values of all planes of A and of B, so B is loaded once for the three planes.  An operand is
+// D[M,N] = (sum over planes and K of A_plane[m,k] B[n,k]) * row[m] * col[n] * scalar * down + bias[n] in fp32, one CTA pair per
+// 256 x BN tile.  A stage holds 64 K values of all planes of A and of B, so B is loaded once for the three planes.  An operand is
 // K-major ([rows, K] in memory: boxes of 64 K values x rows) or MN-major ([K, rows]: boxes of 64 rows x 64 K values).
 struct QatGemmParams {
   float* d;
@@ -275,6 +285,7 @@ struct QatGemmParams {
   const float* scalar;
   const float* bias;
   int32_t* status;
+  float down;  // a power of two
   int32_t M, N, K, planes, a_mn, b_mn, promote;  // promote: stages per accumulator
   int32_t num_m, num_n;
 };
@@ -525,7 +536,10 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         aux->bias[half * C::COLS + i] = (p.bias != nullptr && col0 + i < p.N) ? p.bias[col0 + i] : 0.0f;
       }
       asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-      const float rs = __fmul_rn(scalar, (p.row != nullptr && row0 + lane < p.M) ? p.row[row0 + lane] : 1.0f);
+      float rs = __fmul_rn(scalar, (p.row != nullptr && row0 + lane < p.M) ? p.row[row0 + lane] : 1.0f);
+      // the power of two goes with a factor above 1, and before one below: neither order leaves fp32's range where the result does not
+      float down = p.down;
+      if (fabsf(rs) > 1.0f) rs = __fmul_rn(rs, down), down = 1.0f;
       float run[C::COLS];
       for (int kb = 0; kb < num_kb; kb += p.promote) {
         if (!warp_mbar_wait(&aux->tfull[buf], bph, abort_flag)) {
@@ -565,7 +579,7 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int e = c + 4 * k + j;
-            const float y = __fmul_rn(run[e], __fmul_rn(rs, aux->cs[half * C::COLS + e]));
+            const float y = __fmul_rn(__fmul_rn(run[e], down), __fmul_rn(rs, aux->cs[half * C::COLS + e]));
             w[j] = __float_as_uint(p.bias != nullptr ? __fadd_rn(y, aux->bias[half * C::COLS + e]) : y);
           }
           const uint32_t addr = smem_u32(dst) + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4);
@@ -739,11 +753,13 @@ static int split_block_rows(const qlin_qat_args* a) {
   return need > 16 ? need : 16;
 }
 static int split_row_blocks(const qlin_qat_args* a) { return (a->tokens + split_block_rows(a) - 1) / split_block_rows(a); }
-static float split_huge(const qlin_qat_args* a) {
+static int longer_exp(const qlin_qat_args* a) {
   int e = 0;
   while ((int64_t{1} << e) < (a->tokens > a->out ? a->tokens : a->out)) ++e;
-  return std::ldexp(1.0f, kSumExp - e);
+  return e;
 }
+static float split_huge(const qlin_qat_args* a) { return std::ldexp(1.0f, kSumExp - longer_exp(a)); }
+static float split_far(const qlin_qat_args* a) { return std::ldexp(1.0f, kShift - 36 - longer_exp(a)); }
 static int split_grid(const qlin_qat_args* a) { return split_row_blocks(a) * split_strips(a); }
 
 }  // namespace qlin
@@ -810,7 +826,7 @@ extern "C" int qlin_qat_split(const qlin_qat_args* a, void* stream) {
   if (!aligned16(a->g_planes) || !aligned16(a->scale)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_split: 16-byte alignment");
   if (a->colsum != nullptr && (a->workspace == nullptr || !aligned16(a->workspace))) return fail(QLIN_ERR_NULL, "qlin_qat_split: column sums need a workspace");
   QatSplitParams p = {a->g, a->scale, static_cast<__nv_bfloat16*>(a->g_planes), a->flags + 2 * kQatFlagSlots, a->colsum != nullptr ? a->workspace : nullptr, a->rcp, a->tokens, a->out,
-                      split_block_rows(a), split_huge(a)};
+                      split_block_rows(a), a->step, split_huge(a), split_far(a)};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   qat_split_kernel<<<split_grid(a), kSplitThreads, 0, s>>>(p);
   QLIN_CHECK_LAUNCH("qlin_qat_split");
@@ -859,6 +875,7 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
     a_cols = O, a_rows = T, b_cols = I, b_rows = T;
     f.a = a->g, f.a_m = 1, f.a_k = O, f.b = a->x, f.b_n = 1, f.b_k = I;
   }
+  p.down = which == 0 ? 1.0f : kShiftDown;
   f.M = p.M, f.N = p.N, f.K = p.K;
   // a product looks at the flags of its own two operands: the others may have been left out
   f.n[0] = which == 1 ? 0 : act_grid(a);

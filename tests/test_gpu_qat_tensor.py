@@ -163,7 +163,7 @@ def test_large_gradients_stay_finite(cuda_dev):
         big = go.clone()
         big[:, 5] *= 1.4e36
         all_big = go * (2.0**122 / float(go.abs().max()))
-        large = go * (2.0**108 / float((go * lin.quantize_weight.clip_val.view(1, -1) / 127).abs().max()))
+        large = go * (2.0**36 / float((go * lin.quantize_weight.clip_val.view(1, -1) / 127).abs().max()))
         large[:, 5] = 0
         lin.quantize_weight.clip_val[5] = 0
     for g, flag in ((big, True), (all_big, True), (large, False)):
@@ -172,6 +172,37 @@ def test_large_gradients_stay_finite(cuda_dev):
         grads = torch.autograd.grad(out, [x, w, lin.bias], g)
         assert all(bool(torch.isfinite(v).all()) for v in grads)
         _check(lin, x, w, g, out, grads)
+
+
+@gpu
+@pytest.mark.parametrize("what", ["a few", "a row and a column", "all", "subnormal", "beside a tiny scale"])
+def test_tiny_gradients(cuda_dev, what):
+    """Elements down to the smallest fp32 number, as in the tails of a GELU: the tensor cores carry them, to the last place that
+    fp32 has, unless the weight's scale is so small beside the activations' that lost digits could show."""
+    t, k, n = 300, 264, 200
+    lin, x, w, go = _operands(t, k, n)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    with torch.no_grad():
+        if what in ("a few", "beside a tiny scale"):
+            go[torch.rand(t, n, generator=g, device="cuda") < 0.02] = 1e-35
+            go[:, ::7] *= 1e-12
+            go[1::3, 1::9], go[2, 3] = 1e-42, 2.0**-149
+        elif what == "a row and a column":
+            go[5], go[:, 7] = go[5] * 1e-36, go[:, 7] * 1e-38
+        elif what == "all":
+            go *= 1e-33
+        else:
+            go *= 1e-40
+        if what == "beside a tiny scale":
+            w[3] *= 2.0**-40
+            lin.quantize_weight.clip_val.view(-1)[3] *= 2.0**-40
+    flag = what == "beside a tiny scale"
+    assert _passes(lin, x, w, go) == ((False,) * 4 + (flag,), (False, flag, flag))
+    got = torch.autograd.grad(_run(lin, x, w), [x, w], go)
+    gd, xd, wd = go.double(), x.detach().double(), w.detach().double()
+    for a, want, terms, m in ((got[0], gd @ wd, gd.abs() @ wd.abs(), n), (got[1], gd.t() @ xd, gd.abs().t() @ xd.abs(), t)):
+        # in fp32 each product is rounded to a multiple of 2^-149
+        assert bool(((a.double() - want).abs() <= 8 * m**0.5 * 2.0**-24 * terms + (m if flag else 1) * 2.0**-149).all())
 
 
 @gpu
