@@ -22,8 +22,8 @@
 // What the argument rests on is checked where the operands are made: a value that is not bit for bit what the quantizer makes of a
 // whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element so large that a sum of
 // its products with codes could leave fp32's range (which the product with the operand itself need not), or a tiny one beside a scale at
-// which its lost digits could show raises a flag on the device, and the last kernel of each product, which is always launched, then
-// computes it in fp32 from the operands themselves.  With no flag up it returns at once.
+// which its lost digits could show raises a flag on the device.  Every block of a product reads its flags first, and with one up the
+// product is computed in fp32 from the operands themselves.
 #include <cmath>
 
 #include <cuda.h>
@@ -47,6 +47,7 @@ constexpr int kShift = 72;
 constexpr int kSumExp = 118;
 constexpr float kTiny = 7.888609052210118e-31f;   // 2^-100
 constexpr float kShiftUp = 4722366482869645213696.0f, kShiftDown = 1.0f / kShiftUp;  // 2^72, 2^-72
+constexpr float kApart = 8.8817841970012523e-16f;  // 2^-50
 constexpr int kPrepThreads = 256;
 constexpr int kQatFlagSlots = 1184;  // flags of each kernel that makes an operand
 
@@ -274,6 +275,126 @@ __global__ void __launch_bounds__(256) qat_colsum_kernel(const float* sums, int 
   }
 }
 
+// ------------------------------------------------------------------------------------------------ fp32 product on a flag
+// D[M,N] = sum_k A[m,k] B[n,k] + bias[n] from the fp32 operands, one FMA a term in the order of k.  Each operand is dense along K or along
+// its rows, and the dense side is a multiple of 8.
+struct QatFp32Params {
+  const float* a;
+  const float* b;
+  int64_t a_m, a_k, b_n, b_k;  // element strides
+  int32_t a_vec;               // a starts on a 16-byte boundary
+  int32_t wide;                // tiles of 128 columns
+};
+constexpr int kFpM = 128, kFpK = 16, kFpThreads = 256;
+constexpr int fp_row(int k, int width) { return k * (width + 4); }  // 16-byte rows
+constexpr int fp_buffer_floats(int nt) { return fp_row(kFpK, kFpM) + fp_row(kFpK, 64 * nt); }
+
+// Bound by the FMA pipe and by what shared memory returns (8 x 8 outputs a thread take four 16-byte reads for 32 packed FMAs; with 8 x 4
+// it is three for 16).  Tiles of 128 x 64 NT, two buffers, the next 16 values of k on their way from global memory while these are
+// multiplied.  Forward and backward with a flag up, a kernel of 64 x 64 tiles behind the tensor cores' product -> this in its place
+// (library): one infinity in the gradient, 4096 x 768 x 3072 2992 -> 1234 us (1185), 2048 x 4096 x 4096 10790 -> 3420 (3735); activations
+// with codes past 256 10380 -> 3550 (3735), the forward pass of that alone 4720 -> 1850 (1240).
+// Not inlined: beside it the tensor cores' path would spill.
+template <int NT>
+__device__ __noinline__ void qat_fp32_product(const QatFp32Params f, float* d, const float* bias, int M, int N, int K) {
+  extern __shared__ __align__(1024) uint8_t smem_bytes[];
+  float* smem = reinterpret_cast<float*>(smem_bytes);
+  constexpr int kN = 64 * NT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = (warp & 3) * 32 + (lane >> 3) * 4, tx = (warp >> 2) * 32 * NT + (lane & 7) * 4;  // rows ty .. + 3 and 16 on, columns tx .. + 3 and 32 on
+  const int num_n = (N + kN - 1) / kN, tiles = (M + kFpM - 1) / kFpM * num_n, num_k = (K + kFpK - 1) / kFpK;
+  const bool a_along_k = f.a_k == 1, b_along_k = f.b_k == 1;
+  // a thread brings four values along the dense side from one row, or one k, of each 64 rows
+  const int ar = a_along_k ? tid >> 2 : (tid & 15) * 4, ak = a_along_k ? (tid & 3) * 4 : tid >> 4;
+  const int br = b_along_k ? tid >> 2 : (tid & 15) * 4, bk = b_along_k ? (tid & 3) * 4 : tid >> 4;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int m0 = t / num_n * kFpM, n0 = t % num_n * kN;
+    float4 ra[2], rb[NT];
+    const auto fetch = [&](int k0) {  // four along the dense side are all inside or all outside
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int m = m0 + ar + 64 * c;
+        ra[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (m < M && k0 + ak < K) {
+          const float* src = f.a + m * f.a_m + (k0 + ak) * f.a_k;
+          ra[c] = f.a_vec ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NT; ++c) {
+        const int n = n0 + br + 64 * c;
+        rb[c] = n < N && k0 + bk < K ? *reinterpret_cast<const float4*>(f.b + n * f.b_n + (k0 + bk) * f.b_k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    };
+    const auto put = [](float* dst, int width, bool along_k, int k, int r, float4 v) {
+      if (along_k) {
+        dst[fp_row(k, width) + r] = v.x;
+        dst[fp_row(k + 1, width) + r] = v.y;
+        dst[fp_row(k + 2, width) + r] = v.z;
+        dst[fp_row(k + 3, width) + r] = v.w;
+      } else {
+        *reinterpret_cast<float4*>(dst + fp_row(k, width) + r) = v;
+      }
+    };
+    const auto keep = [&](int buf) {
+      float* sa = smem + buf * fp_buffer_floats(NT);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) put(sa, kFpM, a_along_k, ak, ar + 64 * c, ra[c]);
+#pragma unroll
+      for (int c = 0; c < NT; ++c) put(sa + fp_row(kFpK, kFpM), kN, b_along_k, bk, br + 64 * c, rb[c]);
+    };
+    float2 acc[8][2 * NT];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 2 * NT; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    fetch(0);
+    keep(0);
+    asm volatile("bar.sync 3, 256;" ::: "memory");
+#pragma unroll 1
+    for (int kb = 0; kb < num_k; ++kb) {
+      const bool more = kb + 1 < num_k;
+      if (more) fetch((kb + 1) * kFpK);
+      const float* sa = smem + (kb & 1) * fp_buffer_floats(NT);
+      const float* sb = sa + fp_row(kFpK, kFpM);
+#pragma unroll
+      for (int k = 0; k < kFpK; ++k) {
+        float av[8];
+        float2 bv[2 * NT];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 u = *reinterpret_cast<const float4*>(sa + fp_row(k, kFpM) + ty + 16 * h);
+          av[4 * h] = u.x, av[4 * h + 1] = u.y, av[4 * h + 2] = u.z, av[4 * h + 3] = u.w;
+        }
+#pragma unroll
+        for (int h = 0; h < NT; ++h) {
+          const float4 u = *reinterpret_cast<const float4*>(sb + fp_row(k, kN) + tx + 32 * h);
+          bv[2 * h] = make_float2(u.x, u.y), bv[2 * h + 1] = make_float2(u.z, u.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 2 * NT; ++j) acc[i][j] = __ffma2_rn(make_float2(av[i], av[i]), bv[j], acc[i][j]);
+      }
+      if (more) keep((kb + 1) & 1);
+      asm volatile("bar.sync 3, 256;" ::: "memory");
+    }
+#pragma unroll
+    for (int h = 0; h < NT; ++h) {
+      const int n = n0 + tx + 32 * h;
+      if (n >= N) continue;  // N is a multiple of 8
+      const float4 c = bias == nullptr ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(bias[n], bias[n + 1], bias[n + 2], bias[n + 3]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + ty + (i >> 2) * 16 + (i & 3);
+        float4 o = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+        if (bias != nullptr) o = make_float4(__fadd_rn(o.x, c.x), __fadd_rn(o.y, c.y), __fadd_rn(o.z, c.z), __fadd_rn(o.w, c.w));
+        if (m < M) *reinterpret_cast<float4*>(d + static_cast<int64_t>(m) * N + n) = o;
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ product
 // D[M,N] = (sum over planes and K of A_plane[m,k] B[n,k]) * row[m] * col[n] * scalar * down + bias[n] in fp32, one CTA pair per
 // 256 x BN tile.  A stage holds 64 K values of all planes of A and of B, so B is loaded once for the three planes.  An operand is
@@ -288,6 +409,9 @@ struct QatGemmParams {
   float down;  // a power of two
   int32_t M, N, K, planes, a_mn, b_mn, promote;  // promote: stages per accumulator
   int32_t num_m, num_n;
+  const int32_t* flags;  // three groups of kQatFlagSlots; the first n of each belong to this product's operands
+  int32_t flag_n[3];
+  QatFp32Params f;
 };
 
 struct QatAux {
@@ -319,6 +443,7 @@ struct QatCfg {
   static constexpr int SMEM_BYTES = AUX_OFFSET + static_cast<int>(sizeof(QatAux));
 };
 static_assert(QatCfg<256>::SMEM_BYTES <= 232448, "shared memory budget");
+static_assert(2 * fp_buffer_floats(2) * 4 <= QatCfg<128>::OUT_OFFSET && kFpThreads == QatCfg<128>::EPI_WARPS * 32, "the fp32 product runs in the epilogue warps");
 
 __device__ __forceinline__ void qat_load(uint32_t bar, void* dst, const void* tmap, int32_t x, int32_t y, int32_t z) {
   asm volatile(
@@ -390,6 +515,14 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const bool aligned = (smem_u32(smem) & 1023u) == 0;
+  int up = 0;  // the flags are complete: the kernels that raise them ended before this one began
+#pragma unroll
+  for (int g = 0; g < 3; ++g)
+#pragma unroll
+    for (int i = 0; i < (kQatFlagSlots + C::THREADS - 1) / C::THREADS; ++i) {
+      const int at = i * C::THREADS + static_cast<int>(threadIdx.x);
+      if (at < p.flag_n[g]) up |= p.flags[g * kQatFlagSlots + at];
+    }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -415,8 +548,7 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     tma_prefetch_desc(&tmap_d);
   }
   tc_fence_before();
-  __syncthreads();
-  griddep_launch();  // the kernel that looks at the flags may start as SMs fall free; it waits for this one before it writes
+  const bool again = __syncthreads_or(up) != 0;  // the same in every block
   cluster_arrive_wait();  // both CTAs' barriers exist before either touches the other's
   tc_fence_after();
   const uint32_t tmem_base = aux->tmem_base;
@@ -425,7 +557,15 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int num_kb = (p.K + 63) / 64;
   bool timed_out = false;
 
-  if (!aligned) {
+  if (again) {
+    if (warp < C::EPI_WARPS) {
+      if (p.f.wide) {
+        qat_fp32_product<2>(p.f, p.d, p.bias, p.M, p.N, p.K);
+      } else {
+        qat_fp32_product<1>(p.f, p.d, p.bias, p.M, p.N, p.K);
+      }
+    }
+  } else if (!aligned) {
     if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, static_cast<int32_t>(QLIN_ERR_BAD_ALIGN));
   } else if (warp == C::PRODUCER_WARP) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -537,9 +677,9 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
       asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
       float rs = __fmul_rn(scalar, (p.row != nullptr && row0 + lane < p.M) ? p.row[row0 + lane] : 1.0f);
-      // the power of two goes with a factor above 1, and before one below: neither order leaves fp32's range where the result does not
-      float down = p.down;
-      if (fabsf(rs) > 1.0f) rs = __fmul_rn(rs, down), down = 1.0f;
+      // the power of two goes with the factor, or before one that it would take out of fp32's range
+      const bool apart = fabsf(rs) < kApart;
+      if (!apart) rs = __fmul_rn(rs, p.down);
       float run[C::COLS];
       for (int kb = 0; kb < num_kb; kb += p.promote) {
         if (!warp_mbar_wait(&aux->tfull[buf], bph, abort_flag)) {
@@ -568,6 +708,10 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         if (buf == 0) bph ^= 1u;
       }
       if (!ok) break;
+      if (__any_sync(0xffffffffu, apart)) {
+#pragma unroll
+        for (int e = 0; e < C::COLS; ++e) run[e] = apart ? __fmul_rn(run[e], p.down) : run[e];
+      }
 #pragma unroll
       for (int c = 0; c < C::COLS; c += 16) {
         uint8_t* dst = stage + (piece & 1) * 2048;
@@ -579,7 +723,7 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int e = c + 4 * k + j;
-            const float y = __fmul_rn(__fmul_rn(run[e], down), __fmul_rn(rs, aux->cs[half * C::COLS + e]));
+            const float y = __fmul_rn(run[e], __fmul_rn(rs, aux->cs[half * C::COLS + e]));
             w[j] = __float_as_uint(p.bias != nullptr ? __fadd_rn(y, aux->bias[half * C::COLS + e]) : y);
           }
           const uint32_t addr = smem_u32(dst) + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4);
@@ -623,68 +767,6 @@ qat_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
 }
 
-// ------------------------------------------------------------------------------------------------ fp32 product on a flag
-struct QatFallbackParams {
-  const float* a;
-  const float* b;
-  const float* bias;
-  float* d;
-  const int32_t* flags;        // three groups of kQatFlagSlots; the first n of each belong to this product's operands
-  int64_t a_m, a_k, b_n, b_k;  // element strides
-  int32_t M, N, K, n[3];
-};
-constexpr int kFbTile = 64, kFbK = 16;
-
-__global__ void __launch_bounds__(256) qat_fallback_kernel(const QatFallbackParams p) {
-  int up = 0;
-  for (int g = 0; g < 3; ++g)
-    for (int i = threadIdx.x; i < p.n[g]; i += 256) up |= p.flags[g * kQatFlagSlots + i];
-  griddep_wait();  // the flags were complete before the product started; its result was not
-  if (!__syncthreads_or(up)) return;
-  __shared__ float sa[kFbK][kFbTile + 1], sb[kFbK][kFbTile + 1];
-  const int num_n = (p.N + kFbTile - 1) / kFbTile, tiles = (p.M + kFbTile - 1) / kFbTile * num_n;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int m0 = t / num_n * kFbTile, n0 = t % num_n * kFbTile;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < p.K; k0 += kFbK) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // neighbouring threads read neighbouring addresses: along K or along the rows, whichever is dense
-        const int e = i * 256 + threadIdx.x;
-        const int ka = p.a_k == 1 ? e % kFbK : e / kFbTile, ma = p.a_k == 1 ? e / kFbK : e % kFbTile;
-        const int kb = p.b_k == 1 ? e % kFbK : e / kFbTile, nb = p.b_k == 1 ? e / kFbK : e % kFbTile;
-        sa[ka][ma] = (m0 + ma < p.M && k0 + ka < p.K) ? p.a[(m0 + ma) * p.a_m + (k0 + ka) * p.a_k] : 0.0f;
-        sb[kb][nb] = (n0 + nb < p.N && k0 + kb < p.K) ? p.b[(n0 + nb) * p.b_n + (k0 + kb) * p.b_k] : 0.0f;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < kFbK; ++k) {
-        float x[4], y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          x[i] = sa[k][ty * 4 + i];
-          y[i] = sb[k][tx * 4 + i];
-        }
-        if (k0 + k < p.K) {  // an infinity times the padding would be NaN
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(x[i], y[j], acc[i][j]);
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-        if (m < p.M && n < p.N) p.d[static_cast<int64_t>(m) * p.N + n] = p.bias != nullptr ? __fadd_rn(acc[i][j], p.bias[n]) : acc[i][j];
-      }
-  }
-}
-
 // ------------------------------------------------------------------------------------------------ host side
 static int qat_map(CUtensorMap* tm, const void* base, int64_t cols, int64_t rows, int64_t planes, int box_x, int box_y, bool f32) {
   typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -715,8 +797,11 @@ static int launch_qat_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const C
     if (e != cudaSuccess) return fail(QLIN_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured[dev] = true;
   }
+  // as many pairs as have a tile of this product or of the fp32 one
+  const int64_t tiles = static_cast<int64_t>(p.num_m) * p.num_n, fp_tiles = static_cast<int64_t>((p.M + kFpM - 1) / kFpM) * ((p.N + 63) / 64);
+  const int64_t busy = tiles > (fp_tiles + 1) / 2 ? tiles : (fp_tiles + 1) / 2;
   int pairs = sm_count() / 2;
-  if (pairs > p.num_m * p.num_n) pairs = p.num_m * p.num_n;
+  if (pairs > busy) pairs = static_cast<int>(busy);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs), 1, 1);
   cfg.blockDim = dim3(C::THREADS, 1, 1);
@@ -848,13 +933,13 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
   if (a == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_product: args is NULL");
   if (!qat_shape_ok(a)) return fail(QLIN_ERR_BAD_SHAPE, "qlin_qat: in and out must be positive multiples of 8");
   if (which < 0 || which > 2) return fail(QLIN_ERR_UNSUPPORTED, "qlin_qat_product: which must be 0, 1 or 2");
-  if (a->d == nullptr || !aligned16(a->d)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_product: d must be 16-byte aligned");
+  if (a->d == nullptr || !aligned16(a->d) || !aligned16(a->x) || !aligned16(a->w)) return fail(QLIN_ERR_BAD_ALIGN, "qlin_qat_product: x, w and d must be 16-byte aligned");
   const int64_t T = a->tokens, I = a->in, O = a->out;
   QatGemmParams p = {};
-  QatFallbackParams f = {};
+  QatFp32Params& f = p.f;
   p.status = a->status;
-  p.d = f.d = a->d;
-  f.flags = a->flags;
+  p.d = a->d;
+  p.flags = a->flags;
   const void *pa, *pb;
   int64_t a_cols, a_rows, b_cols, b_rows;
   if (which == 0) {
@@ -862,7 +947,7 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
     p.col = a->scale, p.scalar = a->step, p.bias = a->bias;
     pa = a->x_codes, pb = a->w_codes;
     a_cols = I, a_rows = T, b_cols = I, b_rows = O;
-    f.a = a->x, f.a_m = I, f.a_k = 1, f.b = a->w, f.b_n = I, f.b_k = 1, f.bias = a->bias;
+    f.a = a->x, f.a_m = I, f.a_k = 1, f.b = a->w, f.b_n = I, f.b_k = 1;
   } else if (which == 1) {
     p.M = a->tokens, p.N = a->in, p.K = a->out, p.planes = 3;
     pa = a->g_planes, pb = a->w_codes;
@@ -876,11 +961,14 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
     f.a = a->g, f.a_m = 1, f.a_k = O, f.b = a->x, f.b_n = 1, f.b_k = I;
   }
   p.down = which == 0 ? 1.0f : kShiftDown;
-  f.M = p.M, f.N = p.N, f.K = p.K;
+  f.a_vec = aligned16(f.a);
+  const int64_t rows = (p.M + kFpM - 1) / kFpM, ctas = sm_count() / 2 * 2;
+  const auto rounds = [&](int width) { return (rows * ((p.N + width - 1) / width) + ctas - 1) / ctas; };
+  f.wide = 8 * rounds(128) <= 5 * rounds(64);  // a round of 64 columns took 0.63 of one of 128 (264 and 420 us at 4096 terms)
   // a product looks at the flags of its own two operands: the others may have been left out
-  f.n[0] = which == 1 ? 0 : act_grid(a);
-  f.n[1] = which == 2 ? 0 : weight_grid(a);
-  f.n[2] = which == 0 ? 0 : split_grid(a);
+  p.flag_n[0] = which == 1 ? 0 : act_grid(a);
+  p.flag_n[1] = which == 2 ? 0 : weight_grid(a);
+  p.flag_n[2] = which == 0 ? 0 : split_grid(a);
   if (pa == nullptr || pb == nullptr || f.a == nullptr || f.b == nullptr || a->flags == nullptr) return fail(QLIN_ERR_NULL, "qlin_qat_product: a pointer is NULL");
   const int num_kb = (p.K + 63) / 64;
   // The sums of the forward product are whole numbers, exact in fp32 up to 2^24 and truncated beyond: one accumulator for as
@@ -907,23 +995,5 @@ extern "C" int qlin_qat_product(const qlin_qat_args* a, int32_t which, void* str
   rc = qat_map(&td, a->d, p.N, p.M, 1, 16, 32, true);
   if (rc != QLIN_OK) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  rc = bn == 256 ? launch_qat_gemm<256>(ta, tb, td, p, s) : bn == 192 ? launch_qat_gemm<192>(ta, tb, td, p, s) : launch_qat_gemm<128>(ta, tb, td, p, s);
-  if (rc != QLIN_OK) return rc;
-  const int64_t tiles = static_cast<int64_t>((f.M + kFbTile - 1) / kFbTile) * ((f.N + kFbTile - 1) / kFbTile);
-  const int64_t most = static_cast<int64_t>(sm_count()) * 4;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles < most ? tiles : most), 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, qat_fallback_kernel, f);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(QLIN_ERR_LAUNCH, "qlin_qat_product: %s", cudaGetErrorString(e));
-  }
-  return QLIN_OK;
+  return bn == 256 ? launch_qat_gemm<256>(ta, tb, td, p, s) : bn == 192 ? launch_qat_gemm<192>(ta, tb, td, p, s) : launch_qat_gemm<128>(ta, tb, td, p, s);
 }

@@ -596,7 +596,7 @@ int qlin_peer_barrier(const qlin_peer_barrier_args* args, void* stream);
  * bf16 tensor cores, at fp32 accuracy.  x [tokens, in] and w [out, in] are the fake-quantised operands of a PACT+ activation
  * quantizer and of a per-channel symmetric weight quantizer: whole numbers of steps.  They enter as those whole numbers, a
  * gradient g [tokens, out] as three bf16 parts.  Operands the arithmetic cannot carry (no whole number of steps, scales out of
- * range, infinite, NaN, huge or tiny gradients) raise a flag, and the products they are part of are then computed in fp32 from x, w and g.
+ * range, infinite, NaN or huge gradients, tiny ones in columns of tiny scales) raise a flag, and the products they are part of are then computed in fp32 from x, w and g.
  * Forward: qlin_qat_codes(a, 0), qlin_qat_product(a, 0).  Backward: qlin_qat_codes(a, 1) with the step and scales of the forward
  * pass, qlin_qat_split, qlin_qat_product(a, 1) for gx and (a, 2) for gw.  in and out are multiples of 8; x, w and d dense and 16-byte
  * aligned; g dense.  `flags` holds qlin_qat_flag_count() words for each pass, which the calls of that pass write before they read (an operand that is left out cannot be multiplied, and its words are not read).

@@ -106,6 +106,23 @@ def test_edges(cuda_dev, t, k, n):
 
 
 @gpu
+@pytest.mark.parametrize("t,k,n", [(1, 8, 8), (65, 64, 136), (257, 128, 264), (127, 72, 384), (1000, 200, 392), (129, 1032, 56), (63, 1032, 8), (3001, 520, 1048)])
+def test_edges_of_the_product_in_fp32(cuda_dev, t, k, n):
+    """Operands off the steps: every product is the fp32 one, with edges of its 128 x 64 tiles and 16-term stages, and once with a
+    gradient off a 16-byte boundary."""
+    lin, x, w, go = _operands(t, k, n)
+    with torch.no_grad():
+        x[t // 2, k // 2] += 0.003
+        w[n // 2, k // 2] += 0.0007
+    buf = torch.empty(t * n + 1, device="cuda")
+    buf[1:] = go.flatten()
+    out = _run(lin, x, w)
+    for g in (go, buf[1:].view(t, n)):
+        assert _passes(lin, x, w, g)[1] == (True, True, True)
+        _check(lin, x, w, g, out, torch.autograd.grad(out, [x, w, lin.bias], g, retain_graph=True))
+
+
+@gpu
 @pytest.mark.parametrize("what", ["tiny gradient", "activation off the steps", "weight off the steps", "scales replaced", "gradient off 16 bytes"])
 def test_operands_the_codes_cannot_carry(cuda_dev, what):
     t, k, n = 300, 264, 200
