@@ -127,11 +127,12 @@ __device__ __forceinline__ float bq_block_sum(float v, float* slot) {
 // Resident blocks an SM.  One output fits 64 registers a thread, 1024 threads; the values of two or three between their maximum
 // and their codes, beside the next row, need 80.  At 64 they spill: 16384 x 4096, addend, norm and three outputs 207 us at 1024
 // threads, 170 at 768; two outputs 143 and 131.
-constexpr int bq_resident(int tpb, int nout) { return (nout >= 2 && tpb <= 256 ? 768 : 1024) / tpb; }
+constexpr int bq_resident(int tpb, int nout, bool ahead) { return (ahead && nout >= 2 && tpb <= 256 ? 768 : 1024) / tpb; }
 
-// NOUT: the most outputs this instance takes (their values stay in registers between the maximum and the codes)
-template <int TPB, int NOUT>
-__global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT)) block_quant_kernel(const BlockQuantParams p, int mul_in_smem) {
+// AHEAD: the next row is loaded while this one is reduced and stored, and NOUT is the most outputs this instance takes (their values stay in
+// registers between the maximum and the codes).  Without it a row's outputs follow one another, which takes 64 registers for any number.
+template <int TPB, int NOUT, bool AHEAD>
+__global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT, AHEAD)) block_quant_kernel(const BlockQuantParams p, int mul_in_smem) {
   // The reciprocal SmoothQuant vectors are the same for every row: with `mul_in_smem` the block copies them into shared
   // memory once, quarter-transposed ([output][quarter][slice] of four floats) so that the four 16-byte reads of a
   // thread's slice are conflict free, instead of re-reading them through L1 for every row and output.
@@ -158,17 +159,22 @@ __global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT)) block_quant_kerne
   uint32_t h[8], a[8], nx[8], na[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) h[j] = a[j] = nx[j] = na[j] = 0u;
-  if (active && blockIdx.x < p.rows) {
+  if (AHEAD && active && blockIdx.x < p.rows) {
     bq_load8(p.x + static_cast<int64_t>(blockIdx.x) * p.ldx + ch * 16, nx);
     if (ahead_r) bq_load8(p.r + static_cast<int64_t>(blockIdx.x) * p.ldr + ch * 16, na);
   }
-  int flip = 0;
+  int flip = 0, flip_max = 0;
   for (int row = blockIdx.x; row < p.rows; row += gridDim.x, flip ^= 1) {
+    if (AHEAD) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) h[j] = nx[j], a[j] = na[j];
+      for (int j = 0; j < 8; ++j) h[j] = nx[j], a[j] = na[j];
+    } else if (active) {
+      bq_load8(p.x + static_cast<int64_t>(row) * p.ldx + ch * 16, h);
+      if (ahead_r) bq_load8(p.r + static_cast<int64_t>(row) * p.ldr + ch * 16, a);
+    }
     // issued as soon as this row's inputs are used up, so that the next row needs no registers of its own before
     const auto load_next = [&]() {
-      if (active && p.rows - row > static_cast<int>(gridDim.x)) {
+      if (AHEAD && active && p.rows - row > static_cast<int>(gridDim.x)) {
         const int64_t next = row + static_cast<int>(gridDim.x);
         bq_load8(p.x + next * p.ldx + ch * 16, nx);
         if (ahead_r) bq_load8(p.r + next * p.ldr + ch * 16, na);
@@ -221,95 +227,98 @@ __global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT)) block_quant_kerne
     }
     if (active && p.h_out != nullptr) bq_store8(p.h_out + static_cast<int64_t>(row) * p.ldh + ch * 16, h);
 
-    uint32_t v[NOUT][8];
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) {
-      if (o >= p.nout) break;
-      __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
-      if (active) {
-        if (p.mul[o] != nullptr) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 f = mul_in_smem ? reinterpret_cast<const float4*>(mul_s)[(o * 4 + q) * nchunks + ch] : reinterpret_cast<const float4*>(p.mul[o])[ch * 4 + q];
-            v[o][2 * q] = bq_mul_pack(h[2 * q], make_float2(f.x, f.y));
-            v[o][2 * q + 1] = bq_mul_pack(h[2 * q + 1], make_float2(f.z, f.w));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[o][j] = h[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v[o][j])));
-      }
-      if (p.mode != QLIN_BLOCK_GIVEN_SCALE) {  // non-negative and never NaN: the order of the bit patterns is that of the values
-        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(amax2), __high2float(amax2))));
-        if (lane == 0) red_max[flip][o][warp] = top;
-      }
-    }
-    float s[NOUT], rs[NOUT];
-    if (p.mode == QLIN_BLOCK_GIVEN_SCALE) {  // one output
-      s[0] = p.scale_in[row];
-      // the shards of a row-parallel Linear each reported the scale of their slice: the row's scale is the largest
-      for (int k = 1; k < p.scale_in_parts; ++k) s[0] = fmaxf(s[0], p.scale_in[k * p.scale_in_stride + row]);
-      rs[0] = __frcp_rn(s[0]);
-#pragma unroll
-      for (int o = 1; o < NOUT; ++o) s[o] = s[0], rs[o] = rs[0];
-      if (threadIdx.x == 0 && p.scale_out[0] != nullptr) p.scale_out[0][row] = s[0];
-    } else if (p.nout > 0) {
-      __syncthreads();
-      uint32_t top[NOUT];
-#pragma unroll
-      for (int o = 0; o < NOUT; ++o) top[o] = o < p.nout ? __reduce_max_sync(0xffffffffu, red_max[flip][o][lane & (NW - 1)]) : 0u;
-      uint32_t mine = top[0];
-#pragma unroll
-      for (int o = 1; o < NOUT; ++o) mine = lane == o ? top[o] : mine;
-      const float amax = __uint_as_float(mine);
-      const float sl = Elem<__nv_bfloat16>::rnd(__fdiv_rn(fmaxf(amax, eps), static_cast<float>(p.levels)));
-      const float rsl = __frcp_rn(sl);
-#pragma unroll
-      for (int o = 0; o < NOUT; ++o) s[o] = NOUT == 1 ? sl : __shfl_sync(0xffffffffu, sl, o), rs[o] = NOUT == 1 ? rsl : __shfl_sync(0xffffffffu, rsl, o);
+    for (int ob = 0; ob < (AHEAD ? 1 : p.nout); ob += NOUT, flip_max ^= 1) {  // with AHEAD all outputs in one pass
+      const int slot = AHEAD ? flip : flip_max;
+      uint32_t v[NOUT][8];
 #pragma unroll
       for (int o = 0; o < NOUT; ++o) {
-        if (o >= p.nout) break;
-        if (p.dst_multimem) {
-          if (threadIdx.x == 0) {
-            bq_store_f32_all(reinterpret_cast<float*>(p.dst_base[0] + p.scale_off[o]) + p.dst_row0 + row, s[o]);
-            if (p.ndst > 1) reinterpret_cast<float*>(p.dst_base[1] + p.scale_off[o])[p.dst_row0 + row] = s[o];
+        if (ob + o >= p.nout) break;
+        __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
+        if (active) {
+          if (p.mul[ob + o] != nullptr) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 f = mul_in_smem ? reinterpret_cast<const float4*>(mul_s)[((ob + o) * 4 + q) * nchunks + ch] : reinterpret_cast<const float4*>(p.mul[ob + o])[ch * 4 + q];
+              v[o][2 * q] = bq_mul_pack(h[2 * q], make_float2(f.x, f.y));
+              v[o][2 * q + 1] = bq_mul_pack(h[2 * q + 1], make_float2(f.z, f.w));
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[o][j] = h[j];
           }
-        } else if (p.ndst > 0) {
-          if (static_cast<int>(threadIdx.x) < p.ndst)
-            reinterpret_cast<float*>(p.dst_base[threadIdx.x] + p.scale_off[o])[p.dst_row0 + row] = s[o];
-        } else if (threadIdx.x == 0 && p.scale_out[o] != nullptr) {
-          p.scale_out[o][row] = s[o];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v[o][j])));
+        }
+        if (p.mode != QLIN_BLOCK_GIVEN_SCALE) {  // non-negative and never NaN: the order of the bit patterns is that of the values
+          const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(amax2), __high2float(amax2))));
+          if (lane == 0) red_max[slot][o][warp] = top;
         }
       }
-    }
-    if (p.mode == QLIN_BLOCK_SCALE_ONLY || !active) continue;
+      float s[NOUT], rs[NOUT];
+      if (p.mode == QLIN_BLOCK_GIVEN_SCALE) {  // one output
+        s[0] = p.scale_in[row];
+        // the shards of a row-parallel Linear each reported the scale of their slice: the row's scale is the largest
+        for (int k = 1; k < p.scale_in_parts; ++k) s[0] = fmaxf(s[0], p.scale_in[k * p.scale_in_stride + row]);
+        rs[0] = __frcp_rn(s[0]);
 #pragma unroll
-    for (int o = 0; o < NOUT; ++o) {
-      if (o >= p.nout) break;
-      const float2 rs2 = make_float2(rs[o], rs[o]);
-      const float2 magic = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the sum's low mantissa byte is rint's code
-      uint32_t out[4];
+        for (int o = 1; o < NOUT; ++o) s[o] = s[0], rs[o] = rs[0];
+        if (threadIdx.x == 0 && p.scale_out[0] != nullptr) p.scale_out[0][row] = s[0];
+      } else if (p.nout > 0) {
+        __syncthreads();
+        uint32_t top[NOUT];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const float2 qa = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g], rs2)), magic);
-        const float2 qb = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g + 1], rs2)), magic);
-        out[g] = __byte_perm(__byte_perm(__float_as_uint(qa.x), __float_as_uint(qa.y), 0x0040),
-                             __byte_perm(__float_as_uint(qb.x), __float_as_uint(qb.y), 0x0040), 0x5410);
+        for (int o = 0; o < NOUT; ++o) top[o] = ob + o < p.nout ? __reduce_max_sync(0xffffffffu, red_max[slot][o][lane & (NW - 1)]) : 0u;
+        uint32_t mine = top[0];
+#pragma unroll
+        for (int o = 1; o < NOUT; ++o) mine = lane == o ? top[o] : mine;
+        const float amax = __uint_as_float(mine);
+        const float sl = Elem<__nv_bfloat16>::rnd(__fdiv_rn(fmaxf(amax, eps), static_cast<float>(p.levels)));
+        const float rsl = __frcp_rn(sl);
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) s[o] = NOUT == 1 ? sl : __shfl_sync(0xffffffffu, sl, o), rs[o] = NOUT == 1 ? rsl : __shfl_sync(0xffffffffu, rsl, o);
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) {
+          if (ob + o >= p.nout) break;
+          if (p.dst_multimem) {
+            if (threadIdx.x == 0) {
+              bq_store_f32_all(reinterpret_cast<float*>(p.dst_base[0] + p.scale_off[ob + o]) + p.dst_row0 + row, s[o]);
+              if (p.ndst > 1) reinterpret_cast<float*>(p.dst_base[1] + p.scale_off[ob + o])[p.dst_row0 + row] = s[o];
+            }
+          } else if (p.ndst > 0) {
+            if (static_cast<int>(threadIdx.x) < p.ndst)
+              reinterpret_cast<float*>(p.dst_base[threadIdx.x] + p.scale_off[ob + o])[p.dst_row0 + row] = s[o];
+          } else if (threadIdx.x == 0 && p.scale_out[ob + o] != nullptr) {
+            p.scale_out[ob + o][row] = s[o];
+          }
+        }
       }
-      const uint4 packed = make_uint4(out[0], out[1], out[2], out[3]);
-      if (p.dst_multimem) {
-        const int64_t off = p.codes_off[o] + static_cast<int64_t>(p.dst_row0 + row) * p.ldq[o] + ch * 16;
-        bq_store16_all(p.dst_base[0] + off, packed);
-        // this GPU's own copy also gets a plain store: its own later kernels must not depend on the round trip of the
-        // multicast store through the switch (the copy that arrives that way carries the same bytes)
-        if (p.ndst > 1) *reinterpret_cast<uint4*>(p.dst_base[1] + off) = packed;
-      } else if (p.ndst > 0) {
-        const int64_t off = p.codes_off[o] + static_cast<int64_t>(p.dst_row0 + row) * p.ldq[o] + ch * 16;
-        for (int d = 0; d < p.ndst; ++d) *reinterpret_cast<uint4*>(p.dst_base[d] + off) = packed;
-      } else {
-        *reinterpret_cast<uint4*>(p.codes[o] + static_cast<int64_t>(row) * p.ldq[o] + ch * 16) = packed;
+      if (p.mode == QLIN_BLOCK_SCALE_ONLY || !active) continue;
+#pragma unroll
+      for (int o = 0; o < NOUT; ++o) {
+        if (ob + o >= p.nout) break;
+        const float2 rs2 = make_float2(rs[o], rs[o]);
+        const float2 magic = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the sum's low mantissa byte is rint's code
+        uint32_t out[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const float2 qa = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g], rs2)), magic);
+          const float2 qb = __fadd2_rn(bq_unpack(bq_mul_pack(v[o][2 * g + 1], rs2)), magic);
+          out[g] = __byte_perm(__byte_perm(__float_as_uint(qa.x), __float_as_uint(qa.y), 0x0040),
+                               __byte_perm(__float_as_uint(qb.x), __float_as_uint(qb.y), 0x0040), 0x5410);
+        }
+        const uint4 packed = make_uint4(out[0], out[1], out[2], out[3]);
+        if (p.dst_multimem) {
+          const int64_t off = p.codes_off[ob + o] + static_cast<int64_t>(p.dst_row0 + row) * p.ldq[ob + o] + ch * 16;
+          bq_store16_all(p.dst_base[0] + off, packed);
+          // this GPU's own copy also gets a plain store: its own later kernels must not depend on the round trip of the
+          // multicast store through the switch (the copy that arrives that way carries the same bytes)
+          if (p.ndst > 1) *reinterpret_cast<uint4*>(p.dst_base[1] + off) = packed;
+        } else if (p.ndst > 0) {
+          const int64_t off = p.codes_off[ob + o] + static_cast<int64_t>(p.dst_row0 + row) * p.ldq[ob + o] + ch * 16;
+          for (int d = 0; d < p.ndst; ++d) *reinterpret_cast<uint4*>(p.dst_base[d] + off) = packed;
+        } else {
+          *reinterpret_cast<uint4*>(p.codes[ob + o] + static_cast<int64_t>(row) * p.ldq[ob + o] + ch * 16) = packed;
+        }
       }
     }
   }
@@ -357,19 +366,19 @@ __global__ void __launch_bounds__(256) rope_kernel(const RopeParams p) {
   }
 }
 
-template <int TPB, int NOUT>
-static int launch_block_quant_n(const BlockQuantParams& p, cudaStream_t s) {
+template <int TPB, int NOUT, bool AHEAD>
+static int launch_block_quant_as(const BlockQuantParams& p, cudaStream_t s) {
   static bool configured[64] = {};
   constexpr int kSmemMax = TPB >= 1024 ? 98304 : 49152;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(block_quant_kernel<TPB, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
+    if (cudaFuncSetAttribute(block_quant_kernel<TPB, NOUT, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
       return fail(QLIN_ERR_LAUNCH, "cudaFuncSetAttribute failed for qlin_block_quant");
     configured[dev] = true;
   }
   // the blocks that are resident: each walks over its rows and loads ahead
-  int grid = sm_count() * bq_resident(TPB, NOUT);
+  int grid = sm_count() * bq_resident(TPB, NOUT, AHEAD);
   if (grid > p.rows) grid = p.rows;
   if (p.max_ctas > 0) {  // the cap counts blocks of 256 threads
     int cap = TPB >= 256 ? p.max_ctas : p.max_ctas * (256 / TPB);
@@ -378,9 +387,21 @@ static int launch_block_quant_n(const BlockQuantParams& p, cudaStream_t s) {
   }
   const int smem = p.nout * p.cols * 4;
   const bool in_smem = smem > 0 && smem <= kSmemMax && p.rows >= 8 * grid;
-  block_quant_kernel<TPB, NOUT><<<grid, TPB, in_smem ? smem : 0, s>>>(p, in_smem ? 1 : 0);
+  block_quant_kernel<TPB, NOUT, AHEAD><<<grid, TPB, in_smem ? smem : 0, s>>>(p, in_smem ? 1 : 0);
   QLIN_CHECK_LAUNCH("qlin_block_quant");
   return QLIN_OK;
+}
+
+template <int TPB, int NOUT>
+static int launch_block_quant_n(const BlockQuantParams& p, cudaStream_t s) {
+  // Rows that are all resident at 64 registers a thread but not at 80: a second row for some blocks costs more than the load ahead gives.
+  // Two or three outputs, one at a time -> the other way: 592 x 4096, addend and norm, 8.2 and 10.3 us -> 9.1 and 11.3; 889 x 2048 6.9
+  // and 8.5 -> 7.2 and 9.1; 2048 x 1024 7.4 and 9.0 -> 7.5 and 9.3.  Above, at 888 x 4096, 10.9 and 13.5 -> 9.5 and 11.4.
+  if constexpr (NOUT >= 2 && TPB <= 256) {
+    if (p.max_ctas <= 0 && p.rows > sm_count() * bq_resident(TPB, NOUT, true) && p.rows <= sm_count() * bq_resident(TPB, NOUT, false))
+      return launch_block_quant_as<TPB, 1, false>(p, s);
+  }
+  return launch_block_quant_as<TPB, NOUT, true>(p, s);
 }
 
 template <int TPB>

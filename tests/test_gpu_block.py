@@ -80,6 +80,22 @@ def test_blocks_that_walk_over_rows(cuda_dev, max_ctas, nout, K):
             assert torch.equal(xin, want[2])
 
 
+@pytest.mark.parametrize("rows,K", [(592, 4096), (446, 2064), (889, 2048), (2368, 1024), (3553, 512)])
+@pytest.mark.parametrize("nout", [2, 3])
+def test_rows_that_are_resident_one_output_at_a_time(cuda_dev, rows, K, nout):
+    """The band of rows that runs without the load ahead: same results as blocks that walk over the rows with it."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, r = (torch.randn(rows, K, generator=g, device="cuda") * 2).bfloat16(), torch.randn(rows, K, generator=g, device="cuda").bfloat16()
+    x[3], r[3] = 0, 0
+    w = (1 + 0.1 * torch.randn(K, generator=g, device="cuda")).bfloat16()
+    rcps = [ops.smooth_reciprocal(_smooth(K, 11 + i).float().to(cuda_dev)) for i in range(nout)]
+    rcps[1] = None
+    for kw in (dict(), dict(prologue=L.BLOCK_SILU_MUL, r=r), dict(prologue=L.BLOCK_NORM, r=r, norm_w=w), dict(mode=L.BLOCK_SCALE_ONLY)):
+        got, want = (ops.block_quant(x, smooth_rcps=rcps, want_h=True, store_sum="norm_w" in kw, max_ctas=m, **kw) for m in (0, 100))
+        for a, b in zip((*got[0], *got[1], got[2], got[3]), (*want[0], *want[1], want[2], want[3])):
+            assert (a is None and b is None) or torch.equal(a, b)
+
+
 def test_silu_mul_prologue_and_two_pass_given_scale(cuda_dev):
     T, K = 23, 7168
     g = torch.Generator().manual_seed(2)
