@@ -236,11 +236,19 @@ __global__ void __launch_bounds__(TPB, bq_resident(TPB, NOUT, AHEAD)) block_quan
         __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
         if (active) {
           if (p.mul[ob + o] != nullptr) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float4 f = mul_in_smem ? reinterpret_cast<const float4*>(mul_s)[((ob + o) * 4 + q) * nchunks + ch] : reinterpret_cast<const float4*>(p.mul[ob + o])[ch * 4 + q];
+            const auto scale = [&](int q, float4 f) {
               v[o][2 * q] = bq_mul_pack(h[2 * q], make_float2(f.x, f.y));
               v[o][2 * q + 1] = bq_mul_pack(h[2 * q + 1], make_float2(f.z, f.w));
+            };
+            if (mul_in_smem) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) scale(q, reinterpret_cast<const float4*>(mul_s)[((ob + o) * 4 + q) * nchunks + ch]);
+            } else {  // all four in flight: one at a time behind the choice, SiLU 445 x 14336 took 15.6 us, 888 x 5120 9.9; so 14.9 and 9.5
+              float4 f[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) f[q] = reinterpret_cast<const float4*>(p.mul[ob + o])[ch * 4 + q];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) scale(q, f[q]);
             }
           } else {
 #pragma unroll
