@@ -51,8 +51,8 @@ struct Aux {
   float bias[256];
 };
 
-// SHORT_K: the batched products of attention, whose tiles are a K block or two deep.  They are written as fast as the epilogue
-// goes: sixteen warps and three stages (64 x 2048 x 128 x 2048: 130 us with eight warps and four stages, 108 with sixteen).
+// SHORT_K: batched products whose tiles are a few K blocks deep (attention scores; short_batched has the rule).  They are written
+// as fast as the epilogue goes: sixteen warps and three stages.
 // The CTA-pair kernel, whose main loop counts, lost 3 to 7 % with sixteen warps and the five stages that they leave room for.
 template <bool CHUNKED, bool SHORT_K = false>
 struct Cfg {
@@ -74,12 +74,12 @@ struct Cfg {
   static constexpr int A_BYTES = kBM * kBK;
   static constexpr int B_BYTES = BN * kBK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int COLS_PER_WARP = BN / (EPI_WARPS / 4);  // 128 (unchunked) or 32 (chunked) columns
+  static constexpr int COLS_PER_WARP = BN / (EPI_WARPS / 4);  // 128 columns, 64 (SHORT_K) or 32 (chunked)
   static constexpr int OUT_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int AUX_OFFSET = OUT_OFFSET + EPI_WARPS * kStageOutBytes;
   static constexpr int SMEM_BYTES = AUX_OFFSET + static_cast<int>(sizeof(Aux));
 };
-static_assert(Cfg<false>::SMEM_BYTES <= 232448 && Cfg<true>::SMEM_BYTES <= 232448, "shared memory budget");
+static_assert(Cfg<false>::SMEM_BYTES <= 232448 && Cfg<true>::SMEM_BYTES <= 232448 && Cfg<false, true>::SMEM_BYTES <= 232448, "shared memory budget");
 
 struct GemmParams {
   const void* c;
@@ -659,11 +659,11 @@ __device__ __forceinline__ TileScales fetch_scales(const GemmParams& p, int col,
 // problem's M and N belong to the next problem (or lie outside and read as zeros) and are dropped by the epilogue's
 // bounds checks, and its output goes to D + b * batch_stride_d.
 // TILED: outputs that TMA can address are stored by drain_tile_any (tmap_d); the others, and chunked problems, by emit64 / emit32.
-template <bool F8, bool CHUNKED, bool BATCHED = false, bool TILED = false>
-__global__ void __launch_bounds__(Cfg<CHUNKED, BATCHED && TILED>::THREADS, 1)
+template <bool F8, bool CHUNKED, bool BATCHED = false, bool TILED = false, bool SHORT_K = false>
+__global__ void __launch_bounds__(Cfg<CHUNKED, SHORT_K>::THREADS, 1)
 qlin_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
-  using C = Cfg<CHUNKED, BATCHED && TILED>;
+  using C = Cfg<CHUNKED, SHORT_K>;
   extern __shared__ __align__(1024) uint8_t smem[];
   Aux* aux = reinterpret_cast<Aux*>(smem + C::AUX_OFFSET);
   volatile int* abort_flag = &aux->abort_flag;
@@ -1886,14 +1886,14 @@ struct LaunchCfg {
   }
 };
 
-template <bool F8, bool CHUNKED, bool BATCHED, bool TILED>
+template <bool F8, bool CHUNKED, bool BATCHED, bool TILED, bool SHORT_K>
 static int launch_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, cudaStream_t stream) {
-  using C = Cfg<CHUNKED, BATCHED && TILED>;
+  using C = Cfg<CHUNKED, SHORT_K>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return fail(QLIN_ERR_DEVICE, "device ordinal %d out of range", dev);
-  const auto kernel = qlin_gemm_kernel<F8, CHUNKED, BATCHED, TILED>;
+  const auto kernel = qlin_gemm_kernel<F8, CHUNKED, BATCHED, TILED, SHORT_K>;
   if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return fail(QLIN_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -1910,13 +1910,28 @@ static int launch_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
   }
   return QLIN_OK;
 }
+// Batched products that the epilogue bounds: K of three blocks, and of four where there are few tiles of few columns, whose chain of
+// columns a warp is then half as long.  Heads x m x k x n, four stages and eight warps -> three and sixteen (us).  bf16 out: 64 x 2048 x
+// 128 x 2048 124 -> 102, 64 x 1024 x 256 x 1024 36.5 -> 33.2, 64 x 512 x 512 x 64 10.2 -> 9.9, 64 x 384 x 384 x 128 9.6 -> 8.9, at 64 x 2048 x 384 x
+// 2048 139 -> 145 (fp32 out 230 -> 193); but 64 x 1024 x 1024 x 128 20.8 -> 23.2, 64 x 1536 x 1536 x 64 39.4 -> 44.3, 64 x 2048 x 2048 x 64
+// 60.9 -> 66.6.
+static bool short_batched(const GemmParams& p) {
+  const int64_t tiles = static_cast<int64_t>(p.num_m) * p.num_n * p.batch;
+  return p.kbytes <= 3 * kBK || (p.kbytes <= 4 * kBK && p.N <= 128 && tiles <= 2 * sm_count());
+}
+
 // `td`: the output's map, or null for outputs that TMA does not store.
 template <bool F8, bool CHUNKED, bool BATCHED = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* td, const GemmParams& p, cudaStream_t stream) {
   if constexpr (!CHUNKED) {
-    if (td != nullptr) return launch_as<F8, false, BATCHED, true>(ta, tb, *td, p, stream);
+    if (td != nullptr) {
+      if constexpr (BATCHED) {
+        if (short_batched(p)) return launch_as<F8, false, true, true, true>(ta, tb, *td, p, stream);
+      }
+      return launch_as<F8, false, BATCHED, true, false>(ta, tb, *td, p, stream);
+    }
   }
-  return launch_as<F8, CHUNKED, BATCHED, false>(ta, tb, ta, p, stream);
+  return launch_as<F8, CHUNKED, BATCHED, false, false>(ta, tb, ta, p, stream);
 }
 
 // Largest number of two-CTA clusters of the pair kernel that can be resident at once (cached per device).

@@ -40,3 +40,16 @@ def test_many_batched_tiles_with_ragged_edges(cuda_dev, B, M, N):
     for dt in (torch.float32, torch.float16, torch.bfloat16):
         assert torch.equal(ops.bmm_i8(a, b, (s1, s2), dt), (acc.half() * s1 * s2).to(dt)), dt
     ops.check_status(cuda_dev)
+
+
+@pytest.mark.parametrize("B,M,K,N", [(5, 260, 384, 264), (5, 260, 400, 264), (148, 200, 512, 72), (149, 200, 512, 72), (9, 130, 512, 136), (3, 300, 2064, 64)])
+def test_batched_products_on_both_sides_of_the_short_rule(cuda_dev, B, M, K, N):
+    g = torch.Generator(device="cuda").manual_seed(B + M + K)
+    a, b = _i8(g, B, M, K), _i8(g, B, N, K)
+    acc = torch.matmul(a.double(), b.double().transpose(1, 2)).int()
+    assert torch.equal(ops.bmm_i8(a, b), acc)
+    s1, s2 = torch.tensor([0.0137], device="cuda"), torch.tensor([0.071], device="cuda")
+    small = a // 16  # sums that fp16 holds
+    want = torch.matmul(small.double(), b.double().transpose(1, 2)).half().float() * s1 * s2
+    assert torch.equal(ops.bmm_i8(small, b, (s1, s2), torch.bfloat16), want.bfloat16())
+    ops.check_status(cuda_dev)
