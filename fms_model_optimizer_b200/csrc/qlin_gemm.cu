@@ -2153,10 +2153,11 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
                      (chunk_k32 == 1 || chunk_k32 == 2 || chunk_k32 == 4) && total_k32 % 4 == 0 && low_byte_enabled())
                         ? 1
                         : 0;
-  // unchunked products whose output TMA can address are stored by it; an accumulator input or row-block scatter keeps emit64
+  // unchunked products whose output TMA can address are stored by it; an accumulator input or row-block scatter keeps emit64, and the
+  // few-row kernel stores by itself
   p.chain = pick_chain(p, f8);
   CUtensorMap tmap_d;
-  const CUtensorMap* td = !chunked && p.c == nullptr && p.scatter_rows <= 0 && make_output_map(&tmap_d, p) ? &tmap_d : nullptr;
+  const auto output_map = [&]() -> const CUtensorMap* { return !chunked && p.c == nullptr && p.scatter_rows <= 0 && make_output_map(&tmap_d, p) ? &tmap_d : nullptr; };
   if (batch > 1) {
     if (chunked || a->c != nullptr || a->scatter_rows != 0) return fail(QLIN_ERR_UNSUPPORTED, "qlin_gemm_batched: one launch takes unchunked problems without accumulator input or scatter");
     if (static_cast<int64_t>(batch) * a->M > 0x7fffffff || static_cast<int64_t>(batch) * a->N > 0x7fffffff)
@@ -2166,7 +2167,7 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
     if (rc != QLIN_OK) return rc;
     rc = make_operand_map(&tb, a->b, static_cast<int64_t>(batch) * a->N, a->K, a->ldb, bn);
     if (rc != QLIN_OK) return rc;
-    return f8 ? launch<true, false, true>(ta, tb, td, p, s) : launch<false, false, true>(ta, tb, td, p, s);
+    return f8 ? launch<true, false, true>(ta, tb, output_map(), p, s) : launch<false, false, true>(ta, tb, output_map(), p, s);
   }
   if (!chunked && a->M <= kBM && a->scatter_rows == 0 && a->max_ctas <= 0 && skinny_enabled()) {
     // weight rows as the MMA's M dimension, the few activation rows (padded to 32) as its N dimension
@@ -2182,6 +2183,7 @@ static int gemm_impl(const qlin_gemm_args* a, void* stream, int32_t batch, int64
     p.sk_mt = p.sk_split = p.sk_stages = 0;
   }
 
+  const CUtensorMap* td = output_map();
   CUtensorMap ta, tb;
   int rc = make_operand_map(&ta, a->a, a->M, a->K, a->lda, kBM);
   if (rc != QLIN_OK) return rc;
