@@ -355,6 +355,24 @@ def test_operands_that_are_stored_negated(cuda_dev, which):
 
 
 @gpu
+def test_memory_of_the_backward_pass(cuda_dev):
+    """What the tensor cores' path needs beside the gradients: codes of one operand at a time and the parts of the gradient."""
+    m, k, n = 16384, 4096, 128
+    lin = QLinear(k, n, num_bits_feature=8, qa_mode="pact+", num_bits_weight=8, qw_mode="sawb+perCh", device="cuda").train()
+    x, go = torch.randn(m, k, device="cuda").requires_grad_(True), torch.randn(m, n, device="cuda")
+    assert L.host().qat_takes(x, lin.weight, lin.bias, torch.zeros(n, device="cuda"))
+    for _ in range(2):
+        out = lin(x)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        grads = torch.autograd.grad(out, [x, lin.weight], go)
+        peak = torch.cuda.max_memory_allocated() - before
+        del out, grads
+    assert peak <= 2.5 * (m * k + n * k) * 4 + 6 * m * n
+
+
+@gpu
 def test_rule(cuda_dev):
     host = L.host()
     lin, x, w, _ = _operands(1024, 512, 512)
