@@ -126,7 +126,9 @@ __device__ __forceinline__ float bq_block_sum(float v, float* slot) {
 // them 39 -> 35, 31 -> 29, 16 -> 16 and 55 -> 47.
 // Resident blocks an SM.  One output fits 64 registers a thread, 1024 threads; the values of two or three between their maximum
 // and their codes, beside the next row, need 80.  At 64 they spill: 16384 x 4096, addend, norm and three outputs 207 us at 1024
-// threads, 170 at 768; two outputs 143 and 131.
+// threads, 170 at 768; two outputs 143 and 131.  Blocks of 512 and 1024 threads (rows over 4096) stay at 64 and spill with two and three
+// outputs; addend and norm, spilling, one output at a time, and before the load ahead: 4096 x 8192 two outputs 87.9, 90.5, 90.8 us, three
+// 120.7, 117.4, 121.0, 4096 x 14336 two 170, 185, 180.
 constexpr int bq_resident(int tpb, int nout, bool ahead) { return (ahead && nout >= 2 && tpb <= 256 ? 768 : 1024) / tpb; }
 
 // AHEAD: the next row is loaded while this one is reduced and stored, and NOUT is the most outputs this instance takes (their values stay in

@@ -4,12 +4,13 @@
 //
 // x and w are fake-quantised: x = c step and w = d s[n] with whole numbers c, d of at most 8 bits and a sign, which bf16 holds
 // exactly (up to 256, so the codes 256 and -1 that some clip pairs reach fit, and so does a NaN).  With the zero point taken
-// off beforehand there is no offset that could cancel.  The gradient is any fp32 number: g s[n] (times a power of two that keeps small
-// parts in range), rounded once, is the sum of three bf16 numbers (8 + 8 + 8 bits, each rounded from what the ones before left over).  So the forward product is one
-// bf16 GEMM whose sums are whole numbers, and each gradient is three, with every product exact and the sums in fp32.
+// off beforehand there is no offset that could cancel.  The gradient is any fp32 number: g s[n] (times a power of two that keeps
+// small parts in range), rounded once, is the sum of three bf16 numbers (8 + 8 + 8 bits, each rounded from what the ones before
+// left over).  So the forward product is one bf16 GEMM whose sums are whole numbers, and each gradient is three, with every
+// product exact and the sums in fp32.
 //
 // The tensor core truncates as it adds, which shows after a few hundred terms.  So no accumulator of a gradient lives longer
-// than 64 terms: the epilogue warps read it and add it to running sums in registers, rounded to nearest, while the tensor core
+// than 64 values of K (192 products, three parts each): the epilogue warps read it and add it to running sums in registers, rounded to nearest, while the tensor core
 // fills the other accumulator.  Relative error (2-norm) against 64 bits, tokens x in x out, of the output, gx and gw, and of
 // the fp32 library product in brackets: 4096 x 768 x 3072 5.7e-8, 1.5e-7, 1.6e-7 (4.9e-7, 9.9e-7, 1.1e-6); 64 x 768 x 768
 // 5.6e-8, 9.6e-8, 6.5e-8 (2.3e-7, 2.3e-7, 1.5e-7); 16384 x 1024 x 1024 5.4e-8, 1.0e-7, 3.0e-7 (5.7e-7, 5.7e-7, 2.3e-6).  With
@@ -20,10 +21,10 @@
 // backward of 4096 x 768 x 3072: 1124 us of device time with the library's fp32 GEMMs, 212 with this.
 //
 // What the argument rests on is checked where the operands are made: a value that is not bit for bit what the quantizer makes of a
-// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element so large that a sum of
-// its products with codes could leave fp32's range (which the product with the operand itself need not), or a tiny one beside a scale at
-// which its lost digits could show raises a flag on the device.  Every block of a product reads its flags first, and with one up the
-// product is computed in fp32 from the operands themselves.
+// whole number (another quantizer's output, a hook's), a scale out of range, an infinity or NaN in the gradient, a gradient element
+// so large that a sum of its products with codes could leave fp32's range (which the product with the operand itself need not), or a
+// tiny one beside a scale at which its lost digits could show raises a flag on the device.  Every block of a product reads its
+// flags first, and with one up the product is computed in fp32 from the operands themselves.
 #include <cmath>
 
 #include <cuda.h>

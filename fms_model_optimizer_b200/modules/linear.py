@@ -604,8 +604,8 @@ def _ordinary_call(*tensors) -> bool:
 class QLinear(nn.Linear):
     """Fake-quant Linear for QAT / DQ (fms_mo/modules/linear.py:51-393, forward :248-305):
     ``F.linear(Qa(x / s), Qw(W * s), bias)`` with the SmoothQuant scale ``s`` of :345-368.  The two
-    quantizers run as single CUDA kernels (forward and backward); the matmul itself stays a plain
-    library GEMM, as in the reference."""
+    quantizers run as single CUDA kernels (forward and backward); the product is the library's, as in the
+    reference, or, for large fp32 calls whose operands are whole numbers of steps, this package's (``_product``)."""
 
     def __init__(self, in_features, out_features, bias=True, num_bits_feature=32, qa_mode=None, num_bits_weight=32,
                  qw_mode=None, **kwargs):  # fmt: skip
